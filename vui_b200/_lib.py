@@ -21,7 +21,7 @@ _API_H = os.path.join(_ROOT, "include", "vuib200.h")
 UNITS = {
     "vuib200.cu": ["decode_kernels.cuh", "tc_gemm.cuh", "fused_blocks.cuh", "depth_group.cuh", "prefill_attn.cuh"],
     "codec.cu": ["codec_kernels.cuh"],
-    "codec_enc.cu": ["codec_enc_kernels.cuh"],
+    "codec_enc.cu": ["codec_enc_kernels.cuh", "split_ops.cuh", "split_gemm.cuh"],
 }
 SOURCES = [os.path.join(_CSRC, u) for u in UNITS]
 HEADERS = sorted({os.path.join(_CSRC, h) for hs in UNITS.values() for h in hs}) + [_API_H]

@@ -16,10 +16,12 @@ struct VuibCodecEnc {
     VuibCodecEncConfig cfg;
     VuibCodecEncWeights w;
     unsigned char* ws;
-    bool have_ws, have_w;
+    bool have_ws, have_w, packed;
     int64_t launches;
-    size_t off_a, off_b, off_x, off_n, off_q, off_o, off_g, off_d, off_hs, off_ha, total;
-    int last_frames;
+    size_t off_flag, off_y, off_p[3], off_x, off_q, off_xp, off_gp, off_d, off_dp, off_h, off_rope, off_w, total;
+    struct Packed { vuis::SgWeight c3[4], c1[4], down[4], out, wqkv[VUIB_CODEC_LAYERS], wo[VUIB_CODEC_LAYERS], fc1[VUIB_CODEC_LAYERS],
+                    fc2[VUIB_CODEC_LAYERS], half, books; } pk;
+    int last_frames, num_sms;
     char err[256];
 };
 
@@ -42,21 +44,50 @@ int32_t fail(VuibCodecEnc* c, int32_t code, const char* fmt, ...) {
             return fail(c, VUIB_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(_err));  \
     } while (0)
 
-float* wsf(VuibCodecEnc* c, size_t off) { return reinterpret_cast<float*>(c->ws + off); }
+constexpr int PAD = 8;   // history of a k = 3 or 2-tap convolution, rounded up to the swizzle's period
 
-cudaError_t conv(VuibCodecEnc* c, const float* w, const float* bias, const float* x, float* y, int Cin, int Cout, int K,
-                 int stride, int Tin, bool elu_in, int epi, const float* res, const float* scale, cudaStream_t s) {
-    EConvArgs a = {};
-    a.w = w; a.bias = bias; a.x = x; a.res = res; a.scale = scale; a.y = y;
-    a.Cin = Cin; a.Cout = Cout; a.K = K; a.stride = stride; a.Tin = Tin; a.Tout = Tin / stride;
-    a.elu_in = elu_in ? 1 : 0; a.epi = epi;
-    a.cc = K == 1 ? 32 : 8;
-    const int XW = EC_T * stride + (K - stride);
-    const size_t smem = (size_t)(a.cc * XW + EC_CO * (a.cc * K + 1)) * 4;
-    dim3 grid((a.Tout + EC_T - 1) / EC_T, (Cout + EC_CO - 1) / EC_CO);
-    c->launches++;
-    k_econv<<<grid, EC_THREADS, smem, s>>>(a);
-    return cudaGetLastError();
+// Packs the matrices for the split GEMMs (once per binding, on the legacy default stream; binding happens outside any capture).
+// Column tiles: 128 where a launch has at least a tile per SM in a 10 s buffer, narrower ones where 250 to 2000 rows leave few.
+int32_t pack_weights(VuibCodecEnc* c) {
+    c->packed = false;
+    if (!c->have_ws || !c->have_w) return VUIB_OK;
+    const VuibCodecEncConfig& g = c->cfg;
+    const VuibCodecEncWeights& w = c->w;
+    unsigned char* cur = c->ws + c->off_w;
+    cudaError_t e = cudaSuccess;
+    auto put = [&](const float* src, int mode, int q0, int q1, int N, int C, int taps, int NT) {
+        vuis::SgPack p = {src, nullptr, reinterpret_cast<vuis::bf16*>(cur), mode, q0, q1, N, C, taps, NT};
+        if (e == cudaSuccess) e = vuis::sg_pack(p, 0);
+        vuis::SgWeight r = {p.out, N, C, taps, NT};
+        cur += vuis::sg_weight_bytes(N, C, taps);
+        return r;
+    };
+    int C = g.base_dim;
+    const int nt3[4] = {32, 64, 64, 32}, nt1[4] = {64, 128, 128, 64}, ntd[4] = {128, 128, 64, 32};
+    for (int i = 0; i < 4; ++i, C *= 2) {
+        c->pk.c3[i] = put(w.res[i].c3.w, vuis::SW_ROWS, 0, 0, C / 2, C, 3, nt3[i]);
+        c->pk.c1[i] = put(w.res[i].c1.w, vuis::SW_ROWS, 0, 0, C, C / 2, 1, nt1[i]);
+        c->pk.down[i] = put(w.down[i].w, vuis::SW_STRIDED, g.ratios[i], C, 2 * C, g.ratios[i] * C, 2, ntd[i]);
+    }
+    const int D = g.d_model;
+    c->pk.out = put(w.conv_out.w, vuis::SW_ROWS, 0, 0, D, C, 3, 32);
+    for (int l = 0; l < g.n_layers; ++l) {
+        c->pk.wqkv[l] = put(w.layer[l].wqkv, vuis::SW_ROWS, 0, 0, 3 * D, D, 1, 32);
+        c->pk.wo[l] = put(w.layer[l].wo, vuis::SW_ROWS, 0, 0, D, D, 1, 32);
+        c->pk.fc1[l] = put(w.layer[l].fc1, vuis::SW_ROWS, 0, 0, g.mlp_dim, D, 1, 32);
+        c->pk.fc2[l] = put(w.layer[l].fc2, vuis::SW_ROWS, 0, 0, D, g.mlp_dim, 1, 32);
+    }
+    c->pk.half = put(w.downsample, vuis::SW_STRIDED, 2, D, D, 2 * D, 2, 32);
+    c->pk.books = put(w.sem_in, vuis::SW_ROWS, 0, 0, 256, D, 1, 32);   // the acoustic projection's columns follow the semantic one's
+    put(w.acq_in, vuis::SW_ROWS, 0, 0, 256, D, 1, 32);
+    c->pk.books.N = 512;
+    CK(e);
+    const int T25 = g.max_samples / 960;
+    vuis::k_srope<<<(T25 * 32 + 255) / 256, 256>>>(w.rope_cos, w.rope_sin, reinterpret_cast<float*>(c->ws + c->off_rope), T25);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(0));
+    c->packed = true;
+    return VUIB_OK;
 }
 
 }  // namespace
@@ -75,18 +106,35 @@ extern "C" int32_t vuib_codec_enc_create(const VuibCodecEncConfig* cfg, VuibCode
     memset(c, 0, sizeof(*c));
     c->cfg = g;
     size_t cur = 0;
-    auto take = [&](size_t floats) { size_t o = cur; cur += (floats * 4 + 255) & ~size_t(255); return o; };
-    const size_t T0 = g.max_samples, T25 = T0 / 960, T12 = T0 / 1920;
-    c->off_a = take(64 * T0);        // stage outputs alternate between a and b (largest: 64 x T0)
-    c->off_b = take(64 * T0);
-    c->off_x = take(512 * T25);
-    c->off_n = take(512 * T25);
-    c->off_q = take(3 * 512 * T25);
-    c->off_o = take(512 * T25);
-    c->off_g = take((size_t)g.mlp_dim * T25);
-    c->off_d = take(512 * T12);
-    c->off_hs = take(256 * T12);
-    c->off_ha = take(256 * T12);
+    auto take = [&](size_t bytes) { size_t o = cur; cur += (bytes + 1023) & ~size_t(1023); return o; };
+    const int T0 = g.max_samples, T25 = T0 / 960, T12 = T0 / 1920, D = g.d_model;
+    c->off_flag = take(256);
+    size_t y = 0, p[3] = {0, 0, 0}, w = 0;
+    auto most = [](size_t& v, size_t n) { if (n > v) v = n; };
+    int C = g.base_dim, T = T0;
+    for (int i = 0; i < 4; ++i) {   // a stage: input and its ELU, the residual block's inner half, the strided convolution's input
+        most(y, (size_t)C * T * 4);
+        most(p[0], vuis::sg_plane_bytes(C, T, PAD));
+        most(p[1], vuis::sg_plane_bytes(C / 2, T, PAD));
+        most(p[2], vuis::sg_plane_bytes(C * g.ratios[i], T / g.ratios[i], PAD));
+        w += vuis::sg_weight_bytes(C / 2, C, 3) + vuis::sg_weight_bytes(C, C / 2, 1) + vuis::sg_weight_bytes(2 * C, 2 * C * g.ratios[i], 1);
+        T /= g.ratios[i];
+        C *= 2;
+    }
+    most(p[0], vuis::sg_plane_bytes(C, T, PAD));
+    w += vuis::sg_weight_bytes(D, C, 3) + (size_t)g.n_layers * vuis::sg_weight_bytes(4 * D + 2 * g.mlp_dim, D, 1) +
+         vuis::sg_weight_bytes(D, 2 * D, 2) + vuis::sg_weight_bytes(512, D, 1);
+    c->off_y = take(y);
+    for (int i = 0; i < 3; ++i) c->off_p[i] = take(p[i]);
+    c->off_x = take((size_t)D * T25 * 4);
+    c->off_q = take((size_t)3 * D * T25 * 4);
+    c->off_xp = take(vuis::sg_plane_bytes(2 * D, T25, PAD));
+    c->off_gp = take(vuis::sg_plane_bytes(g.mlp_dim, T25, PAD));
+    c->off_d = take((size_t)D * T12 * 4);
+    c->off_dp = take(vuis::sg_plane_bytes(D, T12, PAD));
+    c->off_h = take((size_t)512 * T12 * 4);
+    c->off_rope = take((size_t)64 * T25 * 4);
+    c->off_w = take(w);
     c->total = cur;
     *out = c;
     return VUIB_OK;
@@ -119,7 +167,7 @@ extern "C" int32_t vuib_codec_enc_bind_workspace(VuibCodecEnc* c, void* dev, siz
                     bytes, dev);
     c->ws = static_cast<unsigned char*>(dev);
     c->have_ws = true;
-    return VUIB_OK;
+    return pack_weights(c);
 }
 
 extern "C" int32_t vuib_codec_enc_bind_weights(VuibCodecEnc* c, const VuibCodecEncWeights* w) {
@@ -131,7 +179,7 @@ extern "C" int32_t vuib_codec_enc_bind_weights(VuibCodecEnc* c, const VuibCodecE
         if (!p[i]) return fail(c, VUIB_ERR_NULL, "encoder weight pointer #%zu is NULL", i);
     c->w = *w;
     c->have_w = true;
-    return VUIB_OK;
+    return pack_weights(c);
 }
 
 extern "C" int32_t vuib_codec_enc_read_latent(VuibCodecEnc* c, float* out_host, int32_t n, void* stream) {
@@ -139,79 +187,121 @@ extern "C" int32_t vuib_codec_enc_read_latent(VuibCodecEnc* c, float* out_host, 
     if (!c->have_ws) return fail(c, VUIB_ERR_UNBOUND, "encoder workspace not bound");
     if (n < 1 || n > 512 * c->last_frames) return fail(c, VUIB_ERR_RANGE, "latent holds %d floats", 512 * c->last_frames);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    CK(cudaMemcpyAsync(out_host, c->ws + c->off_d, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    const int T = c->last_frames;
+    float* tmp = new (std::nothrow) float[(size_t)512 * T];   // [128][T][4] on the device
+    if (!tmp) return fail(c, VUIB_ERR_CUDA, "out of host memory");
+    cudaError_t e = cudaMemcpyAsync(tmp, c->ws + c->off_d, (size_t)512 * T * 4, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    for (int i = 0; e == cudaSuccess && i < n; ++i) {
+        const int ch = i / T, t = i % T;
+        out_host[i] = tmp[((size_t)(ch / 4) * T + t) * 4 + ch % 4];
+    }
+    delete[] tmp;
+    CK(e);
     return VUIB_OK;
 }
 
 extern "C" int32_t vuib_codec_enc_encode(VuibCodecEnc* c, const float* audio_dev, int32_t n_samples, int32_t n_q,
                                          int64_t* codes_out_dev, void* stream) {
     if (!c || !audio_dev || !codes_out_dev) return VUIB_ERR_NULL;
-    if (!c->have_ws || !c->have_w) return fail(c, VUIB_ERR_UNBOUND, "encoder workspace or weights not bound");
+    if (!c->packed) return fail(c, VUIB_ERR_UNBOUND, "encoder workspace or weights not bound");
     if (n_samples < 1920 || n_samples % 1920 || n_samples > c->cfg.max_samples)
         return fail(c, VUIB_ERR_RANGE, "n_samples = %d: need a multiple of 1920 up to %d", n_samples, c->cfg.max_samples);
     if (n_q < 1 || n_q > 16) return fail(c, VUIB_ERR_RANGE, "n_q = %d outside [1, 16]", n_q);
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
     const VuibCodecEncConfig& g = c->cfg;
     const VuibCodecEncWeights& w = c->w;
-    float* a = wsf(c, c->off_a);
-    float* b = wsf(c, c->off_b);
+    if (c->num_sms == 0) {
+        int dev = 0;
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, dev));
+    }
+    using namespace vuis;
+    const SgCtx x = {reinterpret_cast<int*>(c->ws + c->off_flag), c->num_sms, true, static_cast<cudaStream_t>(stream), &c->launches};
+    auto f32 = [&](size_t off) { return reinterpret_cast<float*>(c->ws + off); };
+    auto planes = [&](size_t off, int C, int T) { return sg_planes(c->ws + off, C, T, PAD); };
+    auto out = [&](const float* bias, int Cout, int act, SgPlanes o, int div) {
+        SgOut e = {};
+        e.bias = bias; e.Cout = Cout; e.act = act; e.o = o; e.p_div = div; e.up = 1;
+        return e;
+    };
+    const SgPlanes none = {};
+    float* y = f32(c->off_y);
     int T = n_samples, C = g.base_dim;
     // ---- ConvEncoder (qwen_codec.py:293-311)
-    CK(conv(c, w.conv_in.w, w.conv_in.b, audio_dev, a, 1, C, 7, 1, T, false, EE_BIAS, nullptr, nullptr, s));
+    {
+        EInArgs a = {audio_dev, w.conv_in.w, w.conv_in.b, y, planes(c->off_p[0], C, T), T};
+        CK(sg_run(x, k_ein, dim3((T + 127) / 128), dim3(256), 0, a));
+    }
     for (int i = 0; i < 4; ++i) {
         const int r = g.ratios[i];
-        // ResBlock: a += conv1(ELU(conv3(ELU(a))))
-        CK(conv(c, w.res[i].c3.w, w.res[i].c3.b, a, b, C, C / 2, 3, 1, T, true, EE_BIAS, nullptr, nullptr, s));
-        CK(conv(c, w.res[i].c1.w, w.res[i].c1.b, b, a, C / 2, C, 1, 1, T, true, EE_RES, a, nullptr, s));
-        // ELU, strided convolution
-        CK(conv(c, w.down[i].w, w.down[i].b, a, b, C, 2 * C, 2 * r, r, T, true, EE_BIAS, nullptr, nullptr, s));
-        float* t = a; a = b; b = t;
-        C *= 2;
+        const SgPlanes in = planes(c->off_p[0], C, T), mid = planes(c->off_p[1], C / 2, T), str = planes(c->off_p[2], C * r, T / r);
+        // ResBlock: y + conv1(ELU(conv3(ELU(y)))), kept only as ELU(...) in the order in which the strided convolution reads it
+        CK(sg_launch(x, c->pk.c3[i], in, T, 1, out(w.res[i].c3.b, C / 2, SA_ELU, mid, 1)));
+        SgOut o = out(w.res[i].c1.b, C, SA_ELU, str, r);
+        o.res = y;
+        o.y_rows = T;
+        CK(sg_launch(x, c->pk.c1[i], mid, T, 1, o));
         T /= r;
+        C *= 2;
+        o = out(w.down[i].b, C, SA_ELU, planes(c->off_p[0], C, T), 1);
+        o.y = i < 3 ? y : nullptr;
+        o.y_rows = T;
+        CK(sg_launch(x, c->pk.down[i], str, T, 1, o));
     }
-    float* x = wsf(c, c->off_x);
-    CK(conv(c, w.conv_out.w, w.conv_out.b, a, x, C, g.d_model, 3, 1, T, true, EE_BIAS, nullptr, nullptr, s));
-    // ---- EncTransformer (314-365) on [512][T], T = 25 Hz frames
     const int D = g.d_model, H = g.n_heads;
-    float* nrm = wsf(c, c->off_n);
-    float* q = wsf(c, c->off_q);   // [3 * 512][T]: q, k, v
-    float* o = wsf(c, c->off_o);
-    float* gact = wsf(c, c->off_g);
+    float* xr = f32(c->off_x);
+    {
+        SgOut o = out(w.conv_out.b, D, SA_NONE, none, 1);
+        o.y = xr;
+        o.y_rows = T;
+        CK(sg_launch(x, c->pk.out, planes(c->off_p[0], C, T), T, 1, o));
+    }
+    // ---- EncTransformer (314-365) on 25 Hz frames
+    float* q = f32(c->off_q);
+    const SgPlanes xp = planes(c->off_xp, D, T), gp = planes(c->off_gp, g.mlp_dim, T), half = planes(c->off_xp, 2 * D, T / 2);
     for (int l = 0; l < g.n_layers; ++l) {
         const VuibEncLayerW& lw = w.layer[l];
-        k_elayernorm<<<(T + 31) / 32, 256, 0, s>>>(x, lw.ln1_w, lw.ln1_b, nrm, D, T);
-        c->launches++;
-        // q | k | v rows stacked in one matrix: one launch with three times the CTAs
-        CK(conv(c, lw.wqkv, nullptr, nrm, q, D, 3 * D, 1, 1, T, false, EE_BIAS, nullptr, nullptr, s));
-        k_eattn<<<(H * T + 3) / 4, 128, 0, s>>>(q, q + (size_t)D * T, q + (size_t)2 * D * T, w.rope_cos, w.rope_sin, o, H, T);
-        c->launches++;
-        CK(conv(c, lw.wo, nullptr, o, x, D, D, 1, 1, T, false, EE_SCALE_RES, x, lw.attn_scale, s));
-        k_elayernorm<<<(T + 31) / 32, 256, 0, s>>>(x, lw.ln2_w, lw.ln2_b, nrm, D, T);
-        c->launches++;
-        CK(conv(c, lw.fc1, nullptr, nrm, gact, D, g.mlp_dim, 1, 1, T, false, EE_GELU, nullptr, nullptr, s));
-        CK(conv(c, lw.fc2, nullptr, gact, x, g.mlp_dim, D, 1, 1, T, false, EE_SCALE_RES, x, lw.mlp_scale, s));
+        SNormArgs na = {xr, T, lw.ln1_w, lw.ln1_b, nullptr, nullptr, 1e-5f, xp, T};
+        CK(sg_run(x, k_snorm<SN_LAYER, 512>, dim3((T + 7) / 8), dim3(256), 0, na));
+        SgOut o = out(nullptr, 3 * D, SA_NONE, none, 1);
+        o.y = q;
+        o.y_rows = T;
+        CK(sg_launch(x, c->pk.wqkv[l], xp, T, 1, o));
+        SAttnArgs aa = {q, T, f32(c->off_rope), g.max_samples / 960, xp, T, H, nullptr, nullptr, 0};
+        CK(sg_run(x, k_sattn, dim3((T + SAT_Q - 1) / SAT_Q, H), dim3(256), 0, aa));
+        o = out(nullptr, D, SA_NONE, none, 1);
+        o.res = o.y = xr;
+        o.scale = lw.attn_scale;
+        o.y_rows = T;
+        CK(sg_launch(x, c->pk.wo[l], xp, T, 1, o));
+        na.w = lw.ln2_w;
+        na.b = lw.ln2_b;
+        CK(sg_run(x, k_snorm<SN_LAYER, 512>, dim3((T + 7) / 8), dim3(256), 0, na));
+        CK(sg_launch(x, c->pk.fc1[l], xp, T, 1, out(nullptr, g.mlp_dim, SA_GELU, gp, 1)));
+        o = out(nullptr, D, SA_NONE, l == g.n_layers - 1 ? half : none, 2);   // the last layer's output feeds the stride-2 convolution
+        o.res = o.y = xr;
+        o.scale = lw.mlp_scale;
+        o.y_rows = T;
+        CK(sg_launch(x, c->pk.fc2[l], gp, T, 1, o));
     }
     // ---- downsample to 12.5 Hz, project, quantise
-    float* d = wsf(c, c->off_d);
-    CK(conv(c, w.downsample, nullptr, x, d, D, D, 4, 2, T, false, EE_BIAS, nullptr, nullptr, s));
     T /= 2;
     c->last_frames = T;
-    float* hs = wsf(c, c->off_hs);
-    float* ha = wsf(c, c->off_ha);
-    CK(conv(c, w.sem_in, nullptr, d, hs, D, 256, 1, 1, T, false, EE_BIAS, nullptr, nullptr, s));
+    const SgPlanes dp = planes(c->off_dp, D, T);
+    SgOut o = out(nullptr, D, SA_NONE, dp, 1);
+    o.y = f32(c->off_d);
+    o.y_rows = T;
+    CK(sg_launch(x, c->pk.half, half, T, 1, o));
+    o = out(nullptr, 512, SA_NONE, none, 1);
+    o.y = f32(c->off_h);
+    o.y_rows = T;
+    CK(sg_launch(x, c->pk.books, dp, T, 1, o));
     ERvqArgs r = {};
-    r.h = hs; r.codes = reinterpret_cast<long long*>(codes_out_dev); r.T = T;
-    r.n = 1; r.q0 = 0; r.table[0] = w.codebook[0]; r.norm2[0] = w.codebook_norm2[0];
-    k_ervq<<<T, 256, 0, s>>>(r);
-    c->launches++;
-    if (n_q > 1) {
-        CK(conv(c, w.acq_in, nullptr, d, ha, D, 256, 1, 1, T, false, EE_BIAS, nullptr, nullptr, s));
-        r.h = ha; r.n = n_q - 1; r.q0 = 1;
-        for (int i = 0; i < n_q - 1; ++i) { r.table[i] = w.codebook[1 + i]; r.norm2[i] = w.codebook_norm2[1 + i]; }
-        k_ervq<<<T, 256, 0, s>>>(r);
-        c->launches++;
-    }
-    CK(cudaGetLastError());
+    r.h = f32(c->off_h);
+    r.codes = reinterpret_cast<long long*>(codes_out_dev);
+    r.T = T;
+    r.n_q = n_q;
+    for (int i = 0; i < n_q; ++i) { r.table[i] = w.codebook[i]; r.norm2[i] = w.codebook_norm2[i]; }
+    CK(sg_run(x, k_ervq, dim3((T + RV_F - 1) / RV_F * RV_CL, 2), dim3(32 * RV_WARPS), 0, r));
     return VUIB_OK;
 }
