@@ -1,0 +1,38 @@
+"""The split GEMMs under the codec (split_gemm.cuh) at row counts around their tiles, clusters and splits: whole inputs decoded and
+encoded in one pass against the CPU oracles."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def codec():
+    from oracle.codec_oracle import CodecOracle
+    from vui_b200.codec import QwenCodecDecoder, random_codec_state
+
+    sd = random_codec_state(0)
+    return QwenCodecDecoder(sd, device="cuda"), CodecOracle(sd)
+
+
+@pytest.mark.parametrize("frames,n_q", [(2, 16), (7, 1), (16, 16), (33, 8)])
+def test_decode_in_one_pass(codec, frames, n_q):
+    dec, oracle = codec
+    codes = torch.randint(0, 2048, (1, n_q, frames), generator=torch.Generator().manual_seed(frames))
+    got = dec(codes.cuda()).cpu()
+    dec.check_device()
+    assert dec.position() == frames
+    ref = oracle.decode_offline(codes)
+    assert got.shape == ref.shape and (got - ref).abs().max().item() <= 5e-5 * ref.abs().max().item()
+
+
+@pytest.mark.parametrize("frames", [1, 2, 17, 32])
+def test_encode_in_one_pass(frames):
+    from oracle.codec_enc_oracle import EncoderOracle, test_audio
+    from vui_b200.codec_encoder import QwenCodecEncoder, random_encoder_state
+
+    enc, oracle = QwenCodecEncoder(random_encoder_state(0)), EncoderOracle(random_encoder_state(0))
+    audio = test_audio(frames * 1920, seed=frames)
+    got, ref = enc(audio.cuda())[0].cpu(), oracle.encode(audio)[0]
+    # a code may differ where two are equally near; what follows from it in its frame then differs too
+    assert got.shape == ref.shape and (got != ref).float().mean().item() <= 0.02

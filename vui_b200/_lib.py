@@ -20,7 +20,7 @@ _API_H = os.path.join(_ROOT, "include", "vuib200.h")
 # translation unit -> the headers it includes (a unit is recompiled when one of them changes)
 UNITS = {
     "vuib200.cu": ["decode_kernels.cuh", "tc_gemm.cuh", "fused_blocks.cuh", "depth_group.cuh", "prefill_attn.cuh"],
-    "codec.cu": ["codec_kernels.cuh"],
+    "codec.cu": ["codec_kernels.cuh", "codec_batch.cuh", "split_ops.cuh", "split_gemm.cuh"],
     "codec_enc.cu": ["codec_enc_kernels.cuh", "split_ops.cuh", "split_gemm.cuh"],
 }
 SOURCES = [os.path.join(_CSRC, u) for u in UNITS]
@@ -186,6 +186,7 @@ SYMBOLS = {
     "vuib_codec_bind_weights": (C.c_int32, [_P, C.POINTER(VuibCodecWeights)]),
     "vuib_codec_reset": (C.c_int32, [_P, _P]),
     "vuib_codec_decode_frame": (C.c_int32, [_P, _P, C.c_int32, _P, _P]),
+    "vuib_codec_decode": (C.c_int32, [_P, _P, C.c_int32, C.c_int32, _P, _P]),
     "vuib_codec_position": (C.c_int32, [_P, C.POINTER(C.c_int32), _P]),
     "vuib_codec_check_flag": (C.c_int32, [_P, _P]),
     "vuib_codec_read_tap": (C.c_int32, [_P, C.c_int32, C.POINTER(C.c_float), C.c_int32, _P]),

@@ -3,8 +3,8 @@ reference uses: ``QwenCodecDecoder`` (src/vui/qwen_codec.py:1079-1276) and ``Cod
 
 The decoder keeps the reference module's state-dict keys, so a state dict saved from the reference's
 ``QwenCodecDecoder`` loads unchanged.  One frame (16 codes -> 1920 samples) is one call of
-``vuib_codec_decode_frame``; longer inputs are fed frame by frame, which for a causal model is the same
-function as the reference's batched forward.  fp32 only (the reference's default, engine.py:302), one stream.
+``vuib_codec_decode_frame``; a longer input outside a streaming context is one call of ``vuib_codec_decode``, inside
+one it is fed frame by frame, which for a causal model is the same function.  fp32 only (the reference's default, engine.py:302), one stream.
 There is no CPU fallback.
 """
 
@@ -342,15 +342,20 @@ class QwenCodecDecoder:
         if not 1 <= n_q <= N_CODEBOOKS:
             raise ValueError(f"n_q = {n_q} outside [1, {N_CODEBOOKS}]")
         codes = codes.to(self.device, torch.int64)
-        if not self._streaming:
-            self.reset_streaming()   # an offline forward starts from zero padding (qwen_codec.py:92-102)
+        if not self._streaming:   # an offline forward starts from zero padding (qwen_codec.py:92-102)
             start = 0
+            if T == 1:
+                self.reset_streaming()
         else:
             start = self.position() if T > 1 else None
         if start is not None and start + T > self.max_seq:
             raise ValueError(f"{start} + {T} frames exceed the codec transformer's {self.max_seq} positions; "
                              "decode in windows (CodecCtx does)")
         audio = torch.empty(1, 1, T * DOWNSAMPLE_RATE, dtype=torch.float32, device=self.device)
+        if not self._streaming and T > 1:
+            codes = codes.contiguous()
+            self._check(self._lib.vuib_codec_decode(self._h, codes.data_ptr(), n_q, T, audio.data_ptr(), self._stream()))
+            return audio
         for t in range(T):
             self._frame(codes[0, :, t], audio[0, 0, t * DOWNSAMPLE_RATE:(t + 1) * DOWNSAMPLE_RATE])
         return audio

@@ -10,6 +10,7 @@
 #include <new>
 
 #include "../../include/vuib200.h"
+#include "codec_batch.cuh"
 #include "codec_kernels.cuh"
 
 using namespace vuic;
@@ -31,11 +32,18 @@ struct Layout {
     size_t partial[4];                          // transposed-convolution partials [Cout][rate]
     size_t kc, vc;                              // [layers][heads][max_seq][64]
     size_t h0, y1, x, qkv, attn, g, lat, u[2], z, a4, d0, d0a, p, y[4], ya[4], r1, part;
+    // whole inputs in one pass: packed matrices and activations for max_seq frames (offsets; planes unless fp32 is said)
+    size_t b_w, b_rope, b_e, b_h, b_y1, b_x, b_n, b_qkv, b_a, b_g, b_lat, b_u, b_up[2], b_z, b_a4, b_d0, b_y, b_r[2];
     size_t total;
     int C[5], T[5];                             // channels / columns after decoder.0 and after each block
 };
 
 }  // namespace
+
+struct BatchWeights {
+    vuis::SgWeight proj, pre, in, qkv[VUIB_CODEC_LAYERS], wo[VUIB_CODEC_LAYERS], gu[VUIB_CODEC_LAYERS], down[VUIB_CODEC_LAYERS], out;
+    vuis::SgWeight up[2], pw1[2], pw2[2], dec, tr[4], c7[4][3], c1[4][3];
+};
 
 struct VuibCodec {
     VuibCodecConfig cfg;
@@ -45,6 +53,9 @@ struct VuibCodec {
     bool have_ws, have_w;
     int64_t launches;
     int max_part_floats;
+    BatchWeights bw;
+    bool packed;
+    int num_sms;
     char err[256];
 };
 
@@ -179,6 +190,42 @@ void make_layout(VuibCodec* c) {
     L.r1 = take(cur, ymax * 4);
     c->max_part_floats = part_max;
     L.part = take(cur, (size_t)part_max * 4);
+
+    using vuis::sg_plane_bytes;
+    const int N = g.max_seq, D = g.d_model, HH = g.n_heads * HD;
+    auto planes = [&](int C, int T, int pad) { cur = (cur + 1023) & ~size_t(1023); return take(cur, sg_plane_bytes(C, T, pad)); };
+    L.b_e = planes(2 * g.codebook_dim, N, 8);
+    L.b_h = planes(g.vq_dim, N, 8);
+    L.b_y1 = planes(lat, N, 8);
+    L.b_x = take(cur, (size_t)D * N * 4);        // fp32
+    L.b_n = planes(D, N, 8);
+    L.b_qkv = take(cur, (size_t)3 * HH * N * 4);  // fp32
+    L.b_a = planes(HH, N, 8);
+    L.b_g = planes(g.mlp_dim, N, 8);
+    L.b_lat = planes(lat, N, 8);
+    L.b_u = take(cur, (size_t)lat * 4 * N * 4);   // fp32
+    for (int i = 0; i < 2; ++i) L.b_up[i] = planes(lat, UP_T[i + 1] * N, 8);
+    L.b_z = planes(lat, 4 * N, 8);
+    L.b_a4 = planes(4 * lat, 4 * N, 8);
+    L.b_d0 = planes(L.C[0], 4 * N, 8);
+    size_t by = 0, br = 0;
+    for (int b = 1; b <= 4; ++b) {
+        const size_t y = (size_t)L.C[b] * L.T[b] * N * 4, r = sg_plane_bytes(L.C[b], L.T[b] * N, vuis::SG_PAD);
+        if (y > by) by = y;
+        if (r > br) br = r;
+    }
+    L.b_y = take(cur, by);                        // fp32
+    cur = (cur + 1023) & ~size_t(1023);
+    L.b_r[0] = take(cur, br);
+    cur = (cur + 1023) & ~size_t(1023);
+    L.b_r[1] = take(cur, br);
+    L.b_rope = take(cur, (size_t)64 * N * 4);
+    cur = (cur + 1023) & ~size_t(1023);
+    size_t wn = (size_t)g.vq_dim * 2 * g.codebook_dim + (size_t)lat * g.vq_dim * 3 + (size_t)D * lat + (size_t)lat * D +
+                (size_t)g.n_layers * ((size_t)3 * HH * D + (size_t)D * HH + (size_t)3 * g.mlp_dim * D) +
+                2 * ((size_t)2 * lat * lat + (size_t)8 * lat * lat) + (size_t)L.C[0] * lat * 7;
+    for (int b = 0; b < 4; ++b) wn += (size_t)g.rates[b] * L.C[b + 1] * L.C[b] * 2 + (size_t)3 * L.C[b + 1] * L.C[b + 1] * 8;
+    L.b_w = take(cur, wn * 6);
     L.total = cur;
 }
 
@@ -254,6 +301,59 @@ cudaError_t tile(VuibCodec* c, int KW, const float* wt, const float* bias, TileI
     return cudaErrorInvalidValue;
 }
 
+// Packs the matrices for the split GEMMs (once per binding, on the legacy default stream; binding happens outside any capture).
+// Column tiles: 96 for the decoder blocks (their channel counts are 96 times a power of two), otherwise as narrow as gives about
+// one tile per SM for 125 frames.
+int32_t pack_batch(VuibCodec* c) {
+    c->packed = false;
+    if (!c->have_ws || !c->have_w) return VUIB_OK;
+    using namespace vuis;
+    const VuibCodecConfig& g = c->cfg;
+    const VuibCodecWeights& w = c->w;
+    const Layout& L = c->lay;
+    unsigned char* cur = c->ws + L.b_w;
+    cudaError_t e = cudaSuccess;
+    auto put = [&](const float* src, int N, int C, int taps, int NT, int mode = SW_ROWS, int q0 = 0, int q1 = 0, const float* src2 = nullptr) {
+        SgPack p = {src, src2, reinterpret_cast<bf16*>(cur), mode, q0, q1, N, C, taps, NT};
+        if (e == cudaSuccess) e = sg_pack(p, 0);
+        cur += sg_weight_bytes(N, C, taps);
+        return SgWeight{p.out, N, C, taps, NT};
+    };
+    BatchWeights& B = c->bw;
+    const int lat = g.latent_dim, D = g.d_model, HH = g.n_heads * HD;
+    B.proj = put(w.sem_proj, g.vq_dim, 2 * g.codebook_dim, 1, 32, SW_CAT, 0, 0, w.acq_proj);
+    B.pre = put(w.pre_conv.w, lat, g.vq_dim, 3, 32);
+    B.in = put(w.in_proj.w, D, lat, 1, 32);
+    for (int l = 0; l < g.n_layers; ++l) {
+        const VuibCodecLayerW& lw = w.layer[l];
+        B.qkv[l] = put(lw.wqkv, 3 * HH, D, 1, 32);
+        B.wo[l] = put(lw.wo, D, HH, 1, 32);
+        B.gu[l] = put(lw.gate, 2 * g.mlp_dim, D, 1, 32, SW_PAIR, 0, 0, lw.up);
+        B.down[l] = put(lw.down, D, g.mlp_dim, 1, 32);
+    }
+    B.out = put(w.out_proj.w, lat, D, 1, 32);
+    for (int i = 0; i < 2; ++i) {
+        B.up[i] = put(w.stage[i].up.w, 2 * lat, lat, 1, 32, SW_TR_ROWS, 2, lat);
+        B.pw1[i] = put(w.stage[i].pw1.w, 4 * lat, lat, 1, i ? 128 : 64);
+        B.pw2[i] = put(w.stage[i].pw2.w, lat, 4 * lat, 1, 32);
+    }
+    B.dec = put(w.dec_in.w, L.C[0], lat, 7, 64);
+    for (int b = 0; b < 4; ++b) {
+        const int C = L.C[b + 1], s = g.rates[b];
+        B.tr[b] = put(w.block[b].up.w, s * C, L.C[b], 2, 96, b == 0 ? SW_TR_ROWS : SW_TR_TILES, s, C);
+        for (int r = 0; r < 3; ++r) {
+            B.c7[b][r] = put(w.block[b].res[r].conv1.w, C, C, 7, 96, SW_TILES);
+            B.c1[b][r] = put(w.block[b].res[r].conv2.w, C, C, 1, 96, SW_TILES);
+        }
+    }
+    CK(e);
+    k_srope<<<(g.max_seq * 32 + 255) / 256, 256>>>(w.rope_cos, w.rope_sin, wsp<float>(c, L.b_rope), g.max_seq);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(0));
+    c->packed = true;
+    return VUIB_OK;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------------------------
@@ -303,7 +403,7 @@ extern "C" int32_t vuib_codec_bind_workspace(VuibCodec* c, void* dev, size_t byt
                     c->lay.total, bytes, dev);
     c->ws = static_cast<unsigned char*>(dev);
     c->have_ws = true;
-    return VUIB_OK;
+    return pack_batch(c);
 }
 
 extern "C" int32_t vuib_codec_bind_weights(VuibCodec* c, const VuibCodecWeights* w) {
@@ -318,7 +418,7 @@ extern "C" int32_t vuib_codec_bind_weights(VuibCodec* c, const VuibCodecWeights*
         if ((uintptr_t)p[i] & 15) return fail(c, VUIB_ERR_WORKSPACE, "codec weight pointer #%zu is not 16-byte aligned", i);
     c->w = *w;
     c->have_w = true;
-    return VUIB_OK;
+    return pack_batch(c);
 }
 
 extern "C" int32_t vuib_codec_reset(VuibCodec* c, void* stream) {
@@ -520,5 +620,137 @@ extern "C" int32_t vuib_codec_decode_frame(VuibCodec* c, const int64_t* codes_de
         CK(launch(c, k_final_conv, dim3((a.T + 31) / 32), dim3(128), (size_t)a.C * 40 * 4, s, a));
     }
     CK(launch(c, k_advance, dim3(1), dim3(32), 0, s, ctr));
+    return VUIB_OK;
+}
+
+// ---------------------------------------------------------------------------------------------
+extern "C" int32_t vuib_codec_decode(VuibCodec* c, const int64_t* codes_dev, int32_t n_q, int32_t n_frames, float* audio_out_dev,
+                                     void* stream) {
+    if (!c || !codes_dev || !audio_out_dev) return VUIB_ERR_NULL;
+    if (!c->packed) return fail(c, VUIB_ERR_UNBOUND, "codec workspace or weights not bound");
+    if (n_q < 1 || n_q > c->cfg.n_q) return fail(c, VUIB_ERR_RANGE, "n_q = %d outside [1, %d]", n_q, c->cfg.n_q);
+    if (n_frames < 1 || n_frames > c->cfg.max_seq) return fail(c, VUIB_ERR_RANGE, "n_frames = %d outside [1, %d]", n_frames, c->cfg.max_seq);
+    using namespace vuis;
+    using namespace vuib_codec_batch;
+    const VuibCodecConfig& g = c->cfg;
+    const VuibCodecWeights& w = c->w;
+    const Layout& L = c->lay;
+    const BatchWeights& B = c->bw;
+    if (c->num_sms == 0) {
+        int dev = 0;
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, dev));
+    }
+    int* ctr = wsp<int>(c, L.ctr);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    // the streaming state starts over; only the counters are left as n_frames streamed frames would leave them
+    CK(cudaMemsetAsync(c->ws, 0, L.state_hi, s));
+    const SgCtx x = {ctr + CTR_FLAG, c->num_sms, pdl_enabled(), s, &c->launches};
+    const int T = n_frames, lat = g.latent_dim, D = g.d_model, HH = g.n_heads * HD;
+    auto P = [&](size_t off, int C, int rows, int pad = 8) { return sg_planes(c->ws + off, C, rows, pad); };
+    const SgPlanes none = {};
+    auto out = [&](const float* bias, int Cout, SgPlanes o, float* y, int y_rows) {
+        SgOut e = {};
+        e.bias = bias; e.Cout = Cout; e.o = o; e.p_div = 1; e.up = 1; e.y = y; e.y_rows = y_rows;
+        return e;
+    };
+    const SgPlanes pe = P(L.b_e, 2 * g.codebook_dim, T), ph = P(L.b_h, g.vq_dim, T), py = P(L.b_y1, lat, T), pn = P(L.b_n, D, T),
+                   pa = P(L.b_a, HH, T), pg = P(L.b_g, g.mlp_dim, T);
+    float* xr = wsp<float>(c, L.b_x);
+    float* qkv = wsp<float>(c, L.b_qkv);
+    {   // quantizer.decode, pre_conv, input projection
+        BEmbedArgs a = {};
+        a.codes = reinterpret_cast<const long long*>(codes_dev);
+        a.n_q = n_q; a.T = T;
+        for (int q = 0; q < 16; ++q) a.table[q] = w.codebook[q];
+        a.o = pe; a.flag = ctr + CTR_FLAG; a.flag_bad = FLAG_BAD_CODE; a.ctr = ctr + CTR_FRAME;
+        CK(sg_run(x, k_bembed, dim3(T), dim3(256), 0, a));
+        CK(sg_launch(x, B.proj, pe, T, 1, out(nullptr, g.vq_dim, ph, nullptr, 0)));
+        CK(sg_launch(x, B.pre, ph, T, 1, out(w.pre_conv.b, lat, py, nullptr, 0)));
+        CK(sg_launch(x, B.in, py, T, 1, out(w.in_proj.b, D, none, xr, T)));
+    }
+    for (int l = 0; l < g.n_layers; ++l) {
+        const VuibCodecLayerW& lw = w.layer[l];
+        SNormArgs na = {xr, T, lw.ln1, nullptr, nullptr, nullptr, g.norm_eps, pn, T};
+        CK(sg_run(x, k_snorm<SN_RMS, 512>, dim3((T + 7) / 8), dim3(256), 0, na));
+        CK(sg_launch(x, B.qkv[l], pn, T, 1, out(nullptr, 3 * HH, none, qkv, T)));
+        SAttnArgs aa = {qkv, T, wsp<float>(c, L.b_rope), g.max_seq, pa, T, g.n_heads, nullptr, nullptr, 0};
+        CK(sg_run(x, k_sattn, dim3((T + SAT_Q - 1) / SAT_Q, g.n_heads), dim3(256), 0, aa));
+        SgOut o = out(nullptr, D, none, xr, T);
+        o.res = xr;
+        o.scale = lw.attn_scale;
+        CK(sg_launch(x, B.wo[l], pa, T, 1, o));
+        na.w = lw.ln2;
+        CK(sg_run(x, k_snorm<SN_RMS, 512>, dim3((T + 7) / 8), dim3(256), 0, na));
+        o = out(nullptr, g.mlp_dim, pg, nullptr, 0);
+        o.gated = 1;
+        CK(sg_launch(x, B.gu[l], pn, T, 1, o));
+        o = out(nullptr, D, none, xr, T);
+        o.res = xr;
+        o.scale = lw.mlp_scale;
+        CK(sg_launch(x, B.down[l], pg, T, 1, o));
+    }
+    SgPlanes cur = P(L.b_lat, lat, T);
+    {
+        SNormArgs na = {xr, T, w.norm, nullptr, nullptr, nullptr, g.norm_eps, pn, T};
+        CK(sg_run(x, k_snorm<SN_RMS, 512>, dim3((T + 7) / 8), dim3(256), 0, na));
+        CK(sg_launch(x, B.out, pn, T, 1, out(w.out_proj.b, lat, cur, nullptr, 0)));
+    }
+    int rows = T;
+    float* u = wsp<float>(c, L.b_u);
+    for (int i = 0; i < 2; ++i) {   // transposed convolution x 2, ConvNeXt block
+        const VuibUpStageW& uw = w.stage[i];
+        SgOut o = out(uw.up.b, lat, none, u, 2 * rows);
+        o.up = 2;
+        CK(sg_launch(x, B.up[i], cur, rows, 1, o));
+        rows *= 2;
+        const SgPlanes z = P(L.b_z, lat, rows), a4 = P(L.b_a4, 4 * lat, rows);
+        SNormArgs na = {u, rows, uw.ln_w, uw.ln_b, uw.dw.w, uw.dw.b, 1e-6f, z, rows};
+        CK(sg_run(x, k_snorm<SN_DW_LAYER, 1024>, dim3((rows + 7) / 8), dim3(256), 0, na));
+        o = out(uw.pw1.b, 4 * lat, a4, nullptr, 0);
+        o.act = SA_GELU;
+        CK(sg_launch(x, B.pw1[i], z, rows, 1, o));
+        cur = P(L.b_up[i], lat, rows);
+        o = out(uw.pw2.b, lat, cur, nullptr, rows);
+        o.res = u;
+        o.scale = uw.gamma;
+        CK(sg_launch(x, B.pw2[i], a4, rows, 1, o));
+    }
+    {   // decoder.0 and the first block's SnakeBeta
+        SgOut o = out(w.dec_in.b, L.C[0], P(L.b_d0, L.C[0], rows), nullptr, 0);
+        o.act = SA_SNAKE; o.ea = w.block[0].act.ea; o.ib = w.block[0].act.ib;
+        CK(sg_launch(x, B.dec, cur, rows, 1, o));
+        cur = o.o;
+    }
+    const int dil[3] = {1, 3, 9};
+    float* y = wsp<float>(c, L.b_y);
+    int in = 1;   // b_r[in] holds the block's input (the first block's is in b_d0)
+    for (int b = 0; b < 4; ++b) {
+        const VuibDecBlockW& bw = w.block[b];
+        const int C = L.C[b + 1];
+        const size_t ro = L.b_r[in ^ 1], mo = L.b_r[in];
+        auto act = [](SgOut& o, const VuibSnakeW& a) { o.act = SA_SNAKE; o.ea = a.ea; o.ib = a.ib; };
+        SgOut o = out(bw.up.b, C, P(ro, C, rows * g.rates[b], SG_PAD), y, rows * g.rates[b]);
+        o.up = g.rates[b];
+        act(o, bw.res[0].act1);
+        CK(sg_launch(x, B.tr[b], cur, rows, 1, o));
+        rows *= g.rates[b];
+        const SgPlanes r = P(ro, C, rows, SG_PAD), m = P(mo, C, rows);
+        for (int k = 0; k < 3; ++k) {
+            o = out(bw.res[k].conv1.b, C, m, nullptr, 0);
+            act(o, bw.res[k].act2);
+            CK(sg_launch(x, B.c7[b][k], r, rows, dil[k], o));
+            const bool last = b == 3 && k == 2;   // the last convolution reads fp32
+            o = out(bw.res[k].conv2.b, C, last ? none : k < 2 ? r : P(ro, C, rows), y, rows);
+            o.res = y;
+            o.y_act = last;
+            act(o, k < 2 ? bw.res[k + 1].act1 : b < 3 ? w.block[b + 1].act : w.final_act);
+            CK(sg_launch(x, B.c1[b][k], m, rows, 1, o));
+        }
+        cur = P(ro, C, rows);
+        in ^= 1;
+    }
+    BFinalArgs f = {y, w.final_conv.w, w.final_conv.b, audio_out_dev, rows};
+    CK(sg_run(x, k_bfinal<96>, dim3((rows + 255) / 256), dim3(256), 0, f));
     return VUIB_OK;
 }

@@ -39,7 +39,7 @@ constexpr int SG_THREADS = 384, SG_EPI_WARPS = 8;
 constexpr int SG_M = 128;            // rows of a tile
 constexpr int SG_MAX_A = 8, SG_MAX_B = 12;
 constexpr int SG_PAD = 64;           // most zero rows in front of an input (history of a k = 7, dilation 9 convolution is 54)
-constexpr int SG_SMEM = 212 * 1024;  // dynamic; the exchange of a split tile takes another 12 KB
+constexpr int SG_SMEM = 212 * 1024;
 constexpr int SG_FLAG_WAIT = 4;
 constexpr unsigned SG_SPIN_LIMIT = 1u << 22;
 
@@ -76,7 +76,7 @@ struct SgArgs {
     int dil;
     int M, n_tiles, m_tiles;
     int b_keep;           // a CTA's tiles share one column tile whose weights fit the ring: they are fetched once
-    int splits;           // CTAs of a cluster that share a tile's channels (NT = 32): 1, 2 or 4
+    int splits;           // CTAs of a cluster that share a tile's channels: 1, 2, 4 or 8
     SgOut out;
     int* flag;
     unsigned spin_limit;
@@ -345,7 +345,6 @@ __global__ void __launch_bounds__(SG_THREADS, 1) k_sg(const __grid_constant__ Sg
     __shared__ uint64_t a_full[SG_MAX_A], a_empty[SG_MAX_A], b_full[SG_MAX_B], b_empty[SG_MAX_B], t_full[2], t_empty[2];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_bad;
-    __shared__ __align__(16) float s_part[NT == 32 ? 3 * 2 * 32 * 16 : 4];              // partial sums of a split tile (12 KB)
     constexpr int NC = NT / 2;                                            // columns of an epilogue thread
     // two pairs of accumulators and, where there is room, NT columns in which a finished tile waits for its epilogue
     constexpr bool STASH = NT < 128;
@@ -377,7 +376,6 @@ __global__ void __launch_bounds__(SG_THREADS, 1) k_sg(const __grid_constant__ Sg
     const int rank = S > 1 ? blockIdx.x % S : 0;                       // a cluster's CTAs share a tile, each a range of channels
     const int kc0 = rank * a.kchunks / S, kchunks = (rank + 1) * a.kchunks / S - kc0, chunks = kchunks * TAPS;
     const int tile0 = blockIdx.x / S, tile_step = S > 1 ? tiles : gridDim.x;
-    if (S > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // "I have started", waited for before the exchange
     unsigned limit = a.spin_limit;
     auto wait = [&](uint64_t* bar, unsigned parity) {
         if (sg_bar_wait(bar, parity, limit)) return;
@@ -469,7 +467,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) k_sg(const __grid_constant__ Sg
         const int quarter = warp & 3, half = (warp - 4) >> 2;
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + half * NC;
         const int n_seg = (kchunks + R::SEG - 1) / R::SEG;
-        const int owner = quarter * S / 4;     // of a split tile, CTA r finishes rows [128 r / S, 128 (r + 1) / S)
+        const int part = half * 4 + quarter, per = SG_EPI_WARPS / S, owner = part / per;   // CTA r of a split tile finishes parts [r per, (r + 1) per)
         int seg = 0;
         sg_pdl_wait();   // the residual is read, and the outputs' buffers may still be read by earlier launches
         for (int tile = tile0; tile < tiles; tile += tile_step) {
@@ -508,29 +506,28 @@ __global__ void __launch_bounds__(SG_THREADS, 1) k_sg(const __grid_constant__ Sg
                     if (lane == 0) sg_bar_arrive(&t_empty[buf]);
                 }
             }
-            if constexpr (NT == 32) {
-                if (S > 1) {
-                    // partial sums to the CTA that finishes these rows, then added there in rank order
-                    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-                    const int per = SG_EPI_WARPS / S, w = half * (4 / S) + quarter % (4 / S);   // warps a CTA finishes, this one's place among them
-                    if (owner != rank) {
-                        const int slot = rank < owner ? rank : rank - 1;
+            if (S > 1) {
+                // partial sums to the CTA that finishes this part, then added there in rank order.  They land in its ring: behind the
+                // first barrier every CTA's MMAs, and with them all use of the rings, are over.
+                asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+                __syncwarp();
+                float* const mail = reinterpret_cast<float*>(sA) + ((part % per) * (NC / 4) * 32 + lane) * 4;
+                const int slot_stride = per * NC * 32;
+                if (owner != rank) {
+                    const uint32_t dst = sg_smem(mail + (rank < owner ? rank : rank - 1) * slot_stride);
 #pragma unroll
-                        for (int i = 0; i < NC; i += 4) {
-                            const uint32_t dst = sg_smem(&s_part[(((slot * per + w) * (NC / 4) + i / 4) * 32 + lane) * 4]);
-                            asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\tst.shared::cluster.v4.f32 [r], {%2, %3, %4, %5};\n\t}"
-                                         ::"r"(dst), "r"(owner), "f"(acc[i]), "f"(acc[i + 1]), "f"(acc[i + 2]), "f"(acc[i + 3]) : "memory");
-                        }
-                    }
-                    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-                    __syncwarp();
-                    if (owner != rank) break;
-                    for (int slot = 0; slot < S - 1; ++slot) {
+                    for (int i = 0; i < NC; i += 4)
+                        asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\tst.shared::cluster.v4.f32 [r], {%2, %3, %4, %5};\n\t}"
+                                     ::"r"(dst + i * 128), "r"(owner), "f"(acc[i]), "f"(acc[i + 1]), "f"(acc[i + 2]), "f"(acc[i + 3]) : "memory");
+                }
+                asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+                __syncwarp();
+                if (owner != rank) break;
+                for (int slot = 0; slot < S - 1; ++slot) {
 #pragma unroll
-                        for (int i = 0; i < NC; i += 4) {
-                            const float4 p = *reinterpret_cast<const float4*>(&s_part[(((slot * per + w) * (NC / 4) + i / 4) * 32 + lane) * 4]);
-                            acc[i] += p.x; acc[i + 1] += p.y; acc[i + 2] += p.z; acc[i + 3] += p.w;
-                        }
+                    for (int i = 0; i < NC; i += 4) {
+                        const float4 p = *reinterpret_cast<const float4*>(mail + slot * slot_stride + i * 32);
+                        acc[i] += p.x; acc[i + 1] += p.y; acc[i + 2] += p.z; acc[i + 3] += p.w;
                     }
                 }
             }
@@ -553,7 +550,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) k_sg(const __grid_constant__ Sg
         }
     }
     if (S > 1 && warp < 4)
-        asm volatile("barrier.cluster.wait.acquire;\n\tbarrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;\n\tbarrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (s_bad && tid == 0) atomicOr(a.flag, SG_FLAG_WAIT);
@@ -585,7 +582,8 @@ __device__ __forceinline__ float sg_weight(const SgPack& a, int n, int tap, int 
         case SW_STRIDED: return a.w[((long long)n * a.q1 + c % a.q1) * (2 * a.q0) + tap * a.q0 + c / a.q1];
         case SW_TR_ROWS:
         case SW_TR_TILES: {
-            const int j = n / a.q1, co = n - j * a.q1, row = co * 2 * a.q0 + (tap == 0 ? j + a.q0 : j);
+            // (kernel = stride: one tap, k = j)
+            const int j = n / a.q1, co = n - j * a.q1, row = a.taps == 1 ? co * a.q0 + j : co * 2 * a.q0 + (tap == 0 ? j + a.q0 : j);
             return a.mode == SW_TR_ROWS ? a.w[(long long)row * a.C + c] : a.w[((long long)(row / 96) * a.C + c) * 96 + row % 96];
         }
         case SW_TILES: return a.w[(((long long)(n / 96) * a.C + c) * a.taps + tap) * 96 + n % 96];
@@ -657,10 +655,10 @@ cudaError_t sg_launch_nt(const SgCtx& x, SgArgs a) {
     const int tiles = a.m_tiles * a.n_tiles;
     int grid = tiles < x.num_sms ? tiles : x.num_sms;
     a.splits = 1;
-    // few tiles (250 rows of 512 columns are 32): a cluster of two or four CTAs shares the channels of each
-    if (NT == 32)
-        for (int s = 2; s <= 4; s *= 2)
-            if (tiles * s <= x.num_sms && a.kchunks >= 4 * s) a.splits = s;
+    // Few tiles (125 rows of 512 columns are 16): a cluster of CTAs shares the channels of each, as long as every one has at least
+    // eight chunks (about 4 us of weights to fetch; the exchange costs 2) and all are resident at once (15 clusters of eight).
+    for (int s = 2; s <= 8; s *= 2)
+        if (tiles * s <= (s == 8 ? 120 : x.num_sms) && a.kchunks >= 2 * s && a.kchunks * TAPS >= 8 * s) a.splits = s;
     if (a.splits > 1) grid = tiles * a.splits;
     else if (tiles > grid && a.kchunks <= SgRing<NT, TAPS>::G && a.n_tiles <= grid) {
         a.b_keep = 1;
