@@ -1158,10 +1158,26 @@ struct SampleArgs {
 struct SampleSmem {
     float s_f[8];
     int s_i[8];
-    uint32_t hist[256];
+    alignas(16) uint32_t hist[256];
     uint32_t s_prefix, s_krem;
     int s_pick, s_lastkept;
 };
+
+// The token that follows a code (model.py:922-925, 967-969).
+__device__ __forceinline__ void sample_token(const SampleArgs& a, int r, int choice, int tid) {
+    if (!a.emb_out) return;
+    const bf16* e = a.code_emb + ((size_t)(a.emb_p - 1) * (SAMPLE_THREADS * SAMPLE_EL) + choice) * a.emb_rd;
+    const bf16* pe = a.pos_emb + (size_t)a.emb_p * a.emb_rd;
+    bf16* o = a.emb_out + ((size_t)r * a.emb_row_mul + a.emb_row_add) * a.emb_rd;
+    for (int k = tid * 8; k < a.emb_rd; k += SAMPLE_THREADS * 8) {
+        float x[8], c[8], sum[8];
+        unpack8(__ldg(reinterpret_cast<const uint4*>(e + k)), x);
+        unpack8(__ldg(reinterpret_cast<const uint4*>(pe + k)), c);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum[j] = x[j] + c[j];
+        *reinterpret_cast<uint4*>(o + k) = pack8(sum);
+    }
+}
 
 // Samples row r with a group of SAMPLE_THREADS threads (index `tid` in the group,
 // named barrier bar_id).  Returns the chosen code to every thread of the group.
@@ -1258,50 +1274,97 @@ __device__ __forceinline__ int sample_row(const SampleArgs& a, int r, int tid, S
 #pragma unroll
         for (int j = 0; j < SAMPLE_EL; ++j) keep[j] = true;
         if (top_k > 0) {
-            // radix select of the top_k-th largest key, 8 bits per pass
-            if (tid == 0) { s_prefix = 0u; s_krem = (uint32_t)top_k; }
-            uint32_t key[SAMPLE_EL];
+            // Logits without a penalty are bf16 values, and their order is that of the scaled ones.  The k-th of 2048 lies within
+            // an octave or two of the largest, that is 128 to 256 steps of a bf16: one histogram of the distance to the largest
+            // in steps finds it in one pass (four passes of a radix select with most values in a handful of its bins took
+            // three times as long).  Distances beyond 255 are not counted; if the k-th is among them the general search follows.
+            bool found = false;
+            if (!(is_cb0 && ctl.rep_penalty > 1.0f)) {
+                uint32_t key16[SAMPLE_EL];
 #pragma unroll
-            for (int j = 0; j < SAMPLE_EL; ++j) key[j] = order_key(sc[j]);
-            for (int pass = 0; pass < 4; ++pass) {
-                const int shift = 24 - 8 * pass;
+                for (int j = 0; j < SAMPLE_EL; ++j) key16[j] = order_key(v[j]) >> 16;
+                const uint32_t kmax = order_key(bv) >> 16;
                 hist[tid] = 0u;
                 bar_named(bar_id, SAMPLE_THREADS);
-                const uint32_t prefix = s_prefix;
-                const uint32_t pmask = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
 #pragma unroll
                 for (int j = 0; j < SAMPLE_EL; ++j)
-                    if ((key[j] & pmask) == prefix) atomicAdd(&hist[(key[j] >> shift) & 255u], 1u);
+                    if (kmax - key16[j] < 256u) atomicAdd(&hist[kmax - key16[j]], 1u);
                 bar_named(bar_id, SAMPLE_THREADS);
                 if (warp == 0) {
-                    // lane covers digits 255-8*lane .. 248-8*lane (descending)
-                    uint32_t c8[8], tot = 0u;
+                    const uint4 h0 = *reinterpret_cast<const uint4*>(&hist[8 * lane]), h1 = *reinterpret_cast<const uint4*>(&hist[8 * lane + 4]);
+                    const uint32_t c8[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+                    uint32_t tot = 0u;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) { c8[j] = hist[255 - 8 * lane - j]; tot += c8[j]; }
+                    for (int j = 0; j < 8; ++j) tot += c8[j];
                     uint32_t inc = tot;
 #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) {
                         const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
                         if (lane >= o) inc += t;
                     }
-                    const uint32_t before = inc - tot, krem = s_krem;
-                    if (before < krem && krem <= inc) {
-                        uint32_t cum = before;
+                    uint32_t cum = inc - tot;
+                    if (lane == 31 && inc < (uint32_t)top_k) s_prefix = 0xFFFFFFFFu;
+                    if (cum < (uint32_t)top_k && (uint32_t)top_k <= inc) {
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
-                            if (cum < krem && krem <= cum + c8[j]) {
-                                s_prefix = prefix | ((uint32_t)(255 - 8 * lane - j) << shift);
-                                s_krem = krem - cum;
-                            }
+                            if (cum < (uint32_t)top_k && (uint32_t)top_k <= cum + c8[j]) s_prefix = kmax - (uint32_t)(8 * lane + j);
                             cum += c8[j];
                         }
                     }
                 }
                 bar_named(bar_id, SAMPLE_THREADS);
-            }
-            const uint32_t thr = s_prefix;
+                const uint32_t thr16 = s_prefix;
+                found = thr16 != 0xFFFFFFFFu;
 #pragma unroll
-            for (int j = 0; j < SAMPLE_EL; ++j) keep[j] = key[j] >= thr;
+                for (int j = 0; j < SAMPLE_EL; ++j) keep[j] = key16[j] >= thr16;
+                if (!found) bar_named(bar_id, SAMPLE_THREADS);   // everyone has read s_prefix before it is set again
+            }
+            if (!found) {
+                // radix select of the top_k-th largest key, 8 bits per pass
+                if (tid == 0) { s_prefix = 0u; s_krem = (uint32_t)top_k; }
+                uint32_t key[SAMPLE_EL];
+#pragma unroll
+                for (int j = 0; j < SAMPLE_EL; ++j) key[j] = order_key(sc[j]);
+                for (int pass = 0; pass < 4; ++pass) {
+                    const int shift = 24 - 8 * pass;
+                    hist[tid] = 0u;
+                    bar_named(bar_id, SAMPLE_THREADS);
+                    const uint32_t prefix = s_prefix;
+                    const uint32_t pmask = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
+#pragma unroll
+                    for (int j = 0; j < SAMPLE_EL; ++j)
+                        if ((key[j] & pmask) == prefix) atomicAdd(&hist[(key[j] >> shift) & 255u], 1u);
+                    bar_named(bar_id, SAMPLE_THREADS);
+                    if (warp == 0) {
+                        // lane covers digits 255-8*lane .. 248-8*lane (descending)
+                        uint32_t c8[8], tot = 0u;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) { c8[j] = hist[255 - 8 * lane - j]; tot += c8[j]; }
+                        uint32_t inc = tot;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+                            if (lane >= o) inc += t;
+                        }
+                        const uint32_t before = inc - tot, krem = s_krem;
+                        if (before < krem && krem <= inc) {
+                            uint32_t cum = before;
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) {
+                                if (cum < krem && krem <= cum + c8[j]) {
+                                    s_prefix = prefix | ((uint32_t)(255 - 8 * lane - j) << shift);
+                                    s_krem = krem - cum;
+                                }
+                                cum += c8[j];
+                            }
+                        }
+                    }
+                    bar_named(bar_id, SAMPLE_THREADS);
+                }
+                const uint32_t thr = s_prefix;
+#pragma unroll
+                for (int j = 0; j < SAMPLE_EL; ++j) keep[j] = key[j] >= thr;
+            }
         }
         float p[SAMPLE_EL], loc = 0.f;
 #pragma unroll
@@ -1373,20 +1436,151 @@ __device__ __forceinline__ int sample_row(const SampleArgs& a, int r, int tid, S
         }
         if (a.bump_frame) a.frame_ctr[slot] += 1;
     }
-    if (a.emb_out) {
-        const bf16* e = a.code_emb + ((size_t)(a.emb_p - 1) * CS + choice) * a.emb_rd;
-        const bf16* pe = a.pos_emb + (size_t)a.emb_p * a.emb_rd;
-        bf16* o = a.emb_out + ((size_t)r * a.emb_row_mul + a.emb_row_add) * a.emb_rd;
-        for (int k = tid * 8; k < a.emb_rd; k += SAMPLE_THREADS * 8) {
-            float x[8], c[8], sum[8];
-            unpack8(__ldg(reinterpret_cast<const uint4*>(e + k)), x);
-            unpack8(__ldg(reinterpret_cast<const uint4*>(pe + k)), c);
+    sample_token(a, r, choice, tid);
+    return choice;
+}
+
+// Draw of a depth codebook: what sample_row does for codebook >= 1 (no penalty, no statistics), as a short piece of code with four
+// barriers.  It runs once per codebook between kernels or phases that evict it from the instruction caches, so its size counts:
+// through sample_row a draw took 5.5 us, most of it fetching instructions.
+struct SampleKey {       // of a row, the same for all its codebooks
+    int slot;
+    uint32_t frame_no, seed_lo, seed_hi;
+    float temperature;
+    int top_k;
+};
+
+__device__ __forceinline__ SampleKey sample_key(const SampleArgs& a, int r, bool report) {
+    SampleKey k;
+    k.slot = __ldcg(a.slots + r);
+    if (k.slot < 0 || k.slot >= a.n_slots) {
+        if (a.flag && report) atomicOr(a.flag, FLAG_BAD_SLOT);
+        k.slot = k.slot < 0 ? 0 : a.n_slots - 1;
+    }
+    k.frame_no = (uint32_t)__ldcg(a.frame_ctr + k.slot);
+    k.seed_lo = __ldcg(&a.ctl->seed_lo);
+    k.seed_hi = __ldcg(&a.ctl->seed_hi);
+    k.temperature = __ldcg(&a.ctl->temperature);
+    k.top_k = __ldcg(&a.ctl->top_k_rq);
+    return k;
+}
+
+__device__ __forceinline__ float sample_uniform(const SampleKey& k, int codebook) {
+    uint32_t c[4] = {(uint32_t)k.slot, k.frame_no, (uint32_t)codebook, 0u};
+    philox4x32_10(c, k.seed_lo, k.seed_hi);
+    return (float)(c[0] >> 8) * (1.0f / 16777216.0f);
+}
+
+// raw: this thread's eight logits; u: sample_uniform.  Returns the code to every thread of the group of 256.
+__device__ __forceinline__ int sample_rq(uint4 raw, const SampleKey& k, float u, int tid, SampleSmem& S_, int bar_id) {
+    const int warp = tid >> 5, lane = tid & 31;
+    float v[SAMPLE_EL];
+    unpack8(raw, v);
+    uint32_t key[SAMPLE_EL], best = 0u;     // a logit's order in 16 bits; with its place behind it, the maximum is the first of equals
 #pragma unroll
-            for (int j = 0; j < 8; ++j) sum[j] = x[j] + c[j];
-            *reinterpret_cast<uint4*>(o + k) = pack8(sum);
+    for (int j = 0; j < SAMPLE_EL; ++j) {
+        key[j] = order_key(v[j]) >> 16;
+        best = max(best, key[j] << 16 | (uint32_t)(2047 - (tid * SAMPLE_EL + j)));
+    }
+    best = __reduce_max_sync(0xffffffffu, best);
+    if (lane == 0) S_.s_i[warp] = (int)best;
+    S_.hist[tid] = 0u;
+    if (tid == 0) { S_.s_pick = 0x7fffffff; S_.s_lastkept = -1; }
+    bar_named(bar_id, SAMPLE_THREADS);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) best = max(best, (uint32_t)S_.s_i[w]);
+    const uint32_t kmax = best >> 16;
+    if (k.top_k == 1) {
+        bar_named(bar_id, SAMPLE_THREADS);   // s_i is free again
+        return 2047 - (int)(best & 0xffffu);
+    }
+    uint32_t thr = 0u;
+    if (k.top_k > 0 && k.top_k < SAMPLE_THREADS * SAMPLE_EL) {
+        // as in sample_row: the k-th largest by its distance to the largest, in steps of a bf16; every warp scans the histogram
+#pragma unroll
+        for (int j = 0; j < SAMPLE_EL; ++j)
+            if (kmax - key[j] < 256u) atomicAdd(&S_.hist[kmax - key[j]], 1u);
+        bar_named(bar_id, SAMPLE_THREADS);
+        const uint4 h0 = *reinterpret_cast<const uint4*>(&S_.hist[8 * lane]), h1 = *reinterpret_cast<const uint4*>(&S_.hist[8 * lane + 4]);
+        const uint32_t c8[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w}, want = (uint32_t)k.top_k;
+        uint32_t tot = 0u;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) tot += c8[j];
+        uint32_t inc = tot;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        uint32_t cum = inc - tot, bin = 256u;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (cum < want && want <= cum + c8[j]) bin = (uint32_t)(8 * lane + j);
+            cum += c8[j];
+        }
+        bin = __reduce_min_sync(0xffffffffu, bin);
+        if (bin < 256u) thr = kmax - bin;
+        else {   // further down: the largest threshold that leaves at least k values, bit by bit
+            for (int bit = 15; bit >= 0; --bit) {
+                const uint32_t t = thr | 1u << bit;
+                uint32_t n = 0u;
+#pragma unroll
+                for (int j = 0; j < SAMPLE_EL; ++j) n += key[j] >= t ? 1u : 0u;
+                n = __reduce_add_sync(0xffffffffu, n);
+                bar_named(bar_id, SAMPLE_THREADS);
+                if (lane == 0) S_.s_i[warp] = (int)n;
+                bar_named(bar_id, SAMPLE_THREADS);
+                n = 0u;
+#pragma unroll
+                for (int w = 0; w < 8; ++w) n += (uint32_t)S_.s_i[w];
+                if (n >= want) thr = t;
+            }
         }
     }
-    return choice;
+    // v / T: the product with the reciprocal and one residual correction (Markstein's scheme) is the correctly rounded quotient
+    const float T = k.temperature, rT = 1.0f / T;
+    auto scaled = [&](float x) { const float q = x * rT; return fmaf(fmaf(-q, T, x), rT, q); };
+    const uint32_t kb = kmax << 16;
+    const float smax = scaled(__uint_as_float((kb & 0x80000000u) ? kb & 0x7fff0000u : ~kb & 0xffff0000u));
+    float p[SAMPLE_EL], loc = 0.f;
+#pragma unroll
+    for (int j = 0; j < SAMPLE_EL; ++j) {
+        p[j] = key[j] >= thr ? expf(scaled(v[j]) - smax) : 0.f;
+        loc += p[j];
+    }
+    float inc = loc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) S_.s_f[warp] = inc;
+    bar_named(bar_id, SAMPLE_THREADS);
+    float wbase = 0.f, total = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        if (w < warp) wbase += S_.s_f[w];
+        total += S_.s_f[w];
+    }
+    const float target = u * total;
+    float cum = wbase + inc - loc;
+    int mine = 0x7fffffff, last = -1;
+#pragma unroll
+    for (int j = 0; j < SAMPLE_EL; ++j) {
+        cum += p[j];
+        if (key[j] >= thr) {
+            last = tid * SAMPLE_EL + j;
+            if (cum > target && mine == 0x7fffffff) mine = last;
+        }
+    }
+    mine = __reduce_min_sync(0xffffffffu, mine);
+    last = __reduce_max_sync(0xffffffffu, last);
+    if (lane == 0) {
+        if (mine != 0x7fffffff) atomicMin(&S_.s_pick, mine);
+        if (last >= 0) atomicMax(&S_.s_lastkept, last);
+    }
+    bar_named(bar_id, SAMPLE_THREADS);
+    return S_.s_pick != 0x7fffffff ? S_.s_pick : S_.s_lastkept;
 }
 
 static __global__ void __launch_bounds__(SAMPLE_THREADS) k_sample(SampleArgs a) {
@@ -1394,6 +1588,22 @@ static __global__ void __launch_bounds__(SAMPLE_THREADS) k_sample(SampleArgs a) 
     pdl_wait();
     __shared__ SampleSmem S_;
     sample_row(a, blockIdx.x, threadIdx.x, S_, 0);
+}
+
+static __global__ void __launch_bounds__(SAMPLE_THREADS) k_sample_rq(SampleArgs a) {
+    pdl_trigger();
+    pdl_wait();
+    __shared__ SampleSmem S_;
+    const int r = blockIdx.x, tid = threadIdx.x;
+    const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(a.logits + (size_t)r * a.stride + tid * SAMPLE_EL));
+    const SampleKey k = sample_key(a, r, tid == 0);
+    const int choice = sample_rq(raw, k, sample_uniform(k, a.codebook), tid, S_, 0);
+    sample_token(a, r, choice, tid);
+    if (tid == 0) {
+        a.code_cur[r] = choice;
+        a.codes_out[(size_t)r * a.Q + a.out_col] = (int64_t)choice;
+        if (a.bump_frame) a.frame_ctr[k.slot] += 1;
+    }
 }
 
 }  // namespace vuib

@@ -14,7 +14,7 @@
 #include "decode_kernels.cuh"
 #include "tc_gemm.cuh"
 #include "fused_blocks.cuh"
-#include "depth_group.cuh"
+#include "depth_tc.cuh"
 #include "prefill_attn.cuh"
 
 using namespace vuib;
@@ -25,7 +25,7 @@ struct WsLayout {
     size_t frame_ctr, rep_counts, rep_hist, rep_head, rep_filled;
     size_t trace;
     size_t xn, rq_xn, rq_attn, tc_partial, tc_counters;
-    size_t dg_layers, dg_head;   // box stream of the depth weights for k_depth_group (depth_group.cuh), 0 if none
+    size_t dg_layers, dg_head;   // slot stream of the depth weights for k_depth_tc (depth_tc.cuh), 0 if none
     size_t fx_a, fx_b, fparts_a, fparts_b, rq_fx_a, rq_fx_b, rq_fparts_a, rq_fparts_b;
     size_t att_tiles, att_ntiles;
     size_t total;
@@ -120,6 +120,12 @@ static int32_t fail(VuibEngine* e, int32_t code, const char* fmt, ...) {
 
 static size_t align_up(size_t v) { return (v + 255) & ~(size_t)255; }
 
+// The shapes k_depth_tc is written for: a head and an eighth of everything else per CTA.
+static bool depth_tc_shape(const VuibConfig& c) {
+    return c.rq_d_model == DT_D && c.rq_n_heads == DT_CL && c.rq_n_layers <= DT_LAYERS && c.rq_ffn % (8 * DT_CL) == 0 &&
+           c.rq_ffn / DT_CL <= 192 && c.codebook_size == DT_CL * 256;
+}
+
 static void make_layout(VuibEngine* e) {
     const VuibConfig& c = e->cfg;
     WsLayout& L = e->lay;
@@ -157,11 +163,10 @@ static void make_layout(VuibEngine* e) {
     L.tc_partial = take((size_t)(TC_PARTIAL_TILES + 80) * TC_TILE_N * (R < 256 ? ((R + 15) / 16) * 16 : 256) * 4);
     L.tc_counters = take(2 * 256 * 4);
     L.dg_layers = L.dg_head = 0;
-    if (c.rq_d_model == DG_D && c.rq_n_heads == DG_CL && c.rq_n_layers <= DG_LAYERS && c.rq_ffn % DG_CL == 0 &&
-        c.rq_ffn / DG_CL <= 192 && c.codebook_size == DG_CL * 256) {
-        const int n_ub = (c.rq_ffn / DG_CL + 63) / 64;
-        L.dg_layers = take((size_t)c.rq_n_layers * DG_CL * dg_boxes_per_layer(n_ub) * DG_BOX_BYTES);
-        L.dg_head = take((size_t)(c.n_quantizers - 1) * DG_CL * 32 * DG_BOX_BYTES);
+    if (depth_tc_shape(c)) {
+        const int n_ub = (c.rq_ffn / DT_CL + 63) / 64;
+        L.dg_layers = take((size_t)c.rq_n_layers * DT_CL * dt_slots_per_layer(n_ub) * DT_SLOT);
+        L.dg_head = take((size_t)(c.n_quantizers - 1) * DT_CL * DT_HEAD_SLOTS * DT_SLOT);
     }
     // fused two-kernel layers (single row): x as each block sees it, and the partial rows between blocks
     L.fx_a = take(d * 2);
@@ -508,13 +513,13 @@ static void build_tc_maps(VuibEngine* e) {
     e->tc = t;
 }
 
-// Copies the depth weights into the box stream k_depth_group reads (once per binding; needs both the weights and
+// Copies the depth weights into the slot stream k_depth_tc reads (once per binding; needs both the weights and
 // the workspace).  Runs on the legacy default stream and waits for it: binding happens outside any capture.
 static int32_t build_dg_stream(VuibEngine* e) {
     e->dg_stream_ready = false;
     if (!e->have_w || !e->have_ws || !e->lay.dg_layers) return VUIB_OK;
     const VuibConfig& c = e->cfg;
-    DgStreamBuild b;
+    DtStreamBuild b;
     memset(&b, 0, sizeof(b));
     for (int i = 0; i < c.rq_n_layers; ++i) {
         b.wqkv[i] = static_cast<const bf16*>(e->w.rq_wqkv[i]);
@@ -528,12 +533,12 @@ static int32_t build_dg_stream(VuibEngine* e) {
     b.head_out = e->ws + e->lay.dg_head;
     b.n_layers = c.rq_n_layers;
     b.ffn = c.rq_ffn;
-    b.upc = c.rq_ffn / DG_CL;
+    b.upc = c.rq_ffn / DT_CL;
     b.n_ub = (b.upc + 63) / 64;
     b.CS = c.codebook_size;
     b.n_head_pos = c.n_quantizers - 1;
-    const int boxes = c.rq_n_layers * DG_CL * dg_boxes_per_layer(b.n_ub) + b.n_head_pos * DG_CL * 32;
-    k_build_dg_stream<<<boxes, 256>>>(b);
+    const int slots = c.rq_n_layers * DT_CL * dt_slots_per_layer(b.n_ub) + b.n_head_pos * DT_CL * DT_HEAD_SLOTS;
+    k_build_dt_stream<<<slots, 256>>>(b);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(0));
     e->dg_stream_ready = true;
@@ -1138,44 +1143,50 @@ static int32_t rq_layers(VuibEngine* e, int M, bf16* x, int rows_per_b, int pos_
 }
 
 // ---------------------------------------------------------------------------
-// Many streams: the whole depth loop as one launch (depth_group.cuh).
+// Several streams: the whole depth loop as one launch (depth_tc.cuh).
 // ---------------------------------------------------------------------------
+typedef DepthTcSmem<16, 8, 5> DtSmem8;
+typedef DepthTcSmem<16, 16, 4> DtSmem16;
+typedef DepthTcSmem<32, 18, 3> DtSmem32;
+static_assert(sizeof(DtSmem8) <= 227 * 1024 && sizeof(DtSmem16) <= 227 * 1024 && sizeof(DtSmem32) <= 227 * 1024, "shared memory of k_depth_tc");
+
 static bool depth_group_ok(VuibEngine* e) {
     if (e->depth_group == 0) {
-        const VuibConfig& c = e->cfg;
-        bool ok = e->tc && c.rq_d_model == DG_D && c.rq_n_heads == DG_CL && c.rq_n_layers <= DG_LAYERS &&
-                  c.rq_ffn % DG_CL == 0 && c.rq_ffn / DG_CL <= 192 && c.codebook_size == DG_CL * 256;
+        bool ok = e->tc && depth_tc_shape(e->cfg);
         if (ok) {
-            ok = cudaFuncSetAttribute(k_depth_group<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sizeof(DepthGroupSmem<8>)) == cudaSuccess &&
-                 cudaFuncSetAttribute(k_depth_group<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sizeof(DepthGroupSmem<16>)) == cudaSuccess;
+            ok = cudaFuncSetAttribute(k_depth_tc<16, 8, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DtSmem8)) == cudaSuccess &&
+                 cudaFuncSetAttribute(k_depth_tc<16, 16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DtSmem16)) == cudaSuccess &&
+                 cudaFuncSetAttribute(k_depth_tc<32, 18, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DtSmem32)) == cudaSuccess;
             if (!ok) cudaGetLastError();
         }
         e->depth_group = ok ? 1 : -1;
     }
-    return e->depth_group == 1 && e->dg_stream_ready && !env_off("VUIB_NO_DEPTH_GROUP");
+    return e->depth_group == 1 && e->dg_stream_ready && !env_off("VUIB_NO_DEPTH_GROUP") && !env_off("VUIB_NO_TC");
 }
 
 static int32_t launch_depth_group(VuibEngine* e, int B, const SampleArgs& sa_base, int Qn, cudaStream_t s) {
     const VuibConfig& c = e->cfg;
     const WsLayout& L = e->lay;
-    DepthGroupStream maps;
-    maps.layers = e->ws + L.dg_layers;
-    maps.head = e->ws + L.dg_head;
-    maps.boxes_per_layer = dg_boxes_per_layer((c.rq_ffn / DG_CL + 63) / 64);
-    DepthGroupArgs a;
+    DepthTcArgs a;
     memset(&a, 0, sizeof(a));
+    a.layers = e->ws + L.dg_layers;
+    a.head = e->ws + L.dg_head;
+    a.upc = c.rq_ffn / DT_CL;
+    a.n_ub = (a.upc + 63) / 64;
+    a.slots_per_layer = dt_slots_per_layer(a.n_ub);
     a.B = B;
+    // Streams of a cluster: eight share every step's cost (a warp or a sampling CTA each), and fewer clusters compete for the L2;
+    // beyond 15 clusters of eight, all streams go to the 15 that can be resident at once (a second wave would double the time).
+    int r = B <= 8 * DT_GROUPS ? 8 : (B + DT_GROUPS - 1) / DT_GROUPS;
+    if (r > 18) r = 18;
+    a.r = r;
     a.n_layers = c.rq_n_layers;
     a.Q = c.n_quantizers;
     a.Qn = Qn;
     a.CS = c.codebook_size;
-    a.upc = c.rq_ffn / DG_CL;
     a.max_rows = c.max_rows;
     a.eps = c.rq_norm_eps;
     a.x2 = wsp<bf16>(e, L.rq_x2);
-    a.x1 = wsp<bf16>(e, L.rq_x);
     a.kc = wsp<bf16>(e, L.rq_k);
     a.vc = wsp<bf16>(e, L.rq_v);
     for (int i = 0; i < c.rq_n_layers; ++i) {
@@ -1183,32 +1194,29 @@ static int32_t launch_depth_group(VuibEngine* e, int B, const SampleArgs& sa_bas
         a.mlp_norm[i] = static_cast<const bf16*>(e->w.rq_mlp_norm[i]);
     }
     a.final_norm = static_cast<const bf16*>(e->w.rq_norm);
-    a.logits = wsp<bf16>(e, L.rq_logits);
     a.tap = e->tap_rq;
     a.sa = sa_base;
     a.flag = wsp<int32_t>(e, L.flag);
     a.spin_limit = e->spin_limit;
     a.dbg = env_off("VUIB_TRACE_DEPTH") ? wsp<unsigned long long>(e, L.trace) : nullptr;
-    // groups of 8 streams while they fit the clusters that can be resident at once, else of 16
-    const bool r8 = (B + 7) / 8 <= 15;
-    const int groups = r8 ? (B + 7) / 8 : (B + 15) / 16;
+    const int groups = (B + r - 1) / r;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(groups * DG_CL);
-    cfg.blockDim = dim3(DG_THREADS);
-    cfg.dynamicSmemBytes = r8 ? sizeof(DepthGroupSmem<8>) : sizeof(DepthGroupSmem<16>);
+    cfg.gridDim = dim3(groups * DT_CL);
+    cfg.blockDim = dim3(DT_THREADS);
+    cfg.dynamicSmemBytes = r <= 8 ? sizeof(DtSmem8) : r <= 16 ? sizeof(DtSmem16) : sizeof(DtSmem32);
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = DG_CL;
+    attr[0].val.clusterDim.x = DT_CL;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    prefer_max_smem(reinterpret_cast<const void*>(r8 ? k_depth_group<8> : k_depth_group<16>));
-    if (r8) CK(cudaLaunchKernelEx(&cfg, k_depth_group<8>, maps, a));
-    else CK(cudaLaunchKernelEx(&cfg, k_depth_group<16>, maps, a));
+    const auto kern = r <= 8 ? k_depth_tc<16, 8, 5> : r <= 16 ? k_depth_tc<16, 16, 4> : k_depth_tc<32, 18, 3>;
+    prefer_max_smem(reinterpret_cast<const void*>(kern));
+    CK(cudaLaunchKernelEx(&cfg, kern, a));
     e->launches++;
     return VUIB_OK;
 }
@@ -1277,7 +1285,8 @@ static int32_t run_depth(VuibEngine* e, int B, const int32_t* slots, const bf16*
         EpiProjPos ep{static_cast<const bf16*>(e->w.rq_backbone_proj), c.d_model, pos_emb, x2, rd, 2};
         CK(VUIB_GEMV(c.d_model, e, sc, ep, B, rd, s));
     }
-    if (tc && depth_group_ok(e)) return launch_depth_group(e, B, sa, Qn, s);
+    // one stream has the fused two-kernel layers; without them it runs what several streams run, bit for bit
+    if ((B > 1 || !fused_depth_ok(e)) && depth_group_ok(e)) return launch_depth_group(e, B, sa, Qn, s);
     rc = tc ? rq_layers_tc(e, 2 * B, x2, 2, 0, s) : rq_layers(e, 2 * B, x2, 2, 0, s);
     if (rc) return rc;
 
@@ -1313,7 +1322,7 @@ static int32_t run_depth(VuibEngine* e, int B, const int32_t* slots, const bf16*
         sa.emb_p = i + 2;
         sa.emb_row_mul = 1;
         sa.emb_row_add = 0;
-        CK(launch(k_sample, B, SAMPLE_THREADS, 0, s, sa));
+        CK(launch(k_sample_rq, B, SAMPLE_THREADS, 0, s, sa));
         e->launches++;
         CK(cudaGetLastError());
     }
@@ -1483,7 +1492,7 @@ extern "C" int32_t vuib_sample_rows(VuibEngine* e, int32_t B, const int32_t* slo
     sa.bump_frame = 1;
     sa.n_slots = e->cfg.n_slots;
     sa.flag = wsp<int32_t>(e, L.flag);
-    CK(launch(k_sample, B, SAMPLE_THREADS, 0, static_cast<cudaStream_t>(stream), sa));
+    CK(launch(sa.codebook ? k_sample_rq : k_sample, B, SAMPLE_THREADS, 0, static_cast<cudaStream_t>(stream), sa));
     e->launches++;
     CK(cudaGetLastError());
     return VUIB_OK;
