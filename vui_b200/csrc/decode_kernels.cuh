@@ -820,9 +820,19 @@ __device__ __forceinline__ void bar_named(int id, int n) {
 }
 
 struct AttnSmem {
-    float sm[4][2][8][10];  // [warp][head][s][acc8, m, l]
+    alignas(16) float o[4][2][HD];   // [warp][head][dim]
+    float ml[4][2][2];               // [warp][head]: max, sum
     int s_last;
 };
+
+// Two fp32 multiply-adds in one instruction.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d)
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)), "l"(*reinterpret_cast<unsigned long long*>(&c)));
+    return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 bf2(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 
 // One (split, kv head, row) unit of work for a group of ATT_THREADS threads whose
 // index within the group is `tid`; the group synchronises on named barrier bar_id.
@@ -865,87 +875,107 @@ __device__ __forceinline__ void attn_unit(const AttnArgs& a, int sp, int kvh, in
             vr[it] = make_uint4(0, 0, 0, 0);
         }
     }
-    float (&sm)[4][2][8][10] = S_.sm;
     int& s_last = S_.s_last;
-    float qf[2][8];
+    float2 q2[2][4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const int hq = kvh * G + (h < G ? h : 0);
-        unpack8(__ldcg(reinterpret_cast<const uint4*>(a.q + (size_t)r * a.Hq * HD + hq * HD + s * 8)), qf[h]);
+        const uint4 qw = __ldcg(reinterpret_cast<const uint4*>(a.q + (size_t)r * a.Hq * HD + hq * HD + s * 8));
+        q2[h][0] = bf2(qw.x); q2[h][1] = bf2(qw.y); q2[h][2] = bf2(qw.z); q2[h][3] = bf2(qw.w);
     }
     attn_stamp(a, tid, 1);
-    float m[2] = {NEG_BIG, NEG_BIG}, l[2] = {0.f, 0.f}, acc[2][8];
+    // All scores of the lane's eight keys and two heads first: 16 sums over the eight lanes of a group, halved in every step, so that
+    // lane s ends up with head s >> 2 and keys 2 (s & 3), 2 (s & 3) + 1.  One maximum and one exponential a score then; with a
+    // running softmax in every lane the arithmetic took longer than the keys' way from memory.
+    float d[16];
+#pragma unroll
+    for (int it = 0; it < ATT_ITERS; ++it) {
+        const float2 k2[4] = {bf2(kr[it].x), bf2(kr[it].y), bf2(kr[it].z), bf2(kr[it].w)};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float2 x = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x = fma2(q2[h][j], k2[j], x);
+            d[h * 8 + it] = x.x + x.y;
+        }
+    }
+    const bool b2 = s & 4, b1 = s & 2, b0 = s & 1;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float got = __shfl_xor_sync(0xffffffffu, b2 ? d[i] : d[i + 8], 4);
+        d[i] = (b2 ? d[i + 8] : d[i]) + got;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float got = __shfl_xor_sync(0xffffffffu, b1 ? d[i] : d[i + 4], 2);
+        d[i] = (b1 ? d[i + 4] : d[i]) + got;
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const float got = __shfl_xor_sync(0xffffffffu, b0 ? d[i] : d[i + 2], 1);
+        d[i] = (b0 ? d[i + 2] : d[i]) + got;
+    }
+    float p[2], m = NEG_BIG, l;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int t = t_begin + (2 * (s & 3) + i) * 16 + warp * 4 + g;
+        p[i] = t < t_end ? d[i] * 0.125f : NEG_BIG;
+        m = fmaxf(m, p[i]);
+    }
+#pragma unroll
+    for (int o = 1; o <= 16; o <<= 1)
+        if (o != 4) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) p[i] = p[i] > NEG_BIG ? __expf(p[i] - m) : 0.f;
+    l = p[0] + p[1];
+#pragma unroll
+    for (int o = 1; o <= 16; o <<= 1)
+        if (o != 4) l += __shfl_xor_sync(0xffffffffu, l, o);
+    attn_stamp(a, tid, 2);
+    float2 acc[2][4];
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[h][j] = 0.f;
-
+        for (int j = 0; j < 4; ++j) acc[h][j] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int it = 0; it < ATT_ITERS; ++it) {
-        const int t = t_begin + it * 16 + warp * 4 + g;
-        float kf[8], vf[8];
-        unpack8(kr[it], kf);
-        unpack8(vr[it], vf);
-        float d[2];
+        const float2 v2[4] = {bf2(vr[it].x), bf2(vr[it].y), bf2(vr[it].z), bf2(vr[it].w)};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            float dd = 0.f;
+            const float w = __shfl_sync(0xffffffffu, p[it & 1], (lane & 24) + h * 4 + (it >> 1));
 #pragma unroll
-            for (int j = 0; j < 8; ++j) dd = fmaf(qf[h][j], kf[j], dd);
-            dd += __shfl_xor_sync(0xffffffffu, dd, 1);
-            dd += __shfl_xor_sync(0xffffffffu, dd, 2);
-            dd += __shfl_xor_sync(0xffffffffu, dd, 4);
-            d[h] = dd * 0.125f;
-        }
-        if (t < t_end) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const float mn = fmaxf(m[h], d[h]);
-                const float corr = __expf(m[h] - mn), p = __expf(d[h] - mn);
-                l[h] = l[h] * corr + p;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[h][j] = fmaf(p, vf[j], acc[h][j] * corr);
-                m[h] = mn;
-            }
+            for (int j = 0; j < 4; ++j) acc[h][j] = fma2(make_float2(w, w), v2[j], acc[h][j]);
         }
     }
-    attn_stamp(a, tid, 2);
-    // merge the 4 key groups of the warp
+    // sums over the four key groups of the warp, halved in the same way: group g keeps head g >> 1 and half g & 1 of its eight dims
+    float o8[8];
 #pragma unroll
-    for (int o = 8; o <= 16; o <<= 1) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const float mo = __shfl_xor_sync(0xffffffffu, m[h], o);
-            const float lo = __shfl_xor_sync(0xffffffffu, l[h], o);
-            float ao[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) ao[j] = __shfl_xor_sync(0xffffffffu, acc[h][j], o);
-            softmax_merge(m[h], l[h], acc[h], mo, lo, ao);
-        }
+    for (int j = 0; j < 8; ++j) {
+        const float a0 = j & 1 ? acc[0][j >> 1].y : acc[0][j >> 1].x, a1 = j & 1 ? acc[1][j >> 1].y : acc[1][j >> 1].x;
+        const bool up = g & 2;
+        o8[j] = (up ? a1 : a0) + __shfl_xor_sync(0xffffffffu, up ? a0 : a1, 16);
     }
-    if (g == 0) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) sm[warp][h][s][j] = acc[h][j];
-            sm[warp][h][s][8] = m[h];
-            sm[warp][h][s][9] = l[h];
-        }
+    for (int j = 0; j < 4; ++j) {
+        const bool up = g & 1;
+        const float got = __shfl_xor_sync(0xffffffffu, up ? o8[j] : o8[j + 4], 8);
+        o8[j] = (up ? o8[j + 4] : o8[j]) + got;
     }
+    *reinterpret_cast<float4*>(&S_.o[warp][g >> 1][s * 8 + (g & 1) * 4]) = make_float4(o8[0], o8[1], o8[2], o8[3]);
+    if (g == 0 && (s & 3) == 0) { S_.ml[warp][s >> 2][0] = m; S_.ml[warp][s >> 2][1] = l; }
     attn_stamp(a, tid, 3);
     bar_named(bar_id, ATT_THREADS);
     // thread (h, dim): merge the 4 warps
     const int h = tid >> 6, dim = tid & 63;
-    const int ds = dim >> 3, dj = dim & 7;
     float M_ = NEG_BIG;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) M_ = fmaxf(M_, sm[w][h][ds][8]);
+    for (int w = 0; w < 4; ++w) M_ = fmaxf(M_, S_.ml[w][h][0]);
     float L_ = 0.f, O_ = 0.f;
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-        const float c = __expf(sm[w][h][ds][8] - M_);
-        L_ += sm[w][h][ds][9] * c;
-        O_ += sm[w][h][ds][dj] * c;
+        const float c = __expf(S_.ml[w][h][0] - M_);
+        L_ += S_.ml[w][h][1] * c;
+        O_ += S_.o[w][h][dim] * c;
     }
     const bool head_ok = h < G;
     const int hq = kvh * G + (head_ok ? h : 0);
