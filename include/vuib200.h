@@ -296,9 +296,9 @@ int32_t vuib_read_trace(VuibEngine* e, uint64_t* out_host, int32_t n_stamps);
  * flag is followed by vuib_reset_state before the handle is used again. */
 int32_t vuib_set_wait_limit(VuibEngine* e, uint32_t polls);
 
-/* Test hook for the bound above: presets the arrival counters so that the next tensor-core GEMM
- * launch sees one arrival fewer than it waits for.  Its wait runs out, the flag is recorded, the
- * kernel returns.  Nothing faults or hangs.  Synchronises `stream`. */
+/* Test hook for the bound above: the next tensor-core GEMM whose tiles are shared by a cluster waits for
+ * one value more than is sent to it.  Its wait runs out, the flag is recorded, the kernel returns.
+ * Nothing faults or hangs. */
 int32_t vuib_debug_withhold_arrival(VuibEngine* e, void* stream);
 
 /* Position-only rewind / reset (engine.py:651-654).  Synchronous small copies. */

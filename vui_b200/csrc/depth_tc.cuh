@@ -20,6 +20,7 @@
 // is bounded: a thread whose wait runs out records the device flag and no longer waits.  No load uses cluster multicast.
 #pragma once
 #include "fused_blocks.cuh"
+#include "tc_gemm.cuh"
 
 namespace vuib {
 
@@ -126,12 +127,6 @@ struct DepthTcSmem {
 
 __device__ __forceinline__ void dt_bar() { bar_named(1, DT_CONSUMERS); }
 
-__device__ __forceinline__ bool dt_elect() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
-}
-
 // A thread's bounded waits: after the first that runs out it only looks once.
 struct DtWait {
     int32_t* flag;
@@ -155,39 +150,12 @@ struct DtWait {
     }
 };
 
-__device__ __forceinline__ void dt_push_v4(uint32_t dst, uint32_t bar, float a, float b, float c, float d) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
-                 ::"r"(dst), "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar) : "memory");
-}
 __device__ __forceinline__ void dt_push_b32(uint32_t dst, uint32_t bar, uint32_t v) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst), "r"(v), "r"(bar) : "memory");
 }
-// ---- MMA side: operands K-major in 128-byte swizzle (rows 128 bytes apart, 8-row groups 1024), low descriptor words only
-__device__ __forceinline__ uint32_t dt_desc(const void* smem) { return (smem_u32(smem) >> 4 & 0x3FFF) | 1u << 16; }
-constexpr uint32_t DT_DESC_HI = (1024u >> 4) | 1u << 14 | 2u << 29;
-template <int N>
-constexpr uint32_t DT_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | (8u << 24);
-
-// 64 of K for one tile: four MMAs.  With TEST the barrier of the next stage is tested in front of them and the answer collected
-// behind (a test's 170 cycles would otherwise be the tensor pipe's too).
 template <int N, bool FIRST, bool TEST>
 __device__ __forceinline__ uint32_t dt_mma4(uint32_t d, uint32_t a, uint32_t b, uint32_t bar, uint32_t parity) {
-    uint32_t ok = 0;
-#define DT_BODY(pre, post)                                                                                                        \
-    "{\n\t.reg .pred p;\n\t.reg .b64 x, y;\n\t.reg .b32 t, u;\n\t" pre                                                              \
-    "mov.b64 x, {%2, %4};\n\tmov.b64 y, {%3, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%1], x, y, %5, %8;\n\t"                     \
-    "add.u32 t, %2, 2;\n\tadd.u32 u, %3, 2;\n\tmov.b64 x, {t, %4};\n\tmov.b64 y, {u, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%1], x, y, %5, 1;\n\t" \
-    "add.u32 t, %2, 4;\n\tadd.u32 u, %3, 4;\n\tmov.b64 x, {t, %4};\n\tmov.b64 y, {u, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%1], x, y, %5, 1;\n\t" \
-    "add.u32 t, %2, 6;\n\tadd.u32 u, %3, 6;\n\tmov.b64 x, {t, %4};\n\tmov.b64 y, {u, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%1], x, y, %5, 1;\n\t" \
-    post "}"
-#define DT_OPS : "=r"(ok) : "r"(d), "r"(a), "r"(b), "r"(DT_DESC_HI), "r"(DT_IDESC<N>), "r"(bar), "r"(parity), "n"(FIRST ? 0 : 1) : "memory"
-    if constexpr (TEST)
-        asm volatile(DT_BODY("mbarrier.test_wait.parity.shared::cta.b64 p, [%6], %7;\n\t", "selp.u32 %0, 1, 0, p;\n\t") DT_OPS);
-    else
-        asm volatile(DT_BODY("", "mov.u32 %0, 0;\n\t") DT_OPS);
-#undef DT_BODY
-#undef DT_OPS
-    return ok;
+    return tc_mma4<FIRST, TEST>(d, a, b, tc_idesc(N), bar, parity);
 }
 
 // The first columns of this thread's row of a tile: as many as hold RMAX streams.
@@ -242,17 +210,6 @@ __device__ __forceinline__ void dt_norm(S& sm, const bf16* w, float eps, int nv)
         *reinterpret_cast<uint4*>(row + ((q ^ (n & 7)) << 4)) = pack8(o0);
         *reinterpret_cast<uint4*>(row + (((q + 1) ^ (n & 7)) << 4)) = pack8(o1);
     }
-}
-
-// x / (1 + exp(-x)) without a branch: the divisor's reciprocal with a Newton step, the quotient with a residual correction.  (The
-// compiler's division has a slow path, and with a branch in each the eight streams of a thread followed one another.)
-__device__ __forceinline__ float dt_silu(float x) {
-    const float d = 1.0f + expf(fminf(-x, 80.f));
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    r = fmaf(r, fmaf(-d, r, 1.0f), r);
-    const float q = x * r;
-    return fmaf(r, fmaf(-q, d, x), q);
 }
 
 // What this warp wrote to an MMA operand (and read from tensor memory) is done: one arrival of eight.
@@ -361,14 +318,18 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
 
     if (warp == DT_CONSUMERS / 32) {
         // ---------------------------------------------------------------- producer: the slot stream, stage by stage
-        if (dt_elect()) {
+        if (tc_elect()) {
             DtWait w{a.flag, 16u * a.spin_limit};
             int st = 0;
             unsigned ph = 1;
+            bool waited = false;
             bool filled = false;
             auto stages = [&](const unsigned char* src, int n) {
                 for (int i = 0; i < n; ++i) {
-                    if (filled) w.local(&sm.empty[st], ph);
+                    if (filled) {
+                        if (!waited) { pdl_wait(); waited = true; }   // the ring is full until the dependency is met
+                        w.local(&sm.empty[st], ph);
+                    }
                     mbar_expect_tx(&sm.full[st], DT_STAGE);
                     bulk_g2s(sm.ring[st], src + (size_t)i * DT_STAGE, DT_STAGE, &sm.full[st]);
                     if (++st == STAGES) { st = 0; ph ^= 1; filled = true; }
@@ -384,12 +345,13 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
         cluster_wait();
     } else if (warp == DT_CONSUMERS / 32 + 1) {
         // ---------------------------------------------------------------- MMA thread
-        if (dt_elect()) {
+        if (tc_elect()) {
+            pdl_wait();   // its length is not this thread's barriers' to count
             DtWait w{a.flag, 16u * a.spin_limit};
             int st = 0;
             unsigned ph = 0, ph_h = 0, ph_l = 0;
             uint32_t ok = 0;
-            const uint32_t ring0 = dt_desc(sm.ring[0]), h0 = dt_desc(sm.h[0]), at0 = dt_desc(sm.attn), g0 = dt_desc(sm.g[0]);
+            const uint32_t ring0 = tc_desc(sm.ring[0]), h0 = tc_desc(sm.h[0]), at0 = tc_desc(sm.attn), g0 = tc_desc(sm.g[0]);
             constexpr uint32_t CHUNK = N * 128 >> 4, SLOT = DT_SLOT >> 4;
             uint32_t slot = 0, nbar = 0, nph = 0;
             // the stage's first slot; where the next stage will be
@@ -657,7 +619,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
                         if (shared && (i & 1) != half) continue;
                         const float got = __shfl_xor_sync(0xffffffffu, low ? v[i + HN] : v[i], 16);
                         const float a1 = rbf(low ? v[i] : got), a3 = rbf(low ? got : v[i + HN]);
-                        const float sl = rbf(dt_silu(a1));
+                        const float sl = rbf(silu(a1));
                         const int n = low ? i : i + HN;
                         *reinterpret_cast<bf16*>(sm.g[t] + n * 128 + (((u >> 3) ^ (n & 7)) << 4) + (u & 7) * 2) = f2bf(sl * a3);
                     }

@@ -425,6 +425,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) k_sg(const __grid_constant__ Sg
         __syncwarp();
     } else if (warp == 2) {
         if (sg_elect()) {
+            sg_pdl_wait();   // the windows come behind the dependency: its wait is not this thread's barriers' to count
             const uint32_t a_plane = a_bytes / 3 >> 4, a0 = sg_desc_lo(sg_smem(sA)) + shift0 * 4, b0 = sg_desc_lo(sg_smem(sB));
             int sa = 0, sb = 0, seg = 0, left = 0;      // slots, segments so far, channel groups left in this one
             uint32_t pa = 0, pb = 0, ok = 0, d = 0, fb = 0;   // parities, what is known to be complete, accumulators, first weight stage
@@ -553,7 +554,10 @@ __global__ void __launch_bounds__(SG_THREADS, 1) k_sg(const __grid_constant__ Sg
         asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;\n\tbarrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (s_bad && tid == 0) atomicOr(a.flag, SG_FLAG_WAIT);
+    if (s_bad && tid == 0) {   // gave up somewhere: what may still be on its way to this CTA's shared memory lands before it retires
+        atomicOr(a.flag, SG_FLAG_WAIT);
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    }
     if (warp == 3) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
 }
 

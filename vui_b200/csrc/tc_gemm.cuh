@@ -1,23 +1,18 @@
-// Skinny GEMM for many streams / prefill rows on the 5th-generation tensor cores:
+// GEMM for several streams and for prefill rows on the 5th-generation tensor cores:
 //   D[n][m] = sum_k W[n][k] * X[m][k]      (W: weights (N, K) bf16; X: activations (M, K) bf16)
-// "swap-AB": a tile of 128 weight rows is the MMA's M side, the (padded) batch of 16..256
-// activation rows its N side, so one tcgen05.mma covers every stream at once and each weight
-// byte is read from HBM exactly once per step.
+// "swap-AB": a tile of 128 weight rows is the MMA's M side, MT = 16 .. 128 activation rows its N side, so one tcgen05.mma covers
+// every stream of the tile and each weight byte is read once per row block.
 //
-//  * operands reach shared memory through TMA (cp.async.bulk.tensor.2d, 128-byte swizzle,
-//    K-major), one elected thread issues tcgen05.mma (kind::f16, bf16 x bf16 -> fp32), the
-//    accumulator tile lives in tensor memory and is read back with tcgen05.ld for the epilogue;
-//  * an mbarrier ring (full / empty per stage) decouples the TMA thread from the MMA thread; every
-//    wait is bounded and records FLAG_TC_TIMEOUT instead of hanging;
-//  * one tcgen05.mma of this shape costs ~96 ns whatever the batch, i.e. an SM consumes weights at
-//    only ~42 GB/s, so the K dimension is split over enough CTAs to occupy every SM; the CTAs of a
-//    tile (all resident: the grid never exceeds the SM count times two) publish their partial tile,
-//    meet on a counter with a bounded wait, and EACH adds the splits - in index order, so the result
-//    is deterministic - for its own 1/splits slice of the rows and runs the epilogue functor there
-//    (RoPE + KV append, residual add, SwiGLU, logits);
-//  * launched with programmatic dependent launch: the weight tiles of the first stages are
-//    requested before the kernel waits for its predecessor, the activations after.
-// No TMA load here uses cluster multicast.
+//  * operands reach shared memory through TMA (cp.async.bulk.tensor.2d, 128-byte swizzle, K-major), one elected thread issues
+//    tcgen05.mma (kind::f16, bf16 x bf16 -> fp32; max(MT / 2, 32 + MT / 4) cycles per 16 of K), the accumulator tile lives in tensor
+//    memory and is read back with tcgen05.ld; an mbarrier ring decouples the two;
+//  * few tiles leave most SMs idle, so the CTAs of a cluster (2 or 4) share a tile's K.  Each sends its partial rows to the CTA
+//    that finishes them (st.async into the owner's shared memory, counted on its mbarrier: one hop), which adds them in a
+//    fixed order and runs the epilogue functor (RoPE + KV append, residual add, SwiGLU, logits).  Through global memory and a
+//    counter the exchange took 5 us of a GEMM's 9;
+//  * launched with programmatic dependent launch: the weight tiles of the first stages are requested before the kernel waits for
+//    its predecessor, the activations after.
+// Every wait is bounded and records FLAG_TC_TIMEOUT instead of hanging.  No TMA load here uses cluster multicast.
 #pragma once
 #include <cuda.h>
 
@@ -25,8 +20,9 @@
 
 namespace vuib {
 
-constexpr int TC_THREADS = 128;
-constexpr int TC_TILE_N = 128;      // weight rows per CTA (two TMA boxes of 64 rows)
+constexpr int TC_THREADS = 256;
+constexpr int TC_TILE_N = 128;      // weight rows per CTA
+constexpr int TC_BOX_N = 64;        // rows of a TMA box of weights (PAIRED: 16, w1 and w3 in turn)
 constexpr int TC_KCHUNK = 64;       // bf16 per row per stage = 128 bytes = one swizzle span
 constexpr int TC_MAX_STAGES = 12;     // ring depth is set per launch from the shared memory left
 constexpr int TC_EPI_BYTES_PER_M = 256;  // epilogue staging per activation row (128 bf16)
@@ -70,30 +66,44 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
         : "memory");
 }
 
-// K-major, 128-byte-swizzled operand tile: rows are 128 bytes apart, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t umma_desc_sw128(const void* smem_tile) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_u32(smem_tile) >> 4) & 0x3FFF);  // start address
-    d |= (uint64_t)1 << 16;                                // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;                      // stride byte offset between 8-row groups
-    d |= (uint64_t)1 << 46;                                // descriptor version (sm_100)
-    d |= (uint64_t)2 << 61;                                // SWIZZLE_128B
-    return d;
+// One lane of a converged warp, chosen so that the compiler knows that only one is active: with a comparison of lane numbers it
+// wraps every instruction with uniform operands (TMA copies, MMAs, commits) in a loop over the active lanes.
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
 }
 
+// Descriptor of a K-major, 128-byte-swizzled operand tile (rows 128 bytes apart, 8-row groups 1024): the low word holds the start
+// address in 16-byte units, the high word is the same for all.  The issuing thread adds 32-bit offsets only: the tensor pipe has
+// next to no queue, so that what it spends on 64-bit descriptors and predicates the pipe waits for too.
+__device__ __forceinline__ uint32_t tc_desc(const void* smem) { return (smem_u32(smem) >> 4 & 0x3FFF) | 1u << 16; }
+constexpr uint32_t TC_DESC_HI = (1024u >> 4) | 1u << 14 | 2u << 29;
 // kind::f16 instruction descriptor: bf16 A and B, fp32 accumulate, both K-major, M = 128, N = n.
-__device__ __forceinline__ uint32_t umma_idesc_bf16(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+__host__ __device__ constexpr uint32_t tc_idesc(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (8u << 24);
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
+// 64 of K for one tile: four MMAs.  With TEST the barrier of the next stage is tested in front of them and the answer collected
+// behind (a test's 170 cycles would otherwise be the tensor pipe's too).
+template <bool FIRST, bool TEST>
+__device__ __forceinline__ uint32_t tc_mma4(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t bar, uint32_t parity) {
+    uint32_t ok = 0;
+#define TC_BODY(pre, post)                                                                                                        \
+    "{\n\t.reg .pred p;\n\t.reg .b64 x, y;\n\t.reg .b32 t, u;\n\t" pre                                                              \
+    "mov.b64 x, {%2, %4};\n\tmov.b64 y, {%3, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%1], x, y, %5, %8;\n\t"                     \
+    "add.u32 t, %2, 2;\n\tadd.u32 u, %3, 2;\n\tmov.b64 x, {t, %4};\n\tmov.b64 y, {u, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%1], x, y, %5, 1;\n\t" \
+    "add.u32 t, %2, 4;\n\tadd.u32 u, %3, 4;\n\tmov.b64 x, {t, %4};\n\tmov.b64 y, {u, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%1], x, y, %5, 1;\n\t" \
+    "add.u32 t, %2, 6;\n\tadd.u32 u, %3, 6;\n\tmov.b64 x, {t, %4};\n\tmov.b64 y, {u, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%1], x, y, %5, 1;\n\t" \
+    post "}"
+#define TC_OPS : "=r"(ok) : "r"(d), "r"(a), "r"(b), "r"(TC_DESC_HI), "r"(idesc), "r"(bar), "r"(parity), "n"(FIRST ? 0 : 1) : "memory"
+    if constexpr (TEST)
+        asm volatile(TC_BODY("mbarrier.test_wait.parity.shared::cta.b64 p, [%6], %7;\n\t", "selp.u32 %0, 1, 0, p;\n\t") TC_OPS);
+    else
+        asm volatile(TC_BODY("", "mov.u32 %0, 0;\n\t") TC_OPS);
+#undef TC_BODY
+#undef TC_OPS
+    return ok;
 }
 
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -126,6 +136,17 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// x / (1 + exp(-x)) without a branch: the divisor's reciprocal with a Newton step, the quotient with a residual correction.  (The
+// compiler's division has a slow path, and with a branch in each a thread's values follow one another.)
+__device__ __forceinline__ float silu(float x) {
+    const float d = 1.0f + expf(fminf(-x, 80.f));
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    r = fmaf(r, fmaf(-d, r, 1.0f), r);
+    const float q = x * r;
+    return fmaf(r, fmaf(-q, d, x), q);
 }
 
 // ---------------------------------------------------------------------------
@@ -225,8 +246,8 @@ struct TcEpiResidual {  // x += bf16(acc)
     }
 };
 
-struct TcEpiSwiGLU {    // tile rows 0..63 = w1 rows, 64..127 = w3 rows of the same hidden units
-    bf16* act; int F;  // hidden unit of tile row r (< 64) is tile*64 + r
+struct TcEpiSwiGLU {    // of every 32 tile rows, 16 are w1 rows and 16 the same hidden units' w3 rows
+    bf16* act; int F;
     static constexpr bool PAIRED = true;
     static constexpr bool STAGED = false;
     __host__ __device__ TcEpiSwiGLU shifted(int m) const {
@@ -234,15 +255,14 @@ struct TcEpiSwiGLU {    // tile rows 0..63 = w1 rows, 64..127 = w3 rows of the s
         o.act += (size_t)m * F;
         return o;
     }
-    // a1 = the unit's w1 sums, a3 = its w3 sums, for activation rows m0..m0+7
-    __device__ __forceinline__ void apply_pair(int unit, int m0, int M, const float (&a1)[8],
-                                               const float (&a3)[8]) const {
+    // a1 = the unit's w1 sums, a3 = its w3 sums, for activation rows m0 .. m0 + 3
+    __device__ __forceinline__ void apply_pair(int unit, int m0, int M, const float (&a1)[4], const float (&a3)[4]) const {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < 4; ++j) {
             const int m = m0 + j;
             if (m >= M) continue;
             const float a = rbf(a1[j]), g = rbf(a3[j]);
-            const float sl = rbf(a / (1.0f + expf(-a)));
+            const float sl = rbf(silu(a));
             act[(size_t)m * F + unit] = f2bf(sl * g);
         }
     }
@@ -293,26 +313,74 @@ struct TcEpiProjPos {   // depth position 0: bf16(acc) + pos_emb[0], written to 
 };
 
 struct TcArgs {
-    int N;            // weight rows, a multiple of 128 (PAIRED: hidden units, a multiple of 64)
     int row_off;      // first weight row of tile 0 inside the mapped matrix (stacked depth heads)
-    int M, Mpad;      // activation rows in all; rows per CTA padded to a multiple of 16 (<= 256).  M > Mpad: the
-                      // grid's z dimension walks blocks of Mpad rows (one launch for a whole prefill)
-    int chunks;       // K chunks of 64 in all; split s handles chunks [s*chunks/splits, (s+1)*chunks/splits)
-    int stages;       // TMA ring depth (<= TC_MAX_STAGES, <= chunks)
-    int splits;       // gridDim.x: 1, 2, 4, 8 or 16 (PAIRED: not 2)
-    float* partial;   // (row blocks, tiles, splits, 128, Mpad) fp32 scratch (splits > 1)
-    int32_t* counters;  // (2, row blocks x tiles) arrivals / departures, zero between launches
-    int tiles;
+    int M, MT;        // activation rows in all; rows of a tile, 16 to 128: the grid's z dimension walks blocks of MT rows
+    int chunks;       // K chunks of 64 in all; CTA s of a cluster handles chunks [s*chunks/splits, (s+1)*chunks/splits)
+    int stages;       // TMA ring depth (<= TC_MAX_STAGES, <= the shortest split)
+    int splits;       // gridDim.x = CTAs of a cluster: 1, 2 or 4
+    int segs;         // accumulators per CTA: 1, 2 or 4 equal parts of its chunks, added pairwise (see tc_gemm in vuib200.cu)
+    int withhold;     // test hook: the first CTA expects one value more than is sent to it
     int32_t* flag;
     unsigned long long* dbg;  // optional: device-clock stamps of CTA (0,0) (profiling aid)
     unsigned spin_limit;      // polls after which a wait gives up and records FLAG_TC_TIMEOUT
 };
 
 __device__ __forceinline__ void tc_stamp(const TcArgs& a, int i) {
-    if (a.dbg && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 64) {
+    if (a.dbg && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 64) {
         unsigned long long t;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
         a.dbg[i] = t;
+    }
+}
+
+// Eight sums of tile row `row` (n = tile * 128 + row) for activation rows m0 .. m0 + 7.  PAIRED: lanes l and l + 16 hold one unit's w1
+// and w3 sums; the lower one takes the first four activation rows, the upper one the others.
+template <class Epi>
+__device__ __forceinline__ void tc_apply(const Epi& ep, int tile, int row, int m0, int M, const float (&v)[8], const unsigned char* es) {
+    if constexpr (Epi::PAIRED) {
+        const bool low = (row & 16) == 0;
+        float a1[4], a3[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float got = __shfl_xor_sync(0xffffffffu, low ? v[j + 4] : v[j], 16);
+            a1[j] = low ? v[j] : got;
+            a3[j] = low ? got : v[j + 4];
+        }
+        ep.apply_pair(tile * 64 + (row >> 5) * 16 + (row & 15), low ? m0 : m0 + 4, M, a1, a3);
+    } else {
+        ep.apply(tile * TC_TILE_N + row, m0, M, v, nullptr, es);
+    }
+}
+
+// Eight columns of this thread's row, the sum of Q accumulators MT columns apart, added as a balanced tree.
+template <int Q>
+__device__ __forceinline__ void tc_sum(uint32_t addr, int MT, float (&v)[8]) {
+    if constexpr (Q == 1) tmem_ld8(addr, v);
+    else {
+        float u[8];
+        tc_sum<Q / 2>(addr, MT, v);
+        tc_sum<Q / 2>(addr + Q / 2 * MT, MT, u);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] += u[i];
+    }
+}
+__device__ __forceinline__ void tc_sum_of(int segs, uint32_t addr, int MT, float (&v)[8]) {
+    if (segs == 1) tc_sum<1>(addr, MT, v);
+    else if (segs == 2) tc_sum<2>(addr, MT, v);
+    else tc_sum<4>(addr, MT, v);
+}
+// The same over the mailbox's Q sources.
+template <int Q>
+__device__ __forceinline__ void tc_mail_sum(const float* mail, int src_stride, int row_stride, float (&v)[8]) {
+    if constexpr (Q == 1) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = mail[i * row_stride];
+    } else {
+        float u[8];
+        tc_mail_sum<Q / 2>(mail, src_stride, row_stride, v);
+        tc_mail_sum<Q / 2>(mail + Q / 2 * src_stride, src_stride, row_stride, u);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] += u[i];
     }
 }
 
@@ -321,34 +389,36 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 k_gemm_tc(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ CUtensorMap mapA1,
           const __grid_constant__ CUtensorMap mapX, TcArgs a, Epi ep_all) {
     extern __shared__ unsigned char smem_dyn[];
-    __shared__ uint64_t bar_full[TC_MAX_STAGES], bar_empty[TC_MAX_STAGES], bar_done;
+    __shared__ uint64_t bar_full[TC_MAX_STAGES], bar_empty[TC_MAX_STAGES], bar_done, bar_mail;
     __shared__ uint32_t s_tmem;
     __shared__ int s_bad;
-    __shared__ float xchg[Epi::PAIRED ? 128 * 8 : 1];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int split = blockIdx.x, tile = blockIdx.y;  // the CTAs of one tile are neighbours in launch order
-    const int m_base = blockIdx.z * a.Mpad;           // first activation row of this CTA's block
-    const int Mb = min(a.Mpad, a.M - m_base);         // rows of the block
-    const int tile_id = blockIdx.z * a.tiles + tile;  // index of the (block, tile) pair in the split-K scratch
-    const int all_tiles = gridDim.z * a.tiles;
+    const int S = a.splits, rank = blockIdx.x, tile = blockIdx.y;   // the CTAs of one tile are a cluster
+    const int m_base = blockIdx.z * a.MT;             // first activation row of this CTA's block
+    const int Mb = min(a.MT, a.M - m_base);           // rows of the block
     const Epi ep = ep_all.shifted(m_base);
     tc_stamp(a, 0);
-    const int stages = a.stages;  // <= smallest chunk count of any split
-    const uint32_t a_bytes = TC_TILE_N * TC_KCHUNK * 2, b_bytes = (uint32_t)a.Mpad * TC_KCHUNK * 2;
-    const uint32_t stage_bytes = a_bytes + ((b_bytes + 1023u) & ~1023u);
+    const int stages = a.stages;
+    const uint32_t a_bytes = TC_TILE_N * TC_KCHUNK * 2, stage_bytes = a_bytes + (uint32_t)a.MT * TC_KCHUNK * 2;
     unsigned char* base = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
+    const int rpc = TC_TILE_N / S;                    // tile rows this CTA finishes: [rank * rpc, (rank + 1) * rpc)
+    float* mail = reinterpret_cast<float*>(base + (size_t)stages * stage_bytes);         // [source][MT][rpc] (S > 1)
+    unsigned char* es = reinterpret_cast<unsigned char*>(mail) + (S > 1 ? (size_t)TC_TILE_N * a.MT * 4 : 0);  // epilogue staging
+    const int groups = (Mb + 7) / 8;                  // groups of eight activation rows
 
     if (tid == 0) {
         for (int s = 0; s < stages; ++s) { mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 1); }
         mbar_init(&bar_done, 1);
+        mbar_init(&bar_mail, 1);
         s_bad = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        const bool first = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
+        if (S > 1) mbar_expect_tx(&bar_mail, (uint32_t)(S * groups * 8 * rpc * 4 + (first ? a.withhold * 4 : 0)));
     }
-    int tmem_cols = 32;
-    while (tmem_cols < a.Mpad) tmem_cols <<= 1;
-    if (warp == 0) {
+    const int tmem_cols = a.MT * a.segs < 32 ? 32 : a.MT * a.segs;
+    if (warp == 2) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
                      "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -357,183 +427,136 @@ k_gemm_tc(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ CUt
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
+    if (S > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // waited for before the first push
     tc_stamp(a, 1);
     // Only now may the next kernel's CTAs become resident: every CTA of this grid already owns its
     // tensor-memory columns, so early dependents can never starve it of them.
     pdl_trigger();
 
-    const int k_first = (int)((long long)split * a.chunks / a.splits);  // in chunks
-    const int n_chunks = (int)((long long)(split + 1) * a.chunks / a.splits) - k_first;
-    // weight rows of this tile: PAIRED -> 64 rows of each matrix at unit offset tile*64
-    const int rowA0 = a.row_off + (Epi::PAIRED ? tile * 64 : tile * TC_TILE_N);
-    const int rowA1 = a.row_off + (Epi::PAIRED ? tile * 64 : tile * TC_TILE_N + 64);
-
-    // Roles are per warp: the 31 idle lanes of a role's warp park at __syncwarp(), not in an
-    // mbarrier wait, so they cannot hold back the lane that feeds the pipeline.
+    const int k_first = rank * a.chunks / S, n_chunks = (rank + 1) * a.chunks / S - k_first;
     if (warp == 0) {
-      if (lane == 0) {
-        // ---- TMA producer.  Weights for the first ring pass go out before the dependency wait.
-        for (int c = 0; c < stages; ++c) {
-            unsigned char* st = base + (size_t)c * stage_bytes;
-            mbar_expect_tx(&bar_full[c], a_bytes + b_bytes);
-            tma_load_2d(st, &mapA0, (k_first + c) * TC_KCHUNK, rowA0, &bar_full[c]);
-            tma_load_2d(st + a_bytes / 2, &mapA1, (k_first + c) * TC_KCHUNK, rowA1, &bar_full[c]);
-        }
-        pdl_wait();
-        for (int c = 0; c < stages; ++c)
-            tma_load_2d(base + (size_t)c * stage_bytes + a_bytes, &mapX, (k_first + c) * TC_KCHUNK, m_base, &bar_full[c]);
-        for (int c = stages; c < n_chunks; ++c) {
-            const int s = c % stages;
-            if (!mbar_wait(&bar_empty[s], ((c / stages) & 1) ^ 1, 4 * a.spin_limit)) { s_bad = 1; break; }
-            unsigned char* st = base + (size_t)s * stage_bytes;
-            mbar_expect_tx(&bar_full[s], a_bytes + b_bytes);
-            tma_load_2d(st, &mapA0, (k_first + c) * TC_KCHUNK, rowA0, &bar_full[s]);
-            tma_load_2d(st + a_bytes / 2, &mapA1, (k_first + c) * TC_KCHUNK, rowA1, &bar_full[s]);
-            tma_load_2d(st + a_bytes, &mapX, (k_first + c) * TC_KCHUNK, m_base, &bar_full[s]);
-        }
-      }
-      __syncwarp();
-    } else if (warp == 1) {
-      if (lane == 0) {
-        // ---- MMA issuer
-        const uint32_t idesc = umma_idesc_bf16(a.Mpad);
-        for (int c = 0; c < n_chunks; ++c) {
-            const int s = c % stages;
-            if (!mbar_wait(&bar_full[s], (c / stages) & 1, 4 * a.spin_limit)) { s_bad = 1; break; }
-            if (a.dbg && split == 0 && tile == 0 && c < 8) {
-                unsigned long long t;
-                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-                a.dbg[8 + c] = t;  // when chunk c (< 8) became available to the MMA thread
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            unsigned char* st = base + (size_t)s * stage_bytes;
-            const uint64_t da = umma_desc_sw128(st), db = umma_desc_sw128(st + a_bytes);
+        if (tc_elect()) {
+            // ---- TMA producer.  Weights for the first ring pass go out before the dependency wait.
+            auto weights = [&](int c, int s) {
+                unsigned char* st = base + (size_t)s * stage_bytes;
+                const int x = (k_first + c) * TC_KCHUNK;
+                mbar_expect_tx(&bar_full[s], stage_bytes);
+                if constexpr (Epi::PAIRED) {
 #pragma unroll
-            for (int kk = 0; kk < TC_KCHUNK / 16; ++kk)  // 16 bf16 = 32 bytes = 2 descriptor units per step
-                umma_bf16(tmem, da + 2 * kk, db + 2 * kk, idesc, (c > 0 || kk > 0) ? 1u : 0u);
-            umma_commit(&bar_empty[s]);
+                    for (int i = 0; i < 4; ++i) {
+                        tma_load_2d(st + i * 4096, &mapA0, x, a.row_off + tile * 64 + i * 16, &bar_full[s]);
+                        tma_load_2d(st + i * 4096 + 2048, &mapA1, x, a.row_off + tile * 64 + i * 16, &bar_full[s]);
+                    }
+                } else {
+                    tma_load_2d(st, &mapA0, x, a.row_off + tile * TC_TILE_N, &bar_full[s]);
+                    tma_load_2d(st + a_bytes / 2, &mapA0, x, a.row_off + tile * TC_TILE_N + 64, &bar_full[s]);
+                }
+            };
+            auto acts = [&](int c, int s) {
+                tma_load_2d(base + (size_t)s * stage_bytes + a_bytes, &mapX, (k_first + c) * TC_KCHUNK, m_base, &bar_full[s]);
+            };
+            for (int c = 0; c < stages; ++c) weights(c, c);
+            pdl_wait();
+            for (int c = 0; c < stages; ++c) acts(c, c);
+            unsigned limit = 4 * a.spin_limit, ph = 0;
+            for (int c = stages, s = 0; c < n_chunks; ++c) {
+                if (!mbar_wait(&bar_empty[s], ph, limit)) { s_bad = 1; limit = 16; }
+                weights(c, s);
+                acts(c, s);
+                if (++s == stages) { s = 0; ph ^= 1; }
+            }
         }
-        umma_commit(&bar_done);
-      }
-      __syncwarp();
+        __syncwarp();
+    } else if (warp == 1) {
+        if (tc_elect()) {
+            // ---- MMA issuer.  The activations come behind the dependency: its wait is not this thread's barriers' to count.
+            pdl_wait();
+            const uint32_t idesc = tc_idesc(a.MT), d0 = tc_desc(base);
+            unsigned limit = 4 * a.spin_limit, ph = 0;
+            uint32_t ok = 0;
+            for (int c = 0, s = 0, seg = 0, next = 0; c < n_chunks; ++c) {
+                const bool first = c == next;   // of a segment: the next accumulator
+                if (first) {
+                    ++seg;
+                    next = (rank * a.segs + seg) * a.chunks / (S * a.segs) - k_first;
+                }
+                const uint32_t d = tmem + (seg - 1) * a.MT;
+                if (!ok && !mbar_wait(&bar_full[s], ph, limit)) { s_bad = 1; limit = 16; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t da = d0 + s * (stage_bytes >> 4), db = da + (a_bytes >> 4);
+                uint64_t* const done = &bar_empty[s];
+                if (++s == stages) { s = 0; ph ^= 1; }
+                if (first) ok = tc_mma4<true, true>(d, da, db, idesc, smem_u32(&bar_full[s]), ph);
+                else ok = tc_mma4<false, true>(d, da, db, idesc, smem_u32(&bar_full[s]), ph);
+                umma_commit(done);
+            }
+            umma_commit(&bar_done);
+        }
+        __syncwarp();
     }
     pdl_wait();
     tc_stamp(a, 2);
-    unsigned char* es = base + (size_t)stages * stage_bytes;  // epilogue staging, filled while the MMAs run
-    if constexpr (Epi::STAGED) ep.stage(es, tile, Mb, tid);
+    if constexpr (Epi::STAGED) ep.stage(es, tile, Mb, tid);   // while the MMAs run
     // ---- everyone: wait for the accumulator
     const bool done_ok = mbar_wait(&bar_done, 0, 4 * a.spin_limit);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     __syncthreads();
-    if ((!done_ok || s_bad) && tid == 0) atomicOr(a.flag, FLAG_TC_TIMEOUT);
     tc_stamp(a, 3);
-
-    const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);  // thread tid reads tile row tid (TMEM lane)
-    if (a.splits == 1) {
-        for (int m0 = 0; m0 < a.Mpad; m0 += 8) {
+    // warps w and w + 4 read tile rows 32 (w & 3) ..: every other group of eight activation rows each
+    const int row = (warp & 3) * 32 + lane, half = warp >> 2;
+    const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    bool mail_ok = true;
+    if (S == 1) {
+        for (int g = half; g < groups; g += 2) {
             float v[8];
-            tmem_ld8(trow + m0, v);
-            if constexpr (Epi::PAIRED) {  // rows r and r+64 are the w1 / w3 sums of hidden unit tile*64 + r
-#pragma unroll
-                for (int j = 0; j < 8; ++j) xchg[tid * 8 + j] = v[j];
-                __syncthreads();
-                if (tid < 64) {
-                    float g[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) g[j] = xchg[(tid + 64) * 8 + j];
-                    ep.apply_pair(tile * 64 + tid, m0, Mb, v, g);
-                }
-                __syncthreads();
-            } else {
-                ep.apply(tile * TC_TILE_N + tid, m0, Mb, v, xchg, es);
-            }
+            tc_sum_of(a.segs, trow + g * 8, a.MT, v);
+            tc_apply(ep, tile, row, g * 8, Mb, v, es);
         }
     } else {
-        // partial tile to scratch as [m][n]: the 128 threads of a CTA write 512 contiguous bytes per m
-        float* mine = a.partial + ((size_t)tile_id * a.splits + split) * a.Mpad * TC_TILE_N;
-        int m0 = 0;
-        for (; m0 + 32 <= a.Mpad; m0 += 32) {
-            float v[32];
-            tmem_ld32(trow + m0, v);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) mine[(size_t)(m0 + j) * TC_TILE_N + tid] = v[j];
-        }
-        for (; m0 < a.Mpad; m0 += 8) {
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every peer has set up its mailbox
+        const int owner = row / rpc;
+        uint32_t dst, bar;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(mail + (size_t)rank * a.MT * rpc + row % rpc)), "r"(owner));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(smem_u32(&bar_mail)), "r"(owner));
+        for (int g = half; g < groups; g += 2) {
             float v[8];
-            tmem_ld8(trow + m0, v);
+            tc_sum_of(a.segs, trow + g * 8, a.MT, v);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) mine[(size_t)(m0 + j) * TC_TILE_N + tid] = v[j];
+            for (int j = 0; j < 8; ++j)
+                asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];"
+                             ::"r"(dst + (uint32_t)((g * 8 + j) * rpc * 4)), "f"(v[j]), "r"(bar) : "memory");
         }
         tc_stamp(a, 4);
-        __syncthreads();  // orders every thread's partial stores before thread 0's release below
-        if (tid == 0) {
-            // arrive, then wait (bounded) until every split of this tile has published its partial
-            asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(a.counters + tile_id) : "memory");
-            int v = 0;
-            unsigned spins = 0;
-            for (;;) {
-                asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(a.counters + tile_id) : "memory");
-                if (v >= a.splits) break;
-                if (++spins > a.spin_limit) { atomicOr(a.flag, FLAG_TC_TIMEOUT); break; }
+        {
+            const uint32_t addr = smem_u32(&bar_mail);
+            mail_ok = false;
+            for (unsigned spins = 0; spins < 4 * a.spin_limit && !mail_ok; ++spins) {
+                uint32_t ok;
+                asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                             : "=r"(ok) : "r"(addr) : "memory");
+                mail_ok = ok;
             }
         }
-        __syncthreads();
         tc_stamp(a, 5);
-        // This CTA finishes 128/splits rows of the tile: thread = (row j of the slice, column group mg).
-        const int rpc = TC_TILE_N / a.splits;       // rows per CTA
-        const int j_row = tid % rpc, mg = tid / rpc;  // mg in [0, splits)
-        int row;                                      // row inside the tile
-        if constexpr (Epi::PAIRED) {
-            const int half = rpc / 2;                 // w1 rows, then the matching w3 rows (same warp)
-            row = j_row < half ? split * half + j_row : 64 + split * half + (j_row - half);
-        } else {
-            row = split * rpc + j_row;
+        // thread = (row j of the slice, group of eight activation rows); the functors shuffle, and rpc is 32 or 64: warps stay whole
+        for (int e = tid; e < rpc * groups; e += TC_THREADS) {
+            const int j = e % rpc, g = e / rpc;
+            float v[8];
+            const float* box = mail + (size_t)g * 8 * rpc + j;
+            if (S == 2) tc_mail_sum<2>(box, a.MT * rpc, rpc, v);
+            else tc_mail_sum<4>(box, a.MT * rpc, rpc, v);
+            tc_apply(ep, tile, rank * rpc + j, g * 8, Mb, v, es);
         }
-        const float* all = a.partial + (size_t)tile_id * a.splits * a.Mpad * TC_TILE_N + row;
-        const size_t split_stride = (size_t)a.Mpad * TC_TILE_N;
-        const int n_mchunks = a.Mpad / 8;
-        for (int chunk0 = 0; chunk0 < n_mchunks; chunk0 += a.splits) {  // uniform trip count: the
-            const bool active = chunk0 + mg < n_mchunks;                // epilogues shuffle within a warp
-            const int m0 = (active ? chunk0 + mg : n_mchunks - 1) * 8;
-            const int Meff = active ? Mb : 0;
-            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            for (int s0 = 0; s0 < a.splits; s0 += 8) {  // up to 64 loads in flight, summed in split order
-                float p[8][8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        p[u][j] = (s0 + u < a.splits)
-                                      ? __ldcg(all + (size_t)(s0 + u) * split_stride + (size_t)(m0 + j) * TC_TILE_N)
-                                      : 0.f;
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] += p[u][j];
-            }
-            if constexpr (Epi::PAIRED) {
-                const int half = rpc / 2;
-                float g[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) g[j] = __shfl_xor_sync(0xffffffffu, v[j], half);
-                if (j_row < half) ep.apply_pair(tile * 64 + row, m0, Meff, v, g);
-            } else {
-                ep.apply(tile * TC_TILE_N + row, m0, Meff, v, xchg, es);
-            }
-        }
-        __syncthreads();
-        if (tid == 0) {  // the last CTA to leave re-arms both counters for the next launch
-            const int old = atomicAdd(a.counters + all_tiles + tile_id, 1);
-            if (old == a.splits - 1) {
-                a.counters[tile_id] = 0;
-                a.counters[all_tiles + tile_id] = 0;
-            }
-        }
+    }
+    if (!done_ok || !mail_ok || s_bad) {
+        // gave up somewhere: what may still be on its way to this CTA's shared memory lands before the CTA retires
+        if (lane == 0) atomicOr(a.flag, FLAG_TC_TIMEOUT);
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
     }
     tc_stamp(a, 6);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) {
+    if (warp == 2) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
     }
 }

@@ -24,14 +24,13 @@ struct WsLayout {
     size_t rq_x2, rq_x, rq_q, rq_act, rq_k, rq_v, rq_logits, code_cur;
     size_t frame_ctr, rep_counts, rep_hist, rep_head, rep_filled;
     size_t trace;
-    size_t xn, rq_xn, rq_attn, tc_partial, tc_counters;
+    size_t xn, rq_xn, rq_attn;
     size_t dg_layers, dg_head;   // slot stream of the depth weights for k_depth_tc (depth_tc.cuh), 0 if none
     size_t fx_a, fx_b, fparts_a, fparts_b, rq_fx_a, rq_fx_b, rq_fparts_a, rq_fparts_b;
     size_t att_tiles, att_ntiles;
     size_t total;
 };
 
-constexpr int TC_PARTIAL_TILES = 224;  // most (tile, split) pairs of one GEMM launch
 constexpr int FB_MLP_TH_BACKBONE = 512, FB_MLP_U_BACKBONE = 32;  // threads, hidden units per CTA of the MLP block
 constexpr int FB_MLP_TH_DEPTH = 256, FB_MLP_U_DEPTH = 16;
 constexpr int FUSED_MAX_PARTS = 16;     // most partial rows a fused block leaves (clusters of its grid)
@@ -66,6 +65,7 @@ struct VuibEngine {
     bf16* tap_rq;
     long long launches;
     int num_sms;        // 0 until a launch first asks the device
+    bool withhold;        // the next split GEMM waits for one push more than it gets (vuib_debug_withhold_arrival)
     unsigned spin_limit;  // bound of the waits inside kernels, in polls (vuib_set_wait_limit)
     int fused_backbone;   // 0 = not asked yet, 1 = the two-kernel layers can run here, -1 = they cannot
     int fused_depth;
@@ -160,8 +160,6 @@ static void make_layout(VuibEngine* e) {
     L.xn = take(R * (size_t)(c.ffn > c.d_model ? c.ffn : c.d_model) * 2);
     L.rq_xn = take(2 * RB * rd * 2);
     L.rq_attn = take(2 * RB * rd * 2);
-    L.tc_partial = take((size_t)(TC_PARTIAL_TILES + 80) * TC_TILE_N * (R < 256 ? ((R + 15) / 16) * 16 : 256) * 4);
-    L.tc_counters = take(2 * 256 * 4);
     L.dg_layers = L.dg_head = 0;
     if (depth_tc_shape(c)) {
         const int n_ub = (c.rq_ffn / DT_CL + 63) / 64;
@@ -484,14 +482,14 @@ static void build_tc_maps(VuibEngine* e) {
     const int d = c.d_model, qkv = (c.n_heads + 2 * c.n_kv_heads) * HD, rd = c.rq_d_model;
     for (int i = 0; i < c.n_layers && ok; ++i) {
         ok = ok && make_map(&t->wqkv[i], e->w.wqkv[i], qkv, d, 64) && make_map(&t->out_proj[i], e->w.out_proj[i], d, d, 64) &&
-             make_map(&t->w1[i], e->w.w1[i], c.ffn, d, 64) && make_map(&t->w3[i], e->w.w3[i], c.ffn, d, 64) &&
+             make_map(&t->w1[i], e->w.w1[i], c.ffn, d, 16) && make_map(&t->w3[i], e->w.w3[i], c.ffn, d, 16) &&
              make_map(&t->w2[i], e->w.w2[i], d, c.ffn, 64);
     }
     for (int i = 0; i < c.rq_n_layers && ok; ++i) {
         ok = ok && make_map(&t->rq_wqkv[i], e->w.rq_wqkv[i], 3 * rd, rd, 64) &&
              make_map(&t->rq_out[i], e->w.rq_out_proj[i], rd, rd, 64) &&
-             make_map(&t->rq_w1[i], e->w.rq_w1[i], c.rq_ffn, rd, 64) &&
-             make_map(&t->rq_w3[i], e->w.rq_w3[i], c.rq_ffn, rd, 64) &&
+             make_map(&t->rq_w1[i], e->w.rq_w1[i], c.rq_ffn, rd, 16) &&
+             make_map(&t->rq_w3[i], e->w.rq_w3[i], c.rq_ffn, rd, 16) &&
              make_map(&t->rq_w2[i], e->w.rq_w2[i], rd, c.rq_ffn, 64);
     }
     ok = ok && make_map(&t->codec_head, e->w.codec_head, c.codebook_size, d, 64) &&
@@ -550,34 +548,31 @@ static bool tc_ok(VuibEngine* e, int M) {
     return M > 4 && e->tc && !env_off("VUIB_NO_TC");
 }
 
-// D = W X^T over all M rows in blocks of <= 256, epilogue ep (see tc_gemm.cuh).
+// D = W X^T over all M rows, epilogue ep (see tc_gemm.cuh).
 //  units: weight rows (N, multiple of 128) or, for the paired SwiGLU form, hidden units (multiple of 64).
 template <class Epi>
 static int32_t tc_gemm(VuibEngine* e, const CUtensorMap& a0, const CUtensorMap& a1, const bf16* X, int M, int K,
                        int units, int row_off, const Epi& ep, cudaStream_t s) {
     const WsLayout& L = e->lay;
-    const int tiles = Epi::PAIRED ? units / 64 : units / TC_TILE_N;
-    const int chunks_total = K / TC_KCHUNK;
-    // Split K over enough CTAs to occupy the SMs (one MMA of this shape takes ~96 ns whatever the
-    // batch, so the tensor pipe of ONE SM consumes weights at only ~42 GB/s).  The CTAs of a tile
-    // meet on a counter, so the grid must be resident at once: at most two CTAs per SM.
+    const int tiles = Epi::PAIRED ? units / 64 : units / TC_TILE_N, chunks = K / TC_KCHUNK;
     if (e->num_sms == 0) {
         int dev = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, dev));
     }
-    // Row blocks: up to 256 activation rows per CTA; a prefill of more rows is ONE launch whose grid's z
-    // dimension walks the blocks (every weight tile is then read by its row blocks back to back and stays in
-    // L2), not one launch per block.
-    const int Mpad = M <= 256 ? (M + 15) / 16 * 16 : 256;
-    const int m_blocks = (M + Mpad - 1) / Mpad;
-    int splits = 1;
-    for (int d = 2; d <= 16; d *= 2) {
-        if (d > chunks_total || tiles * m_blocks * d > e->num_sms + e->num_sms / 2) break;
-        if (Epi::PAIRED && d == 2) continue;
-        splits = d;
-    }
-    const int max_smem = 202 * 1024;
+    // Rows of a tile: all of up to 64; beyond, 64 while that leaves at most one tile per SM, else 128 (an MMA of 128 x 64 x 16 takes
+    // 48 cycles, of 128 x 128 x 16 64).
+    int MT = M <= 16 ? 16 : M <= 32 ? 32 : 64;
+    if (MT == 64 && tiles * ((M + 63) / 64) > e->num_sms) MT = 128;
+    const int m_blocks = (M + MT - 1) / MT;
+    // K is cut into `parts` equal parts that are added as a balanced tree, whoever sums them: a row's bits do not depend on how many
+    // rows share the call (the accumulators of 128-row tiles fill tensor memory's 512 columns).  A cluster of two or four CTAs
+    // shares a tile's parts while all find an SM.
+    int parts = Epi::PAIRED ? 2 : 4, splits = 1;
+    while (parts > 1 && chunks < 2 * parts) parts /= 2;
+    for (int d = 2; d <= parts; d *= 2)
+        if (tiles * m_blocks * d <= e->num_sms) splits = d;
+    const int max_smem = 200 * 1024;
     {   // a function attribute belongs to one device's copy of the kernel: set it once per device
         static std::mutex mu;
         static bool attr_set[64];
@@ -590,31 +585,50 @@ static int32_t tc_gemm(VuibEngine* e, const CUtensorMap& a0, const CUtensorMap& 
         }
     }
     CUtensorMap mx;
-    if (!make_map(&mx, X, M, K, Mpad)) return fail(e, VUIB_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    if (!make_map(&mx, X, M, K, MT)) return fail(e, VUIB_ERR_CUDA, "cuTensorMapEncodeTiled failed");
     TcArgs ta;
-    ta.N = units;
     ta.row_off = row_off;
     ta.M = M;
-    ta.Mpad = Mpad;
-    ta.chunks = chunks_total;
+    ta.MT = MT;
+    ta.chunks = chunks;
     ta.splits = splits;
-    ta.tiles = tiles;
-    ta.partial = wsp<float>(e, L.tc_partial);
-    ta.counters = wsp<int32_t>(e, L.tc_counters);
+    ta.segs = parts / splits;
     ta.flag = wsp<int32_t>(e, L.flag);
     ta.dbg = env_off("VUIB_TRACE") ? wsp<unsigned long long>(e, L.trace) : nullptr;
     ta.spin_limit = e->spin_limit;
-    const int min_chunks = chunks_total / splits;  // the shortest split
-    const size_t stage_bytes = TC_TILE_N * TC_KCHUNK * 2 + ((Mpad * TC_KCHUNK * 2 + 1023) & ~1023);
-    const size_t epi_bytes = Epi::STAGED ? (size_t)Mpad * TC_EPI_BYTES_PER_M : 0;
-    // two CTAs per SM when split (all CTAs of the grid must be resident), the whole SM otherwise
-    const size_t budget = (splits > 1 ? 100 : 200) * 1024;
-    int stages = epi_bytes + stage_bytes <= budget ? (int)((budget - epi_bytes) / stage_bytes) : 1;
+    ta.withhold = splits > 1 && e->withhold ? 1 : 0;
+    if (ta.withhold) e->withhold = false;
+    const int min_chunks = chunks / splits;  // the shortest split
+    const size_t stage_bytes = TC_TILE_N * TC_KCHUNK * 2 + (size_t)MT * TC_KCHUNK * 2;
+    const size_t tail = (splits > 1 ? (size_t)TC_TILE_N * MT * 4 : 0) + (Epi::STAGED ? (size_t)MT * TC_EPI_BYTES_PER_M : 0) + 1024;
+    // room for the next kernel's CTA beside this one where that still leaves three stages
+    int stages = (int)((112 * 1024 - tail) / stage_bytes);
+    if (tail + 3 * stage_bytes > 112 * 1024) stages = (int)((max_smem - tail) / stage_bytes);
     if (stages > TC_MAX_STAGES) stages = TC_MAX_STAGES;
     if (stages > min_chunks) stages = min_chunks;
     ta.stages = stages;
-    const size_t smem = (size_t)stages * stage_bytes + epi_bytes + 1024;
-    CK(launch(k_gemm_tc<Epi>, dim3(splits, tiles, m_blocks), TC_THREADS, smem, s, a0, a1, mx, ta, ep));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(splits, tiles, m_blocks);
+    cfg.blockDim = dim3(TC_THREADS);
+    cfg.dynamicSmemBytes = stages * stage_bytes + tail;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (splits > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = splits;
+        attr[na].val.clusterDim.y = attr[na].val.clusterDim.z = 1;
+        ++na;
+    }
+    if (pdl_enabled()) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na].val.programmaticStreamSerializationAllowed = 1;
+        ++na;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = na;
+    prefer_max_smem(reinterpret_cast<const void*>(k_gemm_tc<Epi>));
+    CK(cudaLaunchKernelEx(&cfg, k_gemm_tc<Epi>, a0, a1, mx, ta, ep));
     e->launches++;
     return VUIB_OK;
 }
@@ -1598,7 +1612,6 @@ extern "C" int32_t vuib_reset_state(VuibEngine* e, void* stream) {
     CK(cudaMemsetAsync(e->ws + L.flag, 0, 256, s));
     CK(cudaMemsetAsync(e->ws + L.counters, 0, (size_t)e->R * c.n_kv_heads * 4, s));
     CK(cudaMemsetAsync(e->ws + L.frame_ctr, 0, (size_t)c.n_slots * 4, s));
-    CK(cudaMemsetAsync(e->ws + L.tc_counters, 0, 2 * 256 * 4, s));
     return vuib_rep_reset(e, -1, stream);
 }
 
@@ -1619,12 +1632,8 @@ extern "C" int32_t vuib_set_wait_limit(VuibEngine* e, uint32_t polls) {
 
 extern "C" int32_t vuib_debug_withhold_arrival(VuibEngine* e, void* stream) {
     if (!e) return VUIB_ERR_NULL;
-    if (!e->have_ws) return fail(e, VUIB_ERR_UNBOUND, "bind the workspace first");
-    int32_t minus_one[256];
-    for (int i = 0; i < 256; ++i) minus_one[i] = -1;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    CK(cudaMemcpyAsync(e->ws + e->lay.tc_counters, minus_one, sizeof(minus_one), cudaMemcpyHostToDevice, s));
-    CK(cudaStreamSynchronize(s));  // the source is a stack array
+    (void)stream;
+    e->withhold = true;
     return VUIB_OK;
 }
 
@@ -1655,7 +1664,6 @@ extern "C" int32_t vuib_check_device_flag(VuibEngine* e, void* stream) {
     if (flag) {
         CK(cudaMemsetAsync(e->ws + e->lay.flag, 0, 4, s));
         // a wait that gave up may have left arrival counters half way: re-arm them with the flag
-        CK(cudaMemsetAsync(e->ws + e->lay.tc_counters, 0, 2 * 256 * 4, s));
         CK(cudaMemsetAsync(e->ws + e->lay.counters, 0, (size_t)e->R * e->cfg.n_kv_heads * 4, s));
         return fail(e, VUIB_ERR_DEVICE_FLAG, "device flag 0x%x (1 = slot outside the cache, 2 = position outside [0, max_seq), 4 = code outside the codebook, 16 = a bounded wait inside a kernel ran out)", flag);
     }
