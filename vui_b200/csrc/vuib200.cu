@@ -543,6 +543,9 @@ static int32_t build_dg_stream(VuibEngine* e) {
     return VUIB_OK;
 }
 
+// A prefill takes the tensor cores for any number of rows: its rows then come out the same bit for bit however a prompt is cut.
+static bool prefill_tc_ok(VuibEngine* e) { return e->tc && !env_off("VUIB_NO_TC"); }
+
 static bool tc_ok(VuibEngine* e, int M) {
     // measured: 8 rows take 3.7 ms/frame on the register-tile GEMV, 16 rows 3.4 ms on the tensor cores
     return M > 4 && e->tc && !env_off("VUIB_NO_TC");
@@ -989,8 +992,9 @@ static int32_t run_layers(VuibEngine* e, int M, cudaStream_t s, Residual* out, b
     out->x = wsp<bf16>(e, e->lay.x);
     out->parts = nullptr;
     out->n_parts = 0;
+    if (prefill && prefill_tc_ok(e)) return run_layers_tc(e, M, s, true);
     if (M == 1 && fused_backbone_ok(e)) return run_layers_fused(e, s, out, after, after_bytes);
-    if (tc_ok(e, M)) return run_layers_tc(e, M, s, prefill);
+    if (tc_ok(e, M)) return run_layers_tc(e, M, s, false);
     const VuibConfig& c = e->cfg;
     const WsLayout& L = e->lay;
     bf16* x = wsp<bf16>(e, L.x);
@@ -1060,8 +1064,8 @@ extern "C" int32_t vuib_prefill(VuibEngine* e, int32_t n_rows, const int32_t* ro
     e->launches++;
     CK(cudaMemcpyAsync(e->ws + L.x, emb_dev, (size_t)n_rows * d * 2, cudaMemcpyDeviceToDevice, s));
     Residual res;
-    if (tc_ok(e, n_rows)) {
-        CK(launch(k_prefill_tiles, 1, 256, (size_t)n_rows * 4, s, static_cast<const int32_t*>(wsp<int32_t>(e, L.row_slot)),
+    if (prefill_tc_ok(e)) {
+        CK(launch(k_prefill_tiles, 1, 256, 0, s, static_cast<const int32_t*>(wsp<int32_t>(e, L.row_slot)),
                   static_cast<const int32_t*>(wsp<int32_t>(e, L.row_pos)), n_rows, wsp<int32_t>(e, L.att_tiles),
                   wsp<int32_t>(e, L.att_ntiles)));
         e->launches++;

@@ -525,25 +525,28 @@ class Engine:
         def flush():
             if not pend:
                 return
-            emb = torch.cat([e for _, _, e in pend], dim=0).to(self.dtype).contiguous()
-            slot = torch.cat([torch.full((e.shape[0],), s_, dtype=torch.int32) for s_, _, e in pend])
-            pos = torch.cat([torch.arange(o, o + e.shape[0], dtype=torch.int32) for _, o, e in pend])
-            slot, pos = slot.to(self.device), pos.to(self.device)
+            emb = pend[0][2] if len(pend) == 1 else torch.cat([e for _, _, e in pend], dim=0)
+            emb = emb.to(self.dtype).contiguous()
+            dev, i32 = self.device, torch.int32
+            slot = [torch.full((e.shape[0],), s_, dtype=i32, device=dev) for s_, _, e in pend]
+            pos = [torch.arange(o, o + e.shape[0], dtype=i32, device=dev) for _, o, e in pend]
+            slot, pos = (t[0] if len(t) == 1 else torch.cat(t) for t in (slot, pos))
             out = torch.empty_like(emb)
             P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
             self._ck(self._lib.vuib_prefill(self._handle, emb.shape[0], P(slot), P(pos), P(emb), P(out),
                                             self._stream))
             i = 0
-            for s_, _, e in pend:
+            for s_, o, e in pend:
                 outs.append(out[i:i + e.shape[0]])
-                self.seq_lens[s_] += e.shape[0]
+                ends[s_] = o + e.shape[0]
                 i += e.shape[0]
             pend.clear()
 
-        offsets = {}
+        offsets: dict[int, int] = {}
+        ends: dict[int, int] = {}
         for row, emb in items:
             emb = emb.reshape(-1, self.D)
-            off = offsets.get(row.idx, row.offset)
+            off = offsets[row.idx] if row.idx in offsets else row.offset
             if off + emb.shape[0] > self.max_seq:
                 raise RuntimeError(f"prefill of {emb.shape[0]} positions overflows max_seq={self.max_seq}")
             # a segment longer than one call is cut; a slot may appear several times in a call (its rows
@@ -559,6 +562,12 @@ class Engine:
                 start += n
             offsets[row.idx] = off + emb.shape[0]
         flush()
+        if len(ends) == 1:
+            for s_, n in ends.items():
+                self.seq_lens[s_] = n
+        elif ends:
+            at = torch.tensor([list(ends), list(ends.values())], dtype=torch.int32).to(self.device)
+            self.seq_lens[at[0].long()] = at[1]
         # stitch cut segments back together per input item
         res, k = [], 0
         for row, emb in items:
@@ -687,17 +696,25 @@ class Engine:
             return None
         return self.model.embed_speaker(spk_emb).to(self.dtype)
 
-    def _prefill_speaker_segments(self, row, segments, spk_token, *, final=False) -> None:
-        last = len(segments) - 1
+    def _speaker_segments_emb(self, segments, spk_token, *, final=False) -> list[Tensor]:
+        """[spk] text_i [SC] codes_i of every segment, as embeddings (1, n, d)."""
+        parts, last = [], len(segments) - 1
         for i, seg in enumerate(segments):
             if spk_token is not None:
-                self._prefill_emb(row, spk_token)
+                parts.append(spk_token)
             if seg.text:
-                self._prefill_emb(row, self._text_emb(seg.text, with_cond_bias=False))
+                parts.append(self._text_emb(seg.text, with_cond_bias=False))
             if final and i == last and self._sc_emb is not None:
-                self._prefill_emb(row, self._sc_emb)
+                parts.append(self._sc_emb)
             if seg.codes is not None:
-                self._prefill_emb(row, self._audio_emb(seg.codes))
+                parts.append(self._audio_emb(seg.codes))
+        return parts
+
+    def _prefill_parts(self, row, parts: list[Tensor]) -> Tensor | None:
+        """One prefill of several embeddings (1, n_i, d): the weights are read once for all of them."""
+        if not parts:
+            return None
+        return self._prefill_emb(row, parts[0] if len(parts) == 1 else torch.cat([p.to(self.dtype) for p in parts], dim=1))
 
     def _prefill_row(self, row, segments, spk_emb, segments_2=None, spk_emb_2=None) -> int:
         row._spk_token = self._embed_speaker(spk_emb)
@@ -706,9 +723,10 @@ class Engine:
         all_codes = [s.codes for s in list(segments) + list(segments_2 or []) if s.codes is not None]
         if all_codes and row._codec_ctx is not None:
             row._codec_ctx.set_prompt(torch.cat([c.to(self.device) for c in all_codes], dim=0).T.unsqueeze(0))
-        self._prefill_speaker_segments(row, segments, row._spk_token, final=True)
+        parts = self._speaker_segments_emb(segments, row._spk_token, final=True)
         if segments_2 is not None:
-            self._prefill_speaker_segments(row, segments_2, row._spk_token_2, final=True)
+            parts += self._speaker_segments_emb(segments_2, row._spk_token_2, final=True)
+        self._prefill_parts(row, parts)
         row._prompt_offset = row.offset
         segs = list(segments) + list(segments_2 or [])
         words = sum(len(s.text.split()) for s in segs if s.text)
@@ -718,12 +736,15 @@ class Engine:
         return row._prompt_offset
 
     def _add_user(self, row, text, codes, *, final=True) -> int:
+        parts = []
         if text:
-            self._prefill_emb(row, self._text_emb(text, with_cond_bias=False, noisy=True))
+            parts.append(self._text_emb(text, with_cond_bias=False, noisy=True))
         if final and self._sc_emb is not None:
-            self._prefill_emb(row, self._sc_emb)
+            parts.append(self._sc_emb)
         if codes is not None:
-            self._prefill_emb(row, self._audio_emb(codes))
+            parts.append(self._audio_emb(codes))
+        self._prefill_parts(row, parts)
+        if codes is not None:
             if row._codec_ctx is not None:
                 row._codec_ctx.add(codes.T.unsqueeze(0).to(self.device))
         return row.offset
@@ -735,12 +756,11 @@ class Engine:
 
     def _add_agent_text(self, row, text, *, final=False) -> Tensor:
         spk = self._active_spk_token(row)
-        if spk is not None:
-            self._prefill_emb(row, spk)
-        out = self._prefill_emb(row, self._text_emb(text, with_cond_bias=True))
+        parts = [spk] if spk is not None else []
+        parts.append(self._text_emb(text, with_cond_bias=True))
         if final and self._sc_emb is not None:
-            out = self._prefill_emb(row, self._sc_emb)
-        return out[0, -1]
+            parts.append(self._sc_emb)
+        return self._prefill_parts(row, parts)[0, -1]
 
     # ------------------------------------------------------------ first frame
     def _first_frames(self, rows: list[Row], hidden: Tensor) -> Tensor:
