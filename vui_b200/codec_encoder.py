@@ -20,6 +20,7 @@ from . import _lib
 from .codec import DOWNSAMPLE_RATE, N_CODEBOOKS, SAMPLE_RATE
 
 RATIOS, BASE_DIM, D_MODEL, N_LAYERS, N_HEADS, MLP = (4, 5, 6, 8), 64, 512, 8, 8, 2048
+GRAPH_FRAMES = 16   # step of the lengths a streaming encoder captures: a frame more or less is 7 us of some 600
 
 
 def encoder_param_shapes() -> "OrderedDict[str, tuple]":
@@ -213,8 +214,7 @@ class StreamingCodecEncoder:
         self._audio_buf = torch.zeros(1, 1, self.max_samples, device=self.device, dtype=self.dtype)
         self._pos = 0
         self._emitted = 0
-        self._graph = None
-        self._codes_out = None
+        self._graphs: dict[int, tuple[torch.cuda.CUDAGraph, Tensor]] = {}   # by frames encoded
 
     def _slide(self) -> None:
         self._audio_buf.zero_()
@@ -222,19 +222,24 @@ class StreamingCodecEncoder:
         self._emitted = 0
 
     def setup_graph(self) -> None:
-        """Capture the whole-buffer encode once; feed()/flush() then replay it (qwen_codec.py:725-736)."""
+        """Capture the encode once; feed()/flush() then replay it (qwen_codec.py:725-736).  Everything in the encoder is
+        causal, so the frames known so far need no more than the samples before their end: one graph for every
+        GRAPH_FRAMES frames (the last for the whole buffer), the shortest that holds them is replayed."""
         with torch.inference_mode():
             self.encoder(self._audio_buf)
             torch.cuda.synchronize()
-            self._graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(self._graph):
-                self._codes_out = self.encoder(self._audio_buf)
+            for n in [*range(GRAPH_FRAMES, self.max_frames, GRAPH_FRAMES), self.max_frames]:
+                g = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(g):
+                    codes = self.encoder(self._audio_buf[:, :, : n * DOWNSAMPLE_RATE])
+                self._graphs[n] = g, codes
 
-    def _encode(self) -> Tensor:
-        if self._graph is not None:
-            self._graph.replay()
-            return self._codes_out
-        return self.encoder(self._audio_buf)
+    def _encode(self, n_frames: int) -> Tensor:
+        if self._graphs:
+            g, codes = self._graphs[min(self.max_frames, -(-n_frames // GRAPH_FRAMES) * GRAPH_FRAMES)]
+            g.replay()
+            return codes
+        return self.encoder(self._audio_buf[:, :, : n_frames * DOWNSAMPLE_RATE])
 
     @torch.inference_mode()
     def feed(self, audio: Tensor):
@@ -253,7 +258,7 @@ class StreamingCodecEncoder:
         n_frames = self._pos // DOWNSAMPLE_RATE
         if n_frames <= self._emitted or (self._pos - self._emitted * DOWNSAMPLE_RATE) < self.min_chunk_samples:
             return None
-        new = self._encode()[0, :, self._emitted: n_frames].T.long().cpu()
+        new = self._encode(n_frames)[0, :, self._emitted: n_frames].T.long().cpu()
         self._emitted = n_frames
         return new
 
@@ -265,7 +270,7 @@ class StreamingCodecEncoder:
         n_frames = self._pos // DOWNSAMPLE_RATE
         if n_frames <= self._emitted:
             return None
-        new = self._encode()[0, :, self._emitted: n_frames].T.long().cpu()
+        new = self._encode(n_frames)[0, :, self._emitted: n_frames].T.long().cpu()
         self._emitted = n_frames
         return new
 

@@ -147,7 +147,7 @@ class TTSEngine:
         total = self.stream_enc._emitted
         if total == 0:
             return None
-        return self.stream_enc._encode()[0, :, :total].T.long().cpu()
+        return self.stream_enc._encode(total)[0, :, :total].T.long().cpu()
 
     # ----------------------------------------------------------- KV position, conditioning
     def reset(self) -> None:
