@@ -19,7 +19,7 @@ _OBJ = os.path.join(_CSRC, "_obj")
 _API_H = os.path.join(_ROOT, "include", "vuib200.h")
 # translation unit -> the headers it includes (a unit is recompiled when one of them changes)
 UNITS = {
-    "vuib200.cu": ["decode_kernels.cuh", "tc_gemm.cuh", "fused_blocks.cuh", "depth_tc.cuh", "prefill_attn.cuh"],
+    "vuib200.cu": ["decode_kernels.cuh", "tc_gemm.cuh", "fused_blocks.cuh", "fused_rows.cuh", "depth_tc.cuh", "prefill_attn.cuh"],
     "codec.cu": ["codec_kernels.cuh", "codec_batch.cuh", "split_ops.cuh", "split_gemm.cuh"],
     "codec_enc.cu": ["codec_enc_kernels.cuh", "split_ops.cuh", "split_gemm.cuh"],
 }

@@ -196,10 +196,11 @@ struct StageNorm {
     const bf16* w;   // (K)
     float eps;
     int row_mul, row_add;
-    // single-row form only: the row is x + bf16(sum_p parts[p]), the partial rows (n_parts, K) fp32 that
-    // the fused two-kernel layers leave behind (fused_blocks.cuh), added in row order
+    // row r is x + bf16(sum_p parts[p][r]), the partial rows (n_parts, n_rows, K) fp32 that the fused
+    // two-kernel layers leave behind (fused_blocks.cuh, fused_rows.cuh), added in the order of the parts
     const float* parts = nullptr;
     int n_parts = 0;
+    int n_rows = 1;
     // The norm weights are constants: a kernel fetches them before it waits for its predecessor,
     // so that their L2 round trip is not paid between the reduction and the scaling.
     template <int K>
@@ -217,78 +218,87 @@ struct StageNorm {
     __device__ __forceinline__ void stage(bf16* Xs, int r0, int nr) const {
         stage<K>(Xs, r0, nr, preload<K>());
     }
-    // Single row given as x + bf16(sum of partial rows): the whole CTA adds the rows (every thread a few
-    // consecutive elements, all rows requested at once, added in row order) and normalises together.
+    // Rows given as x + bf16(sum of partial rows): the whole CTA adds them up (every thread a few consecutive
+    // elements, all parts requested at once, added in order) and normalises together, up to four rows per barrier.
     template <int K>
-    __device__ __forceinline__ void stage_parts(bf16* Xs) const {
+    __device__ __forceinline__ void stage_parts(bf16* Xs, int r0, int nr) const {
         constexpr int EPT = K / GEMV_THREADS;  // 2 (K = 512) or 4 (K = 1024)
         static_assert(EPT == 2 || EPT == 4, "partial rows come from the fused layers: K is 512 or 1024");
-        constexpr int MAXP = 16;
-        __shared__ float red[GEMV_WARPS];
+        constexpr int MAXP = 16, MAXR = 4;
+        __shared__ float red[MAXR][GEMV_WARPS];
         const int k0 = threadIdx.x * EPT;
-        const bf16* xr = x + (size_t)row_add * K;
-        float xv[EPT], wv[EPT], sp[EPT];
-#pragma unroll
-        for (int j = 0; j < EPT; ++j) sp[j] = 0.f;
-        if constexpr (EPT == 4) {
-            const uint2 xraw = __ldcg(reinterpret_cast<const uint2*>(xr + k0));
-            const uint2 wraw = __ldg(reinterpret_cast<const uint2*>(w + k0));
-            float4 p[MAXP];
-#pragma unroll
-            for (int u = 0; u < MAXP; ++u)
-                p[u] = u < n_parts ? __ldcg(reinterpret_cast<const float4*>(parts + (size_t)u * K + k0))
-                                   : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int u = 0; u < MAXP; ++u) { sp[0] += p[u].x; sp[1] += p[u].y; sp[2] += p[u].z; sp[3] += p[u].w; }
-            const __nv_bfloat162* xh = reinterpret_cast<const __nv_bfloat162*>(&xraw);
+        float xv[MAXR][EPT], wv[EPT];
+        {
+            uint2 wraw;
+            if constexpr (EPT == 4) wraw = __ldg(reinterpret_cast<const uint2*>(w + k0));
+            else wraw = make_uint2(__ldg(reinterpret_cast<const unsigned*>(w + k0)), 0u);
             const __nv_bfloat162* wh = reinterpret_cast<const __nv_bfloat162*>(&wraw);
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const float2 a = __bfloat1622float2(xh[i]), b = __bfloat1622float2(wh[i]);
-                xv[2 * i] = a.x; xv[2 * i + 1] = a.y; wv[2 * i] = b.x; wv[2 * i + 1] = b.y;
+            for (int i = 0; i < EPT / 2; ++i) {
+                const float2 b = __bfloat1622float2(wh[i]);
+                wv[2 * i] = b.x; wv[2 * i + 1] = b.y;
             }
-        } else {
-            const unsigned xraw = __ldcg(reinterpret_cast<const unsigned*>(xr + k0));
-            const unsigned wraw = __ldg(reinterpret_cast<const unsigned*>(w + k0));
-            float2 p[MAXP];
-#pragma unroll
-            for (int u = 0; u < MAXP; ++u)
-                p[u] = u < n_parts ? __ldcg(reinterpret_cast<const float2*>(parts + (size_t)u * K + k0)) : make_float2(0.f, 0.f);
-#pragma unroll
-            for (int u = 0; u < MAXP; ++u) { sp[0] += p[u].x; sp[1] += p[u].y; }
-            const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xraw));
-            const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wraw));
-            xv[0] = a.x; xv[1] = a.y; wv[0] = b.x; wv[1] = b.y;
         }
-        float ss = 0.f;
 #pragma unroll
-        for (int j = 0; j < EPT; ++j) {
-            xv[j] = rbf(xv[j] + rbf(sp[j]));
-            ss = fmaf(xv[j], xv[j], ss);
+        for (int rr = 0; rr < MAXR; ++rr) {
+            if (rr >= nr) break;
+            const int r = r0 + rr;
+            const bf16* xr = x + ((size_t)r * row_mul + row_add) * K + k0;
+            const float* pr = parts + (size_t)r * K + k0;
+            const size_t ps = (size_t)n_rows * K;
+            float sp[EPT];
+#pragma unroll
+            for (int j = 0; j < EPT; ++j) sp[j] = 0.f;
+            uint2 xraw;
+            if constexpr (EPT == 4) {
+                xraw = __ldcg(reinterpret_cast<const uint2*>(xr));
+                float4 p[MAXP];
+#pragma unroll
+                for (int u = 0; u < MAXP; ++u)
+                    p[u] = u < n_parts ? __ldcg(reinterpret_cast<const float4*>(pr + u * ps)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int u = 0; u < MAXP; ++u) { sp[0] += p[u].x; sp[1] += p[u].y; sp[2] += p[u].z; sp[3] += p[u].w; }
+            } else {
+                xraw = make_uint2(__ldcg(reinterpret_cast<const unsigned*>(xr)), 0u);
+                float2 p[MAXP];
+#pragma unroll
+                for (int u = 0; u < MAXP; ++u)
+                    p[u] = u < n_parts ? __ldcg(reinterpret_cast<const float2*>(pr + u * ps)) : make_float2(0.f, 0.f);
+#pragma unroll
+                for (int u = 0; u < MAXP; ++u) { sp[0] += p[u].x; sp[1] += p[u].y; }
+            }
+            const __nv_bfloat162* xh = reinterpret_cast<const __nv_bfloat162*>(&xraw);
+#pragma unroll
+            for (int i = 0; i < EPT / 2; ++i) {
+                const float2 a = __bfloat1622float2(xh[i]);
+                xv[rr][2 * i] = rbf(a.x + rbf(sp[2 * i]));
+                xv[rr][2 * i + 1] = rbf(a.y + rbf(sp[2 * i + 1]));
+            }
+            float ss = 0.f;
+#pragma unroll
+            for (int j = 0; j < EPT; ++j) ss = fmaf(xv[rr][j], xv[rr][j], ss);
+            ss = warp_sum(ss);
+            if ((threadIdx.x & 31) == 0) red[rr][threadIdx.x >> 5] = ss;
         }
-        ss = warp_sum(ss);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
         __syncthreads();
-        float tot = 0.f;
 #pragma unroll
-        for (int i = 0; i < GEMV_WARPS; ++i) tot += red[i];
-        const float rinv = rsqrtf(tot / (float)K + eps);
-        if constexpr (EPT == 4) {
-            uint2 o;
-            __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
-            oh[0] = __floats2bfloat162_rn(rbf(xv[0] * rinv) * wv[0], rbf(xv[1] * rinv) * wv[1]);
-            oh[1] = __floats2bfloat162_rn(rbf(xv[2] * rinv) * wv[2], rbf(xv[3] * rinv) * wv[3]);
-            *reinterpret_cast<uint2*>(Xs + k0) = o;
-        } else {
-            *reinterpret_cast<__nv_bfloat162*>(Xs + k0) =
-                __floats2bfloat162_rn(rbf(xv[0] * rinv) * wv[0], rbf(xv[1] * rinv) * wv[1]);
+        for (int rr = 0; rr < MAXR; ++rr) {
+            if (rr >= nr) break;
+            float tot = 0.f;
+#pragma unroll
+            for (int i = 0; i < GEMV_WARPS; ++i) tot += red[rr][i];
+            const float rinv = rsqrtf(tot / (float)K + eps);
+            __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(Xs + (size_t)rr * K + k0);
+#pragma unroll
+            for (int i = 0; i < EPT / 2; ++i)
+                o[i] = __floats2bfloat162_rn(rbf(xv[rr][2 * i] * rinv) * wv[2 * i], rbf(xv[rr][2 * i + 1] * rinv) * wv[2 * i + 1]);
         }
     }
     template <int K>
     __device__ __forceinline__ void stage(bf16* Xs, int r0, int nr, const NormW<K>& nw) const {
         if constexpr (K == 512 || K == 1024) {
-            if (n_parts > 0) {  // uniform over the CTA
-                stage_parts<K>(Xs);
+            if (n_parts > 0) {  // uniform over the CTA; at most four rows
+                stage_parts<K>(Xs, r0, nr);
                 return;
             }
         }
@@ -1067,7 +1077,7 @@ static __global__ void __launch_bounds__(128) k_final_norm(const bf16* __restric
     __shared__ __align__(16) bf16 xsum[1024];
     const bf16* xr = x + (size_t)r * d;
     if (n_parts > 0) {
-        // single row, d <= 1024: x + bf16(sum of the fused layers' partial rows), kept for the second pass
+        // d <= 1024: x + bf16(sum of the fused layers' partial rows, a row for every CTA), kept for the second pass
         for (int k = threadIdx.x * 8; k < d; k += 128 * 8) {
             float f[8], sp[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             unpack8(__ldcg(reinterpret_cast<const uint4*>(xr + k)), f);
@@ -1076,7 +1086,7 @@ static __global__ void __launch_bounds__(128) k_final_norm(const bf16* __restric
 #pragma unroll
                 for (int u = 0; u < 16; ++u) {
                     const bool ok = p0 + u < n_parts;
-                    const float* q = parts + (size_t)(ok ? p0 + u : p0) * d + k;
+                    const float* q = parts + ((size_t)(ok ? p0 + u : p0) * gridDim.x + r) * d + k;
                     pa[u] = ok ? __ldcg(reinterpret_cast<const float4*>(q)) : make_float4(0.f, 0.f, 0.f, 0.f);
                     pb[u] = ok ? __ldcg(reinterpret_cast<const float4*>(q + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
@@ -1090,7 +1100,7 @@ static __global__ void __launch_bounds__(128) k_final_norm(const bf16* __restric
             for (int j = 0; j < 8; ++j) f[j] = rbf(f[j] + rbf(sp[j]));
             const uint4 u = pack8(f);
             *reinterpret_cast<uint4*>(xsum + k) = u;
-            if (xsum_out) *reinterpret_cast<uint4*>(xsum_out + k) = u;
+            if (xsum_out) *reinterpret_cast<uint4*>(xsum_out + (size_t)r * d + k) = u;
         }
         __syncthreads();
         xr = xsum;

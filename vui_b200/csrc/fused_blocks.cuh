@@ -401,6 +401,7 @@ struct AttnBlockArgs {
     unsigned spin_limit;
     PrefetchList next;      // the following kernel's matrices
     unsigned long long* dbg;  // optional: device-clock stamps of CTA 0 (profiling aid)
+    int rows, x_stride;     // several rows (fused_rows.cuh): how many, elements between rows of x_in
 };
 
 template <int K, int G>
@@ -814,6 +815,7 @@ struct MlpBlockArgs {
     unsigned spin_limit;
     PrefetchList next;
     unsigned long long* dbg;
+    int rows;               // several rows (fused_rows.cuh)
 };
 
 // U hidden units per CTA; the grid is F / (U * FB_CL) clusters.

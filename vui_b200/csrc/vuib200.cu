@@ -14,6 +14,7 @@
 #include "decode_kernels.cuh"
 #include "tc_gemm.cuh"
 #include "fused_blocks.cuh"
+#include "fused_rows.cuh"
 #include "depth_tc.cuh"
 #include "prefill_attn.cuh"
 
@@ -167,14 +168,14 @@ static void make_layout(VuibEngine* e) {
         L.dg_head = take((size_t)(c.n_quantizers - 1) * DT_CL * DT_HEAD_SLOTS * DT_SLOT);
     }
     // fused two-kernel layers (single row): x as each block sees it, and the partial rows between blocks
-    L.fx_a = take(d * 2);
-    L.fx_b = take(d * 2);
-    L.fparts_a = take((size_t)FUSED_MAX_PARTS * d * 4);
-    L.fparts_b = take((size_t)FUSED_MAX_PARTS * d * 4);
-    L.rq_fx_a = take(rd * 2);
-    L.rq_fx_b = take(rd * 2);
-    L.rq_fparts_a = take((size_t)FUSED_MAX_PARTS * rd * 4);
-    L.rq_fparts_b = take((size_t)FUSED_MAX_PARTS * rd * 4);
+    L.fx_a = take((size_t)FR_ROWS * d * 2);
+    L.fx_b = take((size_t)FR_ROWS * d * 2);
+    L.fparts_a = take((size_t)FR_ROWS * FUSED_MAX_PARTS * d * 4);
+    L.fparts_b = take((size_t)FR_ROWS * FUSED_MAX_PARTS * d * 4);
+    L.rq_fx_a = take((size_t)FR_ROWS * rd * 2);
+    L.rq_fx_b = take((size_t)FR_ROWS * rd * 2);
+    L.rq_fparts_a = take((size_t)FR_ROWS * FUSED_MAX_PARTS * rd * 4);
+    L.rq_fparts_b = take((size_t)FR_ROWS * FUSED_MAX_PARTS * rd * 4);
     // query tiles of a prefill call (first row, rows) and their count
     L.att_tiles = take(2 * R * 4);
     L.att_ntiles = take(256);
@@ -803,26 +804,41 @@ static bool fused_backbone_ok(VuibEngine* e) {
         ok = ok && cluster_kernel_fits(k_mlp_block<1024, 3072, FB_MLP_U_BACKBONE, FB_MLP_TH_BACKBONE>,
                                        3072 / (FB_MLP_U_BACKBONE * FB_CL), FB_MLP_TH_BACKBONE,
                                        sizeof(MlpBlockSmem<1024, 3072, FB_MLP_U_BACKBONE, FB_MLP_TH_BACKBONE>));
+        ok = ok && cluster_kernel_fits(k_attn_rows<1024, 2, false, FR_ATT_TH>, c.n_kv_heads, FR_ATT_TH, sizeof(AttnRowsSmem<1024, 2, false, FR_ATT_TH>));
+        ok = ok && cluster_kernel_fits(k_mlp_rows<1024, 3072, FB_MLP_U_BACKBONE, FB_MLP_TH_BACKBONE>,
+                                       3072 / (FB_MLP_U_BACKBONE * FB_CL), FB_MLP_TH_BACKBONE,
+                                       sizeof(MlpRowsSmem<1024, 3072, FB_MLP_U_BACKBONE, FB_MLP_TH_BACKBONE>));
         e->fused_backbone = ok ? 1 : -1;
     }
-    return e->fused_backbone == 1 && !env_off("VUIB_NO_FUSED");
+    return e->fused_backbone == 1;
+}
+
+template <int F>
+static bool fused_depth_fits(const VuibConfig& c) {
+    constexpr int NCL = F / (FB_MLP_U_DEPTH * FB_CL);
+    return cluster_kernel_fits(k_attn_block<512, 1, true>, c.rq_n_heads, FB_THREADS, sizeof(AttnBlockSmem<512, 1>)) &&
+           cluster_kernel_fits(k_attn_rows<512, 1, true, FB_THREADS>, c.rq_n_heads, FB_THREADS, sizeof(AttnRowsSmem<512, 1, true, FB_THREADS>)) &&
+           cluster_kernel_fits(k_mlp_block<512, F, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>, NCL, FB_MLP_TH_DEPTH,
+                               sizeof(MlpBlockSmem<512, F, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>)) &&
+           cluster_kernel_fits(k_mlp_rows<512, F, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>, NCL, FB_MLP_TH_DEPTH,
+                               sizeof(MlpRowsSmem<512, F, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>));
 }
 
 static bool fused_depth_ok(VuibEngine* e) {
     if (e->fused_depth == 0) {
         const VuibConfig& c = e->cfg;
         bool ok = e->tc && e->tc->fused_depth;
-        ok = ok && cluster_kernel_fits(k_attn_block<512, 1, true>, c.rq_n_heads, FB_THREADS, sizeof(AttnBlockSmem<512, 1>));
-        if (ok && c.rq_ffn == 1408)
-            ok = cluster_kernel_fits(k_mlp_block<512, 1408, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>, 1408 / (FB_MLP_U_DEPTH * FB_CL),
-                                     FB_MLP_TH_DEPTH, sizeof(MlpBlockSmem<512, 1408, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>));
-        else if (ok)
-            ok = cluster_kernel_fits(k_mlp_block<512, 1536, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>, 1536 / (FB_MLP_U_DEPTH * FB_CL),
-                                     FB_MLP_TH_DEPTH, sizeof(MlpBlockSmem<512, 1536, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>));
+        ok = ok && (c.rq_ffn == 1408 ? fused_depth_fits<1408>(c) : fused_depth_fits<1536>(c));
         e->fused_depth = ok ? 1 : -1;
     }
-    return e->fused_depth == 1 && !env_off("VUIB_NO_FUSED");
+    return e->fused_depth == 1;
 }
+
+// Up to four streams take the fused two-kernel layers, one the single-row kernels (switched off for tests: it then runs what
+// several run, bit for bit).  Five streams and more go to the tensor-core GEMMs and k_depth_tc: the fused kernels' columns
+// and partial rows are laid out for four.
+static bool one_row(int M) { return M == 1 && !env_off("VUIB_NO_FUSED"); }
+static bool rows_fit(int M) { return one_row(M) || (M <= FR_ROWS && !env_off("VUIB_NO_TC")); }
 
 static PrefetchList prefetch_of(const void* a, size_t na, const void* b = nullptr, size_t nb = 0, const void* c = nullptr,
                                 size_t nc = 0) {
@@ -834,9 +850,9 @@ static PrefetchList prefetch_of(const void* a, size_t na, const void* b = nullpt
     return p;
 }
 
-// The backbone's blocks for ONE row whose (slot, position) is row 0 of the workspace table and whose
+// The backbone's blocks for up to four rows whose (slot, position) are in the workspace table and whose
 // input is L.x.  `after` names what follows the last block (its matrix is pulled into L2).
-static int32_t run_layers_fused(VuibEngine* e, cudaStream_t s, Residual* out, const void* after, size_t after_bytes) {
+static int32_t run_layers_fused(VuibEngine* e, int M, cudaStream_t s, Residual* out, const void* after, size_t after_bytes) {
     const VuibConfig& c = e->cfg;
     const WsLayout& L = e->lay;
     const int d = c.d_model, qc = c.n_heads * HD, kvc = c.n_kv_heads * HD;
@@ -874,7 +890,12 @@ static int32_t run_layers_fused(VuibEngine* e, cudaStream_t s, Residual* out, co
         // and 19 MB of hints during this block delayed its own loads (0.799 -> 0.788 ms per frame without them)
         aa.next = prefetch_of(nullptr, 0);
         if (env_off("VUIB_TRACE") && (li == 5 || li == 6)) aa.dbg = wsp<unsigned long long>(e, L.trace) + (li - 5) * 32;
-        CK(launch_cluster(k_attn_block<1024, 2, false>, c.n_kv_heads, FB_THREADS, sizeof(AttnBlockSmem<1024, 2>), s, e->tc->f_out[li], aa));
+        aa.rows = M;
+        aa.x_stride = d;
+        if (one_row(M))
+            CK(launch_cluster(k_attn_block<1024, 2, false>, c.n_kv_heads, FB_THREADS, sizeof(AttnBlockSmem<1024, 2>), s, e->tc->f_out[li], aa));
+        else
+            CK(launch_cluster(k_attn_rows<1024, 2, false, FR_ATT_TH>, c.n_kv_heads, FR_ATT_TH, sizeof(AttnRowsSmem<1024, 2, false, FR_ATT_TH>), s, e->tc->f_out[li], aa));
         e->launches++;
 
         MlpBlockArgs ma;
@@ -903,8 +924,13 @@ static int32_t run_layers_fused(VuibEngine* e, cudaStream_t s, Residual* out, co
         ma.next = li + 1 < c.n_layers ? prefetch_of(e->w.wqkv[li + 1], qkv_bytes, e->w.out_proj[li + 1], wo_bytes)
                                       : prefetch_of(after, after_bytes);
         if (env_off("VUIB_TRACE") && (li == 5 || li == 6)) ma.dbg = wsp<unsigned long long>(e, L.trace) + (li - 5) * 32 + 16;
-        CK(launch_cluster(k_mlp_block<1024, 3072, FB_MLP_U_BACKBONE, FB_MLP_TH_BACKBONE>, NCL, FB_MLP_TH_BACKBONE,
-                          sizeof(MlpBlockSmem<1024, 3072, FB_MLP_U_BACKBONE, FB_MLP_TH_BACKBONE>), s, e->tc->f_w2[li], ma));
+        ma.rows = M;
+        if (one_row(M))
+            CK(launch_cluster(k_mlp_block<1024, 3072, FB_MLP_U_BACKBONE, FB_MLP_TH_BACKBONE>, NCL, FB_MLP_TH_BACKBONE,
+                              sizeof(MlpBlockSmem<1024, 3072, FB_MLP_U_BACKBONE, FB_MLP_TH_BACKBONE>), s, e->tc->f_w2[li], ma));
+        else
+            CK(launch_cluster(k_mlp_rows<1024, 3072, FB_MLP_U_BACKBONE, FB_MLP_TH_BACKBONE>, NCL, FB_MLP_TH_BACKBONE,
+                              sizeof(MlpRowsSmem<1024, 3072, FB_MLP_U_BACKBONE, FB_MLP_TH_BACKBONE>), s, e->tc->f_w2[li], ma));
         e->launches++;
     }
     out->x = xb;
@@ -913,9 +939,20 @@ static int32_t run_layers_fused(VuibEngine* e, cudaStream_t s, Residual* out, co
     return VUIB_OK;
 }
 
-// The depth transformer's blocks for ONE stream (row 0) at depth position `pos`, input token x.
-static int32_t rq_layers_fused(VuibEngine* e, const bf16* x, int pos, cudaStream_t s, Residual* out, const void* after,
-                               size_t after_bytes) {
+template <int F>
+static cudaError_t launch_depth_mlp(VuibEngine* e, int li, const MlpBlockArgs& ma, cudaStream_t s) {
+    constexpr int NCL = F / (FB_MLP_U_DEPTH * FB_CL);
+    return one_row(ma.rows)
+               ? launch_cluster(k_mlp_block<512, F, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>, NCL, FB_MLP_TH_DEPTH,
+                                sizeof(MlpBlockSmem<512, F, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>), s, e->tc->f_rq_w2[li], ma)
+               : launch_cluster(k_mlp_rows<512, F, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>, NCL, FB_MLP_TH_DEPTH,
+                                sizeof(MlpRowsSmem<512, F, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>), s, e->tc->f_rq_w2[li], ma);
+}
+
+// The depth transformer's blocks for up to four streams at depth position `pos`; stream b's input token is x + b * x_stride.
+// Without `out` only the positions' keys and values are wanted, and the last layer's MLP block is left out.
+static int32_t rq_layers_fused(VuibEngine* e, int B, const bf16* x, int x_stride, int pos, cudaStream_t s, Residual* out,
+                               const void* after, size_t after_bytes) {
     const VuibConfig& c = e->cfg;
     const WsLayout& L = e->lay;
     const int rd = c.rq_d_model, Q = c.n_quantizers;
@@ -950,8 +987,14 @@ static int32_t rq_layers_fused(VuibEngine* e, const bf16* x, int pos, cudaStream
         aa.spin_limit = e->spin_limit;
         aa.next = prefetch_of(nullptr, 0);   // as in the backbone: the MLP block copies its own matrices early enough
         if (env_off("VUIB_TRACE_DEPTH") && pos == 8 && (li == 1 || li == 2)) aa.dbg = wsp<unsigned long long>(e, L.trace) + (li - 1) * 32;
-        CK(launch_cluster(k_attn_block<512, 1, true>, c.rq_n_heads, FB_THREADS, sizeof(AttnBlockSmem<512, 1>), s, e->tc->f_rq_out[li], aa));
+        aa.rows = B;
+        aa.x_stride = li == 0 ? x_stride : rd;
+        if (one_row(B))
+            CK(launch_cluster(k_attn_block<512, 1, true>, c.rq_n_heads, FB_THREADS, sizeof(AttnBlockSmem<512, 1>), s, e->tc->f_rq_out[li], aa));
+        else
+            CK(launch_cluster(k_attn_rows<512, 1, true, FB_THREADS>, c.rq_n_heads, FB_THREADS, sizeof(AttnRowsSmem<512, 1, true, FB_THREADS>), s, e->tc->f_rq_out[li], aa));
         e->launches++;
+        if (!out && li + 1 == c.rq_n_layers) return VUIB_OK;
 
         MlpBlockArgs ma;
         memset(&ma, 0, sizeof(ma));
@@ -970,17 +1013,11 @@ static int32_t rq_layers_fused(VuibEngine* e, const bf16* x, int pos, cudaStream
         ma.next = li + 1 < c.rq_n_layers ? prefetch_of(e->w.rq_wqkv[li + 1], qkv_bytes, e->w.rq_out_proj[li + 1], wo_bytes)
                                          : prefetch_of(after, after_bytes);
         if (env_off("VUIB_TRACE_DEPTH") && pos == 8 && (li == 1 || li == 2)) ma.dbg = wsp<unsigned long long>(e, L.trace) + (li - 1) * 32 + 16;
-        if (c.rq_ffn == 1408)
-            CK(launch_cluster(k_mlp_block<512, 1408, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>, ncl, FB_MLP_TH_DEPTH,
-                              sizeof(MlpBlockSmem<512, 1408, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>), s, e->tc->f_rq_w2[li], ma));
-        else
-            CK(launch_cluster(k_mlp_block<512, 1536, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>, ncl, FB_MLP_TH_DEPTH,
-                              sizeof(MlpBlockSmem<512, 1536, FB_MLP_U_DEPTH, FB_MLP_TH_DEPTH>), s, e->tc->f_rq_w2[li], ma));
+        ma.rows = B;
+        CK(c.rq_ffn == 1408 ? launch_depth_mlp<1408>(e, li, ma, s) : launch_depth_mlp<1536>(e, li, ma, s));
         e->launches++;
     }
-    out->x = xb;
-    out->parts = pb;
-    out->n_parts = ncl;
+    if (out) *out = {xb, pb, ncl};
     return VUIB_OK;
 }
 
@@ -993,7 +1030,7 @@ static int32_t run_layers(VuibEngine* e, int M, cudaStream_t s, Residual* out, b
     out->parts = nullptr;
     out->n_parts = 0;
     if (prefill && prefill_tc_ok(e)) return run_layers_tc(e, M, s, true);
-    if (M == 1 && fused_backbone_ok(e)) return run_layers_fused(e, s, out, after, after_bytes);
+    if (rows_fit(M) && fused_backbone_ok(e)) return run_layers_fused(e, M, s, out, after, after_bytes);
     if (tc_ok(e, M)) return run_layers_tc(e, M, s, false);
     const VuibConfig& c = e->cfg;
     const WsLayout& L = e->lay;
@@ -1303,18 +1340,23 @@ static int32_t run_depth(VuibEngine* e, int B, const int32_t* slots, const bf16*
         EpiProjPos ep{static_cast<const bf16*>(e->w.rq_backbone_proj), c.d_model, pos_emb, x2, rd, 2};
         CK(VUIB_GEMV(c.d_model, e, sc, ep, B, rd, s));
     }
-    // one stream has the fused two-kernel layers; without them it runs what several streams run, bit for bit
-    if ((B > 1 || !fused_depth_ok(e)) && depth_group_ok(e)) return launch_depth_group(e, B, sa, Qn, s);
-    rc = tc ? rq_layers_tc(e, 2 * B, x2, 2, 0, s) : rq_layers(e, 2 * B, x2, 2, 0, s);
-    if (rc) return rc;
+    const bool fused = rows_fit(B) && fused_depth_ok(e);
+    if (!fused && depth_group_ok(e)) return launch_depth_group(e, B, sa, Qn, s);
+    Residual first{x2 + rd, nullptr, 0};   // depth position 1 after the layers (every other row of x2, or a row a stream with its partial rows)
+    if (fused) {
+        if ((rc = rq_layers_fused(e, B, x2, 2 * rd, 0, s, nullptr, nullptr, 0)) ||
+            (rc = rq_layers_fused(e, B, x2 + rd, 2 * rd, 1, s, &first, e->w.rq_head, (size_t)CS * rd * 2)))
+            return rc;
+    } else if ((rc = tc ? rq_layers_tc(e, 2 * B, x2, 2, 0, s) : rq_layers(e, 2 * B, x2, 2, 0, s))) {
+        return rc;
+    }
 
     bf16* logits = wsp<bf16>(e, L.rq_logits);
     const bf16* head = static_cast<const bf16*>(e->w.rq_head);
-    const bool fused = B == 1 && fused_depth_ok(e);
     for (int i = 0; i < Qn - 1; ++i) {
-        Residual res{i == 0 ? x2 : x1, nullptr, 0};
+        Residual res = i == 0 ? first : Residual{x1, nullptr, 0};
         if (i > 0) {
-            if (fused) rc = rq_layers_fused(e, x1, i + 1, s, &res, head + (size_t)i * CS * rd, (size_t)CS * rd * 2);
+            if (fused) rc = rq_layers_fused(e, B, x1, rd, i + 1, s, &res, head + (size_t)i * CS * rd, (size_t)CS * rd * 2);
             else rc = tc ? rq_layers_tc(e, B, x1, 1, i + 1, s) : rq_layers(e, B, x1, 1, i + 1, s);
             if (rc) return rc;
         }
@@ -1326,8 +1368,8 @@ static int32_t run_depth(VuibEngine* e, int B, const int32_t* slots, const bf16*
             TcEpiLogits el{logits, CS, e->tap_rq ? e->tap_rq + (size_t)i * CS : nullptr, (Q - 1) * CS};
             if ((rc = tc_gemm(e, e->tc->rq_head, e->tc->rq_head, xn, B, rd, CS, i * CS, el, s))) return rc;
         } else {
-            StageNorm sn{res.x, static_cast<const bf16*>(e->w.rq_norm), c.rq_norm_eps,
-                         i == 0 ? 2 : 1, i == 0 ? 1 : 0, res.parts, res.n_parts};
+            StageNorm sn{res.x, static_cast<const bf16*>(e->w.rq_norm), c.rq_norm_eps, i == 0 && !fused ? 2 : 1, 0,
+                         res.parts, res.n_parts, B};
             EpiLogits el{head + (size_t)i * CS * rd, rd, CS, logits, nullptr, nullptr, nullptr,
                          e->tap_rq ? e->tap_rq + (size_t)i * CS : nullptr, (Q - 1) * CS};
             CK(VUIB_GEMV(rd, e, sn, el, B, CS, s));
