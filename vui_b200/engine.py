@@ -219,6 +219,7 @@ class Engine:
         self._handle = C.c_void_p()
         self._graphs: dict[int, torch.cuda.CUDAGraph] = {}
         self._host_frames: set[tuple[int, bool]] = set()   # (rows, with input copy) captured inside the library
+        self._warm: set[int] = set()   # row counts whose kernels have run once
         self._capture_stream = None
         self._sampling_key = None
         self._setup_native()
@@ -377,12 +378,11 @@ class Engine:
             self._handle, B, P(self._g_slot_idx), P(self._g_seq_inc), P(self._g_codes_in),
             P(self._g_hidden_out), P(self._g_cb0_out), P(self._g_eos_out), P(self._g_eos_prob), self._stream))
 
-    def _frame_graph(self, B: int) -> torch.cuda.CUDAGraph:
-        g = self._graphs.get(B)
-        if g is not None:
-            return g
-        # One warm-up outside capture loads the kernels; it runs on the spare slot
-        # with the length frozen, and the sampler state it touched is put back.
+    def _warm_frame(self, B: int) -> None:
+        """A frame outside any capture loads the kernels; it runs on the spare slot with the length frozen, and the
+        state it touched is put back."""
+        if B in self._warm:
+            return
         saved = (self._g_slot_idx.clone(), self._g_seq_inc.clone(), self._g_codes_in.clone(),
                  self.seq_lens.clone(), self._ws.clone())
         self._g_slot_idx.fill_(self._pad_slot)
@@ -396,15 +396,24 @@ class Engine:
             self._frame_call(B)
         torch.cuda.current_stream(self.device).wait_stream(side)
         torch.cuda.synchronize(self.device)
-        g = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(g):
-            self._frame_call(B)
-        torch.cuda.synchronize(self.device)
         self._g_slot_idx.copy_(saved[0])
         self._g_seq_inc.copy_(saved[1])
         self._g_codes_in.copy_(saved[2])
         self.seq_lens.copy_(saved[3])
         self._ws.copy_(saved[4])
+        self._warm.add(B)
+
+    def _frame_graph(self, B: int) -> torch.cuda.CUDAGraph:
+        g = self._graphs.get(B)
+        if g is not None:
+            return g
+        self._warm.discard(B)
+        self._warm_frame(B)
+        torch.cuda.synchronize(self.device)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            self._frame_call(B)
+        torch.cuda.synchronize(self.device)
         self._graphs[B] = g
         return g
 
@@ -426,7 +435,7 @@ class Engine:
         B = _get_bucket(B_active, self._buckets)
         with_in = h_codes_in is not None
         if (B, with_in) not in self._host_frames:
-            self._frame_graph(B)  # runs the frame once outside any capture (kernel loading) and restores the state
+            self._warm_frame(B)
             if self._capture_stream is None:   # the kernels of the graph keep the priority of the stream they were captured on
                 self._capture_stream = torch.cuda.Stream(self.device, priority=-1)
             torch.cuda.synchronize(self.device)
@@ -722,26 +731,30 @@ class Engine:
             return None
         return self._prefill_emb(row, parts[0] if len(parts) == 1 else torch.cat([p.to(self.dtype) for p in parts], dim=1))
 
-    def _prefill_row(self, row, segments, spk_emb, segments_2=None, spk_emb_2=None) -> int:
+    def _prompt_parts(self, row, segments, spk_emb, segments_2=None, spk_emb_2=None) -> list[Tensor]:
+        """Sets the row up for a voice prompt; returns the prompt's embeddings."""
         row._spk_token = self._embed_speaker(spk_emb)
-        row._spk_token_2 = self._embed_speaker(spk_emb_2)
+        row._spk_token_2 = self._embed_speaker(spk_emb_2) if segments_2 is not None else None
         row._active_speaker = 0
-        all_codes = [s.codes for s in list(segments) + list(segments_2 or []) if s.codes is not None]
+        segs = list(segments) + list(segments_2 or [])
+        all_codes = [s.codes for s in segs if s.codes is not None]
         if all_codes and row._codec_ctx is not None:
             row._codec_ctx.set_prompt(torch.cat([c.to(self.device) for c in all_codes], dim=0).T.unsqueeze(0))
+        words = sum(len(s.text.split()) for s in segs if s.text)
+        frames = sum(s.codes.shape[0] for s in segs if s.codes is not None)
+        if words > 0 and frames > 0:
+            row.prompt_wps = words / (frames / FRAME_RATE)
         parts = self._speaker_segments_emb(segments, row._spk_token, final=True)
         if segments_2 is not None:
             parts += self._speaker_segments_emb(segments_2, row._spk_token_2, final=True)
-        self._prefill_parts(row, parts)
+        return parts
+
+    def _prefill_row(self, row, segments, spk_emb, segments_2=None, spk_emb_2=None) -> int:
+        self._prefill_parts(row, self._prompt_parts(row, segments, spk_emb, segments_2, spk_emb_2))
         row._prompt_offset = row.offset
-        segs = list(segments) + list(segments_2 or [])
-        words = sum(len(s.text.split()) for s in segs if s.text)
-        frames = sum(s.codes.shape[0] for s in segs if s.codes is not None)
-        if frames > 0 and words > 0:
-            row.prompt_wps = words / (frames / FRAME_RATE)
         return row._prompt_offset
 
-    def _add_user(self, row, text, codes, *, final=True) -> int:
+    def _user_parts(self, text, codes, *, final=True) -> list[Tensor]:
         parts = []
         if text:
             parts.append(self._text_emb(text, with_cond_bias=False, noisy=True))
@@ -749,10 +762,12 @@ class Engine:
             parts.append(self._sc_emb)
         if codes is not None:
             parts.append(self._audio_emb(codes))
-        self._prefill_parts(row, parts)
-        if codes is not None:
-            if row._codec_ctx is not None:
-                row._codec_ctx.add(codes.T.unsqueeze(0).to(self.device))
+        return parts
+
+    def _add_user(self, row, text, codes, *, final=True) -> int:
+        self._prefill_parts(row, self._user_parts(text, codes, final=final))
+        if codes is not None and row._codec_ctx is not None:
+            row._codec_ctx.add(codes.T.unsqueeze(0).to(self.device))
         return row.offset
 
     def _active_spk_token(self, row):
@@ -760,13 +775,16 @@ class Engine:
             return row._spk_token_2
         return row._spk_token
 
-    def _add_agent_text(self, row, text, *, final=False) -> Tensor:
+    def _agent_parts(self, row, text, *, final=False) -> list[Tensor]:
         spk = self._active_spk_token(row)
         parts = [spk] if spk is not None else []
         parts.append(self._text_emb(text, with_cond_bias=True))
         if final and self._sc_emb is not None:
             parts.append(self._sc_emb)
-        return self._prefill_parts(row, parts)[0, -1]
+        return parts
+
+    def _add_agent_text(self, row, text, *, final=False) -> Tensor:
+        return self._prefill_parts(row, self._agent_parts(row, text, final=final))[0, -1]
 
     # ------------------------------------------------------------ first frame
     def _first_frames(self, rows: list[Row], hidden: Tensor) -> Tensor:
@@ -942,60 +960,91 @@ class Engine:
         pending: deque[int] = deque(range(len(requests)))
         active: dict[int, _ActiveSlot] = {}
         free_slots = set(range(self.max_rows))
-        last_codes: dict[int, Tensor] = {}
         self._apply_cfg(cfg)
         # continuous batching keeps penalty counts without a window (engine.py:606-616)
         self._set_sampling(cfg.temperature, cfg.top_k or 0, RQ_TOP_K, cfg.rep_penalty, 0, cfg.n_codebooks)
+        placed: list[int] = []             # slots whose codes lie in rows 0.. of the static buffers
+        last_codes: dict[int, Tensor] = {}  # codes of slots that are not there yet, (Q,) on the device
 
-        def advance(info: _ActiveSlot) -> bool:
+        def next_text(info: _ActiveSlot) -> list[Tensor] | None:
+            """The next chunk's embeddings, None when there is none."""
             if info.chunk_idx >= len(info.chunks):
-                return False
-            ch = info.chunks[info.chunk_idx]
-            row = info.row
+                return None
+            ch, row = info.chunks[info.chunk_idx], info.row
             if ch["sc"] and row._spk_token_2 is not None:
                 row._active_speaker = 1 - row._active_speaker
             info.max_turn_frames = cfg.max_turn_frames(len(ch["text"].split()), row.prompt_wps)
-            hidden = self._add_agent_text(row, ch["text"])
-            codes = self._first_frames([row], hidden[None])[0]
-            last_codes[row.idx] = codes
+            return self._agent_parts(row, ch["text"])
+
+        def first_frame(info: _ActiveSlot, hidden: Tensor) -> None:
+            codes = self._first_frames([info.row], hidden[None])[0]
+            last_codes[info.row.idx] = codes
             bufs[info.request_idx].append(codes.cpu()[None])
             info.frame_count += 1
             info.turn_count = 1
-            info.seq_offset = row.offset
+
+        def advance(info: _ActiveSlot) -> bool:
+            parts = next_text(info)
+            if parts is None:
+                return False
+            hidden = self._prefill_parts(info.row, parts)[0, -1]
+            info.seq_offset = info.row.offset
+            first_frame(info, hidden)
             return True
 
         def backfill() -> None:
-            while pending and free_slots:
+            """Requests into the free slots: prompts, user turns and first texts of all of them in one prefill, then their
+            first frames, slot by slot as the draws are numbered."""
+            new: list[tuple[_ActiveSlot, Tensor]] = []
+            taken: set[int] = set()
+            while pending and free_slots - taken:
                 ri = pending.popleft()
                 req = requests[ri]
-                slot = min(free_slots)
-                free_slots.remove(slot)
+                slot = min(free_slots - taken)
                 self.seq_lens[slot] = 0
                 self._rep_reset(slot=slot)
                 row = Row(self, slot)
-                self._rows[slot] = row
-                row.prefill(req.segments, spk_emb=req.spk_emb, segments_2=req.segments_2, spk_emb_2=req.spk_emb_2)
+                parts = self._prompt_parts(row, req.segments, req.spk_emb, req.segments_2, req.spk_emb_2)
+                row._prompt_offset = sum(p.shape[1] for p in parts)
                 if req.user_text or req.user_codes is not None:
-                    row.add_user(req.user_text or "", req.user_codes)
+                    parts += self._user_parts(req.user_text or "", req.user_codes)
+                    if req.user_codes is not None and row._codec_ctx is not None:
+                        row._codec_ctx.add(req.user_codes.T.unsqueeze(0).to(self.device))
                 chunks = chunk_text(req.text, min_words=cfg.chunk_words, sentence_only=cfg.sentence_only,
                                     single_speaker=(row._spk_token_2 is None))
                 info = _ActiveSlot(row=row, request_idx=ri, chunks=chunks)
-                if not chunks or not advance(info):
-                    self._rows.pop(slot, None)
-                    free_slots.add(slot)
+                text = next_text(info)
+                if text is None:
                     continue
-                active[slot] = info
+                taken.add(slot)
+                self._rows[slot] = row
+                parts += text
+                info.seq_offset = sum(p.shape[1] for p in parts)
+                new.append((info, torch.cat([p.to(self.dtype) for p in parts], dim=1)))
+            free_slots.difference_update(taken)
+            if new:
+                for (info, _), hidden in zip(new, self._prefill_many([(info.row, emb) for info, emb in new])):
+                    first_frame(info, hidden[-1])
+                    active[info.row.idx] = info
 
         backfill()
         while active:
             slots = sorted(active)
             B = len(slots)
+            # a step leaves its codes where the next one reads them: only rows that moved or began a text are written
+            moved = slots != placed
+            old = self._g_codes_in[: len(placed)].clone() if moved else None
             for qi, s_ in enumerate(slots):
-                self._set_codes_in(qi, last_codes[s_])
-            self._g_slot_idx[:B] = torch.tensor(slots, device=self.device, dtype=torch.int32)
+                if s_ in last_codes:
+                    self._set_codes_in(qi, last_codes[s_])
+                elif moved and placed.index(s_) != qi:
+                    self._set_codes_in(qi, old[placed.index(s_)])
+            last_codes.clear()
+            if moved:
+                self._g_slot_idx[:B] = torch.tensor(slots, device=self.device, dtype=torch.int32)
+                placed = slots
             self._g_seq_inc[:B].fill_(1)
-            self._frame_step(B)
-            h_codes, h_eos = self._read_frame(B)
+            h_codes, h_eos = self._frame_host(B)
             h_codes = h_codes.clone()
             done = []
             for qi, s_ in enumerate(slots):
@@ -1010,7 +1059,6 @@ class Engine:
                     if not advance(info):
                         done.append(s_)
                     continue
-                last_codes[s_] = self._g_codes_in[qi].clone()
                 bufs[info.request_idx].append(h_codes[qi][None])
                 info.frame_count += 1
                 info.turn_count += 1
@@ -1018,7 +1066,8 @@ class Engine:
                 info = active.pop(s_)
                 self._rows.pop(s_, None)
                 free_slots.add(s_)
-            backfill()
+            if done:
+                backfill()
         return [torch.cat(b, dim=0) if b else torch.zeros(0, self.Q, dtype=torch.long) for b in bufs]
 
     # -------------------------------------------------------------- streaming
