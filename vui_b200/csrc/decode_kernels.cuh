@@ -244,7 +244,7 @@ struct StageNorm {
             if (rr >= nr) break;
             const int r = r0 + rr;
             const bf16* xr = x + ((size_t)r * row_mul + row_add) * K + k0;
-            const float* pr = parts + (size_t)r * K + k0;
+            const float* pr = parts + ((size_t)r * row_mul + row_add) * K + k0;
             const size_t ps = (size_t)n_rows * K;
             float sp[EPT];
 #pragma unroll

@@ -402,6 +402,7 @@ struct AttnBlockArgs {
     PrefetchList next;      // the following kernel's matrices
     unsigned long long* dbg;  // optional: device-clock stamps of CTA 0 (profiling aid)
     int rows, x_stride;     // several rows (fused_rows.cuh): how many, elements between rows of x_in
+    int pairs;              // depth loop: rows 2n and 2n + 1 are positions fixed_pos and fixed_pos + 1 of slot n
 };
 
 template <int K, int G>

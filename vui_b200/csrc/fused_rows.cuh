@@ -193,7 +193,8 @@ __device__ __forceinline__ void mma_slice4(const bf16* mat, const bf16* vec, int
 
 // ---------------------------------------------------------------------------
 // Attention block.  AttnBlockArgs with rows: x_in rows are x_stride elements apart, x_out and tap (rows, K),
-// parts_in / parts_out [part][rows][K]; the depth loop's row n uses slot n at fixed_pos.
+// parts_in / parts_out [part][rows][K]; the depth loop's row n uses slot n at fixed_pos,
+// or with `pairs` (fixed_pos = 0 only) position n & 1 of slot n / 2.
 // ---------------------------------------------------------------------------
 template <int K, int G, bool SHORT, int TH>
 struct AttnRowsSmem {
@@ -269,14 +270,15 @@ __global__ void __launch_bounds__(TH, 1) k_attn_rows(const __grid_constant__ CUt
     const int prow = 2 * (pair_live ? tid >> 4 : 0);
     const bool is_q = prow < QR, is_k = !is_q && prow < QR + KR;
     const int sub = is_q ? prow : (is_k ? prow - QR : prow - QR - KR);
-    int pslot = pn, ppos = a.fixed_pos;
+    const int pairs = SHORT && a.pairs ? 1 : 0;
+    int pslot = pn >> pairs, ppos = a.fixed_pos + (pn & pairs);
     float c0 = 1.f, s0 = 0.f, c1 = 1.f, s1 = 0.f;
     // ---- and its keys: a quarter of every CTA's warps for a row (backbone), one (depth loop)
     const int s8 = lane & 7, g4 = lane >> 3;
     const int arow = warp / WPR, asub = warp % WPR;
     const bool row_live = arow < rows;
     const size_t pos_stride = (size_t)kvcols;
-    int slot = arow, pos = a.fixed_pos;
+    int slot = arow >> pairs, pos = a.fixed_pos;   // old keys: those before the pair
     int t_begin = 0, t_end = 0;
     const bf16* kb = nullptr;
     const bf16* vb = nullptr;
@@ -312,7 +314,7 @@ __global__ void __launch_bounds__(TH, 1) k_attn_rows(const __grid_constant__ CUt
     pdl_wait();
     fb_stamp(a.dbg, 1);
 
-    int sl = arow, ps = a.fixed_pos;
+    int sl = arow >> pairs, ps = a.fixed_pos;
     if constexpr (!SHORT) {
         const int r = row_live ? arow : 0;
         sl = __ldcg(a.row_slot + r);
@@ -381,6 +383,17 @@ __global__ void __launch_bounds__(TH, 1) k_attn_rows(const __grid_constant__ CUt
         const float4 q1 = *reinterpret_cast<const float4*>(qkv + h * HD + s8 * 8 + 4);
         qf[h][0] = q0.x; qf[h][1] = q0.y; qf[h][2] = q0.z; qf[h][3] = q0.w;
         qf[h][4] = q1.x; qf[h][5] = q1.y; qf[h][6] = q1.z; qf[h][7] = q1.w;
+    }
+    if constexpr (SHORT) {
+        if (row_live && (arow & pairs)) {   // the second of a pair (of which no key is in the cache) also sees the first one's key
+            const float* first = qkv - QKV + HD + s8 * 8;
+            float kf[8], vf[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) { kf[j] = first[j]; vf[j] = first[HD + j]; }
+            kr[0] = pack8(kf);
+            vr[0] = pack8(vf);
+            t_end = 1;
+        }
     }
     float m[G], l[G], acc[G][8], sc[G][NPRE];
 #pragma unroll

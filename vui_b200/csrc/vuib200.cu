@@ -951,8 +951,9 @@ static cudaError_t launch_depth_mlp(VuibEngine* e, int li, const MlpBlockArgs& m
 
 // The depth transformer's blocks for up to four streams at depth position `pos`; stream b's input token is x + b * x_stride.
 // Without `out` only the positions' keys and values are wanted, and the last layer's MLP block is left out.
+// With `pairs` a stream has two rows, positions 0 and 1 (B counts rows).
 static int32_t rq_layers_fused(VuibEngine* e, int B, const bf16* x, int x_stride, int pos, cudaStream_t s, Residual* out,
-                               const void* after, size_t after_bytes) {
+                               const void* after, size_t after_bytes, bool pairs = false) {
     const VuibConfig& c = e->cfg;
     const WsLayout& L = e->lay;
     const int rd = c.rq_d_model, Q = c.n_quantizers;
@@ -988,6 +989,7 @@ static int32_t rq_layers_fused(VuibEngine* e, int B, const bf16* x, int x_stride
         aa.next = prefetch_of(nullptr, 0);   // as in the backbone: the MLP block copies its own matrices early enough
         if (env_off("VUIB_TRACE_DEPTH") && pos == 8 && (li == 1 || li == 2)) aa.dbg = wsp<unsigned long long>(e, L.trace) + (li - 1) * 32;
         aa.rows = B;
+        aa.pairs = pairs;
         aa.x_stride = li == 0 ? x_stride : rd;
         if (one_row(B))
             CK(launch_cluster(k_attn_block<512, 1, true>, c.rq_n_heads, FB_THREADS, sizeof(AttnBlockSmem<512, 1>), s, e->tc->f_rq_out[li], aa));
@@ -1342,8 +1344,13 @@ static int32_t run_depth(VuibEngine* e, int B, const int32_t* slots, const bf16*
     }
     const bool fused = rows_fit(B) && fused_depth_ok(e);
     if (!fused && depth_group_ok(e)) return launch_depth_group(e, B, sa, Qn, s);
-    Residual first{x2 + rd, nullptr, 0};   // depth position 1 after the layers (every other row of x2, or a row a stream with its partial rows)
-    if (fused) {
+    Residual first{x2, nullptr, 0};   // depth position 1 after the layers: row b * first_mul + first_add
+    int first_mul = 2, first_add = 1;
+    if (fused && 2 * B <= FR_ROWS) {  // both positions as rows of one pass
+        if ((rc = rq_layers_fused(e, 2 * B, x2, rd, 0, s, &first, e->w.rq_head, (size_t)CS * rd * 2, true))) return rc;
+    } else if (fused) {
+        first_mul = 1;
+        first_add = 0;
         if ((rc = rq_layers_fused(e, B, x2, 2 * rd, 0, s, nullptr, nullptr, 0)) ||
             (rc = rq_layers_fused(e, B, x2 + rd, 2 * rd, 1, s, &first, e->w.rq_head, (size_t)CS * rd * 2)))
             return rc;
@@ -1368,8 +1375,8 @@ static int32_t run_depth(VuibEngine* e, int B, const int32_t* slots, const bf16*
             TcEpiLogits el{logits, CS, e->tap_rq ? e->tap_rq + (size_t)i * CS : nullptr, (Q - 1) * CS};
             if ((rc = tc_gemm(e, e->tc->rq_head, e->tc->rq_head, xn, B, rd, CS, i * CS, el, s))) return rc;
         } else {
-            StageNorm sn{res.x, static_cast<const bf16*>(e->w.rq_norm), c.rq_norm_eps, i == 0 && !fused ? 2 : 1, 0,
-                         res.parts, res.n_parts, B};
+            StageNorm sn{res.x, static_cast<const bf16*>(e->w.rq_norm), c.rq_norm_eps, i == 0 ? first_mul : 1,
+                         i == 0 ? first_add : 0, res.parts, res.n_parts, i == 0 ? B * first_mul : B};
             EpiLogits el{head + (size_t)i * CS * rd, rd, CS, logits, nullptr, nullptr, nullptr,
                          e->tap_rq ? e->tap_rq + (size_t)i * CS : nullptr, (Q - 1) * CS};
             CK(VUIB_GEMV(rd, e, sn, el, B, CS, s));
