@@ -543,20 +543,24 @@ def codec_encoder_block(dev, cpu_baseline: bool, reps: int = 5):
     enc = QwenCodecEncoder.random_init(0, device=dev)
     se = StreamingCodecEncoder(enc)
     se.setup_graph()
+    whole, _ = se._graphs[se.max_frames]
+    n0 = enc.launch_count()
+    enc(se._audio_buf)
+    launches = enc.launch_count() - n0
     se._audio_buf.copy_(test_audio(240000, seed=0).to(dev))
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     times = []
     for _ in range(reps):
         torch.cuda.synchronize(dev)
         e0.record()
-        se._graph.replay()
+        whole.replay()
         e1.record()
         torch.cuda.synchronize(dev)
         times.append(e0.elapsed_time(e1))
     ms = statistics.median(times)
     res = {"workload": "codec encoder, 10 s buffer (240000 samples -> 16 x 125 codes), fp32, seeded random weights; "
                        f"median of {reps} graph replays",
-           "ms_per_buffer": ms, "x_realtime": 10e3 / ms, "launches": 75, "gflop": 40.0, "tflops": 40.0 / ms}
+           "ms_per_buffer": ms, "x_realtime": 10e3 / ms, "launches": launches, "gflop": 40.0, "tflops": 40.0 / ms}
     if cpu_baseline:
         from oracle.codec_enc_oracle import EncoderOracle
         from vui_b200.codec_encoder import random_encoder_state
