@@ -154,10 +154,14 @@ __device__ __forceinline__ void mma_rows4(const bf16* mat, const bf16* xs, float
 template <int NROWS, int NW>
 __device__ __forceinline__ float mma_rows4_total(const float* red, int r, int n) {
     constexpr int NT = (NROWS + 15) / 16;
-    float s = 0.f;
+    float s[NW];
 #pragma unroll
-    for (int w = 0; w < NW; ++w) s += red[(w * (NT * 16) + r) * FR_ROWS + n];
-    return s;
+    for (int w = 0; w < NW; ++w) s[w] = red[(w * (NT * 16) + r) * FR_ROWS + n];
+#pragma unroll
+    for (int k = NW / 2; k > 0; k /= 2)   // as a tree: a chain of NW additions is 16 x 4 cycles
+#pragma unroll
+        for (int w = 0; w < k; ++w) s[w] += s[w + k];
+    return s[0];
 }
 
 // A column slice of out_proj or w2 (ROWS x C in shared memory) times the streams' vectors (bf16, C + FR_PAD apart), a warp for every

@@ -162,7 +162,7 @@ static void make_layout(VuibEngine* e) {
     L.rq_xn = take(2 * RB * rd * 2);
     L.rq_attn = take(2 * RB * rd * 2);
     L.dg_layers = L.dg_head = 0;
-    if (depth_tc_shape(c)) {
+    if (depth_tc_shape(c) && c.max_rows > FR_ROWS) {   // up to four streams take the fused layers
         const int n_ub = (c.rq_ffn / DT_CL + 63) / 64;
         L.dg_layers = take((size_t)c.rq_n_layers * DT_CL * dt_slots_per_layer(n_ub) * DT_SLOT);
         L.dg_head = take((size_t)(c.n_quantizers - 1) * DT_CL * DT_HEAD_SLOTS * DT_SLOT);
