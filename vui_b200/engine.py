@@ -207,7 +207,9 @@ class Engine:
         self.max_seq = max_seq or trained
         if self.max_seq > trained:
             raise ValueError(f"max_seq={self.max_seq} exceeds trained ceiling {trained}")
-        self.max_prefill_rows = max_prefill_rows
+        # Rows of one prefill call.  A long prompt in calls of 256 rows reads all weights for each (1.26 ms; 1024 rows take 2.8): unless
+        # fewer are asked for, there is room for 1024 where the cache holds as many (35 KB a row).
+        self.max_prefill_rows = max_prefill_rows if max_prefill_rows < 256 else max(max_prefill_rows, min(1024, self.max_seq))
         if model._cond_bias is None:
             model._cond_bias = torch.zeros(1, 1, self.D, device=self.device, dtype=self.dtype)
         self._cond_bias = model._cond_bias
