@@ -138,15 +138,11 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// x / (1 + exp(-x)) without a branch: the divisor's reciprocal with a Newton step, the quotient with a residual correction.  (The
-// compiler's division has a slow path, and with a branch in each a thread's values follow one another.)
+// x / (1 + exp(-x)) as (x or x exp(x)) / (1 + exp(-|x|)): the divisor lies in [1, 2], so that CUDA's branch-free __fdividef is within
+// its two ulp for every x.
 __device__ __forceinline__ float silu(float x) {
-    const float d = 1.0f + expf(fminf(-x, 80.f));
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    r = fmaf(r, fmaf(-d, r, 1.0f), r);
-    const float q = x * r;
-    return fmaf(r, fmaf(-q, d, x), q);
+    const float e = expf(-fabsf(x));
+    return __fdividef(x < 0.f ? x * e : x, 1.0f + e);
 }
 
 // ---------------------------------------------------------------------------
