@@ -1577,15 +1577,13 @@ __device__ __forceinline__ int sample_rq(uint4 raw, const SampleKey& k, float u,
             }
         }
     }
-    // v / T: the product with the reciprocal and one residual correction (Markstein's scheme) is the correctly rounded quotient
-    const float T = k.temperature, rT = 1.0f / T;
-    auto scaled = [&](float x) { const float q = x * rT; return fmaf(fmaf(-q, T, x), rT, q); };
+    const float T = k.temperature;
     const uint32_t kb = kmax << 16;
-    const float smax = scaled(__uint_as_float((kb & 0x80000000u) ? kb & 0x7fff0000u : ~kb & 0xffff0000u));
+    const float smax = __uint_as_float((kb & 0x80000000u) ? kb & 0x7fff0000u : ~kb & 0xffff0000u) / T;
     float p[SAMPLE_EL], loc = 0.f;
 #pragma unroll
     for (int j = 0; j < SAMPLE_EL; ++j) {
-        p[j] = key[j] >= thr ? expf(scaled(v[j]) - smax) : 0.f;
+        p[j] = key[j] >= thr ? expf(v[j] / T - smax) : 0.f;
         loc += p[j];
     }
     float inc = loc;
