@@ -736,7 +736,7 @@ class Engine:
     def _prompt_parts(self, row, segments, spk_emb, segments_2=None, spk_emb_2=None) -> list[Tensor]:
         """Sets the row up for a voice prompt; returns the prompt's embeddings."""
         row._spk_token = self._embed_speaker(spk_emb)
-        row._spk_token_2 = self._embed_speaker(spk_emb_2) if segments_2 is not None else None
+        row._spk_token_2 = self._embed_speaker(spk_emb_2)   # also without segments of its own: [SC] in a text then switches
         row._active_speaker = 0
         segs = list(segments) + list(segments_2 or [])
         all_codes = [s.codes for s in segs if s.codes is not None]
