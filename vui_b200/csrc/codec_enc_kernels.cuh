@@ -98,6 +98,8 @@ static __global__ void __cluster_dims__(RV_CL, 1, 1) __launch_bounds__(32 * RV_W
     const int part = blockIdx.y, n = part ? a.n_q - 1 : 1, q0 = part ? 1 : 0;
     if (n == 0) return;   // the whole cluster
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, f0 = (blockIdx.x / RV_CL) * RV_F, rank = blockIdx.x % RV_CL;
+    // A peer's shared memory may be touched only once all CTAs of the cluster run: waited for in front of the first store to one.
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     vuis::sg_pdl_wait();
     vuis::sg_pdl_launch();
     float2 r[RV_F][4];
@@ -152,6 +154,7 @@ static __global__ void __cluster_dims__(RV_CL, 1, 1) __launch_bounds__(32 * RV_W
         }
         if ((lane & 3) == 0) { wv[warp][lane >> 2] = bv; wi[warp][lane >> 2] = bi; }
         __syncthreads();
+        if (cb == 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         const int buf = cb & 1;
         if (tid < RV_CL * RV_F) {
             const int f = tid & 7, dst = tid >> 3;
