@@ -41,6 +41,17 @@ def test_buckets():
     assert _get_bucket(9, [1, 2, 4, 8]) == 8
 
 
+def test_prefill_rows_asked_for_are_a_limit():
+    import inspect
+
+    from vui_b200.engine import Engine, _prefill_rows
+
+    assert inspect.signature(Engine.__init__).parameters["max_prefill_rows"].default is None
+    assert [_prefill_rows(None, n) for n in (64, 256, 640, 1024, 2000)] == [256, 256, 640, 1024, 1024]
+    for asked in (1, 16, 256, 512, 4096):
+        assert _prefill_rows(asked, 2000) == asked
+
+
 def test_max_turn_frames():
     c = GenConfig()
     assert c.max_turn_frames(0) == int(15.0 * 12.5)

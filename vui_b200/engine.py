@@ -119,6 +119,12 @@ def _get_bucket(n: int, buckets: list[int]) -> int:
     return buckets[-1]
 
 
+def _prefill_rows(asked: int | None, max_seq: int) -> int:
+    """Rows of one prefill call: as many as are asked for, or room for 1024 where the cache holds as many (35 KB a row).  A long
+    prompt in calls of 256 rows reads all weights for each (1.26 ms; 1024 rows take 2.8)."""
+    return max(256, min(1024, max_seq)) if asked is None else asked
+
+
 class Row:
     """A single conversation slot: index into the shared KV cache, the
     end-of-prompt offset for rewind, and the speaker token(s) from prefill."""
@@ -184,7 +190,7 @@ class Engine:
 
     def __init__(self, name: str = "vui-nano", *, model: VuiB200 | None = None, codec=None,
                  max_rows: int = 1, max_seq: int | None = None, codec_dtype: torch.dtype = torch.float32,
-                 vocoder_ctx: int = 25, max_prefill_rows: int = 256, seed: int = 0):
+                 vocoder_ctx: int = 25, max_prefill_rows: int | None = None, seed: int = 0):
         if not torch.cuda.is_available():
             raise RuntimeError("vui_b200.Engine needs a CUDA device (sm_100a); there is no CPU path")
         if model is None:
@@ -207,9 +213,7 @@ class Engine:
         self.max_seq = max_seq or trained
         if self.max_seq > trained:
             raise ValueError(f"max_seq={self.max_seq} exceeds trained ceiling {trained}")
-        # Rows of one prefill call.  A long prompt in calls of 256 rows reads all weights for each (1.26 ms; 1024 rows take 2.8): unless
-        # fewer are asked for, there is room for 1024 where the cache holds as many (35 KB a row).
-        self.max_prefill_rows = max_prefill_rows if max_prefill_rows < 256 else max(max_prefill_rows, min(1024, self.max_seq))
+        self.max_prefill_rows = _prefill_rows(max_prefill_rows, self.max_seq)
         if model._cond_bias is None:
             model._cond_bias = torch.zeros(1, 1, self.D, device=self.device, dtype=self.dtype)
         self._cond_bias = model._cond_bias
