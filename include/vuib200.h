@@ -415,10 +415,12 @@ int32_t vuib_codec_reset(VuibCodec* c, void* stream);
 int32_t vuib_codec_decode_frame(VuibCodec* c, const int64_t* codes_dev, int32_t n_q, float* audio_out_dev,
                                 void* stream);
 /* codes_dev int64[n_q][n_frames] (n_frames <= max_seq) -> audio_out_dev float[1920 * n_frames] in one pass: QwenCodecDecoder.forward
- * outside a streaming context (qwen_codec.py:1199-1215), from zero left padding.  The streaming state starts over. */
+ * outside a streaming context (qwen_codec.py:1199-1215), from zero left padding.  The streaming state starts over: the next
+ * vuib_codec_decode_frame is a first frame, as after vuib_codec_reset. */
 int32_t vuib_codec_decode(VuibCodec* c, const int64_t* codes_dev, int32_t n_q, int32_t n_frames, float* audio_out_dev,
                           void* stream);
-/* Frames decoded since the last reset (= next transformer position).  Synchronises `stream`. */
+/* Frames decoded since the streaming state last started over (= next transformer position); before the first of them, the
+ * frames of the whole input decoded since the last reset, if any.  Synchronises `stream`. */
 int32_t vuib_codec_position(VuibCodec* c, int32_t* pos, void* stream);
 /* Reads and clears the codec's device flag (code outside [0, 2048), position beyond max_seq: both are
  * clamped, never dereferenced).  Synchronises `stream`. */

@@ -26,6 +26,30 @@ def test_decode_in_one_pass(codec, frames, n_q):
     assert got.shape == ref.shape and (got - ref).abs().max().item() <= 5e-5 * ref.abs().max().item()
 
 
+@pytest.mark.parametrize("frames", [2, 9, 250])
+def test_a_frame_after_a_whole_input_is_a_first_frame(codec, frames):
+    """The library's own calls, without the resets of the Python class between them: 250 is all the positions that there are."""
+    dec, _ = codec
+    codes = torch.randint(0, 2048, (1, 16, frames), generator=torch.Generator().manual_seed(frames)).cuda()
+    nxt = torch.randint(0, 2048, (3, 16), generator=torch.Generator().manual_seed(1)).cuda()
+
+    def stream():
+        out = torch.zeros(3, 1920, device="cuda")
+        for i in range(3):
+            dec._check(dec._lib.vuib_codec_decode_frame(dec._h, nxt[i].data_ptr(), 16, out[i].data_ptr(), dec._stream()))
+            assert dec.position() == i + 1
+        return out
+
+    dec.reset_streaming()
+    fresh = stream()
+    dec(codes)
+    assert dec.position() == frames
+    assert torch.equal(stream(), fresh)
+    dec.check_device()
+    dec.reset_streaming()
+    assert dec.position() == 0
+
+
 @pytest.mark.parametrize("frames", [1, 2, 17, 32])
 def test_encode_in_one_pass(frames):
     from oracle.codec_enc_oracle import EncoderOracle, test_audio

@@ -434,8 +434,10 @@ extern "C" int32_t vuib_codec_position(VuibCodec* c, int32_t* pos, void* stream)
     if (!c || !pos) return VUIB_ERR_NULL;
     if (!c->have_ws) return fail(c, VUIB_ERR_UNBOUND, "codec workspace not bound");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    CK(cudaMemcpyAsync(pos, wsp<int>(c, c->lay.ctr) + CTR_POS, sizeof(int), cudaMemcpyDeviceToHost, s));
+    int ctr[CTR_WHOLE + 1];
+    CK(cudaMemcpyAsync(ctr, wsp<int>(c, c->lay.ctr), sizeof(ctr), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    *pos = ctr[CTR_POS] ? ctr[CTR_POS] : ctr[CTR_WHOLE];
     return VUIB_OK;
 }
 
@@ -643,7 +645,7 @@ extern "C" int32_t vuib_codec_decode(VuibCodec* c, const int64_t* codes_dev, int
     }
     int* ctr = wsp<int>(c, L.ctr);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // the streaming state starts over; only the counters are left as n_frames streamed frames would leave them
+    // the streaming state starts over: a frame that follows is a first frame
     CK(cudaMemsetAsync(c->ws, 0, L.state_hi, s));
     const SgCtx x = {ctr + CTR_FLAG, c->num_sms, pdl_enabled(), s, &c->launches};
     const int T = n_frames, lat = g.latent_dim, D = g.d_model, HH = g.n_heads * HD;
@@ -663,7 +665,7 @@ extern "C" int32_t vuib_codec_decode(VuibCodec* c, const int64_t* codes_dev, int
         a.codes = reinterpret_cast<const long long*>(codes_dev);
         a.n_q = n_q; a.T = T;
         for (int q = 0; q < 16; ++q) a.table[q] = w.codebook[q];
-        a.o = pe; a.flag = ctr + CTR_FLAG; a.flag_bad = FLAG_BAD_CODE; a.ctr = ctr + CTR_FRAME;
+        a.o = pe; a.flag = ctr + CTR_FLAG; a.flag_bad = FLAG_BAD_CODE; a.whole = ctr + CTR_WHOLE;
         CK(sg_run(x, k_bembed, dim3(T), dim3(256), 0, a));
         CK(sg_launch(x, B.proj, pe, T, 1, out(nullptr, g.vq_dim, ph, nullptr, 0)));
         CK(sg_launch(x, B.pre, ph, T, 1, out(w.pre_conv.b, lat, py, nullptr, 0)));

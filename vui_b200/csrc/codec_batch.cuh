@@ -16,7 +16,7 @@ struct BEmbedArgs {
     SgPlanes o;                  // 512 channels: sum of the semantic code vectors, sum of the acoustic ones
     int* flag;                   // set to flag_bad by a code outside [0, 2048)
     int flag_bad;
-    int* ctr;                    // frame counter and position of the streaming state: set to T, as T streamed frames would leave them
+    int* whole;                  // set to T
 };
 
 // SplitResidualVQ.decode's sums (qwen_codec.py:231-238), in codebook order.  A CTA takes one frame.
@@ -48,7 +48,7 @@ static __global__ void __launch_bounds__(256) k_bembed(BEmbedArgs a) {
         for (int i = 0; i < 8; ++i) u[i] = s[c * 8 + i];
         vuis::sg_store8(a.o, a.o.pad + t, c * 8, u);
     }
-    if (t == 0 && c < 2) a.ctr[c] = a.T;
+    if (t == 0 && c == 0) *a.whole = a.T;
 }
 
 struct BFinalArgs {

@@ -29,6 +29,7 @@ namespace vuic {
 constexpr int CTR_FRAME = 0;   // frames decoded since the last reset (its low bit is the state parity)
 constexpr int CTR_POS = 1;     // next transformer position
 constexpr int CTR_FLAG = 2;    // sticky error bits
+constexpr int CTR_WHOLE = 3;   // frames of the last whole input, which are not part of the streaming state
 constexpr int FLAG_BAD_CODE = 1;
 constexpr int FLAG_POS_OVERFLOW = 2;
 constexpr int FLAG_WAIT = 4;        // a bounded wait on an asynchronous copy ran out
