@@ -298,7 +298,7 @@ int32_t vuib_set_wait_limit(VuibEngine* e, uint32_t polls);
 
 /* Test hook for the bound above: the next tensor-core GEMM whose tiles are shared by a cluster waits for
  * one value more than is sent to it.  Its wait runs out, the flag is recorded, the kernel returns.
- * Nothing faults or hangs. */
+ * Nothing faults or hangs.  vuib_reset_state takes an order that no GEMM has used back. */
 int32_t vuib_debug_withhold_arrival(VuibEngine* e, void* stream);
 
 /* Position-only rewind / reset (engine.py:651-654).  Synchronous small copies. */

@@ -719,3 +719,19 @@ def test_bounded_wait_runs_out_and_reports(nano_model):
     again = eng.prefill_ids(row, ids)
     eng.check_device()
     assert torch.equal(again, clean)
+
+
+def test_a_withheld_arrival_does_not_outlive_a_reset(nano_model):
+    """The hook armed, but no GEMM of it run before vuib_reset_state: the calls after that are clean."""
+    from vui_b200 import Engine
+
+    eng = Engine(model=nano_model, max_rows=1, max_seq=64, max_prefill_rows=16)
+    row = eng.new_row()
+    clean = eng.prefill_ids(row, _ids(8, 4)).clone()
+    eng._ck(eng._lib.vuib_set_wait_limit(eng._handle, 20000))
+    eng._ck(eng._lib.vuib_debug_withhold_arrival(eng._handle, eng._stream))
+    eng._ws_reset_counters()
+    eng._rewind_row(row, 0)
+    again = eng.prefill_ids(row, _ids(8, 4))
+    eng.check_device()
+    assert torch.equal(again, clean)

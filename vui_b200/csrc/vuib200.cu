@@ -1665,6 +1665,7 @@ extern "C" int32_t vuib_reset_state(VuibEngine* e, void* stream) {
     CK(cudaMemsetAsync(e->ws + L.flag, 0, 256, s));
     CK(cudaMemsetAsync(e->ws + L.counters, 0, (size_t)e->R * c.n_kv_heads * 4, s));
     CK(cudaMemsetAsync(e->ws + L.frame_ctr, 0, (size_t)c.n_slots * 4, s));
+    e->withhold = false;
     return vuib_rep_reset(e, -1, stream);
 }
 
