@@ -267,7 +267,7 @@ extern "C" int32_t vuib_codec_enc_encode(VuibCodecEnc* c, const float* audio_dev
         o.y = q;
         o.y_rows = T;
         CK(sg_launch(x, c->pk.wqkv[l], xp, T, 1, o));
-        SAttnArgs aa = {q, T, f32(c->off_rope), g.max_samples / 960, xp, T, H, nullptr, nullptr, 0};
+        SAttnArgs aa = {q, T, f32(c->off_rope), g.max_samples / 960, xp, T, H};
         CK(sg_run(x, k_sattn, dim3((T + SAT_Q - 1) / SAT_Q, H), dim3(256), 0, aa));
         o = out(nullptr, D, SA_NONE, none, 1);
         o.res = o.y = xr;

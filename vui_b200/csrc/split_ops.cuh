@@ -98,9 +98,6 @@ struct SAttnArgs {
     int rope_rows;
     SgPlanes o;            // H * 64 channels
     int T, H;
-    float* kc;             // optional: K (after RoPE) and V of every position, [H][max_seq][64]
-    float* vc;
-    int max_seq;
 };
 
 // Rotate-half tables [T][64] (both halves alike) in the order in which k_sattn's lanes, one a row, read them.
@@ -166,14 +163,6 @@ static __global__ void __launch_bounds__(256) k_sattn(SAttnArgs a) {
             for (int q = 0; q < 4; ++q) { ks[k][d + q] = lo[q]; ks[k][d + 32 + q] = hi[q]; }
             *reinterpret_cast<float4*>(&vs[k][d]) = f[it][2];
             *reinterpret_cast<float4*>(&vs[k][d + 32]) = f[it][3];
-            // the CTA whose queries these positions are keeps them for later frames
-            if (a.kc && k0 + k >= q0 && k0 + k < last) {
-                const long long p = ((long long)h * a.max_seq + k0 + k) * 64 + d;
-                *reinterpret_cast<float4*>(a.kc + p) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-                *reinterpret_cast<float4*>(a.kc + p + 32) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<float4*>(a.vc + p) = f[it][2];
-                *reinterpret_cast<float4*>(a.vc + p + 32) = f[it][3];
-            }
         }
         __syncthreads();
         if (k0 + SAT_K < last) fetch(k0 + SAT_K);
