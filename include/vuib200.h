@@ -464,7 +464,7 @@ typedef struct VuibCodecEncWeights {
     const float* downsample;         /* downsample.conv.weight (512, 512, 4), stride 2, no bias */
     const float* sem_in;             /* quantizer.semantic.input_proj.weight (256, 512) */
     const float* acq_in;             /* quantizer.acoustic.input_proj.weight (256, 512) */
-    const float* codebook[16];       /* semantic codebook 0, then acoustic 0..14: (2048, 256) */
+    const float* codebook[16];       /* semantic codebook 0, then acoustic 0..14: (2048, 256), 16-byte aligned */
     const float* codebook_norm2[16]; /* squared norm of every code: (2048) */
 } VuibCodecEncWeights;
 

@@ -60,3 +60,18 @@ def test_encode_in_one_pass(frames):
     got, ref = enc(audio.cuda())[0].cpu(), oracle.encode(audio)[0]
     # a code may differ where two are equally near; what follows from it in its frame then differs too
     assert got.shape == ref.shape and (got != ref).float().mean().item() <= 0.02
+
+
+def test_encoder_takes_weights_at_any_float():
+    """A state dict on the device whose tensors are views one float into their buffers, as slices of one flat parameter buffer are."""
+    from oracle.codec_enc_oracle import test_audio
+    from vui_b200.codec_encoder import QwenCodecEncoder, random_encoder_state
+
+    sd = random_encoder_state(0)
+    odd = {}
+    for name, t in sd.items():
+        flat = torch.empty(t.numel() + 1, device="cuda")
+        odd[name] = flat[1:].view(t.shape).copy_(t)
+        assert odd[name].data_ptr() % 16 == 4
+    audio = test_audio(17 * 1920, seed=17).cuda()
+    assert torch.equal(QwenCodecEncoder(odd)(audio), QwenCodecEncoder(sd)(audio))

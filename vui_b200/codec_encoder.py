@@ -154,7 +154,7 @@ class QwenCodecEncoder:
         w.acq_in = P(sd["quantizer.acoustic.input_proj.weight"].reshape(256, 512))
         books = [sd["quantizer.semantic.codebooks.0.embed"]] + [sd[f"quantizer.acoustic.codebooks.{i}.embed"] for i in range(15)]
         for i, e in enumerate(books):
-            w.codebook[i] = P(e)
+            w.codebook[i] = P(e if e.data_ptr() % 16 == 0 else e.clone())   # read 16 bytes at a time
             w.codebook_norm2[i] = P((e * e).sum(dim=1))
         return w
 

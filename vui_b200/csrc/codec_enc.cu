@@ -14,11 +14,12 @@ using namespace vuie;
 
 struct VuibCodecEnc {
     VuibCodecEncConfig cfg;
-    VuibCodecEncWeights w;
+    VuibCodecEncWeights w;    // as bound
+    VuibCodecEncWeights u;    // with the vectors that are read 16 bytes at a time as the workspace holds them
     unsigned char* ws;
     bool have_ws, have_w, packed;
     int64_t launches;
-    size_t off_flag, off_y, off_p[3], off_x, off_q, off_xp, off_gp, off_d, off_dp, off_h, off_rope, off_w, total;
+    size_t off_flag, off_y, off_p[3], off_x, off_q, off_xp, off_gp, off_d, off_dp, off_h, off_rope, off_v, off_w, total;
     struct Packed { vuis::SgWeight c3[4], c1[4], down[4], out, wqkv[VUIB_CODEC_LAYERS], wo[VUIB_CODEC_LAYERS], fc1[VUIB_CODEC_LAYERS],
                     fc2[VUIB_CODEC_LAYERS], half, books; } pk;
     int last_frames, num_sms;
@@ -81,6 +82,26 @@ int32_t pack_weights(VuibCodecEnc* c) {
     c->pk.books = put(w.sem_in, vuis::SW_ROWS, 0, 0, 256, D, 1, 32);   // the acoustic projection's columns follow the semantic one's
     put(w.acq_in, vuis::SW_ROWS, 0, 0, 256, D, 1, 32);
     c->pk.books.N = 512;
+    // Biases and layer scales are read 16 bytes at a time and a caller's need not lie that way: they are copied behind one another
+    // (their lengths are multiples of 32).
+    c->u = w;
+    float* vec = reinterpret_cast<float*>(c->ws + c->off_v);
+    auto copy = [&](const float*& p, int n) {
+        if (e == cudaSuccess) e = cudaMemcpyAsync(vec, p, (size_t)n * 4, cudaMemcpyDeviceToDevice, 0);
+        p = vec;
+        vec += n;
+    };
+    C = g.base_dim;
+    for (int i = 0; i < 4; ++i, C *= 2) {
+        copy(c->u.res[i].c3.b, C / 2);
+        copy(c->u.res[i].c1.b, C);
+        copy(c->u.down[i].b, 2 * C);
+    }
+    copy(c->u.conv_out.b, D);
+    for (int l = 0; l < g.n_layers; ++l) {
+        copy(c->u.layer[l].attn_scale, D);
+        copy(c->u.layer[l].mlp_scale, D);
+    }
     CK(e);
     const int T25 = g.max_samples / 960;
     vuis::k_srope<<<(T25 * 32 + 255) / 256, 256>>>(w.rope_cos, w.rope_sin, reinterpret_cast<float*>(c->ws + c->off_rope), T25);
@@ -109,7 +130,7 @@ extern "C" int32_t vuib_codec_enc_create(const VuibCodecEncConfig* cfg, VuibCode
     auto take = [&](size_t bytes) { size_t o = cur; cur += (bytes + 1023) & ~size_t(1023); return o; };
     const int T0 = g.max_samples, T25 = T0 / 960, T12 = T0 / 1920, D = g.d_model;
     c->off_flag = take(256);
-    size_t y = 0, p[3] = {0, 0, 0}, w = 0;
+    size_t y = 0, p[3] = {0, 0, 0}, w = 0, v = 0;
     auto most = [](size_t& v, size_t n) { if (n > v) v = n; };
     int C = g.base_dim, T = T0;
     for (int i = 0; i < 4; ++i) {   // a stage: input and its ELU, the residual block's inner half, the strided convolution's input
@@ -118,9 +139,11 @@ extern "C" int32_t vuib_codec_enc_create(const VuibCodecEncConfig* cfg, VuibCode
         most(p[1], vuis::sg_plane_bytes(C / 2, T, PAD));
         most(p[2], vuis::sg_plane_bytes(C * g.ratios[i], T / g.ratios[i], PAD));
         w += vuis::sg_weight_bytes(C / 2, C, 3) + vuis::sg_weight_bytes(C, C / 2, 1) + vuis::sg_weight_bytes(2 * C, 2 * C * g.ratios[i], 1);
+        v += C / 2 + C + 2 * C;
         T /= g.ratios[i];
         C *= 2;
     }
+    v += D + (size_t)g.n_layers * 2 * D;
     most(p[0], vuis::sg_plane_bytes(C, T, PAD));
     w += vuis::sg_weight_bytes(D, C, 3) + (size_t)g.n_layers * vuis::sg_weight_bytes(4 * D + 2 * g.mlp_dim, D, 1) +
          vuis::sg_weight_bytes(D, 2 * D, 2) + vuis::sg_weight_bytes(512, D, 1);
@@ -134,6 +157,7 @@ extern "C" int32_t vuib_codec_enc_create(const VuibCodecEncConfig* cfg, VuibCode
     c->off_dp = take(vuis::sg_plane_bytes(D, T12, PAD));
     c->off_h = take((size_t)512 * T12 * 4);
     c->off_rope = take((size_t)64 * T25 * 4);
+    c->off_v = take(v * 4);
     c->off_w = take(w);
     c->total = cur;
     *out = c;
@@ -177,6 +201,8 @@ extern "C" int32_t vuib_codec_enc_bind_weights(VuibCodecEnc* c, const VuibCodecE
     const void* const* p = reinterpret_cast<const void* const*>(&tmp);
     for (size_t i = 0; i < sizeof(tmp) / sizeof(void*); ++i)
         if (!p[i]) return fail(c, VUIB_ERR_NULL, "encoder weight pointer #%zu is NULL", i);
+    for (int i = 0; i < 16; ++i)
+        if ((uintptr_t)w->codebook[i] & 15) return fail(c, VUIB_ERR_WORKSPACE, "codebook %d is not 16-byte aligned", i);
     c->w = *w;
     c->have_w = true;
     return pack_weights(c);
@@ -209,7 +235,7 @@ extern "C" int32_t vuib_codec_enc_encode(VuibCodecEnc* c, const float* audio_dev
         return fail(c, VUIB_ERR_RANGE, "n_samples = %d: need a multiple of 1920 up to %d", n_samples, c->cfg.max_samples);
     if (n_q < 1 || n_q > 16) return fail(c, VUIB_ERR_RANGE, "n_q = %d outside [1, 16]", n_q);
     const VuibCodecEncConfig& g = c->cfg;
-    const VuibCodecEncWeights& w = c->w;
+    const VuibCodecEncWeights& w = c->u;
     if (c->num_sms == 0) {
         int dev = 0;
         CK(cudaGetDevice(&dev));
