@@ -16,6 +16,9 @@
  *    synchronises the device unless a function says so.
  *  - every kernel is launched on the cudaStream_t the caller passes (as void*),
  *    so the calls can be captured into a CUDA graph and replayed once per frame.
+ *  - the *_bind_weights calls (and a *_bind_workspace after them) lay some weights out a second time in the
+ *    workspace, on the legacy default stream, and wait for that: weights and workspace must be ready by then, outside
+ *    any capture, and weights changed later need another bind call.
  *  - a handle is not thread-safe; use one host thread per engine.
  *  - matrices are bf16, row-major (out_features, in_features), as torch stores
  *    nn.Linear.weight.  Codes are int64.  KV layout is the reference's

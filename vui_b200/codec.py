@@ -156,6 +156,7 @@ class QwenCodecDecoder:
         self._ws = torch.zeros(n.value, dtype=torch.uint8, device=self.device)
         self._check(self._lib.vuib_codec_bind_workspace(self._h, self._ws.data_ptr(), n.value))
         self._w = self._pack(sd)
+        torch.cuda.current_stream(self.device).synchronize()   # binding packs the weights on the default stream
         self._check(self._lib.vuib_codec_bind_weights(self._h, C.byref(self._w)))
         self._codes_in = torch.zeros(N_CODEBOOKS, dtype=torch.int64, device=self.device)
         self._audio = torch.zeros(DOWNSAMPLE_RATE, dtype=torch.float32, device=self.device)

@@ -108,6 +108,7 @@ class QwenCodecEncoder:
         self._ws = torch.zeros(n.value, dtype=torch.uint8, device=self.device)
         self._check(self._lib.vuib_codec_enc_bind_workspace(self._h, self._ws.data_ptr(), n.value))
         self._w = self._pack(sd)
+        torch.cuda.current_stream(self.device).synchronize()   # binding packs the weights on the default stream
         self._check(self._lib.vuib_codec_enc_bind_weights(self._h, C.byref(self._w)))
 
     @classmethod

@@ -286,6 +286,7 @@ class Engine:
             w.rq_attn_norm[i], w.rq_wqkv[i] = P(p + "attn_norm.weight"), P(p + "Wqkv.weight")
             w.rq_out_proj[i], w.rq_mlp_norm[i] = P(p + "out_proj.weight"), P(p + "mlp_norm.weight")
             w.rq_w1[i], w.rq_w3[i], w.rq_w2[i] = P(p + "w1.weight"), P(p + "w3.weight"), P(p + "w2.weight")
+        torch.cuda.current_stream(dev).synchronize()   # binding lays the depth weights out on the default stream
         self._ck(self._lib.vuib_bind_weights(self._handle, C.byref(w)))
         karr = (C.c_void_p * s.n_layers)(*[self._kv[i, 0].data_ptr() for i in range(s.n_layers)])
         varr = (C.c_void_p * s.n_layers)(*[self._kv[i, 1].data_ptr() for i in range(s.n_layers)])
