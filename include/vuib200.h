@@ -483,6 +483,9 @@ int32_t vuib_codec_enc_bind_weights(VuibCodecEnc* c, const VuibCodecEncWeights* 
  * int64[n_q][n_samples / 1920] (n_q <= 16).  Stateless: every call encodes from zero left padding. */
 int32_t vuib_codec_enc_encode(VuibCodecEnc* c, const float* audio_dev, int32_t n_samples, int32_t n_q,
                               int64_t* codes_out_dev, void* stream);
+/* Reads and clears the encoder's device flag: a wait inside a kernel that ran out (its codes are then not to be used).
+ * Synchronises `stream`. */
+int32_t vuib_codec_enc_check_flag(VuibCodecEnc* c, void* stream);
 /* Latents before quantisation of the last call, (512, n_samples / 1920) floats, for parity tests.  Synchronous. */
 int32_t vuib_codec_enc_read_latent(VuibCodecEnc* c, float* out_host, int32_t n, void* stream);
 int64_t vuib_codec_enc_launch_count(VuibCodecEnc* c);

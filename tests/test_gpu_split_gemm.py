@@ -75,3 +75,18 @@ def test_encoder_takes_weights_at_any_float():
         assert odd[name].data_ptr() % 16 == 4
     audio = test_audio(17 * 1920, seed=17).cuda()
     assert torch.equal(QwenCodecEncoder(odd)(audio), QwenCodecEncoder(sd)(audio))
+
+
+def test_encoder_reports_a_wait_that_ran_out():
+    """The flag that the kernels set, set by hand in the workspace: reported once, and the encoder goes on."""
+    from vui_b200 import _lib
+    from vui_b200.codec_encoder import QwenCodecEncoder
+
+    enc = QwenCodecEncoder.random_init(0)
+    enc.check_device()
+    enc._ws[:4].view(torch.int32).fill_(4)
+    with pytest.raises(_lib.VuibError, match="wait") as err:
+        enc.check_device()
+    assert err.value.code == -7
+    enc(torch.zeros(1, 1, 1920, device="cuda"))
+    enc.check_device()

@@ -198,6 +198,7 @@ SYMBOLS = {
     "vuib_codec_enc_bind_workspace": (C.c_int32, [_P, _P, C.c_size_t]),
     "vuib_codec_enc_bind_weights": (C.c_int32, [_P, C.POINTER(VuibCodecEncWeights)]),
     "vuib_codec_enc_encode": (C.c_int32, [_P, _P, C.c_int32, C.c_int32, _P, _P]),
+    "vuib_codec_enc_check_flag": (C.c_int32, [_P, _P]),
     "vuib_codec_enc_read_latent": (C.c_int32, [_P, C.POINTER(C.c_float), C.c_int32, _P]),
     "vuib_codec_enc_launch_count": (C.c_int64, [_P]),
 }

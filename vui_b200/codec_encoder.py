@@ -181,6 +181,10 @@ class QwenCodecEncoder:
                                                          torch.cuda.current_stream(self.device).cuda_stream))
         return torch.tensor(list(buf), dtype=torch.float32).view(512, n_frames)
 
+    def check_device(self) -> None:
+        """Raise if a wait inside a kernel ran out."""
+        self._check(self._lib.vuib_codec_enc_check_flag(self._h, torch.cuda.current_stream(self.device).cuda_stream))
+
     def launch_count(self) -> int:
         return int(self._lib.vuib_codec_enc_launch_count(self._h))
 

@@ -451,9 +451,10 @@ extern "C" int32_t vuib_codec_check_flag(VuibCodec* c, void* stream) {
     if (!flag) return VUIB_OK;
     CK(cudaMemsetAsync(wsp<int>(c, c->lay.ctr) + CTR_FLAG, 0, sizeof(int), s));
     CK(cudaStreamSynchronize(s));
-    return fail(c, VUIB_ERR_DEVICE_FLAG, "codec device flag 0x%x:%s%s", flag,
+    return fail(c, VUIB_ERR_DEVICE_FLAG, "codec device flag 0x%x:%s%s%s", flag,
                 (flag & FLAG_BAD_CODE) ? " code outside [0, 2048)" : "",
-                (flag & FLAG_POS_OVERFLOW) ? " transformer position beyond max_seq" : "");
+                (flag & FLAG_POS_OVERFLOW) ? " transformer position beyond max_seq" : "",
+                (flag & FLAG_WAIT) ? " a bounded wait inside a kernel ran out" : "");
 }
 
 extern "C" int32_t vuib_codec_read_tap(VuibCodec* c, int32_t which, float* out_host, int32_t n, void* stream) {

@@ -102,6 +102,7 @@ int32_t pack_weights(VuibCodecEnc* c) {
         copy(c->u.layer[l].attn_scale, D);
         copy(c->u.layer[l].mlp_scale, D);
     }
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->ws + c->off_flag, 0, 256, 0);
     CK(e);
     const int T25 = g.max_samples / 960;
     vuis::k_srope<<<(T25 * 32 + 255) / 256, 256>>>(w.rope_cos, w.rope_sin, reinterpret_cast<float*>(c->ws + c->off_rope), T25);
@@ -206,6 +207,19 @@ extern "C" int32_t vuib_codec_enc_bind_weights(VuibCodecEnc* c, const VuibCodecE
     c->w = *w;
     c->have_w = true;
     return pack_weights(c);
+}
+
+extern "C" int32_t vuib_codec_enc_check_flag(VuibCodecEnc* c, void* stream) {
+    if (!c) return VUIB_ERR_NULL;
+    if (!c->packed) return fail(c, VUIB_ERR_UNBOUND, "encoder workspace or weights not bound");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    int flag = 0;
+    CK(cudaMemcpyAsync(&flag, c->ws + c->off_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    if (!flag) return VUIB_OK;
+    CK(cudaMemsetAsync(c->ws + c->off_flag, 0, sizeof(int), s));
+    CK(cudaStreamSynchronize(s));
+    return fail(c, VUIB_ERR_DEVICE_FLAG, "encoder device flag 0x%x: a bounded wait inside a kernel ran out", flag);
 }
 
 extern "C" int32_t vuib_codec_enc_read_latent(VuibCodecEnc* c, float* out_host, int32_t n, void* stream) {
