@@ -403,6 +403,9 @@ typedef struct VuibCodecWeights {
 typedef struct VuibCodec VuibCodec;
 
 int32_t vuib_codec_create(const VuibCodecConfig* cfg, VuibCodec** out);
+/* The same without vuib_codec_decode: whole inputs need the matrices a second time and room for max_seq frames of activations
+ * (1.5 GB of workspace at 250 frames), streaming alone 39 MB. */
+int32_t vuib_codec_create_streaming(const VuibCodecConfig* cfg, VuibCodec** out);
 int32_t vuib_codec_destroy(VuibCodec* c);
 int32_t vuib_codec_last_error(VuibCodec* c, char* buf, size_t n);
 /* Streaming state (convolution histories, transposed-convolution partials, transformer KV and position)

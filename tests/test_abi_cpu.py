@@ -68,3 +68,18 @@ def test_struct_sizes_match_header():
     assert C.sizeof(_lib.VuibConfig) == 18 * 4
     assert C.sizeof(_lib.VuibSampling) == 32
     assert C.sizeof(_lib.VuibWeights) == 8 * (5 + 7 * 64 + 5 + 7 * 64)
+
+
+def test_a_streaming_codec_asks_for_streaming_memory_only():
+    lib = _lib.load()
+    cfg = _lib.VuibCodecConfig(16, 2048, 256, 512, 1024, 512, 8, 16, 1024, 250, 1536, (C.c_int32 * 4)(8, 5, 4, 3), 1e-6)
+    sizes = []
+    for create in (lib.vuib_codec_create, lib.vuib_codec_create_streaming):
+        h, n = C.c_void_p(), C.c_size_t()
+        assert create(None, C.byref(h)) == -1 and create(C.byref(cfg), None) == -1
+        assert create(C.byref(cfg), C.byref(h)) == 0
+        assert lib.vuib_codec_workspace_bytes(h, C.byref(n)) == 0
+        sizes.append(n.value)
+        assert lib.vuib_codec_decode(h, C.c_void_p(256), 16, 1, C.c_void_p(256), None) == -4   # nothing bound
+        lib.vuib_codec_destroy(h)
+    assert sizes[1] < 40e6 and 1.4e9 < sizes[0] < 1.6e9

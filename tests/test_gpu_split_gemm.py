@@ -90,3 +90,18 @@ def test_encoder_reports_a_wait_that_ran_out():
     assert err.value.code == -7
     enc(torch.zeros(1, 1, 1920, device="cuda"))
     enc.check_device()
+
+
+def test_a_streaming_decoder_takes_whole_inputs_frame_by_frame(codec):
+    from vui_b200.codec import QwenCodecDecoder, random_codec_state
+
+    whole, _ = codec
+    dec = QwenCodecDecoder(random_codec_state(0), whole_inputs=False)
+    assert dec._ws.numel() < 40e6 < whole._ws.numel()
+    codes = torch.randint(0, 2048, (1, 16, 5), generator=torch.Generator().manual_seed(5)).cuda()
+    for _ in range(2):   # each call starts from zero padding
+        got = dec(codes)
+        assert dec.position() == 5 and (got - whole(codes)).abs().max().item() <= 5e-5 * got.abs().max().item()
+    with dec.streaming(1):
+        assert torch.equal(torch.cat([dec(codes[:, :, t:t + 1]) for t in range(5)], dim=-1), got)
+    dec.check_device()

@@ -185,6 +185,7 @@ SYMBOLS = {
     "vuib_codec_bind_workspace": (C.c_int32, [_P, _P, C.c_size_t]),
     "vuib_codec_bind_weights": (C.c_int32, [_P, C.POINTER(VuibCodecWeights)]),
     "vuib_codec_reset": (C.c_int32, [_P, _P]),
+    "vuib_codec_create_streaming": (C.c_int32, [C.POINTER(VuibCodecConfig), C.POINTER(_P)]),
     "vuib_codec_decode_frame": (C.c_int32, [_P, _P, C.c_int32, _P, _P]),
     "vuib_codec_decode": (C.c_int32, [_P, _P, C.c_int32, C.c_int32, _P, _P]),
     "vuib_codec_position": (C.c_int32, [_P, C.POINTER(C.c_int32), _P]),

@@ -130,13 +130,17 @@ def random_codec_state(seed: int = 0) -> "OrderedDict[str, Tensor]":
 
 
 class QwenCodecDecoder:
-    """Codes (1, n_q, T) int64 -> audio (1, 1, T * 1920) fp32 in [-1, 1]."""
+    """Codes (1, n_q, T) int64 -> audio (1, 1, T * 1920) fp32 in [-1, 1].
 
-    def __init__(self, state_dict: dict, device="cuda", max_seq: int = 250):
+    Decoding whole inputs in one pass takes 1.4 GB more of workspace than streaming does (39 MB); with ``whole_inputs=False`` that
+    memory is not taken and they go through frame by frame."""
+
+    def __init__(self, state_dict: dict, device="cuda", max_seq: int = 250, whole_inputs: bool = True):
         if not torch.cuda.is_available():
             raise RuntimeError("vui_b200.codec needs a CUDA device: there is no CPU path")
         self.device = torch.device(device)
         self.max_seq = int(max_seq)
+        self.whole_inputs = bool(whole_inputs)
         self._lib = _lib.load()
         shapes = codec_param_shapes()
         missing = [k for k in shapes if k not in state_dict]
@@ -150,7 +154,8 @@ class QwenCodecDecoder:
         cfg = _lib.VuibCodecConfig(16, 2048, 256, 512, LATENT, D_MODEL, N_LAYERS, N_HEADS, MLP, self.max_seq, DEC_DIM,
                                    (C.c_int32 * 4)(*RATES), 1e-6)
         self._h = C.c_void_p()
-        self._check(self._lib.vuib_codec_create(C.byref(cfg), C.byref(self._h)))
+        create = self._lib.vuib_codec_create if self.whole_inputs else self._lib.vuib_codec_create_streaming
+        self._check(create(C.byref(cfg), C.byref(self._h)))
         n = C.c_size_t()
         self._check(self._lib.vuib_codec_workspace_bytes(self._h, C.byref(n)))
         self._ws = torch.zeros(n.value, dtype=torch.uint8, device=self.device)
@@ -345,7 +350,7 @@ class QwenCodecDecoder:
         codes = codes.to(self.device, torch.int64)
         if not self._streaming:   # an offline forward starts from zero padding (qwen_codec.py:92-102)
             start = 0
-            if T == 1:
+            if T == 1 or not self.whole_inputs:
                 self.reset_streaming()
         else:
             start = self.position() if T > 1 else None
@@ -353,7 +358,7 @@ class QwenCodecDecoder:
             raise ValueError(f"{start} + {T} frames exceed the codec transformer's {self.max_seq} positions; "
                              "decode in windows (CodecCtx does)")
         audio = torch.empty(1, 1, T * DOWNSAMPLE_RATE, dtype=torch.float32, device=self.device)
-        if not self._streaming and T > 1:
+        if not self._streaming and T > 1 and self.whole_inputs:
             codes = codes.contiguous()
             self._check(self._lib.vuib_codec_decode(self._h, codes.data_ptr(), n_q, T, audio.data_ptr(), self._stream()))
             return audio

@@ -51,6 +51,7 @@ struct VuibCodec {
     Layout lay;
     unsigned char* ws;
     bool have_ws, have_w;
+    bool stream_only;             // no room for whole inputs (vuib_codec_create_streaming)
     int64_t launches;
     int max_part_floats;
     BatchWeights bw;
@@ -190,6 +191,8 @@ void make_layout(VuibCodec* c) {
     L.r1 = take(cur, ymax * 4);
     c->max_part_floats = part_max;
     L.part = take(cur, (size_t)part_max * 4);
+    L.total = cur;
+    if (c->stream_only) return;
 
     using vuis::sg_plane_bytes;
     const int N = g.max_seq, D = g.d_model, HH = g.n_heads * HD;
@@ -306,7 +309,7 @@ cudaError_t tile(VuibCodec* c, int KW, const float* wt, const float* bias, TileI
 // one tile per SM for 125 frames.
 int32_t pack_batch(VuibCodec* c) {
     c->packed = false;
-    if (!c->have_ws || !c->have_w) return VUIB_OK;
+    if (!c->have_ws || !c->have_w || c->stream_only) return VUIB_OK;
     using namespace vuis;
     const VuibCodecConfig& g = c->cfg;
     const VuibCodecWeights& w = c->w;
@@ -357,7 +360,7 @@ int32_t pack_batch(VuibCodec* c) {
 }  // namespace
 
 // ---------------------------------------------------------------------------------------------
-extern "C" int32_t vuib_codec_create(const VuibCodecConfig* cfg, VuibCodec** out) {
+static int32_t create(const VuibCodecConfig* cfg, bool stream_only, VuibCodec** out) {
     if (!cfg || !out) return VUIB_ERR_NULL;
     *out = nullptr;
     const VuibCodecConfig& g = *cfg;
@@ -371,10 +374,14 @@ extern "C" int32_t vuib_codec_create(const VuibCodecConfig* cfg, VuibCodec** out
     if (!c) return VUIB_ERR_NULL;
     memset(c, 0, sizeof(*c));
     c->cfg = g;
+    c->stream_only = stream_only;
     make_layout(c);
     *out = c;
     return VUIB_OK;
 }
+
+extern "C" int32_t vuib_codec_create(const VuibCodecConfig* cfg, VuibCodec** out) { return create(cfg, false, out); }
+extern "C" int32_t vuib_codec_create_streaming(const VuibCodecConfig* cfg, VuibCodec** out) { return create(cfg, true, out); }
 
 extern "C" int32_t vuib_codec_destroy(VuibCodec* c) {
     delete c;
@@ -630,6 +637,7 @@ extern "C" int32_t vuib_codec_decode_frame(VuibCodec* c, const int64_t* codes_de
 extern "C" int32_t vuib_codec_decode(VuibCodec* c, const int64_t* codes_dev, int32_t n_q, int32_t n_frames, float* audio_out_dev,
                                      void* stream) {
     if (!c || !codes_dev || !audio_out_dev) return VUIB_ERR_NULL;
+    if (c->stream_only) return fail(c, VUIB_ERR_UNBOUND, "created by vuib_codec_create_streaming: no room for whole inputs");
     if (!c->packed) return fail(c, VUIB_ERR_UNBOUND, "codec workspace or weights not bound");
     if (n_q < 1 || n_q > c->cfg.n_q) return fail(c, VUIB_ERR_RANGE, "n_q = %d outside [1, %d]", n_q, c->cfg.n_q);
     if (n_frames < 1 || n_frames > c->cfg.max_seq) return fail(c, VUIB_ERR_RANGE, "n_frames = %d outside [1, %d]", n_frames, c->cfg.max_seq);
