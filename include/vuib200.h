@@ -293,10 +293,11 @@ int32_t vuib_reset_state(VuibEngine* e, void* stream);
  * stamps of the last such launch to out_host.  Synchronous. */
 int32_t vuib_read_trace(VuibEngine* e, uint64_t* out_host, int32_t n_stamps);
 
-/* Every wait inside a kernel (the tile counter on which the K-splits of a tensor-core GEMM meet, its
- * mbarrier pipeline) gives up after a bounded number of polls, records the device flag and lets the
- * kernel finish; this sets that bound (default 2^22 polls, at least 16).  A frame that reported the
- * flag is followed by vuib_reset_state before the handle is used again. */
+/* Every wait inside a kernel (mbarrier pipelines, the mailboxes in which the K-splits of a tensor-core GEMM
+ * meet, the exchanges of the cluster kernels) gives up after a bounded number of polls, records the device
+ * flag and lets the kernel finish; this sets that bound (default 2^22 polls; at least 16, 2^18 for the cluster
+ * kernels, at most 2^26).  A frame that reported the flag is followed by vuib_reset_state before the handle is
+ * used again. */
 int32_t vuib_set_wait_limit(VuibEngine* e, uint32_t polls);
 
 /* Test hook for the bound above: the next tensor-core GEMM whose tiles are shared by a cluster waits for

@@ -40,3 +40,15 @@ def test_no_store_to_a_peer_before_the_cluster_has_met(file, name, body):
     first, met = REMOTE.search(body), WAIT.search(body)
     assert met and met.start() < first.start(), f"{file}: {name} stores to a peer before it has waited for the cluster"
     assert ARRIVE.search(body).start() < met.start()
+
+
+def test_a_wait_is_not_given_up_while_peers_are_sending():
+    """The host lets no cluster kernel wait for less than 2^18 polls, and no bound overflow when a kernel multiplies it."""
+    src = open(os.path.join(CSRC, "vuib200.cu")).read()
+    for args in ("aa", "ma", "a"):
+        for m in re.finditer(rf"\b{args}\.spin_limit = ([^;]+);", src):
+            assert m.group(1) == "cluster_limit(e)"
+    assert re.search(r"cluster_limit\(const VuibEngine\* e\) \{ return e->spin_limit > 1u << 18 \? e->spin_limit : 1u << 18; \}", src)
+    assert "e->spin_limit = polls < 1u << 26 ? polls : 1u << 26;" in src
+    factors = [int(f) for name in sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) for f in re.findall(r"\b(\d+)u? \* a\.spin_limit", open(name).read())]
+    assert factors and max(factors) * 2 ** 26 < 2 ** 32

@@ -735,3 +735,26 @@ def test_a_withheld_arrival_does_not_outlive_a_reset(nano_model):
     again = eng.prefill_ids(row, _ids(8, 4))
     eng.check_device()
     assert torch.equal(again, clean)
+
+
+@pytest.mark.parametrize("polls", [16, 2 ** 32 - 1])
+def test_wait_limit_at_its_ends(nano_model, polls):
+    """One to four streams run in kernels whose CTAs send to one another: the shortest limit does not make them give up, and the
+    longest does not overflow into a short one, in them or in the GEMMs of more streams."""
+    from vui_b200 import Engine
+
+    for n in (1, 3) if polls == 16 else (1, 3, 6):
+        eng = Engine(model=nano_model, max_rows=n, max_seq=64)
+        rows = [eng.new_row() for _ in range(n)]
+        out = []
+        for limit in (1 << 22, polls):
+            if limit != 16:   # GEMMs, in a prefill or of five streams and more, do take so short a limit
+                eng._ck(eng._lib.vuib_set_wait_limit(eng._handle, limit))
+            for r in rows:
+                eng._rewind_row(r, 0)
+            h = torch.stack([eng.prefill_ids(r, _ids(5 + i, i)) for i, r in enumerate(rows)])
+            eng._ck(eng._lib.vuib_set_wait_limit(eng._handle, limit))
+            eng._graphs = {}
+            out.append(eng.generate_frames(rows, h, 3, greedy=True))
+            eng.check_device()
+        assert torch.equal(out[0], out[1])

@@ -148,6 +148,11 @@ struct DtWait {
         if (limit > 1) atomicOr(flag, FLAG_COPY_TIMEOUT);
         limit = 1;
     }
+    // A CTA that gave up a wait must not retire with copies or pushes on their way to its shared memory; the launch takes 2 ms at most.
+    __device__ __forceinline__ void linger() const {
+        if (limit == 1)
+            for (int i = 0; i < 1000; ++i) __nanosleep(10000);
+    }
 };
 
 __device__ __forceinline__ void dt_push_b32(uint32_t dst, uint32_t bar, uint32_t v) {
@@ -340,6 +345,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
                     stages(a.layers + (size_t)(l * DT_CL + c) * a.slots_per_layer * DT_SLOT, a.slots_per_layer / 2);
                 if (pos >= 1) stages(a.head + (size_t)((pos - 1) * DT_CL + c) * DT_HEAD_SLOTS * DT_SLOT, DT_HEAD_SLOTS / 2);
             }
+            w.linger();
         }
         __syncwarp();
         cluster_wait();
@@ -440,6 +446,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
                     umma_commit(&sm.d_head[t]);
                 }
             }
+            w.linger();
         }
         __syncwarp();
         cluster_wait();
@@ -455,6 +462,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
             const bf16* src = r == 2 * DT_LAYERS ? a.final_norm : r & 1 ? a.mlp_norm[l] : a.attn_norm[l];
             *reinterpret_cast<uint4*>(&sm.norm_w[r][(i % (DT_D / 8)) * 8]) = __ldg(reinterpret_cast<const uint4*>(src) + i % (DT_D / 8));
         }
+        if (tid < RMAX) sm.codes[tid] = 0;   // an index also where the wait for the codes runs out
         if (tid < mine) sm.keys[tid] = sample_key(a.sa, b0 + c + tid * DT_CL, true);   // read behind many barriers
         const int quarter = warp & 3, half = warp >> 2;
         const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
@@ -685,6 +693,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
             }
             fb_stamp(dbg, 13);
         }
+        w.linger();
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

@@ -266,6 +266,10 @@ static cudaError_t launch_gemv_k(VuibEngine* e, const Stage& st, const Epi& ep, 
             return fail(e, VUIB_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(_err));  \
     } while (0)
 
+// Bound of the waits in kernels whose CTAs push to one another: never so short that a CTA gives up, and retires, while what its peers
+// send is on its way.  They start together and are microseconds apart; 2^18 polls take 3 ms or more.
+static unsigned cluster_limit(const VuibEngine* e) { return e->spin_limit > 1u << 18 ? e->spin_limit : 1u << 18; }
+
 static bool k_supported(int K) {
     return K == 512 || K == 1024 || K == 1408 || K == 1536 || K == 3072;
 }
@@ -885,7 +889,7 @@ static int32_t run_layers_fused(VuibEngine* e, int M, cudaStream_t s, Residual* 
         aa.Hq = c.n_heads;
         aa.Hkv = c.n_kv_heads;
         aa.flag = wsp<int32_t>(e, L.flag);
-        aa.spin_limit = e->spin_limit;
+        aa.spin_limit = cluster_limit(e);
         // no L2 hint for the MLP block's matrices: that kernel is resident two launches ahead and copies them itself,
         // and 19 MB of hints during this block delayed its own loads (0.799 -> 0.788 ms per frame without them)
         aa.next = prefetch_of(nullptr, 0);
@@ -920,7 +924,7 @@ static int32_t run_layers_fused(VuibEngine* e, int M, cudaStream_t s, Residual* 
         ma.kvcols = kvc;
         ma.n_slots = c.n_slots;
         ma.flag = wsp<int32_t>(e, L.flag);
-        ma.spin_limit = e->spin_limit;
+        ma.spin_limit = cluster_limit(e);
         ma.next = li + 1 < c.n_layers ? prefetch_of(e->w.wqkv[li + 1], qkv_bytes, e->w.out_proj[li + 1], wo_bytes)
                                       : prefetch_of(after, after_bytes);
         if (env_off("VUIB_TRACE") && (li == 5 || li == 6)) ma.dbg = wsp<unsigned long long>(e, L.trace) + (li - 5) * 32 + 16;
@@ -985,7 +989,7 @@ static int32_t rq_layers_fused(VuibEngine* e, int B, const bf16* x, int x_stride
         aa.Hq = c.rq_n_heads;
         aa.Hkv = c.rq_n_heads;
         aa.flag = wsp<int32_t>(e, L.flag);
-        aa.spin_limit = e->spin_limit;
+        aa.spin_limit = cluster_limit(e);
         aa.next = prefetch_of(nullptr, 0);   // as in the backbone: the MLP block copies its own matrices early enough
         if (env_off("VUIB_TRACE_DEPTH") && pos == 8 && (li == 1 || li == 2)) aa.dbg = wsp<unsigned long long>(e, L.trace) + (li - 1) * 32;
         aa.rows = B;
@@ -1011,7 +1015,7 @@ static int32_t rq_layers_fused(VuibEngine* e, int B, const bf16* x, int x_stride
         ma.w2 = static_cast<const bf16*>(e->w.rq_w2[li]);
         ma.parts_out = pb;
         ma.flag = wsp<int32_t>(e, L.flag);
-        ma.spin_limit = e->spin_limit;
+        ma.spin_limit = cluster_limit(e);
         ma.next = li + 1 < c.rq_n_layers ? prefetch_of(e->w.rq_wqkv[li + 1], qkv_bytes, e->w.rq_out_proj[li + 1], wo_bytes)
                                          : prefetch_of(after, after_bytes);
         if (env_off("VUIB_TRACE_DEPTH") && pos == 8 && (li == 1 || li == 2)) ma.dbg = wsp<unsigned long long>(e, L.trace) + (li - 1) * 32 + 16;
@@ -1254,7 +1258,7 @@ static int32_t launch_depth_group(VuibEngine* e, int B, const SampleArgs& sa_bas
     a.tap = e->tap_rq;
     a.sa = sa_base;
     a.flag = wsp<int32_t>(e, L.flag);
-    a.spin_limit = e->spin_limit;
+    a.spin_limit = cluster_limit(e);
     a.dbg = env_off("VUIB_TRACE_DEPTH") ? wsp<unsigned long long>(e, L.trace) : nullptr;
     const int groups = (B + r - 1) / r;
     cudaLaunchConfig_t cfg = {};
@@ -1680,7 +1684,7 @@ extern "C" int32_t vuib_read_trace(VuibEngine* e, uint64_t* out_host, int32_t n_
 extern "C" int32_t vuib_set_wait_limit(VuibEngine* e, uint32_t polls) {
     if (!e) return VUIB_ERR_NULL;
     if (polls < 16) return fail(e, VUIB_ERR_RANGE, "wait limit %u below 16 polls", polls);
-    e->spin_limit = polls;
+    e->spin_limit = polls < 1u << 26 ? polls : 1u << 26;   // the kernels multiply it by up to 16
     return VUIB_OK;
 }
 
