@@ -79,3 +79,19 @@ def test_engine_refuses_without_cuda():
 
     with pytest.raises(RuntimeError):
         Engine(model=None)
+
+
+def test_every_change_of_the_lengths_is_announced_to_a_stream_under_way():
+    """Row.stream generates on a stream of the engine's own, which waits for the caller's only when something has changed there."""
+    from types import SimpleNamespace
+
+    from vui_b200.engine import Engine, Row
+
+    eng = SimpleNamespace(_free={0}, _rows={}, max_rows=1, seq_lens=torch.ones(2, dtype=torch.int32), _touched=False, _new_codec_ctx=lambda: None)
+    eng._release_row = lambda row: Engine._release_row(eng, row)
+    row = Engine.new_row(eng)
+    assert isinstance(row, Row) and eng._touched and eng.seq_lens.tolist() == [0, 1]
+    for change in (lambda: Engine._rewind_row(eng, row, 1), lambda: Engine.reset(eng)):
+        eng._touched = False
+        change()
+        assert eng._touched

@@ -504,6 +504,7 @@ class Engine:
         self._free.remove(idx)
         row = Row(self, idx)
         self._rows[idx] = row
+        self._touched = True
         self.seq_lens[idx] = 0
         return row
 
