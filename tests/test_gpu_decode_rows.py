@@ -1,5 +1,6 @@
-"""Decode steps of several streams at the edges of the kernels' row ranges (fused rows up to 4, tensor-core tiles of 16 / 32 / 64,
-clusters of 8 depth streams up to 120) against the register-tile GEMV kernels, on the same caches and input codes."""
+"""Decode steps of one and of several streams at the edges of the kernels' row ranges (one row, fused rows up to 4, tensor-core tiles of
+16 / 32 / 64, clusters of 8 depth streams up to 120) and of their key ranges (64 keys a CTA and 512 a cluster requested in advance,
+splits of 128) against the register-tile GEMV kernels, on the same caches and input codes."""
 import os
 
 import pytest
@@ -8,11 +9,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(scope="module")
-def sure_model(nano_sd):
+def _sure(nano_sd):
     """The seeded weights with every code following from the one before (as in a trained model): no near ties between codes."""
-    from vui_b200 import VuiB200, VuiShape
-
     sd, g = dict(nano_sd), torch.Generator().manual_seed(1)
     code, audio = (sd[n].float() / sd[n].float().std() for n in ("rq_transformer.code_emb.embedding.weight", "audio_emb.embedding.weight"))
     head = torch.empty_like(sd["rq_transformer.head_W"])
@@ -21,15 +19,56 @@ def sure_model(nano_sd):
     sd["rq_transformer.head_W"] = head
     sd["codec_head.weight"] = (audio[torch.randperm(2048, generator=g)] * 0.1).to(head.dtype)
     sd["rq_transformer.code_emb.embedding.weight"], sd["audio_emb.embedding.weight"] = code.to(head.dtype), audio.to(head.dtype)
-    return VuiB200(VuiShape(), sd, device="cuda")
+    return sd
 
 
-@pytest.mark.parametrize("B", [2, 3, 4, 5, 8, 9, 16, 17, 33, 65, 120, 121, 241])
+@pytest.fixture(scope="module")
+def sure_model(nano_sd):
+    from vui_b200 import VuiB200, VuiShape
+
+    return VuiB200(VuiShape(), _sure(nano_sd), device="cuda")
+
+
+@pytest.fixture(scope="module")
+def deep_model(nano_sd):
+    """Five depth layers: more than the one-launch depth loop takes, so that each layer runs as kernels of its own."""
+    from vui_b200 import VuiB200, VuiShape
+
+    sd = _sure(nano_sd)
+    for name in list(sd):
+        if name.startswith("rq_transformer.blocks.0."):
+            sd[name.replace("blocks.0.", "blocks.4.")] = sd[name].flip(0).contiguous()
+    return VuiB200(VuiShape(n_layers=2, rq_n_layers=5), {k: v for k, v in sd.items()}, device="cuda")
+
+
+LENGTHS = [0, 1, 63, 64, 511, 513, 600, 97]
+
+
+@pytest.mark.parametrize("B", [1, 2, 3, 4, 5, 8, 9, 16, 17, 33, 65, 120, 121, 241])
 def test_decode_step_matches_gemv_kernels(sure_model, B):
+    _check_step(sure_model, B, [LENGTHS[i % 8] for i in range(B)], 640)
+
+
+@pytest.mark.parametrize("B,first", [(1, n) for n in range(1, 8)] + [(2, 4), (2, 6), (3, 4), (4, 2), (4, 4)])
+def test_few_streams_at_every_length(sure_model, B, first):
+    _check_step(sure_model, B, [LENGTHS[(first + i) % 8] for i in range(B)], 640)
+
+
+@pytest.mark.parametrize("B", [1, 2, 3, 4, 6, 17])
+def test_long_contexts(sure_model, B):
+    _check_step(sure_model, B, [[2047, 1024, 513, 1537, 2000, 640][i % 6] for i in range(B)], 2048)
+
+
+@pytest.mark.parametrize("B", [5, 16, 33])
+def test_depth_layers_as_kernels_of_their_own(deep_model, B):
+    _check_step(deep_model, B, [LENGTHS[i % 8] for i in range(B)], 640)
+
+
+def _check_step(model, B, lengths, max_seq):
     from vui_b200 import Engine
 
-    eng = Engine(model=sure_model, max_rows=B, max_seq=640)
-    lens = torch.tensor([[0, 1, 63, 64, 511, 513, 600, 97][i % 8] for i in range(B)], dtype=torch.int32)
+    eng = Engine(model=model, max_rows=B, max_seq=max_seq)
+    lens = torch.tensor(lengths, dtype=torch.int32)
     kv = torch.randn(eng._kv[0].shape, device="cuda", dtype=torch.bfloat16, generator=torch.Generator(device="cuda").manual_seed(B)) * 0.5
     codes_in = torch.randint(0, 2048, (B, 16), generator=torch.Generator().manual_seed(B)).cuda()
     eng._apply_cfg(None, greedy=True)

@@ -292,12 +292,12 @@ def test_teacher_forced_32_frames(eng1, oracle_gpu):
 
 def test_batch_invariance_and_ragged(eng8, eng1):
     """Four streams with ragged prompt lengths decoded together give, bit for bit, what each
-    gives alone (every row is computed in the same order whatever the batch; up to 4 rows stay
-    on the GEMV path, more go to the tensor cores, which sum in another order)."""
+    gives alone (every row is computed in the same order whatever the batch; up to 4 rows run
+    in the fused layers' form for several rows, more go to the tensor-core GEMMs, which sum in another order)."""
     lens = [64, 17, 130, 255]
     idss = [_ids(n, 10 + i) for i, n in enumerate(lens)]
-    # a lone row normally takes the two-kernel fused layers, which sum out_proj / w2 in another order:
-    # switch them off here so that one row and four rows run the same kernels
+    # a lone row normally takes kernels of its own, which sum out_proj / w2 in another order: VUIB_NO_FUSED switches
+    # them off, so that one row and four rows run the same kernels
     os.environ["VUIB_NO_FUSED"] = "1"
     eng1._graphs = {}
     try:
@@ -321,19 +321,19 @@ def test_batch_invariance_and_ragged(eng8, eng1):
 
 def test_fused_layers_match_per_phase_kernels(eng1, oracle_fp32):
     """A lone row runs each layer as two cluster kernels (attention block, MLP block; partial sums of
-    out_proj and w2 exchanged as fp32 rows), several rows as five kernels per layer.  Same rounding
-    points, another fp32 summation order: after a prefill + decode steps the residual stream after every
+    out_proj and w2 exchanged as fp32 rows); without them and without the tensor cores it takes five kernels
+    per layer.  Same rounding points, another fp32 summation order: after a prefill + decode steps the residual stream after every
     block, the final hidden, the cb0 and depth logits and the K/V rows written agree closely, both are
     equally close to the fp32 oracle, and the greedy codes agree except at near-ties."""
     eng = eng1
     ids = _ids(200, 77)
     res = {}
     for off in ("1", ""):
-        os.environ["VUIB_NO_FUSED"] = off
         eng._graphs = {}
         eng.reset()
         row = eng.new_row()
-        h = eng.prefill_ids(row, ids)
+        h = eng.prefill_ids(row, ids)   # the same kernels on both sides
+        os.environ["VUIB_NO_FUSED"] = os.environ["VUIB_NO_TC"] = off   # VUIB_NO_FUSED alone: the fused layers' form for several rows
         taps = torch.zeros(24, 1, 1024, device="cuda", dtype=torch.bfloat16)
         rq_tap = torch.zeros(1, 15, 2048, device="cuda", dtype=torch.bfloat16)
         eng._set_taps(taps, rq_tap)
@@ -354,7 +354,7 @@ def test_fused_layers_match_per_phase_kernels(eng1, oracle_fp32):
                         v=torch.stack([eng._kv[li, 1, row.idx, 200:203].clone() for li in (0, 11, 23)]), off=row.offset)
         eng._set_taps(None, None)
         row.close()
-    os.environ["VUIB_NO_FUSED"] = ""
+        os.environ["VUIB_NO_FUSED"] = os.environ["VUIB_NO_TC"] = ""
     eng._graphs = {}
     a, b = res[""], res["1"]  # fused, per-phase
     assert a["off"] == b["off"] == 203 and a["k"].float().abs().max() > 0
@@ -380,10 +380,10 @@ def test_fused_layers_match_per_phase_kernels(eng1, oracle_fp32):
 
 
 def test_tensor_core_path_matches_gemv_path(nano_model, oracle_fp32):
-    """Five rows and more run on the tcgen05 GEMM (TMA-fed, accumulators in tensor memory); up to 4
-    on the register-tile GEMV.  Same rounding points, different fp32 summation order: a 40-token
+    """A prefill, and decode steps of five rows and more, run on the tcgen05 GEMM (TMA-fed, accumulators in tensor
+    memory); with VUIB_NO_TC on the register-tile GEMV.  Same rounding points, different fp32 summation order: a 40-token
     prefill must agree between the two and with the fp32 oracle within the bf16 tolerance, and a
-    16-stream decode step must agree with the same streams decoded one by one."""
+    16-stream decode step must agree with the same streams decoded one by one (in the fused layers)."""
     from vui_b200 import Engine
 
     eng = Engine(model=nano_model, max_rows=16, max_seq=256)
@@ -408,7 +408,7 @@ def test_tensor_core_path_matches_gemv_path(nano_model, oracle_fp32):
     assert _cos(tc, ref) > COS_TOL and _cos(tc, gemv) > COS_TOL
     assert _rel(tc, ref) < REL_TOL_BF16 and _rel(tc, ref) < 1.25 * _rel(gemv, ref) + 2e-3
     assert _rel(tc, gemv) < REL_TOL_BF16
-    # 16 streams in one step (tensor cores) vs each alone (GEMV)
+    # 16 streams in one step (tensor cores) vs each alone (fused layers)
     lens = [20 + 3 * i for i in range(16)]
     eng.reset()
     rows = [eng.new_row() for _ in lens]
@@ -438,7 +438,7 @@ def test_tensor_core_path_matches_gemv_path(nano_model, oracle_fp32):
 
 
 def test_prefill_chunking_equals_single_call(eng8):
-    """A 300-token prompt (cut at max_prefill_rows=256) and token-by-token prefill give the same hidden."""
+    """A 300-token prompt in one call and in pieces of 50 give the same hidden (test_gpu_prefill_cut.py: cut by the engine)."""
     eng = eng8
     ids = _ids(300, 21)
     eng.reset()
@@ -694,8 +694,8 @@ def test_bad_slot_and_position_are_clamped_and_flagged(eng8):
 
 
 def test_bounded_wait_runs_out_and_reports(nano_model):
-    """A wait inside a kernel that cannot complete (one arrival of the tensor-core GEMM's tile counter
-    withheld by a test hook) gives up after the configured number of polls, records the device flag and
+    """A wait inside a kernel that cannot complete (the tensor-core GEMM's mailbox told to expect one value
+    more than is sent to it by a test hook) gives up after the configured number of polls, records the device flag and
     the kernel returns; after vuib_reset_state the same call is bit-identical to a clean run."""
     from vui_b200 import Engine
     from vui_b200._lib import VuibError
