@@ -552,7 +552,8 @@ static int32_t build_dg_stream(VuibEngine* e) {
 static bool prefill_tc_ok(VuibEngine* e) { return e->tc && !env_off("VUIB_NO_TC"); }
 
 static bool tc_ok(VuibEngine* e, int M) {
-    // measured: 8 rows take 3.7 ms/frame on the register-tile GEMV, 16 rows 3.4 ms on the tensor cores
+    // measured at 300 keys: frames of 5 / 8 / 16 rows take 1.56 / 1.65 / 1.71 ms here and 2.99 / 3.49 / 5.95 on the register-tile
+    // GEMVs; 4 rows take 1.01 ms in the fused layers, which are laid out for no more, and 2.42 on the GEMVs
     return M > 4 && e->tc && !env_off("VUIB_NO_TC");
 }
 
@@ -838,8 +839,8 @@ static bool fused_depth_ok(VuibEngine* e) {
     return e->fused_depth == 1;
 }
 
-// Up to four streams take the fused two-kernel layers, one the single-row kernels (switched off for tests: it then runs what
-// several run, bit for bit).  Five streams and more go to the tensor-core GEMMs and k_depth_tc: the fused kernels' columns
+// Up to four streams take the fused two-kernel layers, one the single-row kernels.  For tests VUIB_NO_FUSED has one row run what
+// several run, bit for bit, and with VUIB_NO_TC the per-phase kernels.  Five streams and more go to the tensor-core GEMMs and k_depth_tc: the fused kernels' columns
 // and partial rows are laid out for four.
 static bool one_row(int M) { return M == 1 && !env_off("VUIB_NO_FUSED"); }
 static bool rows_fit(int M) { return one_row(M) || (M <= FR_ROWS && !env_off("VUIB_NO_TC")); }
