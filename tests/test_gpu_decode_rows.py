@@ -64,6 +64,21 @@ def test_depth_layers_as_kernels_of_their_own(deep_model, B):
     _check_step(deep_model, B, [LENGTHS[i % 8] for i in range(B)], 640)
 
 
+@pytest.mark.parametrize("width", [1024, 1536])
+def test_wider_depth_transformers(width):
+    """Widths that the library takes besides the 512 of the one-launch depth loop (VuiShape itself derives no ffn for them)."""
+    from vui_b200 import VuiB200, VuiShape
+    from vui_b200.model import state_dict_shapes
+
+    class Wide(VuiShape):
+        rq_ffn = property(lambda self: 1536)
+
+    shape, g = Wide(n_layers=2, vocab_size=64, rq_d_model=width, rq_n_heads=width // 64), torch.Generator().manual_seed(width)
+    sd = {n: torch.ones(s) if n.endswith("norm.weight") else torch.randn(s, generator=g) * 0.02 for n, s in state_dict_shapes(shape).items()}
+    model = VuiB200(shape, _sure({n: t.to(torch.bfloat16) for n, t in sd.items()}), device="cuda")
+    _check_step(model, 6, LENGTHS[:6], 640)
+
+
 def _check_step(model, B, lengths, max_seq):
     from vui_b200 import Engine
 

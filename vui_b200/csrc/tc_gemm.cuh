@@ -617,11 +617,12 @@ __global__ void __launch_bounds__(128) k_rmsnorm_rows(const bf16* __restrict__ x
 
 // Depth-transformer attention for many rows: one CTA per row, one warp per head
 // (the same arithmetic as StageRqAttn, written to a buffer instead of a GEMV tile).
+template <int K>
 __global__ void __launch_bounds__(256) k_rq_attn_rows(StageRqAttn st, bf16* __restrict__ out) {
     pdl_trigger();
     pdl_wait();
-    // stage<512>() writes row rr of a tile at Xs + rr*K: aim tile row 0 at this row's output
-    st.template stage<512>(out + (size_t)blockIdx.x * 512, blockIdx.x, 1);
+    // stage<K>() writes row rr of a tile at Xs + rr*K: aim tile row 0 at this row's output
+    st.template stage<K>(out + (size_t)blockIdx.x * K, blockIdx.x, 1);
 }
 
 // eos_head for many rows: one warp per row (Linear with bias, model.py:1099).

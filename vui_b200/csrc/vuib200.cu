@@ -727,7 +727,9 @@ static int32_t rq_layers_tc(VuibEngine* e, int M, bf16* x, int rows_per_b, int p
         if ((rc = tc_gemm(e, e->tc->rq_wqkv[li], e->tc->rq_wqkv[li], xn, M, rd, 3 * rd, 0, eq, s))) return rc;
 
         StageRqAttn sa{q, kc, vc, c.rq_n_heads, Q, rows_per_b, pos_base};
-        CK(launch(k_rq_attn_rows, M, 256, 0, s, sa, attn));
+        const auto attend = rd == 512 ? k_rq_attn_rows<512> : rd == 1024 ? k_rq_attn_rows<1024> : rd == 1408 ? k_rq_attn_rows<1408>
+                          : rd == 1536 ? k_rq_attn_rows<1536> : k_rq_attn_rows<3072>;   // the widths of k_supported
+        CK(launch(attend, M, 256, 0, s, sa, attn));
         e->launches++;
 
         TcEpiResidual eo{x, rd, nullptr};
