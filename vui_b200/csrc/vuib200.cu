@@ -642,6 +642,20 @@ static int32_t tc_gemm(VuibEngine* e, const CUtensorMap& a0, const CUtensorMap& 
     return VUIB_OK;
 }
 
+// Few rows: one wave of k_attn_few, whose CTAs are two to an SM.  At 8 / 16 rows of 270 keys 4.8 / 3.8 us of a layer, 7.9 / 8.6 in
+// k_attn_decode; at 64 rows, two waves, no difference (24.5 us alone either way).
+static cudaError_t attn_decode(VuibEngine* e, const AttnArgs& a, int rows, cudaStream_t s) {
+    if (e->num_sms == 0) {
+        int dev = 0;
+        cudaError_t rc = cudaGetDevice(&dev);
+        if (rc == cudaSuccess) rc = cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, dev);
+        if (rc != cudaSuccess) return rc;
+    }
+    if (rows * a.Hkv <= 2 * e->num_sms)
+        return launch(k_attn_few, dim3(a.Hkv, rows, (a.max_seq + AF_SPLIT - 1) / AF_SPLIT), AF_WARPS * 32, 0, s, a);
+    return launch(k_attn_decode, dim3(a.S, a.Hkv, rows), ATT_THREADS, 0, s, a);
+}
+
 static int32_t norm_rows(VuibEngine* e, const bf16* x, const void* w, float eps, bf16* out, int M, int K, int row_mul,
                          int row_add, cudaStream_t s) {
     CK(launch(k_rmsnorm_rows, M, 128, 0, s, x, static_cast<const bf16*>(w), eps, out, K, row_mul, row_add));
@@ -679,8 +693,8 @@ static int32_t run_layers_tc(VuibEngine* e, int M, cudaStream_t s, bool prefill)
         } else {
             AttnArgs aa{q, static_cast<const bf16*>(e->k[li]), static_cast<const bf16*>(e->v[li]),
                         row_slot, row_pos, wsp<float>(e, L.part), wsp<int32_t>(e, L.counters), attn,
-                        c.n_heads, c.n_kv_heads, c.max_seq, e->S, nullptr, c.n_slots, wsp<int32_t>(e, L.flag)};
-            CK(launch(k_attn_decode, dim3(e->S, c.n_kv_heads, M), ATT_THREADS, 0, s, aa));
+                        c.n_heads, c.n_kv_heads, c.max_seq, e->S, c.n_slots, wsp<int32_t>(e, L.flag), prefill ? 0 : 1};
+            CK(attn_decode(e, aa, M, s));
         }
         e->launches++;
 
@@ -1059,8 +1073,8 @@ static int32_t run_layers(VuibEngine* e, int M, cudaStream_t s, Residual* out, b
 
         AttnArgs aa{q, static_cast<const bf16*>(e->k[li]), static_cast<const bf16*>(e->v[li]),
                     row_slot, row_pos, wsp<float>(e, L.part), wsp<int32_t>(e, L.counters), attn,
-                    c.n_heads, c.n_kv_heads, c.max_seq, e->S, nullptr, c.n_slots, wsp<int32_t>(e, L.flag)};
-        CK(launch(k_attn_decode, dim3(e->S, c.n_kv_heads, M), ATT_THREADS, 0, s, aa));
+                    c.n_heads, c.n_kv_heads, c.max_seq, e->S, c.n_slots, wsp<int32_t>(e, L.flag), 0};
+        CK(attn_decode(e, aa, M, s));
         e->launches++;
         CK(cudaGetLastError());
 
@@ -1517,8 +1531,8 @@ extern "C" int32_t vuib_attention(VuibEngine* e, int32_t layer, int32_t n_rows, 
     AttnArgs aa{static_cast<const bf16*>(q_dev), static_cast<const bf16*>(e->k[layer]),
                 static_cast<const bf16*>(e->v[layer]), row_slot_dev, row_pos_dev,
                 wsp<float>(e, e->lay.part), wsp<int32_t>(e, e->lay.counters), static_cast<bf16*>(out_dev),
-                c.n_heads, c.n_kv_heads, c.max_seq, e->S, nullptr, c.n_slots, wsp<int32_t>(e, e->lay.flag)};
-    CK(launch(k_attn_decode, dim3(e->S, c.n_kv_heads, n_rows), ATT_THREADS, 0, static_cast<cudaStream_t>(stream), aa));
+                c.n_heads, c.n_kv_heads, c.max_seq, e->S, c.n_slots, wsp<int32_t>(e, e->lay.flag), 0};
+    CK(attn_decode(e, aa, n_rows, static_cast<cudaStream_t>(stream)));
     e->launches++;
     CK(cudaGetLastError());
     return VUIB_OK;
@@ -1816,8 +1830,8 @@ extern "C" int32_t vuib_attention_noalloc(int32_t n_heads, int32_t n_kv_heads, i
     AttnArgs aa{static_cast<const bf16*>(q_dev), static_cast<const bf16*>(k_cache_dev),
                 static_cast<const bf16*>(v_cache_dev), row_slot_dev, row_pos_dev,
                 reinterpret_cast<float*>(b), reinterpret_cast<int32_t*>(b + NA_PART_BYTES),
-                static_cast<bf16*>(out_dev), n_heads, n_kv_heads, max_seq, S, nullptr, 0, nullptr};
-    k_attn_decode<<<dim3(S, n_kv_heads, n_rows), ATT_THREADS, 0, s>>>(aa);
+                static_cast<bf16*>(out_dev), n_heads, n_kv_heads, max_seq, S, 0, nullptr, 0};
+    k_attn_few<<<dim3(n_kv_heads, n_rows, (max_seq + AF_SPLIT - 1) / AF_SPLIT), AF_WARPS * 32, 0, s>>>(aa);   // as vuib_attention for so few rows
     rc = cudaGetLastError();
     if (rc != cudaSuccess)
         return na_fail(err, err_len, VUIB_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(rc));
