@@ -1072,7 +1072,15 @@ __device__ __forceinline__ uint32_t att_term(float x, float y, int part) {
 // pieces give A fragments of V transposed (16 dims x 16 keys).  The B operand's eight columns are the two query heads, or the two
 // heads' probabilities as three bf16 terms each (high, middle, low: all 24 bits), columns that would be idle otherwise: the products
 // are exact and the sums fp32.  With many rows, where instructions count, this is no faster than the FMA pipe (256 rows: 69 us, 49).
-constexpr int AF_WARPS = 8, AF_SPLIT = 512;
+// Longer contexts are cut into splits of AF_LONG, two tiles a warp (as splits of 512 they took 1 to 5 us a layer more).
+constexpr int AF_WARPS = 8, AF_SPLIT = 512, AF_LONG = 256, AF_MAX_SEQ = 1024;
+__host__ __device__ constexpr int af_split(int len) { return len <= AF_SPLIT ? AF_SPLIT : AF_LONG; }
+// Where it is used.  Frames of 5 / 8 / 16 rows at 300 keys take 1.52 / 1.59 / 1.65 ms with it and 1.63 / 1.67 / 1.70 with k_attn_decode, at
+// 800 keys 1.61 / 1.66 / 1.82 and 1.65 / 1.70 / 1.80; at 2000 keys 1.76 / 1.88 / 2.21 and 1.67 / 1.82 / 2.03, so that caches for more than
+// 1024 positions keep to the other; at 32 rows (two CTAs an SM) 1.85 and 1.84 at 300 keys, 2.19 and 2.03 at 800.
+inline bool af_use(int rows, int Hkv, int max_seq, int num_sms) { return rows * Hkv <= num_sms && max_seq <= AF_MAX_SEQ; }
+__host__ __device__ constexpr int af_splits(int len) { return (len + af_split(len) - 1) / af_split(len); }
+
 
 static __global__ void __launch_bounds__(AF_WARPS * 32, 2) k_attn_few(AttnArgs a) {
     constexpr int STEP = 16 * AF_WARPS;   // a pass of the CTA's warps
@@ -1082,7 +1090,12 @@ static __global__ void __launch_bounds__(AF_WARPS * 32, 2) k_attn_few(AttnArgs a
     pdl_trigger();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int sp = blockIdx.z, kvh = blockIdx.x, r = blockIdx.y, G = a.Hq / a.Hkv;
-    const int pos_stride = a.Hkv * HD, t_begin = sp * AF_SPLIT;
+    const int pos_stride = a.Hkv * HD;
+    int t_begin = 0, t_len = 0;   // the split's first key and most keys: by the row's length
+    auto cut = [&](int p) {
+        t_len = af_split(p + 1);
+        t_begin = sp * t_len;
+    };
     const bf16 *kb, *vb;   // of the split's first key
     auto clamp_slot = [&](int s) { return s < 0 ? 0 : a.n_slots > 0 && s >= a.n_slots ? a.n_slots - 1 : s; };
     auto clamp_pos = [&](int p) { return p < 0 ? 0 : p >= a.max_seq ? a.max_seq - 1 : p; };
@@ -1122,8 +1135,9 @@ static __global__ void __launch_bounds__(AF_WARPS * 32, 2) k_attn_few(AttnArgs a
     if (a.early) {   // with the row's place as memory has it now; it is read again behind the wait
         slot = clamp_slot(__ldcg(a.row_slot + r));
         pos = clamp_pos(__ldcg(a.row_pos + r));
+        cut(pos);
         aim(slot);
-        start(min(pos - t_begin, AF_SPLIT));   // the row's own key is still to come
+        start(min(pos - t_begin, t_len));   // the row's own key is still to come
     }
     pdl_wait();
     uint32_t qf[4][2];   // columns of the B operand: head g & 1
@@ -1144,8 +1158,10 @@ static __global__ void __launch_bounds__(AF_WARPS * 32, 2) k_attn_few(AttnArgs a
             if (s != s_now) atomicOr(a.flag, FLAG_BAD_SLOT);
             if (p != p_now) atomicOr(a.flag, FLAG_BAD_POS);
         }
+        const bool same = a.early && s == slot && p == pos;
+        cut(p);
         if (t_begin > p) return;
-        if (a.early && s == slot && p == pos) {   // only the row's own key is still missing
+        if (same) {   // only the row's own key is still missing
             const int own = p - t_begin;
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -1165,10 +1181,10 @@ static __global__ void __launch_bounds__(AF_WARPS * 32, 2) k_attn_few(AttnArgs a
             slot = s;
             pos = p;
             aim(slot);
-            start(min(p + 1 - t_begin, AF_SPLIT));
+            start(min(p + 1 - t_begin, t_len));
         }
     }
-    const int len = pos + 1, nsplit = (len + AF_SPLIT - 1) / AF_SPLIT, n = min(len - t_begin, AF_SPLIT);
+    const int len = pos + 1, nsplit = af_splits(len), n = min(len - t_begin, t_len);
     float m = NEG_BIG, l = 0.f, o[4][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;

@@ -642,8 +642,6 @@ static int32_t tc_gemm(VuibEngine* e, const CUtensorMap& a0, const CUtensorMap& 
     return VUIB_OK;
 }
 
-// Few rows: one wave of k_attn_few, whose CTAs are two to an SM.  At 8 / 16 rows of 270 keys 4.8 / 3.8 us of a layer, 7.9 / 8.6 in
-// k_attn_decode; at 64 rows, two waves, no difference (24.5 us alone either way).
 static cudaError_t attn_decode(VuibEngine* e, const AttnArgs& a, int rows, cudaStream_t s) {
     if (e->num_sms == 0) {
         int dev = 0;
@@ -651,8 +649,8 @@ static cudaError_t attn_decode(VuibEngine* e, const AttnArgs& a, int rows, cudaS
         if (rc == cudaSuccess) rc = cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, dev);
         if (rc != cudaSuccess) return rc;
     }
-    if (rows * a.Hkv <= 2 * e->num_sms)
-        return launch(k_attn_few, dim3(a.Hkv, rows, (a.max_seq + AF_SPLIT - 1) / AF_SPLIT), AF_WARPS * 32, 0, s, a);
+    if (af_use(rows, a.Hkv, a.max_seq, e->num_sms))
+        return launch(k_attn_few, dim3(a.Hkv, rows, af_splits(a.max_seq)), AF_WARPS * 32, 0, s, a);
     return launch(k_attn_decode, dim3(a.S, a.Hkv, rows), ATT_THREADS, 0, s, a);
 }
 
@@ -1831,7 +1829,14 @@ extern "C" int32_t vuib_attention_noalloc(int32_t n_heads, int32_t n_kv_heads, i
                 static_cast<const bf16*>(v_cache_dev), row_slot_dev, row_pos_dev,
                 reinterpret_cast<float*>(b), reinterpret_cast<int32_t*>(b + NA_PART_BYTES),
                 static_cast<bf16*>(out_dev), n_heads, n_kv_heads, max_seq, S, 0, nullptr, 0};
-    k_attn_few<<<dim3(n_kv_heads, n_rows, (max_seq + AF_SPLIT - 1) / AF_SPLIT), AF_WARPS * 32, 0, s>>>(aa);   // as vuib_attention for so few rows
+    int sms = 0;
+    rc = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (rc != cudaSuccess)
+        return na_fail(err, err_len, VUIB_ERR_CUDA, "cudaDeviceGetAttribute: %s", cudaGetErrorString(rc));
+    if (af_use(n_rows, n_kv_heads, max_seq, sms))
+        k_attn_few<<<dim3(n_kv_heads, n_rows, af_splits(max_seq)), AF_WARPS * 32, 0, s>>>(aa);
+    else
+        k_attn_decode<<<dim3(S, n_kv_heads, n_rows), ATT_THREADS, 0, s>>>(aa);
     rc = cudaGetLastError();
     if (rc != cudaSuccess)
         return na_fail(err, err_len, VUIB_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(rc));
