@@ -688,7 +688,7 @@ extern "C" int32_t vuib_codec_decode(VuibCodec* c, const int64_t* codes_dev, int
         CK(sg_run(x, k_snorm<SN_RMS, 512>, dim3((T + 7) / 8), dim3(256), 0, na));
         CK(sg_launch(x, B.qkv[l], pn, T, 1, out(nullptr, 3 * HH, none, qkv, T)));
         SAttnArgs aa = {qkv, T, wsp<float>(c, L.b_rope), g.max_seq, pa, T, g.n_heads};
-        CK(sg_run(x, k_sattn, dim3((T + SAT_Q - 1) / SAT_Q, g.n_heads), dim3(256), 0, aa));
+        CK(sat_launch(x, aa));
         SgOut o = out(nullptr, D, none, xr, T);
         o.res = xr;
         o.scale = lw.attn_scale;

@@ -310,7 +310,7 @@ extern "C" int32_t vuib_codec_enc_encode(VuibCodecEnc* c, const float* audio_dev
         o.y_rows = T;
         CK(sg_launch(x, c->pk.wqkv[l], xp, T, 1, o));
         SAttnArgs aa = {q, T, f32(c->off_rope), g.max_samples / 960, xp, T, H};
-        CK(sg_run(x, k_sattn, dim3((T + SAT_Q - 1) / SAT_Q, H), dim3(256), 0, aa));
+        CK(sat_launch(x, aa));
         o = out(nullptr, D, SA_NONE, none, 1);
         o.res = o.y = xr;
         o.scale = lw.attn_scale;
@@ -343,7 +343,19 @@ extern "C" int32_t vuib_codec_enc_encode(VuibCodecEnc* c, const float* audio_dev
     r.codes = reinterpret_cast<long long*>(codes_out_dev);
     r.T = T;
     r.n_q = n_q;
+    r.flag = x.flag;
     for (int i = 0; i < n_q; ++i) { r.table[i] = w.codebook[i]; r.norm2[i] = w.codebook_norm2[i]; }
-    CK(sg_run(x, k_ervq, dim3((T + RV_F - 1) / RV_F * RV_CL, 2), dim3(32 * RV_WARPS), 0, r));
+    {
+        static thread_local int ready = -1;   // device whose copy of the kernel this thread has opted into its shared memory
+        int dev = 0;
+        CK(cudaGetDevice(&dev));
+        if (ready != dev) {
+            CK(cudaFuncSetAttribute(k_ervq<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, RV_SMEM));
+            CK(cudaFuncSetAttribute(k_ervq<9>, cudaFuncAttributeMaxDynamicSharedMemorySize, RV_SMEM));
+        }
+        ready = dev;
+    }
+    const int F = T > 8 * 15 && T <= 9 * 15 ? 9 : 8;   // frames of a cluster, see k_ervq
+    CK(sg_run(x, F == 9 ? k_ervq<9> : k_ervq<8>, dim3((T + F - 1) / F * RV_CL, 2), dim3(32 * RV_WARPS), RV_SMEM, r));
     return VUIB_OK;
 }

@@ -654,6 +654,25 @@ cudaError_t sg_run(const SgCtx& x, void (*kern)(KArgs...), dim3 grid, dim3 block
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+template <class... KArgs, class... Args>
+cudaError_t sg_run_cluster(const SgCtx& x, void (*kern)(KArgs...), int cluster, dim3 grid, dim3 block, size_t smem, const Args&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = x.s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = x.pdl ? 2 : 1;
+    ++*x.launches;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
 template <int NT, int TAPS>
 cudaError_t sg_launch_nt(const SgCtx& x, SgArgs a) {
     const int tiles = a.m_tiles * a.n_tiles;
@@ -677,21 +696,7 @@ cudaError_t sg_launch_nt(const SgCtx& x, SgArgs a) {
     }
     if (e != cudaSuccess) return e;
     if (a.splits == 1) return sg_run(x, k_sg<NT, TAPS>, dim3(grid), dim3(SG_THREADS), SG_SMEM, a);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(SG_THREADS);
-    cfg.dynamicSmemBytes = SG_SMEM;
-    cfg.stream = x.s;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = a.splits;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = x.pdl ? 2 : 1;
-    ++*x.launches;
-    return cudaLaunchKernelEx(&cfg, k_sg<NT, TAPS>, a);
+    return sg_run_cluster(x, k_sg<NT, TAPS>, a.splits, dim3(grid), dim3(SG_THREADS), SG_SMEM, a);
 }
 
 // D = X (*) W over M rows.  out.up / out.Cout describe the columns; N = W.N must be a multiple of W.NT.

@@ -98,6 +98,7 @@ struct SAttnArgs {
     int rope_rows;
     SgPlanes o;            // H * 64 channels
     int T, H;
+    int cluster;           // sat_cluster(T)
 };
 
 // Rotate-half tables [T][64] (both halves alike) in the order in which k_sattn's lanes, one a row, read them.
@@ -113,13 +114,24 @@ constexpr int SAT_Q = 16, SAT_K = 64;   // queries of a CTA, keys of a step
 
 // Causal attention with rotate-half RoPE, head size 64: a CTA takes 16 queries of a head (two a warp), keys arrive 64 at a time in
 // shared memory (RoPE applied on the way), softmax with a running maximum per step.  T <= 500, so there are a few hundred CTAs of
-// one to eight steps, each a chain of loads, two products and a softmax: the next step's keys are requested before this one's
-// products, and every load is a row per lane (with the tables as [T][64] a lane fetched a line of its own: 35 us a layer of 250 rows).
-static __global__ void __launch_bounds__(256) k_sattn(SAttnArgs a) {
+// work that is a chain of loads, two products and a softmax, 5 us a step: the steps of 16 queries are shared out over a cluster of up
+// to SAT_CL CTAs, whose states the first one merges in their order (rows 250 / 160 / 96: 13.7 / 9.4 / 8.9 us a layer, 24.7 / 16.9 / 10.6
+// with all steps in one CTA).
+// Every load is a row per lane (with the tables as [T][64] a lane fetched a line of its own: 35 us a layer of 250 rows); a CTA's next
+// step, where it has one, is requested before this one's products.
+constexpr int SAT_CL = 4;
+inline int sat_cluster(int T) { return T <= SAT_K ? 1 : T <= 2 * SAT_K ? 2 : SAT_CL; }
+
+template <int PER_SM>
+static __global__ void __launch_bounds__(256, PER_SM) k_sattn(SAttnArgs a) {
     __shared__ __align__(16) float qs[SAT_Q][64], ks[SAT_K][65], vs[SAT_K][64], ps[8][2][SAT_K];
+    static_assert(sizeof(vs) >= SAT_Q * 66 * sizeof(float), "a CTA's o[64], m, l of every query take the place of its values");
+    const int CL = a.cluster, rank = blockIdx.x % CL;
     sg_pdl_wait();
     sg_pdl_launch();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, q0 = blockIdx.x * SAT_Q, T = a.T;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, q0 = blockIdx.x / CL * SAT_Q, T = a.T;
+    const int last = min(q0 + SAT_Q, T), own = rank * SAT_K, step = CL * SAT_K;   // keys [0, last); this CTA's first, and from step to step
+    if (own >= last) return;   // nothing to add, and nobody looks here
     const float* xq = a.qkv + (long long)h * 16 * a.rows * 4;
     const float* xk = xq + (long long)a.H * 16 * a.rows * 4;
     const float* xv = xk + (long long)a.H * 16 * a.rows * 4;
@@ -140,7 +152,7 @@ static __global__ void __launch_bounds__(256) k_sattn(SAttnArgs a) {
             f[it][4] = table(i, t, 0); f[it][5] = table(i, t, 4);
         }
     };
-    fetch(0);
+    fetch(own);
     if (tid < 128) {
         const int q = tid & 15, i = tid >> 4, t = min(q0 + q, T - 1);
         float lo[4], hi[4];
@@ -151,8 +163,7 @@ static __global__ void __launch_bounds__(256) k_sattn(SAttnArgs a) {
     float m[2], l[2], o[2][2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) { m[i] = -INFINITY; l[i] = 0.f; o[i][0] = o[i][1] = 0.f; }
-    const int last = min(q0 + SAT_Q, T);   // keys [0, last)
-    for (int k0 = 0; k0 < last; k0 += SAT_K) {
+    for (int k0 = own; k0 < last; k0 += step) {
         __syncthreads();
 #pragma unroll
         for (int it = 0; it < 2; ++it) {
@@ -165,7 +176,7 @@ static __global__ void __launch_bounds__(256) k_sattn(SAttnArgs a) {
             *reinterpret_cast<float4*>(&vs[k][d + 32]) = f[it][3];
         }
         __syncthreads();
-        if (k0 + SAT_K < last) fetch(k0 + SAT_K);
+        if (k0 + step < last) fetch(k0 + step);
         float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
 #pragma unroll 4
         for (int d = 0; d < 64; d += 4) {
@@ -189,8 +200,10 @@ static __global__ void __launch_bounds__(256) k_sattn(SAttnArgs a) {
             float mx = fmaxf(s[i][0], s[i][1]);
 #pragma unroll
             for (int w = 16; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
-            const float mn = fmaxf(m[i], mx);          // key 0 is in the first step, so mn is finite from there on
-            const float corr = expf(m[i] - mn), p0 = expf(s[i][0] - mn), p1 = expf(s[i][1] - mn);
+            const float mn = fmaxf(m[i], mx);
+            // a query before all keys of the step (not of the first CTA's first one) has no state yet
+            const float ref = mn == -INFINITY ? 0.f : mn;
+            const float corr = expf(m[i] - ref), p0 = expf(s[i][0] - ref), p1 = expf(s[i][1] - ref);
             ps[warp][i][lane] = p0;
             ps[warp][i][lane + 32] = p1;
             float sum = p0 + p1;
@@ -219,6 +232,48 @@ static __global__ void __launch_bounds__(256) k_sattn(SAttnArgs a) {
             }
         }
     }
+    if (CL > 1) {
+        float* const mine = &vs[0][0];
+        if (rank > 0) {
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                float* p = mine + (warp * 2 + i) * 66;
+                p[lane] = o[i][0];
+                p[lane + 32] = o[i][1];
+                if (lane == 0) { p[64] = m[i]; p[65] = l[i]; }
+            }
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (rank == 0) {
+            float v[SAT_CL - 1][2][4];   // all requested before the first is used
+#pragma unroll
+            for (int r = 1; r < SAT_CL; ++r)
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    if (r < CL && r * SAT_K < last) {
+                        uint32_t src;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(src) : "r"(sg_smem(mine + (warp * 2 + i) * 66)), "r"(r));
+                        asm volatile("ld.shared::cluster.f32 %0, [%4];\n\tld.shared::cluster.f32 %1, [%4 + 128];\n\tld.shared::cluster.f32 %2, [%5 + 256];\n\t"
+                                     "ld.shared::cluster.f32 %3, [%5 + 260];"
+                                     : "=&f"(v[r - 1][i][0]), "=&f"(v[r - 1][i][1]), "=&f"(v[r - 1][i][2]), "=&f"(v[r - 1][i][3])
+                                     : "r"(src + lane * 4), "r"(src) : "memory");
+                    }
+#pragma unroll
+            for (int r = 1; r < SAT_CL; ++r)
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    if (r < CL && r * SAT_K < last) {   // key 0 is in this CTA, so m is finite
+                        const float mn = fmaxf(m[i], v[r - 1][i][2]), c0 = expf(m[i] - mn), c1 = expf(v[r - 1][i][2] - mn);
+                        l[i] = l[i] * c0 + v[r - 1][i][3] * c1;
+                        o[i][0] = o[i][0] * c0 + v[r - 1][i][0] * c1;
+                        o[i][1] = o[i][1] * c0 + v[r - 1][i][1] * c1;
+                        m[i] = mn;
+                    }
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // read before its CTA retires
+        if (rank > 0) return;
+    }
     // through shared memory to eight-channel chunks (a warp's rows of qs are its own)
     __syncwarp();
 #pragma unroll
@@ -234,6 +289,20 @@ static __global__ void __launch_bounds__(256) k_sattn(SAttnArgs a) {
         for (int i = 0; i < 8; ++i) v[i] = qs[q][c + i];
         sg_store8(a.o, a.o.pad + q0 + q, h * 64 + c, v);
     }
+}
+
+inline cudaError_t sat_launch(const SgCtx& x, SAttnArgs a) {
+    a.cluster = sat_cluster(a.T);
+    const dim3 grid((a.T + SAT_Q - 1) / SAT_Q * a.cluster, a.H);
+    if (a.cluster == 1) return sg_run(x, k_sattn<2>, grid, dim3(256), 0, a);
+    // CTAs with keys to look at; where two to an SM (128 registers) are a wave and a bit, three (80): 250 rows of eight heads 13.7 us, not
+    // 17.0, but 160 rows 12.7, not 9.4
+    int busy = 0;
+    for (int q0 = 0; q0 < a.T; q0 += SAT_Q) {
+        const int last = q0 + SAT_Q < a.T ? q0 + SAT_Q : a.T, steps = (last + SAT_K - 1) / SAT_K;
+        busy += steps < a.cluster ? steps : a.cluster;
+    }
+    return sg_run_cluster(x, busy * a.H > 2 * x.num_sms ? k_sattn<3> : k_sattn<2>, a.cluster, grid, dim3(256), 0, a);
 }
 
 }  // namespace vuis
