@@ -16,6 +16,7 @@ this library's own kernels); pass it, or any object with ``decode(codes_bqt)`` a
 from __future__ import annotations
 
 import ctypes as C
+import weakref
 from collections import deque
 from collections.abc import Iterator
 from dataclasses import dataclass
@@ -146,7 +147,7 @@ class Row:
 
     @property
     def offset(self) -> int:
-        return int(self._engine.seq_lens[self._idx].item())
+        return self._engine._row_len(self._idx)
 
     def prefill(self, segments, spk_emb=None, segments_2=None, spk_emb_2=None) -> int:
         return self._engine._prefill_row(self, segments, spk_emb, segments_2, spk_emb_2)
@@ -181,6 +182,52 @@ class Row:
 
     def __exit__(self, *exc):
         self.close()
+
+
+class _KnownLengths:
+    """The slots' lengths as far as the host itself wrote them last (resets, rewinds, prefills).  They are known without a device
+    read, which would wait for everything before it: a prompt's host work then runs beside the GPU's on the one before.  Any other
+    write to the tensor moves its version and ends that knowledge, and so does every step that advances lengths (forget)."""
+
+    def __init__(self, seq_lens: Tensor):
+        self.seq_lens, self.version, self.lens = seq_lens, seq_lens._version, {}
+
+    def forget(self) -> None:
+        self.lens.clear()
+        self.version = self.seq_lens._version
+
+    def get(self, slot: int) -> int:
+        if self.seq_lens._version != self.version:
+            self.forget()
+        n = self.lens.get(slot)
+        return int(self.seq_lens[slot].item()) if n is None else n
+
+    def wrote(self, slot: int, n: int, version_before: int) -> None:
+        if version_before != self.version:
+            self.lens.clear()
+        self.lens[slot] = int(n)
+        self.version = self.seq_lens._version
+
+
+def _set_len(engine, slot: int, n: int) -> None:
+    """Writes a slot's length: a fill on the device (an assignment copies a scalar from the host, 10 us more)."""
+    known = getattr(engine, "_known", None)
+    before = known and known.seq_lens._version
+    engine.seq_lens[slot].fill_(n)
+    if known:
+        known.wrote(slot, n, before)
+
+
+class _FrameGraph(torch.cuda.CUDAGraph):
+    """A captured frame: its replay advances the engine's lengths."""
+
+    engine = staticmethod(lambda: None)   # a weak reference to it, set by _frame_graph
+
+    def replay(self):
+        engine = self.engine()
+        if engine is not None:
+            engine._lens_moved()
+        super().replay()
 
 
 class Engine:
@@ -255,7 +302,9 @@ class Engine:
         # KV: one allocation, per-layer views in the reference's FlashKVCache layout
         self._kv = torch.zeros(s.n_layers, 2, n_slots, self.max_seq, s.n_kv_heads, s.head_dim,
                                device=dev, dtype=torch.bfloat16)
-        self.seq_lens = torch.zeros(n_slots, device=dev, dtype=torch.int32)
+        with torch.inference_mode(False):   # a tensor that counts its in-place writes, whoever makes them: see _KnownLengths
+            self.seq_lens = torch.zeros(n_slots, device=dev, dtype=torch.int32)
+        self._known = _KnownLengths(self.seq_lens)
         # this engine's caches; model.decoder.flash_kv_caches (where the reference keeps them, model.py:473-495)
         # points at the caches of the engine built last on the model
         self.flash_kv_caches = [
@@ -380,6 +429,7 @@ class Engine:
 
     # ----------------------------------------------------------------- graphs
     def _frame_call(self, B: int) -> None:
+        self._lens_moved()
         P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
         self._ck(self._lib.vuib_decode_frame(
             self._handle, B, P(self._g_slot_idx), P(self._g_seq_inc), P(self._g_codes_in),
@@ -417,7 +467,8 @@ class Engine:
         self._warm.discard(B)
         self._warm_frame(B)
         torch.cuda.synchronize(self.device)
-        g = torch.cuda.CUDAGraph()
+        g = _FrameGraph()
+        g.engine = weakref.ref(self)
         with torch.cuda.graph(g):
             self._frame_call(B)
         torch.cuda.synchronize(self.device)
@@ -463,6 +514,7 @@ class Engine:
                 self._h_codes_in[: h_codes_in.shape[0]].copy_(h_codes_in)
                 h_codes_in = self._h_codes_in
             src = C.c_void_p(h_codes_in.data_ptr())
+        self._lens_moved()
         self._ck(self._lib.vuib_frame_host(self._handle, B, int(with_in), src, C.c_void_p(self._h_codes.data_ptr()),
                                            C.c_void_p(self._h_eos.data_ptr()), self._stream))
         return self._h_codes[:B_active], self._h_eos[:B_active]
@@ -479,6 +531,7 @@ class Engine:
         """Backbone-only step over all max_rows slots (engine.py:850-853)."""
         P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
         self._g_slot_idx.copy_(torch.arange(self.max_rows, device=self.device, dtype=torch.int32))
+        self._lens_moved()
         self._ck(self._lib.vuib_backbone_step(
             self._handle, self.max_rows, P(self._g_slot_idx), None, P(self._g_codes_in),
             P(self._g_hidden_out), P(self._g_cb0_out), P(self._g_eos_out), self._stream))
@@ -520,9 +573,15 @@ class Engine:
         self._touched = True
         self.seq_lens.zero_()
 
+    def _row_len(self, slot: int) -> int:
+        return self._known.get(slot)
+
+    def _lens_moved(self) -> None:
+        self._known.forget()
+
     def _rewind_row(self, row: Row, offset: int) -> int:
         self._touched = True
-        self.seq_lens[row.idx] = offset
+        _set_len(self, row.idx, offset)
         return offset
 
     def set_conditioning(self, *, sq_scores=None, wps_score: float = 0.0) -> None:
@@ -587,7 +646,7 @@ class Engine:
         flush()
         if len(ends) == 1:
             for s_, n in ends.items():
-                self.seq_lens[s_] = n
+                _set_len(self, s_, n)
         elif ends:
             at = torch.tensor([list(ends), list(ends.values())], dtype=torch.int32).to(self.device)
             self.seq_lens[at[0].long()] = at[1]
@@ -1009,7 +1068,7 @@ class Engine:
                 ri = pending.popleft()
                 req = requests[ri]
                 slot = min(free_slots - taken)
-                self.seq_lens[slot] = 0
+                _set_len(self, slot, 0)
                 self._rep_reset(slot=slot)
                 row = Row(self, slot)
                 parts = self._prompt_parts(row, req.segments, req.spk_emb, req.segments_2, req.spk_emb_2)
