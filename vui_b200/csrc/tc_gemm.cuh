@@ -25,7 +25,8 @@ constexpr int TC_TILE_N = 128;      // weight rows per CTA
 constexpr int TC_BOX_N = 64;        // rows of a TMA box of weights (PAIRED: 16, w1 and w3 in turn)
 constexpr int TC_KCHUNK = 64;       // bf16 per row per stage = 128 bytes = one swizzle span
 constexpr int TC_MAX_STAGES = 12;     // ring depth is set per launch from the shared memory left
-constexpr int TC_EPI_BYTES_PER_M = 256;  // epilogue staging per activation row (128 bf16)
+constexpr int TC_MAX_M = 128;            // most activation rows of a tile
+constexpr int TC_EPI_BYTES_PER_M = 256, TC_EPI_HEAD = TC_MAX_M * 8;  // epilogue staging: 128 bf16 per activation row behind a number each
 constexpr int FLAG_TC_TIMEOUT = 16;
 constexpr unsigned TC_SPIN_LIMIT = 1u << 22;  // default bound of every wait below, in polls (TcArgs::spin_limit)
 
@@ -121,6 +122,16 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                   "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
 // 32 consecutive accumulator columns of this thread's TMEM lane in one instruction.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     uint32_t r[32];
@@ -158,10 +169,16 @@ struct TcEpiQkv {      // RoPE on q,k + K/V append (EpiQkv of the GEMV path)
     int m_off;  // row index of m = 0 in the depth-transformer addressing
     static constexpr bool PAIRED = false;
     static constexpr bool STAGED = true;
-    // While the MMAs run: RoPE rows [cos,sin] x 64 of every activation row's position -> es[m][128].
+    // While the MMAs run: the cache row of every activation row, and the RoPE rows [cos,sin] x 64 of its position -> es[m][128].  (With
+    // slot and position read in apply() a round trip to the L2 stood in front of every eight rows' stores.)
     __device__ __forceinline__ void stage(unsigned char* es, int tile, int M, int tid) const {
+        if (tid < M) {
+            const int slot = row_slot ? __ldcg(row_slot + tid) : (tid + m_off) / rows_per_b;
+            const int pos = row_slot ? __ldcg(row_pos + tid) : pos_base + (tid + m_off) % rows_per_b;
+            reinterpret_cast<long long*>(es)[tid] = (long long)slot * max_seq + pos;
+        }
         if (!rope) return;
-        uint4* dst = reinterpret_cast<uint4*>(es);
+        uint4* dst = reinterpret_cast<uint4*>(es + TC_EPI_HEAD);
         for (int i = tid; i < M * 16; i += TC_THREADS) {
             const int m = i >> 4, c = i & 15;
             const int pos = row_slot ? __ldcg(row_pos + m) : pos_base + (m + m_off) % rows_per_b;
@@ -180,32 +197,37 @@ struct TcEpiQkv {      // RoPE on q,k + K/V append (EpiQkv of the GEMV path)
         const bool odd = n & 1;
         const bool do_rope = rope && n < q_cols + kv_cols;
         const bool to_cache = n >= q_cols;
-        int slot[8], pos[8];
-        if (to_cache) {
+        const long long* cache_row = reinterpret_cast<const long long*>(es);
+        const __nv_bfloat162* rs = reinterpret_cast<const __nv_bfloat162*>(es + TC_EPI_HEAD);
+        // exchanges, table reads and arithmetic of the eight rows beside one another, then the stores: row by row, with a branch at the
+        // end of the rows, each waited for the one before (1.5 us more)
+        float t[8], other[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {  // loads first: they do not depend on one another
-                const int m = m0 + j < M ? m0 + j : (M > 0 ? M - 1 : 0);
-                if (row_slot) { slot[j] = __ldcg(row_slot + m); pos[j] = __ldcg(row_pos + m); }
-                else { slot[j] = (m + m_off) / rows_per_b; pos[j] = pos_base + (m + m_off) % rows_per_b; }
-            }
-        }
-        const __nv_bfloat162* rs = reinterpret_cast<const __nv_bfloat162*>(es);
+        for (int j = 0; j < 8; ++j) t[j] = rbf(v[j]);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int m = m0 + j;
-            float t = rbf(v[j]);
-            const float other = __shfl_xor_sync(0xffffffffu, t, 1);
-            if (m >= M) continue;
-            if (do_rope) {
-                const __nv_bfloat162 f = rs[m * 64 + (n & (HD - 1))];
+        for (int j = 0; j < 8; ++j) other[j] = __shfl_xor_sync(0xffffffffu, t[j], 1);
+        if (do_rope) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const __nv_bfloat162 f = rs[min(m0 + j, M - 1) * 64 + (n & (HD - 1))];
                 const float c = __low2float(f), sn = __high2float(f);
-                t = odd ? rbf(rbf(t * c) + rbf(other * sn)) : rbf(rbf(t * c) + rbf((-other) * sn));
+                t[j] = odd ? rbf(rbf(t[j] * c) + rbf(other[j] * sn)) : rbf(rbf(t[j] * c) + rbf((-other[j]) * sn));
             }
-            const bf16 o = f2bf(t);
-            if (!to_cache) q_out[(size_t)m * q_cols + n] = o;
-            else if (n < q_cols + kv_cols) k_cache[((size_t)slot[j] * max_seq + pos[j]) * kv_cols + (n - q_cols)] = o;
-            else v_cache[((size_t)slot[j] * max_seq + pos[j]) * kv_cols + (n - q_cols - kv_cols)] = o;
         }
+        bf16* out;
+        size_t at[8];
+        if (!to_cache) {
+            out = q_out + n;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) at[j] = (size_t)(m0 + j) * q_cols;
+        } else {
+            out = n < q_cols + kv_cols ? k_cache + (n - q_cols) : v_cache + (n - q_cols - kv_cols);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) at[j] = (size_t)cache_row[min(m0 + j, M - 1)] * kv_cols;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (m0 + j < M) out[at[j]] = f2bf(t[j]);
     }
 };
 
@@ -253,14 +275,12 @@ struct TcEpiSwiGLU {    // of every 32 tile rows, 16 are w1 rows and 16 the same
     }
     // a1 = the unit's w1 sums, a3 = its w3 sums, for activation rows m0 .. m0 + 3
     __device__ __forceinline__ void apply_pair(int unit, int m0, int M, const float (&a1)[4], const float (&a3)[4]) const {
+        bf16 o[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int m = m0 + j;
-            if (m >= M) continue;
-            const float a = rbf(a1[j]), g = rbf(a3[j]);
-            const float sl = rbf(silu(a));
-            act[(size_t)m * F + unit] = f2bf(sl * g);
-        }
+        for (int j = 0; j < 4; ++j) o[j] = f2bf(rbf(silu(rbf(a1[j]))) * rbf(a3[j]));
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (m0 + j < M) act[(size_t)(m0 + j) * F + unit] = o[j];
     }
 };
 
@@ -348,22 +368,47 @@ __device__ __forceinline__ void tc_apply(const Epi& ep, int tile, int row, int m
     }
 }
 
-// Eight columns of this thread's row, the sum of Q accumulators MT columns apart, added as a balanced tree.
-template <int Q>
-__device__ __forceinline__ void tc_sum(uint32_t addr, int MT, float (&v)[8]) {
-    if constexpr (Q == 1) tmem_ld8(addr, v);
-    else {
-        float u[8];
+// N columns of this thread's row, the sum of Q accumulators MT columns apart, added as a balanced tree.
+template <int Q, int N>
+__device__ __forceinline__ void tc_sum(uint32_t addr, int MT, float (&v)[N]) {
+    if constexpr (Q == 1) {
+        if constexpr (N == 8) tmem_ld8(addr, v);
+        else tmem_ld16(addr, v);
+    } else {
+        float u[N];
         tc_sum<Q / 2>(addr, MT, v);
         tc_sum<Q / 2>(addr + Q / 2 * MT, MT, u);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] += u[i];
+        for (int i = 0; i < N; ++i) v[i] += u[i];
     }
 }
-__device__ __forceinline__ void tc_sum_of(int segs, uint32_t addr, int MT, float (&v)[8]) {
+template <int N>
+__device__ __forceinline__ void tc_sum_of(int segs, uint32_t addr, int MT, float (&v)[N]) {
     if (segs == 1) tc_sum<1>(addr, MT, v);
     else if (segs == 2) tc_sum<2>(addr, MT, v);
     else tc_sum<4>(addr, MT, v);
+}
+// f(first column, eight sums) for columns [c0, c1) in eights, read from tensor memory one by one or, with BATCH 16, two at a time: the
+// way from there is paid less often, but 16 registers more leave less room beside for the next kernels' CTAs.
+template <int BATCH, class F>
+__device__ __forceinline__ void tc_columns(int segs, uint32_t addr, int MT, int c0, int c1, F f) {
+    auto batch = [&](auto size) {
+        constexpr int N = decltype(size)::value;
+        float v[N];
+        tc_sum_of(segs, addr + c0, MT, v);
+#pragma unroll
+        for (int i = 0; i < N; i += 8) {
+            const float v8[8] = {v[i], v[i + 1], v[i + 2], v[i + 3], v[i + 4], v[i + 5], v[i + 6], v[i + 7]};
+            f(c0 + i, v8);
+        }
+        c0 += N;
+    };
+    if constexpr (BATCH == 16) {
+#pragma unroll 1
+        while (c0 + 16 <= c1) batch(std::integral_constant<int, 16>{});
+    }
+#pragma unroll 1
+    while (c0 < c1) batch(std::integral_constant<int, 8>{});
 }
 // The same over the mailbox's Q sources.
 template <int Q>
@@ -380,7 +425,7 @@ __device__ __forceinline__ void tc_mail_sum(const float* mail, int src_stride, i
     }
 }
 
-template <class Epi>
+template <class Epi, int BATCH>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_gemm_tc(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ CUtensorMap mapA1,
           const __grid_constant__ CUtensorMap mapX, TcArgs a, Epi ep_all) {
@@ -498,30 +543,24 @@ k_gemm_tc(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ CUt
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     __syncthreads();
     tc_stamp(a, 3);
-    // warps w and w + 4 read tile rows 32 (w & 3) ..: every other group of eight activation rows each
-    const int row = (warp & 3) * 32 + lane, half = warp >> 2;
+    // warps w and w + 4 read tile rows 32 (w & 3) ..: a half of the groups of eight activation rows each
+    const int row = (warp & 3) * 32 + lane, split = (groups + 1) / 2 * 8, c0 = warp >> 2 ? split : 0, c1 = warp >> 2 ? groups * 8 : split;
     const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     bool mail_ok = true;
     if (S == 1) {
-        for (int g = half; g < groups; g += 2) {
-            float v[8];
-            tc_sum_of(a.segs, trow + g * 8, a.MT, v);
-            tc_apply(ep, tile, row, g * 8, Mb, v, es);
-        }
+        tc_columns<BATCH>(a.segs, trow, a.MT, c0, c1, [&](int m0, const float (&v)[8]) { tc_apply(ep, tile, row, m0, Mb, v, es); });
     } else {
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every peer has set up its mailbox
         const int owner = row / rpc;
         uint32_t dst, bar;
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(mail + (size_t)rank * a.MT * rpc + row % rpc)), "r"(owner));
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(smem_u32(&bar_mail)), "r"(owner));
-        for (int g = half; g < groups; g += 2) {
-            float v[8];
-            tc_sum_of(a.segs, trow + g * 8, a.MT, v);
+        tc_columns<BATCH>(a.segs, trow, a.MT, c0, c1, [&](int m0, const float (&v)[8]) {
 #pragma unroll
             for (int j = 0; j < 8; ++j)
                 asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];"
-                             ::"r"(dst + (uint32_t)((g * 8 + j) * rpc * 4)), "f"(v[j]), "r"(bar) : "memory");
-        }
+                             ::"r"(dst + (uint32_t)((m0 + j) * rpc * 4)), "f"(v[j]), "r"(bar) : "memory");
+        });
         tc_stamp(a, 4);
         {
             const uint32_t addr = smem_u32(&bar_mail);

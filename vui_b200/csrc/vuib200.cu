@@ -582,6 +582,9 @@ static int32_t tc_gemm(VuibEngine* e, const CUtensorMap& a0, const CUtensorMap& 
     for (int d = 2; d <= parts; d *= 2)
         if (tiles * m_blocks * d <= e->num_sms) splits = d;
     const int max_smem = 200 * 1024;
+    // Tiles of 64 rows and more read their sums in sixteens (240 rows: SUMS), narrower ones in eights: at 16 rows a frame's layers took
+    // 1.3 us more each with the registers that sixteens need.
+    const auto kern = MT >= 64 ? k_gemm_tc<Epi, 16> : k_gemm_tc<Epi, 8>;
     {   // a function attribute belongs to one device's copy of the kernel: set it once per device
         static std::mutex mu;
         static bool attr_set[64];
@@ -589,7 +592,8 @@ static int32_t tc_gemm(VuibEngine* e, const CUtensorMap& a0, const CUtensorMap& 
         CK(cudaGetDevice(&dev));
         std::lock_guard<std::mutex> lock(mu);
         if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-            CK(cudaFuncSetAttribute(k_gemm_tc<Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+            CK(cudaFuncSetAttribute(k_gemm_tc<Epi, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+            CK(cudaFuncSetAttribute(k_gemm_tc<Epi, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
             if (dev >= 0 && dev < 64) attr_set[dev] = true;
         }
     }
@@ -609,7 +613,7 @@ static int32_t tc_gemm(VuibEngine* e, const CUtensorMap& a0, const CUtensorMap& 
     if (ta.withhold) e->withhold = false;
     const int min_chunks = chunks / splits;  // the shortest split
     const size_t stage_bytes = TC_TILE_N * TC_KCHUNK * 2 + (size_t)MT * TC_KCHUNK * 2;
-    const size_t tail = (splits > 1 ? (size_t)TC_TILE_N * MT * 4 : 0) + (Epi::STAGED ? (size_t)MT * TC_EPI_BYTES_PER_M : 0) + 1024;
+    const size_t tail = (splits > 1 ? (size_t)TC_TILE_N * MT * 4 : 0) + (Epi::STAGED ? (size_t)MT * TC_EPI_BYTES_PER_M + TC_EPI_HEAD : 0) + 1024;
     // room for the next kernel's CTA beside this one where that still leaves three stages
     int stages = (int)((112 * 1024 - tail) / stage_bytes);
     if (tail + 3 * stage_bytes > 112 * 1024) stages = (int)((max_smem - tail) / stage_bytes);
@@ -636,8 +640,8 @@ static int32_t tc_gemm(VuibEngine* e, const CUtensorMap& a0, const CUtensorMap& 
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    prefer_max_smem(reinterpret_cast<const void*>(k_gemm_tc<Epi>));
-    CK(cudaLaunchKernelEx(&cfg, k_gemm_tc<Epi>, a0, a1, mx, ta, ep));
+    prefer_max_smem(reinterpret_cast<const void*>(kern));
+    CK(cudaLaunchKernelEx(&cfg, kern, a0, a1, mx, ta, ep));
     e->launches++;
     return VUIB_OK;
 }
