@@ -179,6 +179,7 @@ struct TcEpiQkv {      // RoPE on q,k + K/V append (EpiQkv of the GEMV path)
         }
         if (!rope) return;
         uint4* dst = reinterpret_cast<uint4*>(es + TC_EPI_HEAD);
+#pragma unroll 4
         for (int i = tid; i < M * 16; i += TC_THREADS) {
             const int m = i >> 4, c = i & 15;
             const int pos = row_slot ? __ldcg(row_pos + m) : pos_base + (m + m_off) % rows_per_b;
@@ -199,35 +200,26 @@ struct TcEpiQkv {      // RoPE on q,k + K/V append (EpiQkv of the GEMV path)
         const bool to_cache = n >= q_cols;
         const long long* cache_row = reinterpret_cast<const long long*>(es);
         const __nv_bfloat162* rs = reinterpret_cast<const __nv_bfloat162*>(es + TC_EPI_HEAD);
-        // exchanges, table reads and arithmetic of the eight rows beside one another, then the stores: row by row, with a branch at the
-        // end of the rows, each waited for the one before (1.5 us more)
-        float t[8], other[8];
+        bf16* const out = !to_cache ? q_out + n : n < q_cols + kv_cols ? k_cache + (n - q_cols) : v_cache + (n - q_cols - kv_cols);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) t[j] = rbf(v[j]);
+        for (int half = 0; half < 8 / 8; ++half) {
+            float t[8], other[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) other[j] = __shfl_xor_sync(0xffffffffu, t[j], 1);
-        if (do_rope) {
+            for (int j = 0; j < 8; ++j) t[j] = rbf(v[half * 8 + j]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) other[j] = __shfl_xor_sync(0xffffffffu, t[j], 1);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const __nv_bfloat162 f = rs[min(m0 + j, M - 1) * 64 + (n & (HD - 1))];
-                const float c = __low2float(f), sn = __high2float(f);
-                t[j] = odd ? rbf(rbf(t[j] * c) + rbf(other[j] * sn)) : rbf(rbf(t[j] * c) + rbf((-other[j]) * sn));
+                const int m = m0 + half * 8 + j, mm = min(m, M - 1);
+                if (do_rope) {
+                    const __nv_bfloat162 f = rs[mm * 64 + (n & (HD - 1))];
+                    const float c = __low2float(f), sn = odd ? __high2float(f) : -__high2float(f);
+                    t[j] = rbf(rbf(t[j] * c) + rbf(other[j] * sn));
+                }
+                const size_t at = to_cache ? (size_t)cache_row[mm] * kv_cols : (size_t)m * q_cols;
+                if (m < M) out[at] = f2bf(t[j]);
             }
         }
-        bf16* out;
-        size_t at[8];
-        if (!to_cache) {
-            out = q_out + n;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) at[j] = (size_t)(m0 + j) * q_cols;
-        } else {
-            out = n < q_cols + kv_cols ? k_cache + (n - q_cols) : v_cache + (n - q_cols - kv_cols);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) at[j] = (size_t)cache_row[min(m0 + j, M - 1)] * kv_cols;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (m0 + j < M) out[at[j]] = f2bf(t[j]);
     }
 };
 
@@ -238,6 +230,7 @@ struct TcEpiResidual {  // x += bf16(acc)
     // While the MMAs run: this tile's slice of the residual stream, x[m][tile*128 .. +128) -> es[m][128].
     __device__ __forceinline__ void stage(unsigned char* es, int tile, int M, int tid) const {
         uint4* dst = reinterpret_cast<uint4*>(es);
+#pragma unroll 4
         for (int i = tid; i < M * 16; i += TC_THREADS) {
             const int m = i >> 4, c = i & 15;
             dst[i] = __ldcg(reinterpret_cast<const uint4*>(x + (size_t)m * N + tile * TC_TILE_N) + c);
@@ -574,6 +567,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ CUt
         }
         tc_stamp(a, 5);
         // thread = (row j of the slice, group of eight activation rows); the functors shuffle, and rpc is 32 or 64: warps stay whole
+#pragma unroll 1
         for (int e = tid; e < rpc * groups; e += TC_THREADS) {
             const int j = e % rpc, g = e / rpc;
             float v[8];

@@ -582,8 +582,8 @@ static int32_t tc_gemm(VuibEngine* e, const CUtensorMap& a0, const CUtensorMap& 
     for (int d = 2; d <= parts; d *= 2)
         if (tiles * m_blocks * d <= e->num_sms) splits = d;
     const int max_smem = 200 * 1024;
-    // Tiles of 64 rows and more read their sums in sixteens (240 rows: SUMS), narrower ones in eights: at 16 rows a frame's layers took
-    // 1.3 us more each with the registers that sixteens need.
+    // Tiles of 64 rows and more read their sums in sixteens (a SwiGLU of 240 rows 4.8 -> 3.8 us behind its MMAs), narrower ones in
+    // eights: at 16 rows a frame's layers took 2.5 us more each with the registers that sixteens need.
     const auto kern = MT >= 64 ? k_gemm_tc<Epi, 16> : k_gemm_tc<Epi, 8>;
     {   // a function attribute belongs to one device's copy of the kernel: set it once per device
         static std::mutex mu;
