@@ -614,9 +614,13 @@ static int32_t tc_gemm(VuibEngine* e, const CUtensorMap& a0, const CUtensorMap& 
     const int min_chunks = chunks / splits;  // the shortest split
     const size_t stage_bytes = TC_TILE_N * TC_KCHUNK * 2 + (size_t)MT * TC_KCHUNK * 2;
     const size_t tail = (splits > 1 ? (size_t)TC_TILE_N * MT * 4 : 0) + (Epi::STAGED ? (size_t)MT * TC_EPI_BYTES_PER_M + TC_EPI_HEAD : 0) + 1024;
-    // room for the next kernel's CTA beside this one where that still leaves three stages
-    int stages = (int)((112 * 1024 - tail) / stage_bytes);
-    if (tail + 3 * stage_bytes > 112 * 1024) stages = (int)((max_smem - tail) / stage_bytes);
+    // Room for the next kernel's CTA beside this one where that still leaves three stages, unless this GEMM leaves a third of the SMs
+    // for it: three stages of 64 rows are a round trip every 3 x 64 of K (w1 / w3 at 37 rows 3.6 us behind the dependency, 2.8 with all
+    // eight chunks in the ring; at 240 rows 5.9 and 4.5).  Narrow tiles have five stages as it is, and what follows them wants the room
+    // (16 streams: 20 frames 30.4 ms, 30.7 with more).
+    const size_t beside = MT >= 64 && splits * tiles * m_blocks * 3 <= e->num_sms * 2 ? max_smem : 112 * 1024;
+    int stages = (int)((beside - tail) / stage_bytes);
+    if (tail + 3 * stage_bytes > beside) stages = (int)((max_smem - tail) / stage_bytes);
     if (stages > TC_MAX_STAGES) stages = TC_MAX_STAGES;
     if (stages > min_chunks) stages = min_chunks;
     ta.stages = stages;
