@@ -34,6 +34,7 @@ constexpr int DT_D = 512;
 constexpr int DT_XS = DT_D + 8;                // padded row stride of the residual rows (elements)
 constexpr int DT_GROUPS = 15;                  // clusters of 8 that can be resident at once with one CTA per SM
 constexpr int DT_HEAD_SLOTS = 16;
+constexpr int DT_QKV_SLOTS = 12;               // a layer's first slots: q | k, v
 
 // Slots of a layer and CTA, in order of use: q | k rows of head c per 64 of K (8); v rows, two K-chunks a slot (4); the head's K-slice
 // of out_proj per 128 output rows (4); w1 / w3 of 64 hidden units per tile and K-chunk (8 n_ub); the CTA's K-slice of w2 per 128
@@ -287,6 +288,9 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
     const int mine = (nv - c + DT_CL - 1) / DT_CL;     // streams this CTA samples (may be 0)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n_pos = a.Qn, n_ub = a.n_ub;             // depth positions 0 .. Qn - 1; position p >= 1 yields codebook p
+    // Position 0 yields no codebook: of its last layer the others need the keys and values alone (12 frames of 256 streams 41.96 -> 41.66
+    // ms; of 16 and 64 streams the same as before).
+    const auto keys_only = [&](int pos, int l) { return pos == 0 && l == a.n_layers - 1; };
     if (tid == 0) {
         for (int i = 0; i < STAGES; ++i) { mbar_init(&sm.full[i], 1); mbar_init(&sm.empty[i], 1); }
         mbar_init(&sm.h_ready, DT_CONSUMERS / 32);
@@ -342,7 +346,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
             };
             for (int pos = 0; pos < n_pos; ++pos) {
                 for (int l = 0; l < a.n_layers; ++l)
-                    stages(a.layers + (size_t)(l * DT_CL + c) * a.slots_per_layer * DT_SLOT, a.slots_per_layer / 2);
+                    stages(a.layers + (size_t)(l * DT_CL + c) * a.slots_per_layer * DT_SLOT, keys_only(pos, l) ? DT_QKV_SLOTS / 2 : a.slots_per_layer / 2);
                 if (pos >= 1) stages(a.head + (size_t)((pos - 1) * DT_CL + c) * DT_HEAD_SLOTS * DT_SLOT, DT_HEAD_SLOTS / 2);
             }
             w.linger();
@@ -389,7 +393,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
                 }
             };
             for (int pos = 0; pos < n_pos; ++pos) {
-                for (int l = 0; l < a.n_layers; ++l, ph_l ^= 1) {
+                for (int l = 0; l < a.n_layers; ++l) {
                     need(&sm.h_ready, ph_h);
                     ph_h ^= 1;
                     tile8(t_qk);
@@ -405,6 +409,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
                         close();
                     }
                     umma_commit(&sm.d_v);
+                    if (keys_only(pos, l)) break;
                     need(&sm.attn_ready, ph_l);
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
@@ -437,6 +442,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
                         }
                         close();
                     }
+                    ph_l ^= 1;
                 }
                 if (pos == 0) continue;
                 need(&sm.h_ready, ph_h);
@@ -466,7 +472,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
         if (tid < mine) sm.keys[tid] = sample_key(a.sa, b0 + c + tid * DT_CL, true);   // read behind many barriers
         const int quarter = warp & 3, half = warp >> 2;
         const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-        unsigned phase = 0, ph_l = 0, ph_pos = 0;
+        unsigned phase = 0, ph_q = 0, ph_l = 0, ph_pos = 0;   // parities of the q/k/v tiles and of a layer's others
         uint32_t peer[DT_CL];   // this CTA's shared memory at every CTA of the cluster
 #pragma unroll
         for (int q = 0; q < DT_CL; ++q) peer[q] = peer_addr(&sm, q);
@@ -515,7 +521,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
                 }
             }
             __syncwarp();
-            for (int l = 0; l < a.n_layers; ++l, ph_l ^= 1) {
+            for (int l = 0; l < a.n_layers; ++l, ph_q ^= 1) {
                 bf16* kcl = a.kc + (size_t)l * a.max_rows * a.Q * DT_D;
                 bf16* vcl = a.vc + (size_t)l * a.max_rows * a.Q * DT_D;
                 unsigned long long* dbg = (pos == 8 && l == 1) ? a.dbg : nullptr;
@@ -524,7 +530,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
                 dt_publish(&sm.h_ready);
                 fb_stamp(dbg, 1);
                 // ---- q and k rows to warps 0-3, v rows to warps 4 and 5
-                dt_wait_tile(w, half ? &sm.d_v : &sm.d_qk, ph_l);
+                dt_wait_tile(w, half ? &sm.d_v : &sm.d_qk, ph_q);
                 if (half == 0 || quarter < 2) {
                     float v[DT_COLS<RMAX>];
                     dt_tile((half ? t_v : t_qk) + lanes, v);
@@ -540,6 +546,16 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
                 }
                 dt_bar();
                 fb_stamp(dbg, 2);
+                auto fetch_next = [&] {   // the next layer's keys and values, or the next position's first layer's
+                    const bool wrap = l == a.n_layers - 1;
+#pragma unroll
+                    for (int i = 0; i < SETS; ++i)
+                        if (warp + 8 * i < nv) fetch(kr[i], vr[i], wrap ? 0 : l + 1, warp + 8 * i, wrap ? pos + 1 : pos);
+                };
+                if (keys_only(pos, l)) {
+                    fetch_next();
+                    continue;
+                }
                 // ---- attention of head c: one warp per stream, keys [0, pos) + the new key
                 auto attend = [&](int n, const uint4 (&k4)[4], const uint4 (&v4)[4]) {
                     // Group g4 of eight lanes has keys g4, g4 + 4, .. and lane s8 of it eight of the 64 dimensions; the new key is every
@@ -597,12 +613,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
                     attend(n, k4, v4);
                 }
                 dt_publish(&sm.attn_ready);
-                {   // the next layer's, or the next position's first layer's
-                    const bool wrap = l == a.n_layers - 1;
-#pragma unroll
-                    for (int i = 0; i < SETS; ++i)
-                        if (warp + 8 * i < nv) fetch(kr[i], vr[i], wrap ? 0 : l + 1, warp + 8 * i, wrap ? pos + 1 : pos);
-                }
+                fetch_next();
                 fb_stamp(dbg, 3);
                 dt_push_partials<N, RMAX>(sm, w, sm.d_out, ph_l, t_out, c, nv);
                 fb_stamp(dbg, 4);
@@ -638,6 +649,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
                 fb_stamp(dbg, 8);
                 dt_residual_exchange<RMAX>(sm, w, c, phase, nv, peer);
                 fb_stamp(dbg, 9);
+                ph_l ^= 1;
             }
             if (pos == 0) continue;
             unsigned long long* dbg = pos == 8 ? a.dbg : nullptr;
