@@ -697,9 +697,11 @@ static int32_t run_layers_tc(VuibEngine* e, int M, cudaStream_t s, bool prefill)
             if (c.n_heads == 2 * c.n_kv_heads) CK(launch(k_prefill_attn<2>, dim3(gx, c.n_kv_heads), 256, 0, s, pa));
             else CK(launch(k_prefill_attn<1>, dim3(gx, c.n_kv_heads), 128, 0, s, pa));
         } else {
+            // A frame's old keys may be asked for before the preceding kernel has ended (AttnArgs::early): they were written a whole pass over
+            // the layers ago, whose GEMMs cannot all be resident (124 CTAs a layer or more, two an SM at most; so not with fewer than four layers).
             AttnArgs aa{q, static_cast<const bf16*>(e->k[li]), static_cast<const bf16*>(e->v[li]),
                         row_slot, row_pos, wsp<float>(e, L.part), wsp<int32_t>(e, L.counters), attn,
-                        c.n_heads, c.n_kv_heads, c.max_seq, e->S, c.n_slots, wsp<int32_t>(e, L.flag), prefill ? 0 : 1};
+                        c.n_heads, c.n_kv_heads, c.max_seq, e->S, c.n_slots, wsp<int32_t>(e, L.flag), !prefill && c.n_layers >= 4};
             CK(attn_decode(e, aa, M, s));
         }
         e->launches++;
