@@ -51,3 +51,77 @@ def test_lengths_are_what_the_device_has(nano_model, rows, mode):
         with pytest.raises(RuntimeError, match="overflows"):
             eng.prefill_ids(rs[-1], ids)
     eng.check_device()
+
+
+def _data(eng, slot, n):
+    eng.seq_lens.data[slot] = n
+
+
+def _dlpack(eng, slot, n):
+    torch.from_dlpack(torch.utils.dlpack.to_dlpack(eng.seq_lens.view(-1)))[slot] = n
+
+
+def _c_abi(eng, slot, n):
+    eng._ck(eng._lib.vuib_set_seq_len(eng._handle, slot, n))
+
+
+def _replayed_write(eng, slot, n):
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        eng.seq_lens[slot].fill_(n)
+    eng.seq_lens[slot] = 3
+    eng._rows[slot].rewind()   # the host's own write is the last that it sees
+    g.replay()
+
+
+def _c_step(eng, slot, n, call=None):
+    """The backbone step of the C ABI on the engine's handle, `n` - 1 -> `n`."""
+    import ctypes as C
+
+    P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    eng._rows[slot]._prompt_offset = n - 1
+    eng._rows[slot].rewind()
+    slots = torch.tensor([slot], dtype=torch.int32, device="cuda")
+    codes = torch.zeros(1, eng.Q, dtype=torch.long, device="cuda")
+    step = lambda: eng._ck(eng._lib.vuib_backbone_step(  # noqa: E731
+        eng._handle, 1, P(slots), None, P(codes), P(eng._g_hidden_out), P(eng._g_cb0_out), P(eng._g_eos_out), eng._stream))
+    if call is None:
+        step()
+    else:
+        call(step)
+    torch.cuda.synchronize()
+
+
+def _replayed_step(eng, slot, n):
+    def call(step):
+        step()   # outside of a capture first: it loads the kernels
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            step()
+        eng._rows[slot].rewind()
+        g.replay()
+
+    _c_step(eng, slot, n, call)
+
+
+@pytest.mark.parametrize("write", [_data, _dlpack, _c_abi, _replayed_write, _c_step, _replayed_step])
+def test_writers_that_the_host_does_not_see(nano_model, write):
+    """Lengths written behind the Engine's back, just after it wrote them itself: the next prefill goes where the device says."""
+    from vui_b200 import Engine
+
+    eng = Engine(model=nano_model, max_rows=3, max_seq=128)
+    rows = [eng.new_row() for _ in range(3)]
+    ids = torch.randint(0, 1000, (9,), generator=torch.Generator().manual_seed(2))
+    row, n = rows[1], 40
+    eng.prefill_ids(row, ids)
+    write(eng, row.idx, n)
+    assert row.offset == n
+    eng._kv.zero_()
+    eng.prefill_ids(row, ids)
+    assert row.offset == n + 9
+    written = eng._kv[-1, 0, row.idx].flatten(1).any(dim=1).nonzero().flatten().tolist()
+    assert written == list(range(n, n + 9))
+    assert row.prefill([]) == n + 9 and row._prompt_offset == n + 9
+    write(eng, row.idx, n)
+    assert row.add_user("") == n
+    eng.check_device()

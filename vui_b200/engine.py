@@ -16,7 +16,6 @@ this library's own kernels); pass it, or any object with ``decode(codes_bqt)`` a
 from __future__ import annotations
 
 import ctypes as C
-import weakref
 from collections import deque
 from collections.abc import Iterator
 from dataclasses import dataclass
@@ -147,7 +146,7 @@ class Row:
 
     @property
     def offset(self) -> int:
-        return self._engine._row_len(self._idx)
+        return int(self._engine.seq_lens[self._idx].item())
 
     def prefill(self, segments, spk_emb=None, segments_2=None, spk_emb_2=None) -> int:
         return self._engine._prefill_row(self, segments, spk_emb, segments_2, spk_emb_2)
@@ -184,50 +183,9 @@ class Row:
         self.close()
 
 
-class _KnownLengths:
-    """The slots' lengths as far as the host itself wrote them last (resets, rewinds, prefills).  They are known without a device
-    read, which would wait for everything before it: a prompt's host work then runs beside the GPU's on the one before.  Any other
-    write to the tensor moves its version and ends that knowledge, and so does every step that advances lengths (forget)."""
-
-    def __init__(self, seq_lens: Tensor):
-        self.seq_lens, self.version, self.lens = seq_lens, seq_lens._version, {}
-
-    def forget(self) -> None:
-        self.lens.clear()
-        self.version = self.seq_lens._version
-
-    def get(self, slot: int) -> int:
-        if self.seq_lens._version != self.version:
-            self.forget()
-        n = self.lens.get(slot)
-        return int(self.seq_lens[slot].item()) if n is None else n
-
-    def wrote(self, slot: int, n: int, version_before: int) -> None:
-        if version_before != self.version:
-            self.lens.clear()
-        self.lens[slot] = int(n)
-        self.version = self.seq_lens._version
-
-
 def _set_len(engine, slot: int, n: int) -> None:
     """Writes a slot's length: a fill on the device (an assignment copies a scalar from the host, 10 us more)."""
-    known = getattr(engine, "_known", None)
-    before = known and known.seq_lens._version
     engine.seq_lens[slot].fill_(n)
-    if known:
-        known.wrote(slot, n, before)
-
-
-class _FrameGraph(torch.cuda.CUDAGraph):
-    """A captured frame: its replay advances the engine's lengths."""
-
-    engine = staticmethod(lambda: None)   # a weak reference to it, set by _frame_graph
-
-    def replay(self):
-        engine = self.engine()
-        if engine is not None:
-            engine._lens_moved()
-        super().replay()
 
 
 class Engine:
@@ -302,9 +260,7 @@ class Engine:
         # KV: one allocation, per-layer views in the reference's FlashKVCache layout
         self._kv = torch.zeros(s.n_layers, 2, n_slots, self.max_seq, s.n_kv_heads, s.head_dim,
                                device=dev, dtype=torch.bfloat16)
-        with torch.inference_mode(False):   # a tensor that counts its in-place writes, whoever makes them: see _KnownLengths
-            self.seq_lens = torch.zeros(n_slots, device=dev, dtype=torch.int32)
-        self._known = _KnownLengths(self.seq_lens)
+        self.seq_lens = torch.zeros(n_slots, device=dev, dtype=torch.int32)
         # this engine's caches; model.decoder.flash_kv_caches (where the reference keeps them, model.py:473-495)
         # points at the caches of the engine built last on the model
         self.flash_kv_caches = [
@@ -429,7 +385,6 @@ class Engine:
 
     # ----------------------------------------------------------------- graphs
     def _frame_call(self, B: int) -> None:
-        self._lens_moved()
         P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
         self._ck(self._lib.vuib_decode_frame(
             self._handle, B, P(self._g_slot_idx), P(self._g_seq_inc), P(self._g_codes_in),
@@ -467,8 +422,7 @@ class Engine:
         self._warm.discard(B)
         self._warm_frame(B)
         torch.cuda.synchronize(self.device)
-        g = _FrameGraph()
-        g.engine = weakref.ref(self)
+        g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
             self._frame_call(B)
         torch.cuda.synchronize(self.device)
@@ -514,7 +468,6 @@ class Engine:
                 self._h_codes_in[: h_codes_in.shape[0]].copy_(h_codes_in)
                 h_codes_in = self._h_codes_in
             src = C.c_void_p(h_codes_in.data_ptr())
-        self._lens_moved()
         self._ck(self._lib.vuib_frame_host(self._handle, B, int(with_in), src, C.c_void_p(self._h_codes.data_ptr()),
                                            C.c_void_p(self._h_eos.data_ptr()), self._stream))
         return self._h_codes[:B_active], self._h_eos[:B_active]
@@ -531,7 +484,6 @@ class Engine:
         """Backbone-only step over all max_rows slots (engine.py:850-853)."""
         P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
         self._g_slot_idx.copy_(torch.arange(self.max_rows, device=self.device, dtype=torch.int32))
-        self._lens_moved()
         self._ck(self._lib.vuib_backbone_step(
             self._handle, self.max_rows, P(self._g_slot_idx), None, P(self._g_codes_in),
             P(self._g_hidden_out), P(self._g_cb0_out), P(self._g_eos_out), self._stream))
@@ -573,12 +525,6 @@ class Engine:
         self._touched = True
         self.seq_lens.zero_()
 
-    def _row_len(self, slot: int) -> int:
-        return self._known.get(slot)
-
-    def _lens_moved(self) -> None:
-        self._known.forget()
-
     def _rewind_row(self, row: Row, offset: int) -> int:
         self._touched = True
         _set_len(self, row.idx, offset)
@@ -598,9 +544,11 @@ class Engine:
             self._cond_bias.add_(torch.nn.functional.linear(v, sd["wps_proj.proj.weight"]).reshape(1, 1, -1))
 
     # ---------------------------------------------------------------- prefill
-    def _prefill_many(self, items: list[tuple[Row, Tensor]]) -> list[Tensor]:
+    def _prefill_many(self, items: list[tuple[Row, Tensor]], ends: dict[int, int] | None = None) -> list[Tensor]:
         """Prefill several (row, emb (T_i, d)) pairs in as few calls as fit
-        max_prefill_rows.  Returns each row's final-norm output (T_i, d)."""
+        max_prefill_rows.  Returns each row's final-norm output (T_i, d); ``ends``
+        receives the length that each row's slot has afterwards, so that a caller
+        who needs it does not wait for the prefill to read it back."""
         outs = []
         pend: list[tuple[int, int, Tensor]] = []  # slot, offset, emb
 
@@ -624,11 +572,14 @@ class Engine:
                 i += e.shape[0]
             pend.clear()
 
+        # The lengths are the device's: kernels, captured graphs and callers of the C ABI write them unseen by the host.  One read a
+        # call, and the embeddings of the items are under way by then.
+        lens = self.seq_lens.tolist()
         offsets: dict[int, int] = {}
-        ends: dict[int, int] = {}
+        ends = {} if ends is None else ends
         for row, emb in items:
             emb = emb.reshape(-1, self.D)
-            off = offsets[row.idx] if row.idx in offsets else row.offset
+            off = offsets[row.idx] if row.idx in offsets else lens[row.idx]
             if off + emb.shape[0] > self.max_seq:
                 raise RuntimeError(f"prefill of {emb.shape[0]} positions overflows max_seq={self.max_seq}")
             # a segment longer than one call is cut; a slot may appear several times in a call (its rows
@@ -660,10 +611,10 @@ class Engine:
             res.append(torch.cat(parts, dim=0) if len(parts) > 1 else parts[0])
         return res
 
-    def _prefill_emb(self, row: Row, emb: Tensor) -> Tensor:
+    def _prefill_emb(self, row: Row, emb: Tensor, ends: dict[int, int] | None = None) -> Tensor:
         """Write (1, T, d) embeddings into the row's slot at its current offset;
         returns the decoder's final-norm output (1, T, d) (engine.py:674-694)."""
-        return self._prefill_many([(row, emb)])[0].unsqueeze(0)
+        return self._prefill_many([(row, emb)], ends)[0].unsqueeze(0)
 
     def prefill_ids(self, row: Row, ids: Tensor) -> Tensor:
         """Tokenizer-free prefill of text token ids; returns the last position's hidden (d,)."""
@@ -792,11 +743,14 @@ class Engine:
                 parts.append(self._audio_emb(seg.codes))
         return parts
 
-    def _prefill_parts(self, row, parts: list[Tensor]) -> Tensor | None:
-        """One prefill of several embeddings (1, n_i, d): the weights are read once for all of them."""
+    def _prefill_parts(self, row, parts: list[Tensor]) -> tuple[Tensor | None, int]:
+        """One prefill of several embeddings (1, n_i, d): the weights are read once for all of them.  Returns the
+        final-norm output (None without embeddings) and the row's length afterwards."""
         if not parts:
-            return None
-        return self._prefill_emb(row, parts[0] if len(parts) == 1 else torch.cat([p.to(self.dtype) for p in parts], dim=1))
+            return None, row.offset
+        ends: dict[int, int] = {}
+        out = self._prefill_emb(row, parts[0] if len(parts) == 1 else torch.cat([p.to(self.dtype) for p in parts], dim=1), ends)
+        return out, ends[row.idx]
 
     def _prompt_parts(self, row, segments, spk_emb, segments_2=None, spk_emb_2=None) -> list[Tensor]:
         """Sets the row up for a voice prompt; returns the prompt's embeddings."""
@@ -817,8 +771,7 @@ class Engine:
         return parts
 
     def _prefill_row(self, row, segments, spk_emb, segments_2=None, spk_emb_2=None) -> int:
-        self._prefill_parts(row, self._prompt_parts(row, segments, spk_emb, segments_2, spk_emb_2))
-        row._prompt_offset = row.offset
+        _, row._prompt_offset = self._prefill_parts(row, self._prompt_parts(row, segments, spk_emb, segments_2, spk_emb_2))
         return row._prompt_offset
 
     def _user_parts(self, text, codes, *, final=True) -> list[Tensor]:
@@ -832,10 +785,10 @@ class Engine:
         return parts
 
     def _add_user(self, row, text, codes, *, final=True) -> int:
-        self._prefill_parts(row, self._user_parts(text, codes, final=final))
+        _, end = self._prefill_parts(row, self._user_parts(text, codes, final=final))
         if codes is not None and row._codec_ctx is not None:
             row._codec_ctx.add(codes.T.unsqueeze(0).to(self.device))
-        return row.offset
+        return end
 
     def _active_spk_token(self, row):
         if row._active_speaker == 1 and row._spk_token_2 is not None:
@@ -851,7 +804,7 @@ class Engine:
         return parts
 
     def _add_agent_text(self, row, text, *, final=False) -> Tensor:
-        return self._prefill_parts(row, self._agent_parts(row, text, final=final))[0, -1]
+        return self._prefill_parts(row, self._agent_parts(row, text, final=final))[0][0, -1]
 
     # ------------------------------------------------------------ first frame
     def _first_frames(self, rows: list[Row], hidden: Tensor) -> Tensor:
@@ -1054,9 +1007,8 @@ class Engine:
             parts = next_text(info)
             if parts is None:
                 return False
-            hidden = self._prefill_parts(info.row, parts)[0, -1]
-            info.seq_offset = info.row.offset
-            first_frame(info, hidden)
+            out, info.seq_offset = self._prefill_parts(info.row, parts)
+            first_frame(info, out[0, -1])
             return True
 
         def backfill() -> None:

@@ -250,7 +250,6 @@ class VuiB200(torch.nn.Module):
             eng._rewind_row(self._decode_row, int(pos))
             self._decode_graph = g
         self._decode_graph.replay()
-        eng._lens_moved()
         return eng._g_hidden_out[:1], eng._g_cb0_out[:1], eng._g_eos_out[:1].reshape(1, 1)
 
     def weight_bytes_per_step(self) -> int:
