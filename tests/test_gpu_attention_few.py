@@ -57,3 +57,26 @@ def test_infinite_values_stay_infinite(eng, rows):
     assert (out[:, :, 3] == float("inf")).all()
     out[:, :, 3] = 1.0
     assert (out == 1.0).all()
+
+
+@pytest.mark.parametrize("rows", [1, 5, 18])
+@pytest.mark.parametrize("moved", ["not", "position", "slot", "wildly"])
+def test_keys_requested_before_the_place_is_final(eng, rows, moved):
+    """As a step asks for them: where the table changes behind the early look (or does not), the result is that of the final place."""
+    import ctypes as C
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    layer = 3
+    eng.flash_kv_caches[layer].k_cache.normal_(generator=g)
+    eng.flash_kv_caches[layer].v_cache.normal_(generator=g)
+    q = torch.randn(rows, 1024, device="cuda", generator=g).to(torch.bfloat16)
+    P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    for first in range(0, len(LENGTHS), rows):
+        pos = torch.tensor([LENGTHS[(first + i) % len(LENGTHS)] - 1 for i in range(rows)], dtype=torch.int32, device="cuda")
+        slots = torch.tensor([(5 * i) % 64 for i in range(rows)], dtype=torch.int32, device="cuda")
+        old_pos = {"position": (pos - 1).clamp(min=0), "wildly": (pos * 7919) % 3000 - 900}.get(moved, pos).to(torch.int32)
+        old_slots = {"slot": (slots + 1) % 64, "wildly": slots - 40}.get(moved, slots).to(torch.int32)
+        out = torch.empty_like(q)
+        eng._ck(eng._lib.vuib_debug_attention_moved(eng._handle, layer, rows, P(q), P(old_slots), P(old_pos), P(slots), P(pos), P(out), eng._stream))
+        assert torch.equal(out, eng._attention(layer, q, slots, pos))
+    eng.check_device()

@@ -96,14 +96,20 @@ __device__ __forceinline__ float pick(const float (&a)[RT], int r) {
 // ---------------------------------------------------------------------------
 // Embedding gather-sum for a decode step (AudioEmbedding.forward, model.py:559-563)
 // plus the per-row (slot, position) table every later kernel of the step reads.
+// A step begins here, and its other kernels start only once every CTA of this one
+// has met its dependency: then all that was launched before the step has ended,
+// and the cache rows of earlier steps may be read before a kernel's own pdl_wait()
+// (k_attn_block, k_attn_rows, AttnArgs::early).  The order of the two lines below
+// is that guarantee; in a frame graph, whose first kernel waits for nothing, it
+// costs nothing.
 // ---------------------------------------------------------------------------
 static __global__ void __launch_bounds__(128) k_embed_codes(
     const int64_t* __restrict__ codes, const int32_t* __restrict__ slots,
     const int32_t* __restrict__ seq_lens, const bf16* __restrict__ table, bf16* __restrict__ x,
     int32_t* __restrict__ row_slot, int32_t* __restrict__ row_pos, int d, int Q, int CS,
     int n_slots, int max_seq, int32_t* __restrict__ flag) {
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     const int r = blockIdx.x;
     if (slots) {  // decode step: also publish the row's (slot, position)
         int slot = slots[r];
@@ -153,6 +159,18 @@ static __global__ void __launch_bounds__(128) k_embed_codes(
             }
         }
         *reinterpret_cast<uint4*>(x + (size_t)r * d + k) = pack8(acc);
+    }
+}
+
+// Writes a (slot, position) table 20 us after its successor may have started: the successor's early look at the table then finds
+// what was there before.  For tests of that case.
+static __global__ void __launch_bounds__(256) k_move_rows(const int32_t* slot_in, const int32_t* pos_in, int32_t* row_slot, int32_t* row_pos, int n) {
+    pdl_trigger();
+    pdl_wait();
+    __nanosleep(20000);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        row_slot[i] = slot_in[i];
+        row_pos[i] = pos_in[i];
     }
 }
 
@@ -804,7 +822,7 @@ struct AttnArgs {
     int Hq, Hkv, max_seq, S;
     int n_slots;              // slots in the cache; 0 = unknown (only negative slots can then be caught)
     int32_t* flag;            // device error word (may be NULL)
-    int early;                // keys before row_pos were written long before the preceding kernel: requested before its end
+    int early;                // keys before row_pos are of earlier steps, which have ended (k_embed_codes): requested before pdl_wait()
 };
 
 __device__ __forceinline__ void softmax_merge(float& m, float& l, float (&acc)[8], float mo,

@@ -525,8 +525,8 @@ __global__ void __launch_bounds__(FB_THREADS, 1) k_attn_block(const __grid_const
             s1 = bf2f(__ushort_as_bfloat16((unsigned short)(f.y >> 16)));
         }
     };
-    // A stream's rows before its position were written by earlier frames, so for the backbone they can be requested
-    // BEFORE the dependency wait, with the position as it stands in memory now.  It is read again after the wait: if
+    // A stream's rows before its position were written by earlier frames, which have ended (k_embed_codes), so for the backbone
+    // they can be requested BEFORE the dependency wait, with the position as it stands in memory now.  It is read again after the wait: if
     // the kernel that sets it had not finished (first layer of a frame), the requests are simply made again.
     bool early = false;
     if constexpr (!SHORT) {

@@ -697,11 +697,9 @@ static int32_t run_layers_tc(VuibEngine* e, int M, cudaStream_t s, bool prefill)
             if (c.n_heads == 2 * c.n_kv_heads) CK(launch(k_prefill_attn<2>, dim3(gx, c.n_kv_heads), 256, 0, s, pa));
             else CK(launch(k_prefill_attn<1>, dim3(gx, c.n_kv_heads), 128, 0, s, pa));
         } else {
-            // A frame's old keys may be asked for before the preceding kernel has ended (AttnArgs::early): they were written a whole pass over
-            // the layers ago, whose GEMMs cannot all be resident (124 CTAs a layer or more, two an SM at most; so not with fewer than four layers).
             AttnArgs aa{q, static_cast<const bf16*>(e->k[li]), static_cast<const bf16*>(e->v[li]),
                         row_slot, row_pos, wsp<float>(e, L.part), wsp<int32_t>(e, L.counters), attn,
-                        c.n_heads, c.n_kv_heads, c.max_seq, e->S, c.n_slots, wsp<int32_t>(e, L.flag), !prefill && c.n_layers >= 4};
+                        c.n_heads, c.n_kv_heads, c.max_seq, e->S, c.n_slots, wsp<int32_t>(e, L.flag), !prefill};
             CK(attn_decode(e, aa, M, s));
         }
         e->launches++;
@@ -1542,6 +1540,30 @@ extern "C" int32_t vuib_attention(VuibEngine* e, int32_t layer, int32_t n_rows, 
                 c.n_heads, c.n_kv_heads, c.max_seq, e->S, c.n_slots, wsp<int32_t>(e, e->lay.flag), 0};
     CK(attn_decode(e, aa, n_rows, static_cast<cudaStream_t>(stream)));
     e->launches++;
+    CK(cudaGetLastError());
+    return VUIB_OK;
+}
+
+extern "C" int32_t vuib_debug_attention_moved(VuibEngine* e, int32_t layer, int32_t n_rows, const void* q_dev,
+                                              const int32_t* old_slot_dev, const int32_t* old_pos_dev,
+                                              const int32_t* row_slot_dev, const int32_t* row_pos_dev,
+                                              void* out_dev, void* stream) {
+    if (!e || !q_dev || !old_slot_dev || !old_pos_dev || !row_slot_dev || !row_pos_dev || !out_dev) return VUIB_ERR_NULL;
+    if (!e->have_kv || !e->have_ws) return fail(e, VUIB_ERR_UNBOUND, "bind kv and workspace first");
+    const VuibConfig& c = e->cfg;
+    if (layer < 0 || layer >= c.n_layers) return fail(e, VUIB_ERR_RANGE, "layer %d out of range", layer);
+    if (n_rows < 1 || n_rows > e->R) return fail(e, VUIB_ERR_RANGE, "n_rows %d outside [1, %d]", n_rows, e->R);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    int32_t *slot = wsp<int32_t>(e, e->lay.row_slot), *pos = wsp<int32_t>(e, e->lay.row_pos);
+    CK(cudaMemcpyAsync(slot, old_slot_dev, (size_t)n_rows * 4, cudaMemcpyDeviceToDevice, s));
+    CK(cudaMemcpyAsync(pos, old_pos_dev, (size_t)n_rows * 4, cudaMemcpyDeviceToDevice, s));
+    CK(launch(k_move_rows, 1, 256, 0, s, row_slot_dev, row_pos_dev, slot, pos, n_rows));
+    AttnArgs aa{static_cast<const bf16*>(q_dev), static_cast<const bf16*>(e->k[layer]),
+                static_cast<const bf16*>(e->v[layer]), slot, pos,
+                wsp<float>(e, e->lay.part), wsp<int32_t>(e, e->lay.counters), static_cast<bf16*>(out_dev),
+                c.n_heads, c.n_kv_heads, c.max_seq, e->S, c.n_slots, wsp<int32_t>(e, e->lay.flag), 1};
+    CK(attn_decode(e, aa, n_rows, s));
+    e->launches += 2;
     CK(cudaGetLastError());
     return VUIB_OK;
 }
