@@ -1,5 +1,5 @@
-"""Decode attention at the edges of its tiles (16 keys a warp, 128 a pass, 512 a CTA, splits of 256 beyond; splits of 128 with more
-rows or in longer caches), against softmax attention in 64 bits, and with infinite values."""
+"""Decode attention at the edges of its tiles (4 keys a step of a warp, splits of 128; for few rows in caches of up to 1024 positions four
+splits a CTA, else one), against softmax attention in 64 bits and against itself with other rows, and with infinite values."""
 import pytest
 import torch
 
@@ -80,3 +80,47 @@ def test_keys_requested_before_the_place_is_final(eng, rows, moved):
         eng._ck(eng._lib.vuib_debug_attention_moved(eng._handle, layer, rows, P(q), P(old_slots), P(old_pos), P(slots), P(pos), P(out), eng._stream))
         assert torch.equal(out, eng._attention(layer, q, slots, pos))
     eng.check_device()
+
+
+def test_a_rows_bits_are_its_own(nano_model):
+    """Whatever kernel the number of rows or the size of the cache leads to: a row alone, among few, among many, in a longer cache."""
+    from vui_b200 import Engine
+
+    layer, outs = 0, []
+    for max_seq in (1024, 1088):
+        eng = Engine(model=nano_model, max_rows=64, max_seq=max_seq)
+        g = torch.Generator(device="cuda").manual_seed(7)
+        for c in (eng.flash_kv_caches[layer].k_cache, eng.flash_kv_caches[layer].v_cache):
+            c[:, :1024] = torch.randn(65, 1024, 8, 64, device="cuda", generator=g)
+        q = torch.randn(46, 1024, device="cuda", generator=g).to(torch.bfloat16)
+        pos = torch.tensor([LENGTHS[i % len(LENGTHS)] - 1 for i in range(46)], dtype=torch.int32)
+        slots = torch.arange(46, dtype=torch.int32) % 23
+        outs.append(eng._attention(layer, q, slots, pos))
+        for first, n in [(i, 1) for i in range(23)] + [(0, 5), (18, 5), (0, 18), (5, 18), (0, 19), (20, 24)]:
+            part = slice(first, first + n)
+            assert torch.equal(eng._attention(layer, q[part], slots[part], pos[part]), outs[0][part]), (max_seq, first, n)
+    assert torch.equal(*outs)
+
+
+def test_a_streams_step_does_not_depend_on_the_others(nano_model):
+    """The backbone's step from five rows on, bit for bit: few and many rows, caches on either side of the rule."""
+    from vui_b200 import Engine
+
+    seen = {}
+    for max_seq in (1024, 1088):
+        eng = Engine(model=nano_model, max_rows=33, max_seq=max_seq)
+        g = torch.Generator(device="cuda").manual_seed(8)
+        eng._kv[:, :, :, :1024] = torch.randn(eng._kv[:, :, :, :1024].shape, device="cuda", generator=g, dtype=torch.bfloat16) * 0.5
+        codes = torch.randint(0, 2048, (33, 16), generator=torch.Generator().manual_seed(8)).cuda()
+        lens = torch.tensor([(37 * i + 3) % 700 for i in range(33)], dtype=torch.int32, device="cuda")
+        eng._g_slot_idx[:] = torch.arange(33, dtype=torch.int32, device="cuda")
+        eng._g_seq_inc.fill_(1)
+        for B in (33, 19, 18, 5):
+            eng.seq_lens[:33] = lens
+            eng._g_codes_in.copy_(codes)
+            eng._apply_cfg(None, greedy=True)
+            eng._frame_call(B)
+            got = (eng._g_hidden_out[:B].clone(), torch.stack([eng._kv[:, :, b, int(lens[b])] for b in range(B)]))
+            for a, b in zip(got, seen.setdefault("first", got)):
+                assert torch.equal(a, b[:B]), (max_seq, B)
+        eng.check_device()

@@ -18,8 +18,8 @@ typedef __nv_bfloat16 bf16;
 constexpr int HD = 64;             // head_dim of backbone and depth transformer
 constexpr int GEMV_THREADS = 256;  // 8 warps; one work item (1-2 weight rows) per warp
 constexpr int GEMV_WARPS = 8;
-constexpr int ATT_SPLIT = 128;     // keys per CTA in the backbone attention
-constexpr int ATT_THREADS = 128;
+constexpr int ATT_SPLIT = 128;     // keys per split in the backbone attention
+constexpr int ATT_THREADS = 128;   // threads per split
 constexpr int ATT_ITERS = ATT_SPLIT / 16;  // 4 warps x 4 key groups per pass
 constexpr int PART_STRIDE = HD + 2;        // acc[64], m, l
 constexpr int SAMPLE_THREADS = 256;
@@ -804,11 +804,12 @@ __global__ void __launch_bounds__(GEMV_THREADS, (RT >= 4 ? 2 : 1)) k_gemv(Stage 
 
 // ---------------------------------------------------------------------------
 // Backbone decode attention (flash_attn_with_kvcache call, model.py:247-257):
-// ragged per-row length row_pos[r]+1, GQA 2:1, scale 1/8, fp32 softmax.  One CTA
-// = (split of ATT_SPLIT keys, kv head, row); partial (acc, m, l) per split go to
-// scratch and the last CTA of a (row, kv head) merges them in split order, so the
-// result does not depend on arrival order.  k_attn_decode is for many rows,
-// k_attn_few below for few.
+// ragged per-row length row_pos[r]+1, GQA 2:1, scale 1/8, fp32 softmax.  Four warps
+// = (split of ATT_SPLIT keys, kv head, row).  The splits' states (acc, m, l) are
+// merged in split order, whichever is done last, so a row's bits depend on its own
+// keys alone: not on arrival, on the other rows of the call, on the size of the cache
+// or on the kernel.  k_attn_decode has one split a CTA and is for many rows,
+// k_attn_wide has four and is for few.
 // ---------------------------------------------------------------------------
 struct AttnArgs {
     const bf16* q;        // (R, Hq*64)
@@ -840,11 +841,14 @@ __device__ __forceinline__ void bar_named(int id, int n) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
-struct AttnSmem {
+struct AttnSmem {   // of one split
     alignas(16) float o[4][2][HD];   // [warp][head][dim]
     float ml[4][2][2];               // [warp][head]: max, sum
-    int s_last;
 };
+
+__host__ __device__ constexpr int att_splits(int len, int per_cta = 1) { return (len + ATT_SPLIT * per_cta - 1) / (ATT_SPLIT * per_cta); }
+__device__ __forceinline__ int att_slot(const AttnArgs& a, int v) { return v < 0 ? 0 : a.n_slots > 0 && v >= a.n_slots ? a.n_slots - 1 : v; }
+__device__ __forceinline__ int att_pos(const AttnArgs& a, int v) { return v < 0 ? 0 : v >= a.max_seq ? a.max_seq - 1 : v; }
 
 // Two fp32 multiply-adds in one instruction.
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
@@ -855,84 +859,11 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 }
 __device__ __forceinline__ float2 bf2(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 
-// A (row, head)'s splits in index order; 16 splits' worth of loads are in flight at a time.
-__device__ __forceinline__ void att_merge_splits(const AttnArgs& a, int r, int hq, int dim, int nsplit) {
-    const float* pb = a.part + ((size_t)r * a.Hq + hq) * a.S * PART_STRIDE;
-    float Mx = NEG_BIG, Ls = 0.f, Os = 0.f;
-    for (int i0 = 0; i0 < nsplit; i0 += 16) {
-        float ms[16], ls[16], os[16];
-#pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const bool ok = i0 + u < nsplit;
-            const float* q = pb + (size_t)(ok ? i0 + u : i0) * PART_STRIDE;
-            ms[u] = ok ? __ldcg(q + HD) : NEG_BIG;
-            ls[u] = ok ? __ldcg(q + HD + 1) : 0.f;
-            os[u] = ok ? __ldcg(q + dim) : 0.f;
-        }
-        float Mn = Mx;
-#pragma unroll
-        for (int u = 0; u < 16; ++u) Mn = fmaxf(Mn, ms[u]);
-        const float c0 = __expf(Mx - Mn);
-        Ls *= c0;
-        Os *= c0;
-#pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const float c = __expf(ms[u] - Mn);
-            Ls += ls[u] * c;
-            Os += os[u] * c;
-        }
-        Mx = Mn;
-    }
-    a.out[(size_t)r * a.Hq * HD + hq * HD + dim] = f2bf(Os / Ls);
-}
-
-// With the bound of five CTAs an SM (94 or 96 registers allow them either way; the schedule differs) 256 rows take 44.8 us, not 49.1.
-static __global__ void __launch_bounds__(ATT_THREADS, 5) k_attn_decode(AttnArgs a) {
-    __shared__ AttnSmem S_;
-    pdl_trigger();
-    const int sp = blockIdx.x, kvh = blockIdx.y, r = blockIdx.z;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int s = lane & 7, g = lane >> 3;
-    const int G = a.Hq / a.Hkv;  // q heads per kv head (2)
-    const int t_begin = sp * ATT_SPLIT;
-    const size_t pos_stride = (size_t)a.Hkv * HD;
-    auto clamp_slot = [&](int v) { return v < 0 ? 0 : a.n_slots > 0 && v >= a.n_slots ? a.n_slots - 1 : v; };
-    auto clamp_pos = [&](int v) { return v < 0 ? 0 : v >= a.max_seq ? a.max_seq - 1 : v; };
-    const bf16 *kb, *vb;
-    // all K and V requests of this lane in flight before any arithmetic
-    uint4 kr[ATT_ITERS], vr[ATT_ITERS];
-    auto key_of = [&](int it) { return t_begin + it * 16 + warp * 4 + g; };
-    auto request = [&](int slot, int end) {
-        const size_t base = (size_t)slot * a.max_seq * pos_stride + kvh * HD + s * 8;
-        kb = a.kc + base;
-        vb = a.vc + base;
-#pragma unroll
-        for (int it = 0; it < ATT_ITERS; ++it) {
-            const int t = key_of(it);
-            if (t < end) {
-                kr[it] = ldg_stream(kb + (size_t)t * pos_stride);
-                vr[it] = ldg_stream(vb + (size_t)t * pos_stride);
-            } else {
-                kr[it] = make_uint4(0, 0, 0, 0);
-                vr[it] = make_uint4(0, 0, 0, 0);
-            }
-        }
-    };
-    pdl_wait();
-    const int s_now = __ldcg(a.row_slot + r);  // both requests in flight before the first use
-    const int p_now = __ldcg(a.row_pos + r);
-    // A slot or position outside the cache is recorded and clamped, never followed: a position past
-    // max_seq would also ask for more splits than the grid has, and the merge would never run.
-    const int len = clamp_pos(p_now) + 1;
-    if (a.flag && tid == 0 && sp == 0 && kvh == 0) {
-        if (clamp_slot(s_now) != s_now) atomicOr(a.flag, FLAG_BAD_SLOT);
-        if (clamp_pos(p_now) != p_now) atomicOr(a.flag, FLAG_BAD_POS);
-    }
-    const int nsplit = (len + ATT_SPLIT - 1) / ATT_SPLIT;
-    if (sp >= nsplit) return;
-    const int t_end = min(len, t_begin + ATT_SPLIT);
-    request(clamp_slot(s_now), t_end);
-    int& s_last = S_.s_last;
+// A split's states of its four warps from the keys and values in registers: lane (g, s) of a warp has dims 8 s .. 8 s + 7 of keys
+// t_begin + it * 16 + warp * 4 + g.
+__device__ __forceinline__ void att_split(const AttnArgs& a, int r, int kvh, int t_begin, int t_end, int warp, int lane,
+                                          const uint4 (&kr)[ATT_ITERS], const uint4 (&vr)[ATT_ITERS], AttnSmem& S_) {
+    const int s = lane & 7, g = lane >> 3, G = a.Hq / a.Hkv;
     float2 q2[2][4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -1018,27 +949,58 @@ static __global__ void __launch_bounds__(ATT_THREADS, 5) k_attn_decode(AttnArgs 
     }
     *reinterpret_cast<float4*>(&S_.o[warp][g >> 1][s * 8 + (g & 1) * 4]) = make_float4(o8[0], o8[1], o8[2], o8[3]);
     if (g == 0 && (s & 3) == 0) { S_.ml[warp][s >> 2][0] = m; S_.ml[warp][s >> 2][1] = l; }
-    __syncthreads();
-    // thread (h, dim): merge the 4 warps
-    const int h = tid >> 6, dim = tid & 63;
-    float M_ = NEG_BIG;
+}
+
+// Thread (h, dim) of a split: its four warps' states as one.
+__device__ __forceinline__ void att_merge_warps(const AttnSmem& S_, int h, int dim, float& M_, float& L_, float& O_) {
+    M_ = NEG_BIG;
 #pragma unroll
     for (int w = 0; w < 4; ++w) M_ = fmaxf(M_, S_.ml[w][h][0]);
-    float L_ = 0.f, O_ = 0.f;
+    L_ = O_ = 0.f;
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
         const float c = __expf(S_.ml[w][h][0] - M_);
         L_ += S_.ml[w][h][1] * c;
         O_ += S_.o[w][h][dim] * c;
     }
-    const bool head_ok = h < G;
-    const int hq = kvh * G + (head_ok ? h : 0);
-    if (nsplit == 1) {
-        if (head_ok) a.out[(size_t)r * a.Hq * HD + hq * HD + dim] = f2bf(O_ / L_);
-        return;
+}
+
+// A (row, head)'s splits in index order, U splits' loads in flight at a time: state(i, ok, m, l, o) reads split i where ok.
+template <int U, class State>
+__device__ __forceinline__ float att_merge_splits(int nsplit, State state) {
+    float Mx = NEG_BIG, Ls = 0.f, Os = 0.f;
+    for (int i0 = 0; i0 < nsplit; i0 += U) {
+        float ms[U], ls[U], os[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool ok = i0 + u < nsplit;
+            ms[u] = NEG_BIG;
+            ls[u] = os[u] = 0.f;
+            state(ok ? i0 + u : i0, ok, ms[u], ls[u], os[u]);
+        }
+        float Mn = Mx;
+#pragma unroll
+        for (int u = 0; u < U; ++u) Mn = fmaxf(Mn, ms[u]);
+        const float c0 = __expf(Mx - Mn);
+        Ls *= c0;
+        Os *= c0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const float c = __expf(ms[u] - Mn);
+            Ls += ls[u] * c;
+            Os += os[u] * c;
+        }
+        Mx = Mn;
     }
-    float* pp = a.part + (((size_t)r * a.Hq + hq) * a.S + sp) * PART_STRIDE;
-    if (head_ok) {
+    return Os / Ls;
+}
+
+// Writes a split's state for the merge; the return value says whether the row's other CTAs, `ctas` in all, have written theirs.  Every
+// thread of the CTA calls it; `tid` counts them.
+__device__ __forceinline__ bool att_publish(const AttnArgs& a, int r, int kvh, int hq, bool mine, int sp, int dim, float M_, float L_, float O_,
+                                            int ctas, int tid, int& s_last) {
+    if (mine) {
+        float* pp = a.part + (((size_t)r * a.Hq + hq) * a.S + sp) * PART_STRIDE;
         pp[dim] = O_;
         if (dim == 0) {
             pp[HD] = M_;
@@ -1049,11 +1011,71 @@ static __global__ void __launch_bounds__(ATT_THREADS, 5) k_attn_decode(AttnArgs 
     if (tid == 0) {
         int old;
         asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(old) : "l"(a.counters + r * a.Hkv + kvh) : "memory");
-        s_last = (old == nsplit - 1);
+        s_last = (old == ctas - 1);
     }
     __syncthreads();
-    if (!s_last) return;
-    if (head_ok) att_merge_splits(a, r, hq, dim, nsplit);
+    return s_last;
+}
+
+__device__ __forceinline__ void att_finish(const AttnArgs& a, int r, int hq, int dim, int nsplit) {
+    const float* part = a.part + ((size_t)r * a.Hq + hq) * a.S * PART_STRIDE;
+    a.out[(size_t)r * a.Hq * HD + hq * HD + dim] = f2bf(att_merge_splits<16>(nsplit, [&](int i, bool ok, float& m, float& l, float& o) {
+        const float* q = part + (size_t)i * PART_STRIDE;
+        if (ok) { m = __ldcg(q + HD); l = __ldcg(q + HD + 1); o = __ldcg(q + dim); }
+    }));
+}
+
+// Many rows.  What bounds it is arithmetic per key beside the bytes: 256 rows of 64 to 512 keys take 52 us, 3.0 TB/s.  (With the bound of
+// five CTAs an SM; 96 registers allow them either way, but the schedule without it takes 10 % longer.)
+static __global__ void __launch_bounds__(ATT_THREADS, 5) k_attn_decode(AttnArgs a) {
+    __shared__ AttnSmem S_;
+    __shared__ int s_last;
+    pdl_trigger();
+    const int sp = blockIdx.x, kvh = blockIdx.y, r = blockIdx.z;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int s = lane & 7, g = lane >> 3;
+    const int G = a.Hq / a.Hkv;  // q heads per kv head (2)
+    const int t_begin = sp * ATT_SPLIT;
+    pdl_wait();
+    const int s_now = __ldcg(a.row_slot + r);  // both requests in flight before the first use
+    const int p_now = __ldcg(a.row_pos + r);
+    // A slot or position outside the cache is recorded and clamped, never followed: a position past
+    // max_seq would also ask for more splits than the grid has, and the merge would never run.
+    const int slot = att_slot(a, s_now), len = att_pos(a, p_now) + 1;
+    if (a.flag && tid == 0 && sp == 0 && kvh == 0) {
+        if (slot != s_now) atomicOr(a.flag, FLAG_BAD_SLOT);
+        if (len - 1 != p_now) atomicOr(a.flag, FLAG_BAD_POS);
+    }
+    const int nsplit = att_splits(len);
+    if (sp >= nsplit) return;
+    const int t_end = min(len, t_begin + ATT_SPLIT);
+    // all K and V requests of this lane in flight before any arithmetic
+    const size_t pos_stride = (size_t)a.Hkv * HD, base = (size_t)slot * a.max_seq * pos_stride + kvh * HD + s * 8;
+    uint4 kr[ATT_ITERS], vr[ATT_ITERS];
+#pragma unroll
+    for (int it = 0; it < ATT_ITERS; ++it) {
+        const int t = t_begin + it * 16 + warp * 4 + g;
+        if (t < t_end) {
+            kr[it] = ldg_stream(a.kc + base + (size_t)t * pos_stride);
+            vr[it] = ldg_stream(a.vc + base + (size_t)t * pos_stride);
+        } else {
+            kr[it] = make_uint4(0, 0, 0, 0);
+            vr[it] = make_uint4(0, 0, 0, 0);
+        }
+    }
+    att_split(a, r, kvh, t_begin, t_end, warp, lane, kr, vr, S_);
+    __syncthreads();
+    const int h = tid >> 6, dim = tid & 63;
+    float M_, L_, O_;
+    att_merge_warps(S_, h, dim, M_, L_, O_);
+    const bool head_ok = h < G;
+    const int hq = kvh * G + (head_ok ? h : 0);
+    if (nsplit == 1) {
+        if (head_ok) a.out[(size_t)r * a.Hq * HD + hq * HD + dim] = f2bf(O_ / L_);
+        return;
+    }
+    if (!att_publish(a, r, kvh, hq, head_ok, sp, dim, M_, L_, O_, nsplit, tid, s_last)) return;
+    if (head_ok) att_finish(a, r, hq, dim, nsplit);
     if (tid == 0) a.counters[r * a.Hkv + kvh] = 0;
 }
 
@@ -1064,250 +1086,79 @@ __device__ __forceinline__ void ldg_stream_if(uint4& r, const void* p, bool ok) 
                  : "=&r"(r.x), "=&r"(r.y), "=&r"(r.z), "=&r"(r.w) : "l"(p), "r"((uint32_t)ok));
 }
 
-// c += A B, m16n8k16
-__device__ __forceinline__ void att_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
+// Few rows.  What bounds it then is round trips: the keys' way from memory behind the preceding kernel, and the merge through global
+// memory.  A CTA takes four splits, so up to 512 keys are merged in shared memory; old keys are requested before the preceding kernel has
+// ended; and there is an SM for each (row, kv head), since a CTA's keys and values fill its registers.  Frames of 5 / 8 / 16 / 18 rows
+// at 300 keys take 1.52 / 1.55 / 1.58 / 1.60 ms, with k_attn_decode 1.52 / 1.59 / 1.64 / 1.64.
+// Beyond 512 keys a row has two CTAs and more than nine rows no SM for each: 800 keys in caches of 1024 take 1.57 / 1.60 / 1.74 / 1.78 ms, with
+// k_attn_decode 1.54 / 1.65 / 1.71 / 1.74.  Where the cache ends at 1024 a row that fills it spends as many steps on either side and the sum is
+// in favour or even; in caches of 1536 (16 rows: 1.60, 1.74, 1.90 ms at 300, 800 and 1500 keys, with the other 1.62, 1.71, 1.81) it is not.
+constexpr int ATT_WIDE = 4;   // splits of a CTA
+inline bool att_wide(int rows, int Hkv, int max_seq, int num_sms) { return rows * Hkv <= num_sms && max_seq <= 2 * ATT_WIDE * ATT_SPLIT; }
 
-// Term `part` (0 high, 1 middle, 2 low) of two fp32 values whose sum of bf16 terms they are; 0 for part 3.
-__device__ __forceinline__ uint32_t att_term(float x, float y, int part) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    x -= __low2float(h);
-    y -= __high2float(h);
-    const __nv_bfloat162 m = __floats2bfloat162_rn(x, y);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(x - __low2float(m), y - __high2float(m));
-    const uint32_t a = *reinterpret_cast<const uint32_t*>(&h), b = *reinterpret_cast<const uint32_t*>(&m), c = *reinterpret_cast<const uint32_t*>(&l);
-    return part < 2 ? (part ? b : a) : (part == 2 ? c : 0u);
-}
-
-// Few rows (attn_decode in vuib200.cu): what it costs then is round trips, so a CTA of eight warps takes up to AF_SPLIT keys of a (row,
-// kv head) and contexts of that length need no merge through global memory; rows before the row's own key are requested before the
-// preceding kernel has ended.  At 16 rows of 270 keys 3.8 us of a frame's layer, 8.6 as splits of 128 asked for behind it.
-//
-// A warp's tile is 16 keys and both products are mma.sync m16n8k16 straight from registers.  The order of k in a dot product is free,
-// so the 16 bytes that a lane loads of a K row are halves of two A fragments (16 keys x 16 dims), and byte permutes of two keys' V
-// pieces give A fragments of V transposed (16 dims x 16 keys).  The B operand's eight columns are the two query heads, or the two
-// heads' probabilities as three bf16 terms each (high, middle, low: all 24 bits), columns that would be idle otherwise: the products
-// are exact and the sums fp32.  With many rows, where instructions count, this is no faster than the FMA pipe (256 rows: 69 us, 49).
-// Longer contexts are cut into splits of AF_LONG, two tiles a warp (as splits of 512 they took 1 to 5 us a layer more).
-constexpr int AF_WARPS = 8, AF_SPLIT = 512, AF_LONG = 256, AF_MAX_SEQ = 1024;
-__host__ __device__ constexpr int af_split(int len) { return len <= AF_SPLIT ? AF_SPLIT : AF_LONG; }
-// Where it is used.  Frames of 5 / 8 / 16 rows at 300 keys take 1.52 / 1.59 / 1.65 ms with it and 1.63 / 1.67 / 1.70 with k_attn_decode, at
-// 800 keys 1.61 / 1.66 / 1.82 and 1.65 / 1.70 / 1.80; at 2000 keys 1.76 / 1.88 / 2.21 and 1.67 / 1.82 / 2.03, so that caches for more than
-// 1024 positions keep to the other; at 32 rows (two CTAs an SM) 1.85 and 1.84 at 300 keys, 2.19 and 2.03 at 800.
-inline bool af_use(int rows, int Hkv, int max_seq, int num_sms) { return rows * Hkv <= num_sms && max_seq <= AF_MAX_SEQ; }
-__host__ __device__ constexpr int af_splits(int len) { return (len + af_split(len) - 1) / af_split(len); }
-
-
-static __global__ void __launch_bounds__(AF_WARPS * 32, 2) k_attn_few(AttnArgs a) {
-    constexpr int STEP = 16 * AF_WARPS;   // a pass of the CTA's warps
-    __shared__ __align__(16) float s_o[AF_WARPS][2][HD];
-    __shared__ float s_ml[AF_WARPS][2][2];
+static __global__ void __launch_bounds__(ATT_WIDE * ATT_THREADS, 1) k_attn_wide(AttnArgs a) {
+    __shared__ AttnSmem S_[ATT_WIDE];
     __shared__ int s_last;
     pdl_trigger();
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int sp = blockIdx.z, kvh = blockIdx.x, r = blockIdx.y, G = a.Hq / a.Hkv;
-    const int pos_stride = a.Hkv * HD;
-    int t_begin = 0, t_len = 0;   // the split's first key and most keys: by the row's length
-    auto cut = [&](int p) {
-        t_len = af_split(p + 1);
-        t_begin = sp * t_len;
-    };
-    const bf16 *kb, *vb;   // of the split's first key
-    auto clamp_slot = [&](int s) { return s < 0 ? 0 : a.n_slots > 0 && s >= a.n_slots ? a.n_slots - 1 : s; };
-    auto clamp_pos = [&](int p) { return p < 0 ? 0 : p >= a.max_seq ? a.max_seq - 1 : p; };
-    auto aim = [&](int slot) {
-        const size_t base = ((size_t)slot * a.max_seq + t_begin) * pos_stride + kvh * HD;
-        kb = a.kc + base + t * 8;
-        vb = a.vc + base + g * 8;
-    };
-    // A tile in registers.  K: lane (g, t) has 16-byte pieces t and t + 4 of keys g and g + 8; V: piece g of keys 2 t, 2 t + 1, 2 t + 8,
-    // 2 t + 9.  Two tiles are in flight: 8 KB a warp.
-    uint4 kr[2][2][2], vr[2][4];
-    auto v_key = [&](int i) { return 2 * t + (i & 1) + (i >> 1) * 8; };
-    auto request_k = [&](uint4 (&k4)[2][2], int k0, int end) {
+    const int kvh = blockIdx.x, r = blockIdx.y, wsp = threadIdx.x / ATT_THREADS, sp = blockIdx.z * ATT_WIDE + wsp;   // split of the CTA, of the row
+    const int tid = threadIdx.x % ATT_THREADS, warp = tid >> 5, lane = tid & 31;
+    const int G = a.Hq / a.Hkv, t_begin = sp * ATT_SPLIT, t_first = t_begin + warp * 4 + (lane >> 3);
+    const size_t pos_stride = (size_t)a.Hkv * HD;
+    const bf16 *kb, *vb;   // of the lane's first key
+    uint4 kr[ATT_ITERS], vr[ATT_ITERS];
+    auto request = [&](int slot, int end) {
+        const size_t base = ((size_t)slot * a.max_seq + t_first) * pos_stride + kvh * HD + (lane & 7) * 8;
+        kb = a.kc + base;
+        vb = a.vc + base;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int k = k0 + i * 8 + g;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) ldg_stream_if(k4[i][h], kb + k * pos_stride + h * 32, k < end);
+        for (int it = 0; it < ATT_ITERS; ++it) {
+            const bool ok = t_first + it * 16 < end;
+            ldg_stream_if(kr[it], kb + it * 16 * pos_stride, ok);
+            ldg_stream_if(vr[it], vb + it * 16 * pos_stride, ok);
         }
     };
-    auto request_v = [&](uint4 (&v4)[4], int k0, int end) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int k = k0 + v_key(i);
-            ldg_stream_if(v4[i], vb + k * pos_stride, k < end);
-        }
-    };
-    const int first = warp * 16;
-    auto start = [&](int end) {
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            request_k(kr[u], first + u * STEP, end);
-            request_v(vr[u], first + u * STEP, end);
-        }
-    };
-    int slot = 0, pos = -1;
+    int s_old = -1, p_old = -1;
     if (a.early) {   // with the row's place as memory has it now; it is read again behind the wait
-        slot = clamp_slot(__ldcg(a.row_slot + r));
-        pos = clamp_pos(__ldcg(a.row_pos + r));
-        cut(pos);
-        aim(slot);
-        start(min(pos - t_begin, t_len));   // the row's own key is still to come
+        s_old = att_slot(a, __ldcg(a.row_slot + r));
+        p_old = att_pos(a, __ldcg(a.row_pos + r));
+        request(s_old, p_old);
     }
     pdl_wait();
-    uint32_t qf[4][2];   // columns of the B operand: head g & 1
-    {
-        const int hq = kvh * G + ((g & 1) < G ? g & 1 : 0);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint4 w = __ldcg(reinterpret_cast<const uint4*>(a.q + (size_t)r * a.Hq * HD + hq * HD + t * 8 + h * 32));
-            qf[2 * h][0] = w.x; qf[2 * h][1] = w.y; qf[2 * h + 1][0] = w.z; qf[2 * h + 1][1] = w.w;
-        }
+    const int s_now = __ldcg(a.row_slot + r), p_now = __ldcg(a.row_pos + r);
+    const int slot = att_slot(a, s_now), len = att_pos(a, p_now) + 1;   // as in k_attn_decode
+    if (a.flag && threadIdx.x == 0 && blockIdx.z == 0 && kvh == 0) {
+        if (slot != s_now) atomicOr(a.flag, FLAG_BAD_SLOT);
+        if (len - 1 != p_now) atomicOr(a.flag, FLAG_BAD_POS);
     }
-    {
-        const int s_now = __ldcg(a.row_slot + r), p_now = __ldcg(a.row_pos + r);
-        // A slot or position outside the cache is recorded and clamped, never followed: a position past max_seq would also ask for more
-        // splits than the grid has, and the merge would never run.
-        const int s = clamp_slot(s_now), p = clamp_pos(p_now);
-        if (a.flag && tid == 0 && sp == 0 && kvh == 0) {
-            if (s != s_now) atomicOr(a.flag, FLAG_BAD_SLOT);
-            if (p != p_now) atomicOr(a.flag, FLAG_BAD_POS);
-        }
-        const bool same = a.early && s == slot && p == pos;
-        cut(p);
-        if (t_begin > p) return;
-        if (same) {   // only the row's own key is still missing
-            const int own = p - t_begin;
+    const int nsplit = att_splits(len);
+    if (blockIdx.z * ATT_WIDE >= nsplit) return;
+    if (slot != s_old || len - 1 != p_old) {
+        request(slot, len);
+    } else {   // only the row's own key is missing, which the preceding kernel wrote
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int k0 = first + u * STEP;
-                if (own < k0 || own >= k0 + 16) continue;
-#pragma unroll
-                for (int i = 0; i < 2; ++i)
-                    if (own == k0 + i * 8 + g) {
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) kr[u][i][h] = __ldcg(reinterpret_cast<const uint4*>(kb + own * pos_stride + h * 32));
-                    }
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (own == k0 + v_key(i)) vr[u][i] = __ldcg(reinterpret_cast<const uint4*>(vb + own * pos_stride));
+        for (int it = 0; it < ATT_ITERS; ++it)
+            if (t_first + it * 16 == p_old) {
+                kr[it] = __ldcg(reinterpret_cast<const uint4*>(kb + it * 16 * pos_stride));
+                vr[it] = __ldcg(reinterpret_cast<const uint4*>(vb + it * 16 * pos_stride));
             }
-        } else {
-            slot = s;
-            pos = p;
-            aim(slot);
-            start(min(p + 1 - t_begin, t_len));
-        }
     }
-    const int len = pos + 1, nsplit = af_splits(len), n = min(len - t_begin, t_len);
-    float m = NEG_BIG, l = 0.f, o[4][4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
-    auto step = [&](uint4 (&k4)[2][2], uint4 (&v4)[4], int k0) {
-        float s[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            att_mma(s, k4[0][h].x, k4[1][h].x, k4[0][h].y, k4[1][h].y, qf[2 * h][0], qf[2 * h][1]);
-            att_mma(s, k4[0][h].z, k4[1][h].z, k4[0][h].w, k4[1][h].w, qf[2 * h + 1][0], qf[2 * h + 1][1]);
-        }
-        request_k(k4, k0 + 2 * STEP, n);
-        // every lane has both heads' scores of keys g and g + 8 and keeps those of head t & 1: one maximum and one exponential a score
-        const float s0 = k0 + g < n ? ((t & 1) ? s[1] : s[0]) * 0.125f : NEG_BIG;
-        const float s1 = k0 + 8 + g < n ? ((t & 1) ? s[3] : s[2]) * 0.125f : NEG_BIG;
-        float mn = fmaxf(s0, s1);
-#pragma unroll
-        for (int x = 4; x <= 16; x <<= 1) mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, x));
-        mn = fmaxf(m, mn);
-        const float c = __expf(m - mn);
-        const float p0 = s0 > NEG_BIG ? __expf(s0 - mn) : 0.f, p1 = s1 > NEG_BIG ? __expf(s1 - mn) : 0.f;
-        m = mn;
-        l = fmaf(l, c, p0 + p1);
-        // lane (g, t) of the second product: head g & 1, term g >> 1, keys 2 t, 2 t + 1, 2 t + 8, 2 t + 9; its columns are 2 t, 2 t + 1
-        const int from = 8 * t + (g & 1);
-        const float e0 = __shfl_sync(0xffffffffu, p0, from), e1 = __shfl_sync(0xffffffffu, p0, from + 4);
-        const float f0 = __shfl_sync(0xffffffffu, p1, from), f1 = __shfl_sync(0xffffffffu, p1, from + 4);
-        const float c_other = __shfl_xor_sync(0xffffffffu, c, 1);
-        const float c0 = (t & 1) ? c_other : c, c1 = (t & 1) ? c : c_other;
-        const uint32_t b0 = att_term(e0, e1, g >> 1), b1 = att_term(f0, f1, g >> 1);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) { o[j][0] *= c0; o[j][1] *= c1; o[j][2] *= c0; o[j][3] *= c1; }
-        const uint32_t* w0 = reinterpret_cast<const uint32_t*>(&v4[0]);
-        const uint32_t* w1 = reinterpret_cast<const uint32_t*>(&v4[1]);
-        const uint32_t* w2 = reinterpret_cast<const uint32_t*>(&v4[2]);
-        const uint32_t* w3 = reinterpret_cast<const uint32_t*>(&v4[3]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j)   // rows of product j: dims 8 g + 2 j and 8 g + 2 j + 1
-            att_mma(o[j], __byte_perm(w0[j], w1[j], 0x5410), __byte_perm(w0[j], w1[j], 0x7632), __byte_perm(w2[j], w3[j], 0x5410),
-                    __byte_perm(w2[j], w3[j], 0x7632), b0, b1);
-        request_v(v4, k0 + 2 * STEP, n);
-    };
-    for (int k0 = first; k0 < n; k0 += 2 * STEP) {
-        step(kr[0], vr[0], k0);
-        if (k0 + STEP < n) step(kr[1], vr[1], k0 + STEP);
-    }
-#pragma unroll
-    for (int x = 4; x <= 16; x <<= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
-    // Columns 2 t and 2 t + 1 are term t of the heads: added up while the lanes share out heads and dims.  An infinite value makes the
-    // smaller terms 0 x inf: the first one carries it.
-    if (t > 0) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (!(fabsf(o[j][i]) < INFINITY)) o[j][i] = 0.f;
-    }
-    {
-        const bool h1 = t & 1, up = t & 2;
-        float v8[8], v4[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int i = 0; i < 2; ++i)   // dim 8 g + 2 j + i of head t & 1
-                v8[2 * j + i] = (h1 ? o[j][2 * i + 1] : o[j][2 * i]) + __shfl_xor_sync(0xffffffffu, h1 ? o[j][2 * i] : o[j][2 * i + 1], 1);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v4[j] = (up ? v8[j + 4] : v8[j]) + __shfl_xor_sync(0xffffffffu, up ? v8[j] : v8[j + 4], 2);
-        *reinterpret_cast<float4*>(&s_o[warp][t & 1][8 * g + (up ? 4 : 0)]) = make_float4(v4[0], v4[1], v4[2], v4[3]);
-        if (g == 0 && t < 2) { s_ml[warp][t][0] = m; s_ml[warp][t][1] = l; }
-    }
+    const bool live = sp < nsplit;
+    if (live) att_split(a, r, kvh, t_begin, len, warp, lane, kr, vr, S_[wsp]);
     __syncthreads();
-    // thread (h, dim): the warps' states in their order
-    const int h = tid >> 6, dim = tid & 63, hq = kvh * G + h;
-    const bool mine = h < G;
-    if (mine) {
-        float Mx = NEG_BIG, Ls = 0.f, Os = 0.f;
-#pragma unroll
-        for (int w = 0; w < AF_WARPS; ++w) Mx = fmaxf(Mx, s_ml[w][h][0]);
-#pragma unroll
-        for (int w = 0; w < AF_WARPS; ++w) {
-            const float e = __expf(s_ml[w][h][0] - Mx);
-            Ls = fmaf(s_ml[w][h][1], e, Ls);
-            Os = fmaf(s_o[w][h][dim], e, Os);
-        }
-        if (nsplit == 1) {
-            a.out[(size_t)r * a.Hq * HD + hq * HD + dim] = f2bf(Os / Ls);
-        } else {
-            float* pp = a.part + (((size_t)r * a.Hq + hq) * a.S + sp) * PART_STRIDE;
-            pp[dim] = Os;
-            if (dim == 0) {
-                pp[HD] = Mx;
-                pp[HD + 1] = Ls;
-            }
-        }
+    const int h = tid >> 6, dim = tid & 63, hq = kvh * G + (h < G ? h : 0);
+    const bool writer = h < G && wsp == 0;
+    if (nsplit <= ATT_WIDE) {   // all of the row's keys are here
+        if (writer)
+            a.out[(size_t)r * a.Hq * HD + hq * HD + dim] = f2bf(att_merge_splits<ATT_WIDE>(nsplit, [&](int i, bool ok, float& m, float& l, float& o) {
+                if (ok) att_merge_warps(S_[i], h, dim, m, l, o);
+            }));
+        return;
     }
-    if (nsplit == 1) return;
-    __syncthreads();  // every thread's partial stores precede thread 0's release below
-    if (tid == 0) {
-        int old;
-        asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(old) : "l"(a.counters + r * a.Hkv + kvh) : "memory");
-        s_last = (old == nsplit - 1);
-    }
-    __syncthreads();
-    if (!s_last) return;
-    if (mine) att_merge_splits(a, r, hq, dim, nsplit);
-    if (tid == 0) a.counters[r * a.Hkv + kvh] = 0;
+    float M_, L_, O_;
+    if (live) att_merge_warps(S_[wsp], h, dim, M_, L_, O_);
+    if (!att_publish(a, r, kvh, hq, h < G && live, sp, dim, M_, L_, O_, att_splits(len, ATT_WIDE), threadIdx.x, s_last)) return;
+    if (writer) att_finish(a, r, hq, dim, nsplit);
+    if (threadIdx.x == 0) a.counters[r * a.Hkv + kvh] = 0;
 }
 
 // ---------------------------------------------------------------------------

@@ -657,8 +657,8 @@ static cudaError_t attn_decode(VuibEngine* e, const AttnArgs& a, int rows, cudaS
         if (rc == cudaSuccess) rc = cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, dev);
         if (rc != cudaSuccess) return rc;
     }
-    if (af_use(rows, a.Hkv, a.max_seq, e->num_sms))
-        return launch(k_attn_few, dim3(a.Hkv, rows, af_splits(a.max_seq)), AF_WARPS * 32, 0, s, a);
+    if (att_wide(rows, a.Hkv, a.max_seq, e->num_sms))
+        return launch(k_attn_wide, dim3(a.Hkv, rows, att_splits(a.max_seq, ATT_WIDE)), ATT_WIDE * ATT_THREADS, 0, s, a);
     return launch(k_attn_decode, dim3(a.S, a.Hkv, rows), ATT_THREADS, 0, s, a);
 }
 
@@ -1865,8 +1865,8 @@ extern "C" int32_t vuib_attention_noalloc(int32_t n_heads, int32_t n_kv_heads, i
     rc = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (rc != cudaSuccess)
         return na_fail(err, err_len, VUIB_ERR_CUDA, "cudaDeviceGetAttribute: %s", cudaGetErrorString(rc));
-    if (af_use(n_rows, n_kv_heads, max_seq, sms))
-        k_attn_few<<<dim3(n_kv_heads, n_rows, af_splits(max_seq)), AF_WARPS * 32, 0, s>>>(aa);
+    if (att_wide(n_rows, n_kv_heads, max_seq, sms))
+        k_attn_wide<<<dim3(n_kv_heads, n_rows, att_splits(max_seq, ATT_WIDE)), ATT_WIDE * ATT_THREADS, 0, s>>>(aa);
     else
         k_attn_decode<<<dim3(S, n_kv_heads, n_rows), ATT_THREADS, 0, s>>>(aa);
     rc = cudaGetLastError();
