@@ -1,4 +1,4 @@
-"""The quantiser and the codec's attention where their split changes: frames of a cluster (8, or 9 from 121 frames on), one and several
+"""The quantiser and the codec's attention where their split changes: frames of a cluster (8, or 9 where that saves a wave), one and several
 clusters, 64 keys a CTA.  The codes against the nearest ones in 64 bits for the encoder's own latents, followed codebook by codebook as long
 as the distance to the runner-up leaves no doubt; a prefix's frames against those of the whole."""
 import pytest
@@ -19,9 +19,25 @@ def _sound(n):
     return (torch.randn(1, 1, n * 1920, generator=torch.Generator().manual_seed(3)) * 0.1).cuda()
 
 
+@pytest.fixture(scope="module")
+def long_encoder(encoder):
+    """Of 20 s, the longest buffer."""
+    from vui_b200.codec_encoder import QwenCodecEncoder
+
+    return QwenCodecEncoder(encoder[1], max_secs=20.0), encoder[1]
+
+
 @pytest.mark.parametrize("frames", [1, 7, 8, 9, 31, 32, 33, 64, 65, 120, 121, 125])
 def test_codes_are_the_nearest(encoder, frames):
-    enc, sd = encoder
+    _check_nearest(*encoder, frames)
+
+
+@pytest.mark.parametrize("frames", [120, 121, 135, 136, 240, 241, 250])
+def test_codes_of_long_inputs_are_the_nearest(long_encoder, frames):
+    _check_nearest(*long_encoder, frames)
+
+
+def _check_nearest(enc, sd, frames):
     codes = enc(_sound(frames))[0].cpu()
     lat = enc.read_latent(frames).double()
     followed = 0

@@ -355,7 +355,8 @@ extern "C" int32_t vuib_codec_enc_encode(VuibCodecEnc* c, const float* audio_dev
         }
         ready = dev;
     }
-    const int F = T > 8 * 15 && T <= 9 * 15 ? 9 : 8;   // frames of a cluster, see k_ervq
+    const auto waves = [&](int f) { return ((T + f - 1) / f + RV_RESIDENT - 1) / RV_RESIDENT; };
+    const int F = waves(9) < waves(8) ? 9 : 8;   // frames of a cluster, see k_ervq
     CK(sg_run(x, F == 9 ? k_ervq<9> : k_ervq<8>, dim3((T + F - 1) / F * RV_CL, 2), dim3(32 * RV_WARPS), RV_SMEM, r));
     return VUIB_OK;
 }

@@ -75,6 +75,7 @@ struct ERvqArgs {
 };
 
 constexpr int RV_CL = 8;                   // CTAs of a cluster
+constexpr int RV_RESIDENT = 15;   // clusters of 8 CTAs with this much shared memory that run at once
 constexpr int RV_WARPS = 16, RV_CODES = 4, RV_STAGES = 3;   // a ring stage: four codes (4 KB) of one warp
 constexpr int RV_SMEM = RV_WARPS * RV_STAGES * RV_CODES * 1024;
 
@@ -88,8 +89,8 @@ constexpr int RV_SMEM = RV_WARPS * RV_STAGES * RV_CODES * 1024;
 //    shuffles, but each 16-byte load is four passes of shared memory however many lanes share it: 8.4 us a codebook.
 //  * The winners of the CTAs are pushed into every CTA's shared memory and counted there (one hop; two buffers and two barriers in
 //    turn: a CTA pushes for codebook i + 2 only once it has this one's push for i + 1, which comes after i was read).
-// grid (8 * ceil(T / F), 2): acoustic codebooks first, the semantic one beside.  At most 15 clusters of 8 are resident, so F is 9 where
-// eight frames each would be a second wave (121 to 135 frames, the 10 s buffer among them).
+// grid (8 * ceil(T / F), 2): acoustic codebooks first, the semantic one beside.  F is 9 where that takes a wave of resident clusters less
+// than 8 (121 to 135 frames, the 10 s buffer among them; 241 to 250: an encode of 250 frames 2.23 -> 2.20 ms).
 // 13 frames 107 us (140 with loads in the loop and a cluster barrier a codebook), 80 frames 114 (137), 125 frames 156 (266).
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     unsigned long long d;
