@@ -171,16 +171,8 @@ template <int K>
 __device__ __forceinline__ void dt_tile(uint32_t addr, float (&v)[K]) {
     static_assert(K == 8 || K == 16 || K == 32, "columns");
     if constexpr (K == 32) tmem_ld32(addr, v);
-    else if constexpr (K == 8) tmem_ld8(addr, v);
-    else {
-        uint32_t r[16];
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                       "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(addr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-    }
+    else if constexpr (K == 16) tmem_ld16(addr, v);
+    else tmem_ld8(addr, v);
 }
 
 // A load that stays where it is written: the compiler may move __ldcg down to the first use of its result.

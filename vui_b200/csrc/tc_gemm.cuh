@@ -201,24 +201,21 @@ struct TcEpiQkv {      // RoPE on q,k + K/V append (EpiQkv of the GEMV path)
         const long long* cache_row = reinterpret_cast<const long long*>(es);
         const __nv_bfloat162* rs = reinterpret_cast<const __nv_bfloat162*>(es + TC_EPI_HEAD);
         bf16* const out = !to_cache ? q_out + n : n < q_cols + kv_cols ? k_cache + (n - q_cols) : v_cache + (n - q_cols - kv_cols);
+        float t[8], other[8];
 #pragma unroll
-        for (int half = 0; half < 8 / 8; ++half) {
-            float t[8], other[8];
+        for (int j = 0; j < 8; ++j) t[j] = rbf(v[j]);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) t[j] = rbf(v[half * 8 + j]);
+        for (int j = 0; j < 8; ++j) other[j] = __shfl_xor_sync(0xffffffffu, t[j], 1);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) other[j] = __shfl_xor_sync(0xffffffffu, t[j], 1);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int m = m0 + half * 8 + j, mm = min(m, M - 1);
-                if (do_rope) {
-                    const __nv_bfloat162 f = rs[mm * 64 + (n & (HD - 1))];
-                    const float c = __low2float(f), sn = odd ? __high2float(f) : -__high2float(f);
-                    t[j] = rbf(rbf(t[j] * c) + rbf(other[j] * sn));
-                }
-                const size_t at = to_cache ? (size_t)cache_row[mm] * kv_cols : (size_t)m * q_cols;
-                if (m < M) out[at] = f2bf(t[j]);
+        for (int j = 0; j < 8; ++j) {
+            const int m = m0 + j, mm = min(m, M - 1);
+            if (do_rope) {
+                const __nv_bfloat162 f = rs[mm * 64 + (n & (HD - 1))];
+                const float c = __low2float(f), sn = odd ? __high2float(f) : -__high2float(f);
+                t[j] = rbf(rbf(t[j] * c) + rbf(other[j] * sn));
             }
+            const size_t at = to_cache ? (size_t)cache_row[mm] * kv_cols : (size_t)m * q_cols;
+            if (m < M) out[at] = f2bf(t[j]);
         }
     }
 };
