@@ -244,11 +244,13 @@ int32_t vuib_attention_noalloc(int32_t n_heads, int32_t n_kv_heads, int32_t max_
                                const int32_t* row_slot_dev, const int32_t* row_pos_dev, void* out_dev,
                                void* stream, char* err, size_t err_len);
 
-/* Test hook: vuib_attention as a step runs it, with keys requested before the preceding kernel has ended.  The kernel finds
- * the rows at (old_slot, old_pos) first and at (row_slot, row_pos) when that kernel has ended; out is vuib_attention's. */
+/* Test hook: vuib_attention as a step runs it, with keys requested before the preceding kernel has ended.  That kernel moves
+ * the rows from (old_slot, old_pos) to (row_slot, row_pos) and writes their own keys and values there, k_new and v_new:
+ * bf16 (n_rows, n_kv_heads * head_dim).  out is vuib_attention's. */
 int32_t vuib_debug_attention_moved(VuibEngine* e, int32_t layer, int32_t n_rows, const void* q_dev,
                                    const int32_t* old_slot_dev, const int32_t* old_pos_dev,
-                                   const int32_t* row_slot_dev, const int32_t* row_pos_dev, void* out_dev, void* stream);
+                                   const int32_t* row_slot_dev, const int32_t* row_pos_dev, const void* k_new_dev,
+                                   const void* v_new_dev, void* out_dev, void* stream);
 
 /* Gather-sum of codec codes alone: out[r] = sum_q audio_emb[q*CS + codes[r,q]]
  * (AudioEmbedding.forward, model.py:559-563; Engine._audio_emb, engine.py:705-709).

@@ -25,3 +25,16 @@ def test_early_requests_only_in_steps():
     last = [m.strip() for m in re.findall(r"AttnArgs aa\{.*?,\s*([^,{}]+)\};", src, flags=re.S)]
     tables = {"!prefill": 1, "0": len(last) - 2, "1": 1}   # 1: the test hook
     assert {v: last.count(v) for v in set(last)} == tables
+
+
+def test_early_requests_are_coherent():
+    """The preceding kernel may be writing what a stale place leads to, and the second look must see it: no read-only loads."""
+    for name, kernel in (("decode_kernels.cuh", "k_attn_wide("), ("fused_blocks.cuh", "k_attn_block("), ("fused_rows.cuh", "k_attn_rows(")):
+        src = _source(name)
+        body = src[src.index("{", src.index(kernel)):]
+        body = body[: body.index("\n}")]
+        assert "ld_l2" in body[: body.index("pdl_wait()")] and not re.search(r"ldg_stream|\.nc\b|__ldg\([^)]*(?:kb|vb|k_cache|v_cache)", body)
+    src = _source("decode_kernels.cuh")
+    for load in ("uint4 ld_l2(", "void ld_l2_if("):
+        body = src[src.index(load):]
+        assert "ld.global.cg.v4" in body[: body.index("\n}")]

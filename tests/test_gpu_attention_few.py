@@ -60,9 +60,10 @@ def test_infinite_values_stay_infinite(eng, rows):
 
 
 @pytest.mark.parametrize("rows", [1, 5, 18])
-@pytest.mark.parametrize("moved", ["not", "position", "slot", "wildly"])
+@pytest.mark.parametrize("moved", ["not", "on", "back", "slot", "wildly"])
 def test_keys_requested_before_the_place_is_final(eng, rows, moved):
-    """As a step asks for them: where the table changes behind the early look (or does not), the result is that of the final place."""
+    """As a step asks for them: where the table changes behind the early look (or does not), the result is that of the final place, with
+    the row's own key as the preceding kernel wrote it, also where the early look has seen what was there before (back)."""
     import ctypes as C
 
     g = torch.Generator(device="cuda").manual_seed(rows)
@@ -74,11 +75,16 @@ def test_keys_requested_before_the_place_is_final(eng, rows, moved):
     for first in range(0, len(LENGTHS), rows):
         pos = torch.tensor([LENGTHS[(first + i) % len(LENGTHS)] - 1 for i in range(rows)], dtype=torch.int32, device="cuda")
         slots = torch.tensor([(5 * i) % 64 for i in range(rows)], dtype=torch.int32, device="cuda")
-        old_pos = {"position": (pos - 1).clamp(min=0), "wildly": (pos * 7919) % 3000 - 900}.get(moved, pos).to(torch.int32)
+        old_pos = {"on": (pos - 1).clamp(min=0), "back": (pos + 40).clamp(max=1023), "wildly": (pos * 7919) % 3000 - 900}.get(moved, pos).to(torch.int32)
         old_slots = {"slot": (slots + 1) % 64, "wildly": slots - 40}.get(moved, slots).to(torch.int32)
         out = torch.empty_like(q)
-        eng._ck(eng._lib.vuib_debug_attention_moved(eng._handle, layer, rows, P(q), P(old_slots), P(old_pos), P(slots), P(pos), P(out), eng._stream))
+        own = torch.randn(2, rows, 512, device="cuda", generator=g).to(torch.bfloat16)
+        own[0] = q.view(rows, 8, 2, 64)[:, :, 0].reshape(rows, 512)   # a key that weighs: the head's own query
+        eng._ck(eng._lib.vuib_debug_attention_moved(eng._handle, layer, rows, P(q), P(old_slots), P(old_pos), P(slots), P(pos), P(own[0]), P(own[1]),
+                                                    P(out), eng._stream))
         assert torch.equal(out, eng._attention(layer, q, slots, pos))
+        ref = _reference(eng, layer, q, slots, pos)
+        assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all()   # as above
     eng.check_device()
 
 

@@ -162,7 +162,7 @@ SYMBOLS = {
     "vuib_frame_host_capture": (C.c_int32, [_P, C.c_int32, C.c_int32, _P, _P, _P, _P, _P, _P, _P, _P]),
     "vuib_frame_host": (C.c_int32, [_P, C.c_int32, C.c_int32, _P, _P, _P, _P]),
     "vuib_attention": (C.c_int32, [_P, C.c_int32, C.c_int32, _P, _P, _P, _P, _P]),
-    "vuib_debug_attention_moved": (C.c_int32, [_P, C.c_int32, C.c_int32, _P, _P, _P, _P, _P, _P, _P]),
+    "vuib_debug_attention_moved": (C.c_int32, [_P, C.c_int32, C.c_int32, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "vuib_attention_noalloc": (C.c_int32, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P, _P, _P, _P, _P, _P, _P,
                                            C.c_char_p, C.c_size_t]),
     "vuib_embed_codes": (C.c_int32, [_P, C.c_int32, _P, _P, _P]),

@@ -52,11 +52,19 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
     return r;
 }
 
+// 16 bytes from the L2, which other SMs' writes reach, where it is written: the compiler may move __ldcg down to the first use of its result.
+__device__ __forceinline__ uint4 ld_l2(const void* p) {
+    uint4 r;
+    asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+    return r;
+}
+
 // Programmatic dependent launch: a kernel launched with the stream-serialization
 // attribute may start while its predecessor still runs.  pdl_trigger() lets the
 // successor be scheduled; pdl_wait() blocks until the predecessor has finished
-// and its writes are visible.  Everything a kernel does before pdl_wait() must
-// touch only constants (weights).  Both are no-ops for an ordinary launch.
+// and its writes are visible.  What a kernel reads before pdl_wait() is constant
+// (weights) or is read by ld_l2 and, where it may have changed since, read again by
+// ld_l2 behind it (cache rows, see k_embed_codes).  Both are no-ops for an ordinary launch.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -162,15 +170,23 @@ static __global__ void __launch_bounds__(128) k_embed_codes(
     }
 }
 
-// Writes a (slot, position) table 20 us after its successor may have started: the successor's early look at the table then finds
-// what was there before.  For tests of that case.
-static __global__ void __launch_bounds__(256) k_move_rows(const int32_t* slot_in, const int32_t* pos_in, int32_t* row_slot, int32_t* row_pos, int n) {
+// Writes a (slot, position) table and the rows' own keys and values 20 us after its successor may have started: the successor's early
+// look then finds what was there before.  For tests of that case.
+static __global__ void __launch_bounds__(256) k_move_rows(const int32_t* slot_in, const int32_t* pos_in, int32_t* row_slot, int32_t* row_pos, int n,
+                                                          const bf16* k_new, const bf16* v_new, bf16* kc, bf16* vc, int cols, int n_slots, int max_seq) {
     pdl_trigger();
     pdl_wait();
     __nanosleep(20000);
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         row_slot[i] = slot_in[i];
         row_pos[i] = pos_in[i];
+    }
+    for (int i = threadIdx.x; i < n * cols; i += blockDim.x) {
+        const int r = i / cols, slot = slot_in[r], pos = pos_in[r];
+        if (slot < 0 || slot >= n_slots || pos < 0 || pos >= max_seq) continue;
+        const size_t at = ((size_t)slot * max_seq + pos) * cols + i % cols;
+        kc[at] = k_new[i];
+        vc[at] = v_new[i];
     }
 }
 
@@ -1079,11 +1095,11 @@ static __global__ void __launch_bounds__(ATT_THREADS, 5) k_attn_decode(AttnArgs 
     if (tid == 0) a.counters[r * a.Hkv + kvh] = 0;
 }
 
-// ldg_stream where `ok`, zeros elsewhere, without a branch around the load.
-__device__ __forceinline__ void ldg_stream_if(uint4& r, const void* p, bool ok) {
+// ld_l2 where `ok`, zeros elsewhere, without a branch around the load.
+__device__ __forceinline__ void ld_l2_if(uint4& r, const void* p, bool ok) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
-                 "@p ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
-                 : "=&r"(r.x), "=&r"(r.y), "=&r"(r.z), "=&r"(r.w) : "l"(p), "r"((uint32_t)ok));
+                 "@p ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
+                 : "=&r"(r.x), "=&r"(r.y), "=&r"(r.z), "=&r"(r.w) : "l"(p), "r"((uint32_t)ok) : "memory");
 }
 
 // Few rows.  What bounds it then is round trips: the keys' way from memory behind the preceding kernel, and the merge through global
@@ -1105,6 +1121,8 @@ static __global__ void __launch_bounds__(ATT_WIDE * ATT_THREADS, 1) k_attn_wide(
     const int G = a.Hq / a.Hkv, t_begin = sp * ATT_SPLIT, t_first = t_begin + warp * 4 + (lane >> 3);
     const size_t pos_stride = (size_t)a.Hkv * HD;
     const bf16 *kb, *vb;   // of the lane's first key
+    // From the L2 both times: a stale place can lie behind the row's own key, which the preceding kernel then writes while this one reads
+    // it, and the read-only path of k_attn_decode need not see that on the second look.
     uint4 kr[ATT_ITERS], vr[ATT_ITERS];
     auto request = [&](int slot, int end) {
         const size_t base = ((size_t)slot * a.max_seq + t_first) * pos_stride + kvh * HD + (lane & 7) * 8;
@@ -1113,8 +1131,8 @@ static __global__ void __launch_bounds__(ATT_WIDE * ATT_THREADS, 1) k_attn_wide(
 #pragma unroll
         for (int it = 0; it < ATT_ITERS; ++it) {
             const bool ok = t_first + it * 16 < end;
-            ldg_stream_if(kr[it], kb + it * 16 * pos_stride, ok);
-            ldg_stream_if(vr[it], vb + it * 16 * pos_stride, ok);
+            ld_l2_if(kr[it], kb + it * 16 * pos_stride, ok);
+            ld_l2_if(vr[it], vb + it * 16 * pos_stride, ok);
         }
     };
     int s_old = -1, p_old = -1;
@@ -1138,8 +1156,8 @@ static __global__ void __launch_bounds__(ATT_WIDE * ATT_THREADS, 1) k_attn_wide(
 #pragma unroll
         for (int it = 0; it < ATT_ITERS; ++it)
             if (t_first + it * 16 == p_old) {
-                kr[it] = __ldcg(reinterpret_cast<const uint4*>(kb + it * 16 * pos_stride));
-                vr[it] = __ldcg(reinterpret_cast<const uint4*>(vb + it * 16 * pos_stride));
+                kr[it] = ld_l2(kb + it * 16 * pos_stride);
+                vr[it] = ld_l2(vb + it * 16 * pos_stride);
             }
     }
     const bool live = sp < nsplit;

@@ -175,13 +175,6 @@ __device__ __forceinline__ void dt_tile(uint32_t addr, float (&v)[K]) {
     else tmem_ld8(addr, v);
 }
 
-// A load that stays where it is written: the compiler may move __ldcg down to the first use of its result.
-__device__ __forceinline__ uint4 dt_load(const bf16* p) {
-    uint4 v;
-    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-    return v;
-}
-
 // RMSNorm of the residual rows into the MMA operand h: warp w takes streams w, w + 8, ...
 template <class S>
 __device__ __forceinline__ void dt_norm(S& sm, const bf16* w, float eps, int nv) {   // w in shared memory
@@ -481,8 +474,8 @@ __global__ void __launch_bounds__(DT_THREADS, 1) k_depth_tc(const __grid_constan
                 const bool ok = tk < n_keys;
                 k4[u] = v4[u] = make_uint4(0, 0, 0, 0);
                 if (ok) {
-                    k4[u] = dt_load(a.kc + row + (size_t)tk * DT_D);
-                    v4[u] = dt_load(a.vc + row + (size_t)tk * DT_D);
+                    k4[u] = ld_l2(a.kc + row + (size_t)tk * DT_D);
+                    v4[u] = ld_l2(a.vc + row + (size_t)tk * DT_D);
                 }
             }
         };

@@ -509,8 +509,8 @@ __global__ void __launch_bounds__(FB_THREADS, 1) k_attn_block(const __grid_const
             // SHORT: warp 0 alone takes all (<= 16) keys, four per pass
             const int t = SHORT ? (warp == 0 ? it * 4 + g4 : t_end) : t_begin + it * 32 + warp * 4 + g4;
             if (t < t_end) {
-                kr[it] = ldg_stream(kb + (size_t)t * pos_stride);
-                vr[it] = ldg_stream(vb + (size_t)t * pos_stride);
+                kr[it] = ld_l2(kb + (size_t)t * pos_stride);
+                vr[it] = ld_l2(vb + (size_t)t * pos_stride);
             } else {
                 kr[it] = make_uint4(0, 0, 0, 0);
                 vr[it] = make_uint4(0, 0, 0, 0);
@@ -711,8 +711,8 @@ __global__ void __launch_bounds__(FB_THREADS, 1) k_attn_block(const __grid_const
         for (int tb = t_begin + FB_ATT_PRE * 32; tb < t_end; tb += 32) {  // longer caches: the rest, block by block
             const int t = tb + warp * 4 + g4;
             const bool ok = t < t_end;
-            const uint4 kraw = ok ? ldg_stream(kb + (size_t)t * pos_stride) : make_uint4(0, 0, 0, 0);
-            const uint4 vraw = ok ? ldg_stream(vb + (size_t)t * pos_stride) : make_uint4(0, 0, 0, 0);
+            const uint4 kraw = ok ? ld_l2(kb + (size_t)t * pos_stride) : make_uint4(0, 0, 0, 0);
+            const uint4 vraw = ok ? ld_l2(vb + (size_t)t * pos_stride) : make_uint4(0, 0, 0, 0);
             consume(kraw, vraw, ok);
         }
         // merge the warp's 4 key groups, then the CTA's 8 warps

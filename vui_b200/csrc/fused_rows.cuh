@@ -302,8 +302,8 @@ __global__ void __launch_bounds__(TH, 1) k_attn_rows(const __grid_constant__ CUt
         for (int it = 0; it < NPRE; ++it) {
             const int t = key_of(it);
             const bool ok = t < t_end;
-            kr[it] = ok ? ldg_stream(kb + (size_t)t * pos_stride) : make_uint4(0, 0, 0, 0);
-            vr[it] = ok ? ldg_stream(vb + (size_t)t * pos_stride) : make_uint4(0, 0, 0, 0);
+            kr[it] = ok ? ld_l2(kb + (size_t)t * pos_stride) : make_uint4(0, 0, 0, 0);
+            vr[it] = ok ? ld_l2(vb + (size_t)t * pos_stride) : make_uint4(0, 0, 0, 0);
         }
     };
     bool early = false;
@@ -480,8 +480,8 @@ __global__ void __launch_bounds__(TH, 1) k_attn_rows(const __grid_constant__ CUt
             const int t = tb + asub * 4 + g4;
             const bool ok = t < t_end;
             float kf[8], vf[8];
-            unpack8(ok ? ldg_stream(kb + (size_t)t * pos_stride) : make_uint4(0, 0, 0, 0), kf);
-            unpack8(ok ? ldg_stream(vb + (size_t)t * pos_stride) : make_uint4(0, 0, 0, 0), vf);
+            unpack8(ok ? ld_l2(kb + (size_t)t * pos_stride) : make_uint4(0, 0, 0, 0), kf);
+            unpack8(ok ? ld_l2(vb + (size_t)t * pos_stride) : make_uint4(0, 0, 0, 0), vf);
 #pragma unroll
             for (int h = 0; h < G; ++h) {
                 float d = 0.f;

@@ -1547,8 +1547,8 @@ extern "C" int32_t vuib_attention(VuibEngine* e, int32_t layer, int32_t n_rows, 
 extern "C" int32_t vuib_debug_attention_moved(VuibEngine* e, int32_t layer, int32_t n_rows, const void* q_dev,
                                               const int32_t* old_slot_dev, const int32_t* old_pos_dev,
                                               const int32_t* row_slot_dev, const int32_t* row_pos_dev,
-                                              void* out_dev, void* stream) {
-    if (!e || !q_dev || !old_slot_dev || !old_pos_dev || !row_slot_dev || !row_pos_dev || !out_dev) return VUIB_ERR_NULL;
+                                              const void* k_new_dev, const void* v_new_dev, void* out_dev, void* stream) {
+    if (!e || !q_dev || !old_slot_dev || !old_pos_dev || !row_slot_dev || !row_pos_dev || !k_new_dev || !v_new_dev || !out_dev) return VUIB_ERR_NULL;
     if (!e->have_kv || !e->have_ws) return fail(e, VUIB_ERR_UNBOUND, "bind kv and workspace first");
     const VuibConfig& c = e->cfg;
     if (layer < 0 || layer >= c.n_layers) return fail(e, VUIB_ERR_RANGE, "layer %d out of range", layer);
@@ -1557,7 +1557,8 @@ extern "C" int32_t vuib_debug_attention_moved(VuibEngine* e, int32_t layer, int3
     int32_t *slot = wsp<int32_t>(e, e->lay.row_slot), *pos = wsp<int32_t>(e, e->lay.row_pos);
     CK(cudaMemcpyAsync(slot, old_slot_dev, (size_t)n_rows * 4, cudaMemcpyDeviceToDevice, s));
     CK(cudaMemcpyAsync(pos, old_pos_dev, (size_t)n_rows * 4, cudaMemcpyDeviceToDevice, s));
-    CK(launch(k_move_rows, 1, 256, 0, s, row_slot_dev, row_pos_dev, slot, pos, n_rows));
+    CK(launch(k_move_rows, 1, 256, 0, s, row_slot_dev, row_pos_dev, slot, pos, n_rows, static_cast<const bf16*>(k_new_dev),
+              static_cast<const bf16*>(v_new_dev), static_cast<bf16*>(e->k[layer]), static_cast<bf16*>(e->v[layer]), c.n_kv_heads * HD, c.n_slots, c.max_seq));
     AttnArgs aa{static_cast<const bf16*>(q_dev), static_cast<const bf16*>(e->k[layer]),
                 static_cast<const bf16*>(e->v[layer]), slot, pos,
                 wsp<float>(e, e->lay.part), wsp<int32_t>(e, e->lay.counters), static_cast<bf16*>(out_dev),
