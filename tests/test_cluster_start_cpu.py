@@ -52,3 +52,12 @@ def test_a_wait_is_not_given_up_while_peers_are_sending():
     assert "e->spin_limit = polls < 1u << 26 ? polls : 1u << 26;" in src
     factors = [int(f) for name in sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) for f in re.findall(r"\b(\d+)u? \* a\.spin_limit", open(name).read())]
     assert factors and max(factors) * 2 ** 26 < 2 ** 32
+
+
+def test_the_quantisers_winners_have_two_buffers():
+    """Between a thread's reads of a codebook's winners and the next codebook's writes stands no barrier of the CTA: the wait in between is
+    for the peers' answers to this CTA, and the reading thread may be answering another.  So the codebooks take turns."""
+    body = next(k[2] for k in CLUSTERED if k[1] == "k_ervq")
+    assert re.search(r"\bwon\[2\]\[RV_WARPS\]\[F\];", body)
+    uses = re.findall(r"\bwon\[(\w+)\]", body)
+    assert uses.pop(0) == "2" and len(uses) >= 2 and set(uses) == {"buf"} and "const int buf = cb & 1;" in body

@@ -109,7 +109,9 @@ template <int F>
 static __global__ void __cluster_dims__(RV_CL, 1, 1) __launch_bounds__(32 * RV_WARPS) k_ervq(ERvqArgs a) {
     static_assert(F == 8 || F == 9, "eight frames by halves, a ninth by itself");
     extern __shared__ __align__(128) unsigned char rv_ring[];   // [warp][stage][code][256]
-    __shared__ unsigned long long won[RV_WARPS][F];              // this CTA's best of each warp
+    // This CTA's best of each warp, two buffers in turn: a warp that has the peers' answers writes codebook i + 1's while a thread that answers
+    // another CTA may still be reading i's; that thread passes the barrier of i + 1 before anything of i + 2 is written.
+    __shared__ unsigned long long won[2][RV_WARPS][F];
     __shared__ __align__(8) unsigned long long peers[2][RV_CL][F];
     __shared__ uint64_t full[RV_WARPS][RV_STAGES], got[2];
     constexpr int PER = 256 / RV_WARPS, LOADS = PER / RV_CODES;
@@ -206,16 +208,16 @@ static __global__ void __cluster_dims__(RV_CL, 1, 1) __launch_bounds__(32 * RV_W
             if (lane == 0 && load + RV_STAGES < loads) request(load + RV_STAGES);
         }
         if (cb + 1 < n) n2 = __ldg(a.norm2[q0 + cb + 1] + first + lane % PER);
-        if ((lane & 3) == 0) won[warp][lane >> 2] = rv_key(bv, bi);
-        if (F == 9 && lane == 0) won[warp][8] = rv_key(bv8, bi8);
+        const int buf = cb & 1;
+        if ((lane & 3) == 0) won[buf][warp][lane >> 2] = rv_key(bv, bi);
+        if (F == 9 && lane == 0) won[buf][warp][8] = rv_key(bv8, bi8);
         __syncthreads();
         if (cb == 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-        const int buf = cb & 1;
         if (tid < RV_CL * F) {
             const int f = tid % F, dst = tid / F;
             unsigned long long w[RV_WARPS];
 #pragma unroll
-            for (int i = 0; i < RV_WARPS; ++i) w[i] = won[i][f];
+            for (int i = 0; i < RV_WARPS; ++i) w[i] = won[buf][i][f];
 #pragma unroll
             for (int k = RV_WARPS / 2; k > 0; k /= 2)
 #pragma unroll
