@@ -1104,11 +1104,13 @@ __device__ __forceinline__ void ld_l2_if(uint4& r, const void* p, bool ok) {
 
 // Few rows.  What bounds it then is round trips: the keys' way from memory behind the preceding kernel, and the merge through global
 // memory.  A CTA takes four splits, so up to 512 keys are merged in shared memory; old keys are requested before the preceding kernel has
-// ended; and there is an SM for each (row, kv head), since a CTA's keys and values fill its registers.  Frames of 5 / 8 / 16 / 18 rows
-// at 300 keys take 1.52 / 1.55 / 1.58 / 1.60 ms, with k_attn_decode 1.52 / 1.59 / 1.64 / 1.64.
-// Beyond 512 keys a row has two CTAs and more than nine rows no SM for each: 800 keys in caches of 1024 take 1.57 / 1.60 / 1.74 / 1.78 ms, with
-// k_attn_decode 1.54 / 1.65 / 1.71 / 1.74.  Where the cache ends at 1024 a row that fills it spends as many steps on either side and the sum is
-// in favour or even; in caches of 1536 (16 rows: 1.60, 1.74, 1.90 ms at 300, 800 and 1500 keys, with the other 1.62, 1.71, 1.81) it is not.
+// ended; and there is an SM for each (row, kv head), since a CTA's keys and values fill its registers.  Frames of 5 / 8 / 12 / 16 / 18 rows
+// at 305 keys take 1.52 / 1.59 / 1.55 / 1.56 / 1.59 ms, with k_attn_decode 1.51 / 1.59 / 1.60 / 1.62 / 1.64; at 505 keys 1.54 / 1.56 / 1.58 / 1.61 / 1.66
+// and 1.53 / 1.60 / 1.65 / 1.66 / 1.67.
+// Beyond 512 keys a row has two CTAs and more than nine rows no SM for each: at 805 keys 1.58 / 1.61 / 1.70 / 1.75 / 1.78 ms, with k_attn_decode
+// 1.54 / 1.62 / 1.64 / 1.72 / 1.75.  Where the cache ends at 1024 a row that fills it spends as many steps on either side, and the three lengths
+// together are 1 to 1.5 % in favour (five rows: 1 % against); in caches of 1536 (16 rows: 1.60, 1.74, 1.90 ms at 300, 800 and 1500 keys, with the
+// other 1.62, 1.71, 1.81) they are not.
 constexpr int ATT_WIDE = 4;   // splits of a CTA
 inline bool att_wide(int rows, int Hkv, int max_seq, int num_sms) { return rows * Hkv <= num_sms && max_seq <= 2 * ATT_WIDE * ATT_SPLIT; }
 

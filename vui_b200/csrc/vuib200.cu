@@ -552,8 +552,8 @@ static int32_t build_dg_stream(VuibEngine* e) {
 static bool prefill_tc_ok(VuibEngine* e) { return e->tc && !env_off("VUIB_NO_TC"); }
 
 static bool tc_ok(VuibEngine* e, int M) {
-    // measured at 300 keys: frames of 5 / 8 / 16 rows take 1.58 / 1.61 / 1.64 ms here and 2.99 / 3.49 / 5.95 on the register-tile
-    // GEMVs; 4 rows take 1.01 ms in the fused layers, which are laid out for no more, and 2.42 on the GEMVs
+    // measured at 300 keys: frames of 5 / 8 / 16 rows take 1.52 / 1.59 / 1.56 ms here and 2.99 / 3.49 / 5.95 on the register-tile
+    // GEMVs; 4 rows take 1.00 ms in the fused layers, which are laid out for no more, and 2.42 on the GEMVs
     return M > 4 && e->tc && !env_off("VUIB_NO_TC");
 }
 
